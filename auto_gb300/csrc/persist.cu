@@ -47,6 +47,13 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
     return v;
 }
 
+// the larger of a column item's tile and a row item's packed rows
+template <int N>
+FFT_CHD constexpr size_t persist_seq_floats2() {
+    constexpr size_t row = (size_t)row_seqs(N, false) * seq_stride(N), col = col_seq_floats2<N>();
+    return row > col ? row : col;
+}
+
 template <int N, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     persist_class(const DevWorld* __restrict__ worlds, const ColItem* __restrict__ cols, const RowItem* __restrict__ rows,
@@ -54,9 +61,8 @@ __global__ void __launch_bounds__(NT, MINB)
     extern __shared__ float4 smem_raw[];
     __shared__ long long s_item;
     __shared__ int s_stop;
-    constexpr int SEQ = seq_stride(N), NSEQ = row_seqs(N, false) > TC ? row_seqs(N, false) : TC;
     float2* X = reinterpret_cast<float2*>(smem_raw);
-    float2* stw = X + NSEQ * SEQ;  // after the column pass's tile sequences and the row pass's packed rows
+    float2* stw = X + persist_seq_floats2<N>();  // after the column pass's tile sequences and the row pass's packed rows
     // the row items' stage tables, then the column items' (their plans may differ: CMR)
     float2* stwc = stw + tw_table_size(N) + 1;
     fill_stage_twiddles<N>(stw, tw, threadIdx.x, NT);
@@ -150,8 +156,7 @@ constexpr int persist_minb() { return (V == 0 ? 1024 : 512) / persist_nt<N>() < 
 
 template <int N>
 size_t persist_smem() {
-    constexpr int NSEQ = row_seqs(N, false) > TC ? row_seqs(N, false) : TC;
-    return (size_t)NSEQ * seq_stride(N) * sizeof(float2) + stage_table_bytes<N>() + stage_table_bytes<N, CMR>() +
+    return persist_seq_floats2<N>() * sizeof(float2) + stage_table_bytes<N>() + stage_table_bytes<N, CMR>() +
            col_khat_bytes<N>();
 }
 

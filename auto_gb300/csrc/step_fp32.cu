@@ -18,7 +18,8 @@ size_t col_smem_bytes(int H) {
     const int t32 = lfft::tw_table_size(H, CMR), t16 = lfft::tw_table_size(H);
     const size_t scalar_tables = ((t32 > t16 ? t32 : t16) + 1) * sizeof(float2);
     const size_t paired_tables = (lfft::tw_table_size(H, PMR) + 1) * sizeof(lfft::tw2);
-    return (size_t)TC * lfft::seq_stride(H) * sizeof(float2) + (scalar_tables > paired_tables ? scalar_tables : paired_tables) +
+    const int stride = col_stride(H) > lfft::seq_stride(H) ? col_stride(H) : lfft::seq_stride(H);
+    return (size_t)TC * stride * sizeof(float2) + (scalar_tables > paired_tables ? scalar_tables : paired_tables) +
            col_khat_bytes_of(H);
 }
 size_t row_smem_bytes(int W, int acc_planes) {

@@ -442,9 +442,9 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     float2* Z = reinterpret_cast<float2*>(smem_raw);
     float2* stw = Z + S * SEQ;
     float* extra = row_extra_smem<W>(stw);
-    fill_stage_twiddles<W>(stw, tw, threadIdx.x, NT);
     const RowItem it = items[blockIdx.x];
     const DevWorld& wd = worlds[it.world];
+    fill_stage_twiddles<W>(stw, tw, threadIdx.x, NT);
     const int H = wd.H, C = wd.C, K = wd.K, r0 = it.row0;
     const size_t plane = (size_t)W * H, cplane = (size_t)(W / 2) * H;
     // Lenia items cover one target channel; SmoothLife and MNCA items every channel
@@ -643,6 +643,85 @@ __device__ __noinline__ void col_item_unchained(float2* X, const float2* stw, co
     store_tile<H, NT>(X, dst);
 }
 
+// Stride between a column item's two sequences in shared memory: 8 mod 16 float2, so that the eight
+// butterflies of both columns that a half-warp works on (see col_chained) touch all 32 banks once.
+FFT_CHD constexpr int col_stride(int n) { return n + n / 16 + ((24 - (n + n / 16) % 16) % 16); }
+
+// Stages [I, I1) of both columns of a tile in shared memory, as fft_stages, but with the column in the
+// lowest bit of the butterfly index.
+template <int N, int NT, bool INV, int I, int I1, int MR>
+__device__ __forceinline__ void col_stages(float2* X, const float2* stw) {
+    if constexpr (I < I1) {
+        constexpr int R = plan_radix(N, I, MR), L = plan_L(N, I, MR);
+        constexpr int TOT = TC * (N / R), PER = (TOT + NT - 1) / NT, CS = col_stride(N);
+        float2 v[PER][R];
+#pragma unroll
+        for (int p = 0; p < PER; p++) {
+            const int b = threadIdx.x + p * NT;
+            if ((TOT % NT) == 0 || b < TOT)
+                stage_load<N, R, L, INV>(X + (b & 1) * CS, b >> 1, v[p], stw + stage_tw_offset(N, I, MR));
+        }
+        __syncthreads();
+#pragma unroll
+        for (int p = 0; p < PER; p++) {
+            const int b = threadIdx.x + p * NT;
+            if ((TOT % NT) == 0 || b < TOT) stage_store<N, R, L>(X + (b & 1) * CS, b >> 1, v[p]);
+        }
+        __syncthreads();
+        col_stages<N, NT, INV, I + 1, I1, MR>(X, stw);
+    }
+}
+
+// The chained column item.  The first stage of a plan reads elements j + m H/R and the last stage
+// leaves butterfly j the same elements, so with thread t on butterfly j = t / 2 of column t % 2 a
+// warp's access to the tile (H rows of two columns) is 256 contiguous bytes: the forward transform's
+// first stage takes its inputs straight from global memory and the inverse's last stage writes its
+// outputs there.  That leaves 2 (stages - 1) sweeps of the tile through shared memory and
+// 4 stages - 5 barriers, two sweeps and four barriers fewer than staging the tile both ways.  The item is
+// bound by shared-memory instructions and barriers; measured, per generation: 60 worlds of 384 x 384
+// 60.7 -> 55.3 us, 41 of 512 x 512 47.2 -> 44.7, one of 4096 x 4096 107.5 -> 103.3, of 8192 x 8192 576 -> 552.
+template <int H, int NT, bool CG, int MR>
+__device__ __forceinline__ void col_chained(float2* X, const float2* stw, const float2* __restrict__ src,
+                                            float2* __restrict__ dst, const float* ksm) {
+    constexpr int LAST = plan_len(H, MR) - 1, R = plan_radix(H, 0, MR), NB = H / R, CS = col_stride(H);
+    constexpr int HQC = khat_cols_stride<H>();
+    static_assert(TC == 2 && fusable<H, MR>() && TC * NB <= NT, "one outer butterfly per thread, two columns");
+    const int c = threadIdx.x & 1, j = threadIdx.x >> 1;
+    const bool on = TC * NB == NT || threadIdx.x < TC * NB;
+    float2* Xc = X + c * CS;
+    float2 v[R];
+    if (on) {
+        const uint64_t keep = hint::policy_keep();
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = hint::ld2c<CG>(src + threadIdx.x + TC * NB * m, keep);
+        Dft<R, false>::run(v);
+        stage_store<H, R, 1>(Xc, j, v);
+    }
+    cp_async_wait_all();  // the khat columns
+    __syncthreads();
+    col_stages<H, NT, false, 1, LAST, MR>(X, stw);
+    if (on) {
+        stage_load<H, R, NB, false>(Xc, j, v, stw + stage_tw_offset(H, LAST, MR));
+        const float* kc = ksm + c * HQC;
+#pragma unroll
+        for (int m = 0; m < R; m++) {
+            const int ky = j + m * NB;
+            v[m] = cscale(v[m], kc[ky <= H / 2 ? ky : H - ky]);
+        }
+        Dft<R, true>::run(v);
+    }
+    __syncthreads();
+    if (on) stage_store<H, R, 1>(Xc, j, v);
+    __syncthreads();
+    col_stages<H, NT, true, 1, LAST, MR>(X, stw);
+    if (on) {
+        stage_load<H, R, NB, true>(Xc, j, v, stw + stage_tw_offset(H, LAST, MR));
+        const uint64_t keep = hint::policy_keep();
+#pragma unroll
+        for (int m = 0; m < R; m++) hint::st2(dst + threadIdx.x + TC * NB * m, v[m], keep);
+    }
+}
+
 // One column item: tile `tile` (TC spectrum columns) of channel `chan`, convolved with kernel
 // `kernel` (which reads that channel).  A channel read by several kernels has one item per kernel, each
 // repeating the channel's forward column transform: that keeps every item on the chained path and
@@ -655,30 +734,23 @@ __device__ __forceinline__ void col_item(const DevWorld& wd, const ColItem it, f
     const float2* src = wd.spec + c * cplane + (size_t)t * H * TC;
     // Tiles without the packed DC/Nyquist column: the khat multiply runs in registers between the
     // forward and the inverse column FFT, and the tile's two khat columns (contiguous, HQ floats
-    // each) are copied to shared memory while the tile loads.
+    // each) are copied to shared memory while the first stage runs.
     constexpr int HQC = khat_cols_stride<H>();
     const float* kh = wd.khat + ((size_t)k * (W / 2 + 1) + (size_t)TC * t) * HQC;
     if (fusable<H, MR>() && t != 0 && wd.HQ == HQC && ((uintptr_t)kh & 15) == 0) {
         float* ksm = col_khat_smem<H, MR>(stw);
         for (int e = threadIdx.x; e < TC * HQC / 4; e += NT) cp_async16(ksm + 4 * e, kh + 4 * e);
-        load_tile<H, NT, CG>(X, src);
-        cp_async_wait_all();
-        __syncthreads();
-        fft_fused<H, TC, NT, false, true, MR>(X, stw, [&](int s, int j, float2* v) {
-            constexpr int R = plan_radix(H, 0, MR), NB = H / R;
-            const float* kc = ksm + s * HQC;
-#pragma unroll
-            for (int m = 0; m < R; m++) {
-                const int ky = j + m * NB;
-                v[m] = cscale(v[m], kc[ky <= H / 2 ? ky : H - ky]);
-            }
-        });
-        store_tile<H, NT>(X, wd.conv + k * cplane + (size_t)t * H * TC);
+        // the stage tables are read after col_chained's first barrier
+        col_chained<H, NT, CG, MR>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC, ksm);
         return;
     }
     col_item_unchained<H, NT, CG, MR>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC,
                                   wd.khat + (size_t)k * (W / 2 + 1) * HQ, HQ, W, t);
 }
+
+// Shared memory of a column item's two sequences (the unchained item strides them by seq_stride).
+template <int H>
+FFT_CHD constexpr int col_seq_floats2() { return TC * (col_stride(H) > seq_stride(H) ? col_stride(H) : seq_stride(H)); }
 
 // MR: the radix cap of the build's plans (CMR; 16 for the radix-16 build of sizes whose CMR plan has
 // radix 32, launch variant 3)
@@ -686,11 +758,10 @@ template <int H, int NT, int MINB, int MR = CMR>
 __global__ void __launch_bounds__(NT, MINB) col_pass(const DevWorld* __restrict__ worlds, const ColItem* __restrict__ items,
                                                 const float2* __restrict__ tw) {
     extern __shared__ float4 smem_raw[];
-    constexpr int SEQ = seq_stride(H);
     float2* X = reinterpret_cast<float2*>(smem_raw);
-    float2* stw = X + TC * SEQ;
-    fill_stage_twiddles<H, float2, 0, MR>(stw, tw, threadIdx.x, NT);
+    float2* stw = X + col_seq_floats2<H>();
     const ColItem it = items[blockIdx.x];
+    fill_stage_twiddles<H, float2, 0, MR>(stw, tw, threadIdx.x, NT);
     col_item<H, NT, false, MR>(worlds[it.world], it, X, stw);
 }
 
@@ -775,15 +846,63 @@ __device__ __noinline__ void col_item_unchained_pair(cpair* X, const tw2* stw, c
     store_tile_pair<H, NT>(X, dst);
 }
 
+// The chained paired item: as col_chained, with one butterfly of both columns per thread (a warp's access
+// to the tile is 512 contiguous bytes).
+template <int H, int NT>
+__device__ __forceinline__ void col_chained_pair(cpair* X, const tw2* stw, const float2* __restrict__ src,
+                                                 float2* __restrict__ dst, const float* ksm) {
+    constexpr int LAST = plan_len(H, PMR) - 1, R = plan_radix(H, 0, PMR), NB = H / R;
+    constexpr int HQC = khat_cols_stride<H>();
+    static_assert(fusable<H, PMR>() && NB <= NT, "one outer butterfly per thread");
+    const int j = threadIdx.x;
+    const bool on = NB == NT || j < NB;
+    const tw2* last = stw + stage_tw_offset(H, LAST, PMR);
+    cpair v[R];
+    if (on) {
+        const float4* s4 = reinterpret_cast<const float4*>(src) + j;
+        const uint64_t keep = hint::policy_keep();
+#pragma unroll
+        for (int m = 0; m < R; m++) {
+            const float4 q = hint::ld4(s4 + m * NB, keep);
+            v[m] = cpair{make_float2(q.x, q.z), make_float2(q.y, q.w)};
+        }
+        Dft<R, false>::run(v);
+        stage_store<H, R, 1>(X, j, v);
+    }
+    cp_async_wait_all();  // the khat columns
+    __syncthreads();
+    fft_stages<H, 1, NT, false, 1, LAST>(X, stw);
+    if (on) {
+        stage_load<H, R, NB, false>(X, j, v, last);
+#pragma unroll
+        for (int m = 0; m < R; m++) {
+            const int ky = j + m * NB, kk = ky <= H / 2 ? ky : H - ky;
+            v[m] = cscale2(v[m], make_float2(ksm[kk], ksm[HQC + kk]));
+        }
+        Dft<R, true>::run(v);
+    }
+    __syncthreads();
+    if (on) stage_store<H, R, 1>(X, j, v);
+    __syncthreads();
+    fft_stages<H, 1, NT, true, 1, LAST>(X, stw);
+    if (on) {
+        stage_load<H, R, NB, true>(X, j, v, last);
+        float4* d4 = reinterpret_cast<float4*>(dst) + j;
+        const uint64_t keep = hint::policy_keep();
+#pragma unroll
+        for (int m = 0; m < R; m++) hint::st4(d4 + m * NB, make_float4(v[m].re.x, v[m].im.x, v[m].re.y, v[m].im.y), keep);
+    }
+}
+
 template <int H, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) col_pass_pair(const DevWorld* __restrict__ worlds,
                                                      const ColItem* __restrict__ items, const float2* __restrict__ tw) {
     extern __shared__ float4 smem_raw[];
     cpair* X = reinterpret_cast<cpair*>(smem_raw);
     tw2* stw = reinterpret_cast<tw2*>(X + seq_stride(H));
-    fill_stage_twiddles<H>(stw, tw, threadIdx.x, NT);
     const ColItem it = items[blockIdx.x];
     const DevWorld& wd = worlds[it.world];
+    fill_stage_twiddles<H>(stw, tw, threadIdx.x, NT);
     const int W = wd.W, c = it.chan, t = it.tile, k = it.kernel, HQ = wd.HQ;
     const size_t cplane = (size_t)(W / 2) * H;
     const float2* src = wd.spec + c * cplane + (size_t)t * H * TC;
@@ -793,18 +912,7 @@ __global__ void __launch_bounds__(NT, MINB) col_pass_pair(const DevWorld* __rest
     if (fusable<H, PMR>() && t != 0 && wd.HQ == HQC && ((uintptr_t)kh & 15) == 0) {
         float* ksm = col_khat_smem_pair<H>(stw);
         for (int e = threadIdx.x; e < TC * HQC / 4; e += NT) cp_async16(ksm + 4 * e, kh + 4 * e);
-        load_tile_pair<H, NT>(X, src);
-        cp_async_wait_all();
-        __syncthreads();
-        fft_fused<H, 1, NT, false, true>(X, stw, [&](int, int j, cpair* v) {
-            constexpr int R = plan_radix(H, 0, PMR), NB = H / R;
-#pragma unroll
-            for (int m = 0; m < R; m++) {
-                const int ky = j + m * NB, kk = ky <= H / 2 ? ky : H - ky;
-                v[m] = cscale2(v[m], make_float2(ksm[kk], ksm[HQC + kk]));
-            }
-        });
-        store_tile_pair<H, NT>(X, dst);
+        col_chained_pair<H, NT>(X, stw, src, dst, ksm);
         return;
     }
     col_item_unchained_pair<H, NT>(X, stw, src, dst, wd.khat + (size_t)k * (W / 2 + 1) * HQ, HQ, W, t);
@@ -843,7 +951,7 @@ template <int N> constexpr int minb_pair_of() { return 512 / nt_pair_of<N>() < 1
 // its first launch and before any stream capture that contains it; a zero-item call does just that.
 template <int H, int NT, int MINB, int MR = CMR>
 bool col_go(const DevWorld* worlds, const ColItem* items, int nitems, const float2* tw, cudaStream_t s) {
-    const size_t smem = (size_t)TC * seq_stride(H) * sizeof(float2) + stage_table_bytes<H, MR>() + col_khat_bytes<H>();
+    const size_t smem = col_seq_floats2<H>() * sizeof(float2) + stage_table_bytes<H, MR>() + col_khat_bytes<H>();
     static int attr_max = 0;
     if ((int)smem > attr_max) {
         if (cudaFuncSetAttribute(col_pass<H, NT, MINB, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
