@@ -34,7 +34,7 @@ thread_local std::string g_create_error;
 // of streaming them from HBM twice per generation.
 struct Chunk {
     int col0 = 0, ncol = 0, tcg0 = 0, ntcg = 0, row0 = 0, nrow = 0;
-    size_t bytes = 0;
+    size_t bytes = 0, cells = 0;
 };
 
 struct SizeClass {
@@ -411,10 +411,11 @@ int flush_spectra(LeniaCtx* ctx) {
     return 0;
 }
 
-// The column pass of one class (or one world's slice of it).
+// The column pass of one class (or one world's slice of it).  overlap: the launch directly follows an
+// FP32 pass on s (overlap and early as in LaunchOn).
 bool launch_columns(LeniaCtx* ctx, const SizeClass& cl, const ColItem* col, int ncol, const ColItem* tcg, int ntcg,
-                    int variant, int var_tc, cudaStream_t s) {
-    if (ntcg <= 0) return launch_col_fp32(cl.H, variant, ctx->d_worlds, col, ncol, ctx->d_tw, s);
+                    int variant, int var_tc, cudaStream_t s, bool overlap = false, bool early = false) {
+    if (ntcg <= 0) return launch_col_fp32(cl.H, variant, ctx->d_worlds, col, ncol, ctx->d_tw, LaunchOn(s, overlap, early));
     // Tensor-core paths: the FP32 items (each channel's first tile group, which holds the packed
     // DC/Nyquist column) are few.  After the tensor-core launch they ran on an otherwise idle GPU
     // (a 4096-point column item takes about as long as a quarter of the whole tensor-core launch),
@@ -436,12 +437,14 @@ bool launch_columns(LeniaCtx* ctx, const SizeClass& cl, const ColItem* col, int 
 
 // The row pass of one step over a run of a class's row items: on the tensor cores where the class
 // takes them, else the FP32 pass.
-bool launch_rows_step(LeniaCtx* ctx, const SizeClass& cl, int variant, const RowItem* items, int nrow, cudaStream_t s) {
+bool launch_rows_step(LeniaCtx* ctx, const SizeClass& cl, int variant, const RowItem* items, int nrow, cudaStream_t s,
+                      bool overlap = false, bool early = false) {
     if (cl.tc_rows) {
         const int st = cl.tc_row_stride, ngroups = st > 0 ? nrow / st : nrow * -st;
         return launch_row_tc(ctx->tc, ctx->path, cl.W, ctx->d_worlds, items, st, ngroups, ctx->d_tw, s);
     }
-    return launch_row_fp32(cl.W, variant, MODE_STEP, cl.general, ctx->d_worlds, items, nrow, cl.planes, ctx->d_tw, s);
+    return launch_row_fp32(cl.W, variant, MODE_STEP, cl.general, ctx->d_worlds, items, nrow, cl.planes, ctx->d_tw,
+                           LaunchOn(s, overlap, early));
 }
 
 // A launch shape of one size class: launch variants, chunks and the lanes the chunks run on.
@@ -451,6 +454,17 @@ struct Shape {
     int lanes;
 };
 Shape shape_of(const SizeClass& cl) { return Shape{cl.var_col, cl.var_row, cl.var_tc, &cl.chunks, cl.lanes}; }
+
+// Whether a chunk's passes let each other start early (LaunchOn::early).  CTAs that start early take the slots
+// that are free while the pass ahead still runs.  With at most one CTA per SM there is room everywhere
+// (128 x 128: 5.1 -> 4.6 us a generation); with many small CTAs that all fit the GPU together the
+// places even out (54 worlds of 128 x 128: 8.9 -> 8.0 us, 63 of 192 x 192: 18.6 -> 17.6 us).  In between a few
+// SMs get several CTAs and others none (1024 x 1024, 256 and 128 CTAs: 11.1 -> 14.1 us), and passes of
+// several waves lose slots to waiting CTAs (4096 x 4096: 104.6 -> 106.5 us).
+bool early_dependents(const LeniaCtx* ctx, const Chunk& ch) {
+    const int most = std::max(ch.ncol, ch.nrow), least = std::min(ch.ncol, ch.nrow);
+    return most <= ctx->sms || (least >= 4 * ctx->sms && ch.cells <= (4u << 20));
+}
 
 // `steps` steps of one size class, chunk after chunk, in the given launch shape; a resident class is
 // one launch for all its worlds and steps.
@@ -480,11 +494,14 @@ int enqueue_class(LeniaCtx* ctx, const SizeClass& cl, const Shape& sh, int steps
     for (int c = 0; c < nch; c++) {
         const Chunk& ch = (*sh.chunks)[c];
         cudaStream_t on = lanes > 1 ? ctx->lane[c % lanes] : s;
+        // every FP32 launch but a stream's first follows another FP32 pass on that stream
+        const bool fp32 = ch.ntcg == 0 && !cl.tc_rows && ch.ncol > 0;
+        const bool early = fp32 && early_dependents(ctx, ch);
         for (int st = 0; st < steps; st++) {
             bool ok = launch_columns(ctx, cl, cl.d_col + ch.col0, ch.ncol, cl.d_tcg + ch.tcg0, ch.ntcg, sh.var_col,
-                                     sh.var_tc, on);
+                                     sh.var_tc, on, fp32 && (st > 0 || c >= lanes), early);
             if (!ok) return fail(ctx, LENIA_ECUDA, "column launch failed (H=%d)", cl.H);
-            ok = launch_rows_step(ctx, cl, sh.var_row, cl.d_row + ch.row0, ch.nrow, on);
+            ok = launch_rows_step(ctx, cl, sh.var_row, cl.d_row + ch.row0, ch.nrow, on, fp32, early);
             if (!ok) return fail(ctx, LENIA_ECUDA, "row launch failed (W=%d)", cl.W);
         }
     }
@@ -526,6 +543,7 @@ std::vector<Chunk> make_chunks(const LeniaCtx* ctx, const SizeClass& cl, size_t 
             ch.ntcg += b.ntcg;
             ch.nrow += b.nrow;
             ch.bytes += world_step_bytes(ctx->desc[wi]);
+            ch.cells += state_count(ctx->desc[wi]);
         }
         col += ch.ncol;
         tcg += ch.ntcg;

@@ -50,6 +50,35 @@ struct RowItem { int world, row0, chan, pad; };
 
 enum RowMode { MODE_STEP = 0, MODE_FORWARD = 1, MODE_U = 2 };
 
+// Where and how a pass is launched.
+// overlap: a programmatic dependent launch, whose CTAs may start before the kernel ahead of it on the
+// stream has finished; only for a launch that directly follows another FP32 pass on the same
+// stream (every pass waits for the kernel ahead of it, griddepcontrol.wait, before it touches what that
+// kernel reads or writes).  A CTA's set-up (its item, the world, stage tables, the kernel spectrum's
+// columns) then runs before that wait: 0.5 us a launch at every size, 1024 x 1024 alone 11.95 -> 11.1 us
+// a generation.
+// early: the pass lets the launch after it start before its own last stage or its spectrum stores, not
+// only as its CTAs end.
+struct LaunchOn {
+    cudaStream_t s;
+    bool overlap, early;
+    LaunchOn(cudaStream_t stream, bool overlap_ = false, bool early_ = false) : s(stream), overlap(overlap_), early(early_) {}
+};
+template <class... P, class... A>
+bool launch_pass(void (*kernel)(P...), int grid, int threads, size_t smem, LaunchOn on, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = on.s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = on.overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+}
+
 // Fused FP32 path (step_fp32_*.cu).  Every size is built in two launch variants with the same
 // threads per CTA: variant 0 caps registers at 64 per thread (more resident CTAs), variant 1 at
 // 128.  The column pass has a third, variant 2: the paired build (both columns of a tile in one
@@ -57,9 +86,9 @@ enum RowMode { MODE_STEP = 0, MODE_FORWARD = 1, MODE_U = 2 };
 // launcher picks its general build from its `general` argument.  Launchers return false if the
 // size is not built.
 bool launch_col_fp32(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
-                     const float2* tw, cudaStream_t s);
+                     const float2* tw, LaunchOn s);
 bool launch_row_fp32(int W, int variant, int mode, int general, const DevWorld* worlds, const RowItem* items,
-                     int nitems, int acc_planes, const float2* tw, cudaStream_t s);
+                     int nitems, int acc_planes, const float2* tw, LaunchOn s);
 size_t col_smem_bytes(int H);
 size_t row_smem_bytes(int W, int acc_planes);
 // Column-pass launch variants (launch_col_fp32): 0, 1 scalar builds at two register caps, 2 the paired

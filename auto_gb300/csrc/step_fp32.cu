@@ -44,13 +44,13 @@ int max_smem_optin() {
 }
 
 bool launch_col_fp32(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
-                     const float2* tw, cudaStream_t s) {
+                     const float2* tw, LaunchOn s) {
     return launch_col_group_small(H, variant, worlds, items, nitems, tw, s) ||
            launch_col_group_large(H, variant, worlds, items, nitems, tw, s);
 }
 
 bool launch_row_fp32(int W, int variant, int mode, int general, const DevWorld* worlds, const RowItem* items,
-                     int nitems, int acc_planes, const float2* tw, cudaStream_t s) {
+                     int nitems, int acc_planes, const float2* tw, LaunchOn s) {
     if (general)
         return launch_row_group_small_general(W, variant, mode, general, acc_planes, worlds, items, nitems, tw, s) ||
                launch_row_group_large_general(W, variant, mode, general, acc_planes, worlds, items, nitems, tw, s);

@@ -29,6 +29,14 @@
 namespace lenia {
 using namespace lfft;
 
+// Programmatic dependent launch (LaunchOn::overlap): grid_wait returns when the kernel before this one has
+// finished and its writes are visible (at once in a launch without overlap); grid_trigger
+// (LaunchOn::early) lets the next kernel's CTAs start once every CTA of this one has called it or
+// ended.  Every CTA of an overlapped pass waits, so a pass that has finished implies that every pass
+// before it has.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // 16-byte asynchronous global -> shared copy: nothing is held in registers while it is in flight.
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
@@ -388,7 +396,7 @@ __device__ __noinline__ void row_item_u(float2* Z, const float2* stw, const DevW
 // sequences, stw: the stage tables.  CG: spectrum and state loads bypass L1 (the persistent step,
 // where another CTA of the same launch wrote them).
 template <int W, int NT, bool CG>
-__device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, float2* Z, const float2* stw) {
+__device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, float2* Z, const float2* stw, bool early = false) {
     constexpr int S = row_seqs(W, false), ROWS = 2 * S;
     const int H = wd.H;
     const DevKernel kp = wd.kern[0];
@@ -404,6 +412,7 @@ __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, floa
     constexpr int R = plan_radix(W, 0), NB = W / R;
     static_assert(S * NB <= NT, "one butterfly per thread in the fused stage");
     if (threadIdx.x == 0) tc::bulk_prefetch_l2(st, ROWS * W * (uint32_t)sizeof(float));
+    if constexpr (!CG) grid_wait();
     load_rows_spectrum<W, S, NT, CG>(Z, wd.conv, H, r0);
     __syncthreads();
     float sa[R], sb[R];
@@ -426,6 +435,7 @@ __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, floa
                 sb[m] = hint::ld1_atc<(W + decltype(m)::value * NB) * 4, CG>(ga, stream);
             });
         });
+    if (!CG && early) grid_trigger();
     store_rows_spectrum<W, S, NT>(Z, wd.spec, H, r0);
 }
 
@@ -435,7 +445,7 @@ __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, floa
 // does not set the budget of the common path.
 template <int W, int NT, int MINB, bool GEN>
 __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict__ worlds, const RowItem* __restrict__ items,
-                                                int mode, int general, const float2* __restrict__ tw) {
+                                                int mode, int general, const float2* __restrict__ tw, bool early) {
     constexpr int S = row_seqs(W, GEN), ROWS = 2 * S;
     extern __shared__ float4 smem_raw[];
     constexpr int SEQ = seq_stride(W);
@@ -451,6 +461,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     const bool per_chan = wd.rule == LENIA_RULE_LENIA;
     const int d0 = per_chan ? it.chan : 0, d1 = per_chan ? it.chan + 1 : C;
 
+    if constexpr (GEN) grid_wait();
     if (mode == MODE_FORWARD) {
         row_item_forward<W, NT, S>(Z, stw, wd, r0, d0, d1);
         return;
@@ -461,7 +472,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     }
 
     if constexpr (!GEN) {
-        row_item_simple<W, NT, false>(wd, r0, Z, stw);
+        row_item_simple<W, NT, false>(wd, r0, Z, stw, early);
         return;
     }
 
@@ -559,6 +570,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
                 sb[m] = hint::ld1(ga + W + m * NB, stream);
             }
         });
+    if (early) grid_trigger();
     store_rows_spectrum<W, S, NT>(Z, wd.spec + d0 * cplane, H, r0);
 }
 
@@ -633,12 +645,13 @@ __device__ __forceinline__ void store_tile(const float2* X, float2* __restrict__
 // in W/4 takes this path, and as a separate function its registers do not add to the chained path's.
 template <int H, int NT, bool CG = false, int MR = CMR>
 __device__ __noinline__ void col_item_unchained(float2* X, const float2* stw, const float2* src, float2* dst,
-                                                const float* kh, int HQ, int W, int t) {
+                                                const float* kh, int HQ, int W, int t, bool early) {
     load_tile<H, NT, CG>(X, src);
     __syncthreads();
     fft_seqs<H, TC, NT, false, MR>(X, stw);
     multiply_khat<H, NT>(X, X, kh, HQ, W, t);
     __syncthreads();
+    if (!CG && early) grid_trigger();
     fft_seqs<H, TC, NT, true, MR>(X, stw);
     store_tile<H, NT>(X, dst);
 }
@@ -682,7 +695,7 @@ __device__ __forceinline__ void col_stages(float2* X, const float2* stw) {
 // 60.7 -> 55.3 us, 41 of 512 x 512 47.2 -> 44.7, one of 4096 x 4096 107.5 -> 103.3, of 8192 x 8192 576 -> 552.
 template <int H, int NT, bool CG, int MR>
 __device__ __forceinline__ void col_chained(float2* X, const float2* stw, const float2* __restrict__ src,
-                                            float2* __restrict__ dst, const float* ksm) {
+                                            float2* __restrict__ dst, const float* ksm, bool early) {
     constexpr int LAST = plan_len(H, MR) - 1, R = plan_radix(H, 0, MR), NB = H / R, CS = col_stride(H);
     constexpr int HQC = khat_cols_stride<H>();
     static_assert(TC == 2 && fusable<H, MR>() && TC * NB <= NT, "one outer butterfly per thread, two columns");
@@ -713,6 +726,7 @@ __device__ __forceinline__ void col_chained(float2* X, const float2* stw, const 
     __syncthreads();
     if (on) stage_store<H, R, 1>(Xc, j, v);
     __syncthreads();
+    if (!CG && early) grid_trigger();
     col_stages<H, NT, true, 1, LAST, MR>(X, stw);
     if (on) {
         stage_load<H, R, NB, true>(Xc, j, v, stw + stage_tw_offset(H, LAST, MR));
@@ -728,7 +742,7 @@ __device__ __forceinline__ void col_chained(float2* X, const float2* stw, const 
 // multiplies the items, which the multichannel world needs more than it needs the saved transforms.
 // CG: the tile loads bypass L1 (the persistent step, where another CTA of the same launch wrote them).
 template <int H, int NT, bool CG, int MR = CMR>
-__device__ __forceinline__ void col_item(const DevWorld& wd, const ColItem it, float2* X, float2* stw) {
+__device__ __forceinline__ void col_item(const DevWorld& wd, const ColItem it, float2* X, float2* stw, bool early = false) {
     const int W = wd.W, c = it.chan, t = it.tile, k = it.kernel, HQ = wd.HQ;
     const size_t cplane = (size_t)(W / 2) * H;
     const float2* src = wd.spec + c * cplane + (size_t)t * H * TC;
@@ -740,12 +754,14 @@ __device__ __forceinline__ void col_item(const DevWorld& wd, const ColItem it, f
     if (fusable<H, MR>() && t != 0 && wd.HQ == HQC && ((uintptr_t)kh & 15) == 0) {
         float* ksm = col_khat_smem<H, MR>(stw);
         for (int e = threadIdx.x; e < TC * HQC / 4; e += NT) cp_async16(ksm + 4 * e, kh + 4 * e);
+        if constexpr (!CG) grid_wait();
         // the stage tables are read after col_chained's first barrier
-        col_chained<H, NT, CG, MR>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC, ksm);
+        col_chained<H, NT, CG, MR>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC, ksm, early);
         return;
     }
+    if constexpr (!CG) grid_wait();
     col_item_unchained<H, NT, CG, MR>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC,
-                                  wd.khat + (size_t)k * (W / 2 + 1) * HQ, HQ, W, t);
+                                  wd.khat + (size_t)k * (W / 2 + 1) * HQ, HQ, W, t, early);
 }
 
 // Shared memory of a column item's two sequences (the unchained item strides them by seq_stride).
@@ -756,13 +772,13 @@ FFT_CHD constexpr int col_seq_floats2() { return TC * (col_stride(H) > seq_strid
 // radix 32, launch variant 3)
 template <int H, int NT, int MINB, int MR = CMR>
 __global__ void __launch_bounds__(NT, MINB) col_pass(const DevWorld* __restrict__ worlds, const ColItem* __restrict__ items,
-                                                const float2* __restrict__ tw) {
+                                                const float2* __restrict__ tw, bool early) {
     extern __shared__ float4 smem_raw[];
     float2* X = reinterpret_cast<float2*>(smem_raw);
     float2* stw = X + col_seq_floats2<H>();
     const ColItem it = items[blockIdx.x];
     fill_stage_twiddles<H, float2, 0, MR>(stw, tw, threadIdx.x, NT);
-    col_item<H, NT, false, MR>(worlds[it.world], it, X, stw);
+    col_item<H, NT, false, MR>(worlds[it.world], it, X, stw, early);
 }
 
 // ------------------------------------------------------------------ paired column pass
@@ -836,12 +852,13 @@ __device__ __forceinline__ void multiply_khat_pair(cpair* X, const float* __rest
 
 template <int H, int NT>
 __device__ __noinline__ void col_item_unchained_pair(cpair* X, const tw2* stw, const float2* src, float2* dst,
-                                                     const float* kh, int HQ, int W, int t) {
+                                                     const float* kh, int HQ, int W, int t, bool early) {
     load_tile_pair<H, NT>(X, src);
     __syncthreads();
     fft_seqs<H, 1, NT, false>(X, stw);
     multiply_khat_pair<H, NT>(X, kh, HQ, W, t);
     __syncthreads();
+    if (early) grid_trigger();
     fft_seqs<H, 1, NT, true>(X, stw);
     store_tile_pair<H, NT>(X, dst);
 }
@@ -850,7 +867,7 @@ __device__ __noinline__ void col_item_unchained_pair(cpair* X, const tw2* stw, c
 // to the tile is 512 contiguous bytes).
 template <int H, int NT>
 __device__ __forceinline__ void col_chained_pair(cpair* X, const tw2* stw, const float2* __restrict__ src,
-                                                 float2* __restrict__ dst, const float* ksm) {
+                                                 float2* __restrict__ dst, const float* ksm, bool early) {
     constexpr int LAST = plan_len(H, PMR) - 1, R = plan_radix(H, 0, PMR), NB = H / R;
     constexpr int HQC = khat_cols_stride<H>();
     static_assert(fusable<H, PMR>() && NB <= NT, "one outer butterfly per thread");
@@ -884,6 +901,7 @@ __device__ __forceinline__ void col_chained_pair(cpair* X, const tw2* stw, const
     __syncthreads();
     if (on) stage_store<H, R, 1>(X, j, v);
     __syncthreads();
+    if (early) grid_trigger();
     fft_stages<H, 1, NT, true, 1, LAST>(X, stw);
     if (on) {
         stage_load<H, R, NB, true>(X, j, v, last);
@@ -896,7 +914,8 @@ __device__ __forceinline__ void col_chained_pair(cpair* X, const tw2* stw, const
 
 template <int H, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) col_pass_pair(const DevWorld* __restrict__ worlds,
-                                                     const ColItem* __restrict__ items, const float2* __restrict__ tw) {
+                                                     const ColItem* __restrict__ items, const float2* __restrict__ tw,
+                                                     bool early) {
     extern __shared__ float4 smem_raw[];
     cpair* X = reinterpret_cast<cpair*>(smem_raw);
     tw2* stw = reinterpret_cast<tw2*>(X + seq_stride(H));
@@ -912,10 +931,12 @@ __global__ void __launch_bounds__(NT, MINB) col_pass_pair(const DevWorld* __rest
     if (fusable<H, PMR>() && t != 0 && wd.HQ == HQC && ((uintptr_t)kh & 15) == 0) {
         float* ksm = col_khat_smem_pair<H>(stw);
         for (int e = threadIdx.x; e < TC * HQC / 4; e += NT) cp_async16(ksm + 4 * e, kh + 4 * e);
-        col_chained_pair<H, NT>(X, stw, src, dst, ksm);
+        grid_wait();
+        col_chained_pair<H, NT>(X, stw, src, dst, ksm, early);
         return;
     }
-    col_item_unchained_pair<H, NT>(X, stw, src, dst, wd.khat + (size_t)k * (W / 2 + 1) * HQ, HQ, W, t);
+    grid_wait();
+    col_item_unchained_pair<H, NT>(X, stw, src, dst, wd.khat + (size_t)k * (W / 2 + 1) * HQ, HQ, W, t, early);
 }
 
 // Sizes built: each TU instantiates one group.  Threads per CTA: one first-stage butterfly per
@@ -950,7 +971,7 @@ template <int N> constexpr int minb_pair_of() { return 512 / nt_pair_of<N>() < 1
 // Launch one instantiation.  Dynamic shared memory above 48 KB must be enabled per kernel before
 // its first launch and before any stream capture that contains it; a zero-item call does just that.
 template <int H, int NT, int MINB, int MR = CMR>
-bool col_go(const DevWorld* worlds, const ColItem* items, int nitems, const float2* tw, cudaStream_t s) {
+bool col_go(const DevWorld* worlds, const ColItem* items, int nitems, const float2* tw, LaunchOn s) {
     const size_t smem = col_seq_floats2<H>() * sizeof(float2) + stage_table_bytes<H, MR>() + col_khat_bytes<H>();
     static int attr_max = 0;
     if ((int)smem > attr_max) {
@@ -959,8 +980,7 @@ bool col_go(const DevWorld* worlds, const ColItem* items, int nitems, const floa
             return false;
         attr_max = (int)smem;
     }
-    if (nitems > 0) col_pass<H, NT, MINB, MR><<<nitems, NT, smem, s>>>(worlds, items, tw);
-    return true;
+    return nitems <= 0 || launch_pass(col_pass<H, NT, MINB, MR>, nitems, NT, smem, s, worlds, items, tw, s.early);
 }
 
 template <int H>
@@ -969,7 +989,7 @@ constexpr size_t col_pair_smem() {
 }
 
 template <int H, int NT, int MINB>
-bool col_go_pair(const DevWorld* worlds, const ColItem* items, int nitems, const float2* tw, cudaStream_t s) {
+bool col_go_pair(const DevWorld* worlds, const ColItem* items, int nitems, const float2* tw, LaunchOn s) {
     const size_t smem = col_pair_smem<H>();
     static int attr_max = 0;
     if ((int)smem > attr_max) {
@@ -978,8 +998,7 @@ bool col_go_pair(const DevWorld* worlds, const ColItem* items, int nitems, const
             return false;
         attr_max = (int)smem;
     }
-    if (nitems > 0) col_pass_pair<H, NT, MINB><<<nitems, NT, smem, s>>>(worlds, items, tw);
-    return true;
+    return nitems <= 0 || launch_pass(col_pass_pair<H, NT, MINB>, nitems, NT, smem, s, worlds, items, tw, s.early);
 }
 
 // Shared memory of a row-pass launch: sequences, stage tables, then the general path's
@@ -993,7 +1012,7 @@ constexpr size_t row_smem(int general, int planes) {
 
 template <int W, int NT, int MINB, bool GEN>
 bool row_go(int mode, int general, int planes, const DevWorld* worlds, const RowItem* items, int nitems,
-            const float2* tw, cudaStream_t s) {
+            const float2* tw, LaunchOn s) {
     const size_t smem = row_smem<W, GEN>(general, planes);
     static int attr_max = 0;
     if ((int)smem > attr_max) {
@@ -1002,8 +1021,7 @@ bool row_go(int mode, int general, int planes, const DevWorld* worlds, const Row
             return false;
         attr_max = (int)smem;
     }
-    if (nitems > 0) row_pass<W, NT, MINB, GEN><<<nitems, NT, smem, s>>>(worlds, items, mode, general, tw);
-    return true;
+    return nitems <= 0 || launch_pass(row_pass<W, NT, MINB, GEN>, nitems, NT, smem, s, worlds, items, mode, general, tw, s.early);
 }
 
 // Column-pass builds: variant 0 and 1 are the scalar build at 64 (80 with a radix-32 plan) and 128
@@ -1011,7 +1029,7 @@ bool row_go(int mode, int general, int planes, const DevWorld* worlds, const Row
 // 64 registers where the scalar plan has radix 32 (elsewhere variant 0).
 template <int N>
 bool col_go_variant(int variant, const DevWorld* worlds, const ColItem* items, int nitems, const float2* tw,
-                    cudaStream_t s) {
+                    LaunchOn s) {
     if (variant == 2) return col_go_pair<N, nt_pair_of<N>(), minb_pair_of<N>()>(worlds, items, nitems, tw, s);
     if (variant == 1) return col_go<N, nt_of<N>(), minb_of<N, 1>()>(worlds, items, nitems, tw, s);
     if constexpr (col_r32<N>())
@@ -1065,12 +1083,12 @@ int row_local_bytes_large_simple(int W, int variant);
 int row_local_bytes_large_general(int W, int variant);
 
 bool launch_col_group_small(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
-                            const float2* tw, cudaStream_t s);
+                            const float2* tw, LaunchOn s);
 bool launch_col_group_large(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
-                            const float2* tw, cudaStream_t s);
+                            const float2* tw, LaunchOn s);
 #define LENIA_ROW_GROUP_DECL(NAME)                                                                       \
     bool NAME(int W, int variant, int mode, int general, int planes, const DevWorld* worlds, const RowItem* items, \
-              int nitems, const float2* tw, cudaStream_t s);
+              int nitems, const float2* tw, LaunchOn s);
 LENIA_ROW_GROUP_DECL(launch_row_group_small_simple)
 LENIA_ROW_GROUP_DECL(launch_row_group_small_general)
 LENIA_ROW_GROUP_DECL(launch_row_group_large_simple)

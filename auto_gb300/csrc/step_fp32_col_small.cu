@@ -4,7 +4,7 @@
 namespace lenia {
 
 bool launch_col_group_small(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
-                            const float2* tw, cudaStream_t s) {
+                            const float2* tw, LaunchOn s) {
     switch (H) { LENIA_SIZES_SMALL(LENIA_COL_CASE) }
     return false;
 }
