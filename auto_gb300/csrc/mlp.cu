@@ -7,10 +7,10 @@
 // (scripts/life_screen.py:143-179), which is the baseline this proposer is compared with.
 //
 // Parameters: FP32 master weights updated by Adam; BF16 copies feed every GEMM; activations are
-// stored in BF16 for the backward pass; every GEMM accumulates in FP32.  The GEMMs of the two
-// 256-wide layers -- forward h1 and h2, backward dh1 and the weight gradients dW1 and dW2 -- run on
-// the 5th-generation tensor cores (gemm_tc: tcgen05 MMAs, TMEM accumulators); the 3-wide output
-// layer's (z, dW3, dh2) on the CUDA cores.
+// rounded to BF16; every GEMM accumulates in FP32.  The GEMMs of the two 256-wide layers -- forward h1
+// and h2, backward dh1 and the weight gradients dW1 and dW2 -- run on the 5th-generation tensor cores
+// (tcgen05 MMAs, TMEM accumulators), the 3-wide output layer in the hand-overs between them, all in
+// one kernel (mlp_tile) that keeps a tile's activations in shared memory.
 //   layer 1: W1 [256 x 16],  b1 [256]      h1 = relu(x W1^T + b1)
 //   layer 2: W2 [256 x 256], b2 [256]      h2 = relu(h1 W2^T + b2)
 //   layer 3: W3 [3 x 256],   b3 [3]        z  = h2 W3^T + b3,  p = sigmoid(z)
@@ -35,266 +35,381 @@ constexpr int P_W1 = 0, P_B1 = P_W1 + HID * IN, P_W2 = P_B1 + HID, P_B2 = P_W2 +
 
 using bf16 = __nv_bfloat16;
 
-// C[M x N] = A[M x K] * B^T (B is [N x K]) with bf16 operands and FP32 accumulation, when
-// TRANS_B is false; C = A * B (B is [K x N]) when TRANS_B is true.  TRANS_A reads A as [K x M].
-// Epilogue: + bias[n], relu, and output in f32 and/or bf16 (and bf16 transposed, CbT[n * ldt + m]).
-// 64 x 64 tiles, 256 threads, 4 x 4 outputs per thread, K in steps of 16 through shared memory: the
-// CUDA-core GEMM of the 3-wide output layer, where an MMA tile would be almost all padding.
-template <bool TRANS_A, bool TRANS_B>
-__global__ void __launch_bounds__(256) gemm_bf16(const bf16* __restrict__ A, const bf16* __restrict__ B, int M, int N,
-                                                 int K, const float* __restrict__ bias, int relu, float* __restrict__ Cf,
-                                                 bf16* __restrict__ Cb, const bf16* __restrict__ mask,
-                                                 bf16* __restrict__ CbT = nullptr, int ldt = 0) {
-    __shared__ float As[16][64 + 1];
-    __shared__ float Bs[16][64 + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int i = threadIdx.x; i < 16 * 64; i += 256) {
-            const int kk = i / 64, mm = i % 64;
-            const int m = m0 + mm, k = k0 + kk;
-            float a = 0.f;
-            if (m < M && k < K) a = __bfloat162float(TRANS_A ? A[(size_t)k * M + m] : A[(size_t)m * K + k]);
-            As[kk][mm] = a;
-            const int n = n0 + mm;
-            float b = 0.f;
-            if (n < N && k < K) b = __bfloat162float(TRANS_B ? B[(size_t)k * N + n] : B[(size_t)n * K + k]);
-            Bs[kk][mm] = b;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (m >= M || n >= N) continue;
-            float v = acc[i][j] + (bias ? bias[n] : 0.f);
-            if (relu) v = fmaxf(v, 0.f);
-            if (mask && __bfloat162float(mask[(size_t)m * N + n]) <= 0.f) v = 0.f;
-            if (Cf) Cf[(size_t)m * N + n] = v;
-            if (Cb) Cb[(size_t)m * N + n] = __float2bfloat16_rn(v);
-            if (CbT) CbT[(size_t)n * ldt + m] = __float2bfloat16_rn(v);
-        }
+// ------------------------------------------------------------------ the network on a tile of rows
+// One CTA takes 128 rows through the whole network: forward to the logits and, with GRAD, back to every
+// gradient.  Nothing but the inputs, the weights and the results touches global memory.
+//
+// All operands sit in shared memory in the canonical layout without swizzle (8-row x 16-byte core
+// matrices, K-adjacent ones 128 bytes apart, 8-row groups one after another: tc::kmajor_offset).  A
+// matrix stored [r][c] that way is a K-major operand with K = c (LBO 128, SBO one row group) and, read
+// with the roles exchanged, an MN-major operand with K = r (LBO one row group, SBO 128): the same bytes
+// serve h1, dh2, dh1 and W2 in both of their products, so nothing is transposed or stored twice.
+//
+//   D      = x W1^T                       A x [m][i]        B W1 [o][i]      N = 256, K = 16
+//   h1     = relu(D + b1)                 -> R2
+//   D      = h1 W2^T                      A h1              B W2 [o][i]      N = 256, K = 256
+//   h2     = relu(D + b2), z = h2 W3^T + b3                                  (CUDA cores, per row)
+//   dz     = (sigmoid(z) - y) / (3 B), dh2 = (dz W3) * (h2 > 0) -> R1
+//   D      = dh2 W2                       A dh2             B W2 (MN-major)  N = 256, K = 256
+//   dh1    = D * (h1 > 0)                 -> R0
+//   dW2   += dh2^T h1                     A dh2 (MN-major)  B h1 (MN-major)  M = 2 x 128, N = 256, K = 128 rows
+//   dW1   += dh1^T x                      A dh1 (MN-major)  B x (MN-major)   M = 2 x 128, N = 16,  K = 128 rows
+//
+// The bias gradients are column sums of the unrounded FP32 dh2 and dh1 (transposed by shuffles), dW3
+// of dz h2; weight gradients of several tiles meet in global memory with vector reductions.  256
+// threads: warp w reads TMEM lanes 32 (w % 4) .. + 31 (the tile's rows) and columns 128 (w / 4) .. + 127.
+//
+// W2 takes R0 and R1 (128 KB); the backward pass needs R1 for dh2 and fetches W2's rows 128..255
+// again into R0.  One CTA per SM (214 KB of shared memory, all 512 TMEM columns).  A tile is a chain of
+// two (five) waits on the tensor cores with a hand-over after each, so it is bound by that latency: 71
+// tiles forward take 14 us (W2's load included), 8 tiles forward and back 40 us.  As separate GEMM
+// launches, whose hand-overs wrote h1 and h2 (and their transposes) to global memory with 2-byte stores
+// one row stride apart per lane, a 4096-row chunk took 155 us forward and 1000 rows 520 us forward and
+// back: lenia_mlp_predict of 250001 rows went from 11.1 to 0.39 ms, lenia_mlp_gradients of 1000 from 560
+// to 98 us (the rest is copies and synchronisation).
+//
+// Every barrier wait is bounded; a CTA that gives up waits (bounded) for its MMAs and copies, raises *err,
+// frees its TMEM and returns.
+constexpr int TILE = 128, NTHR = 256;
+constexpr uint32_t GROUP = HID * 2 * 8;    // bytes of eight 256-wide rows
+constexpr uint32_t XGROUP = IN * 2 * 8;    // bytes of eight 16-wide rows
+constexpr uint32_t REGION = TILE * HID * 2;  // 64 KB
+constexpr uint32_t S_W1 = 3 * REGION, S_X = S_W1 + HID * IN * 2, S_F = S_X + TILE * IN * 2;
+// floats from S_F: b1, b2, W3, the second column half's logits (then dz), and the sums db2, db1, dW3, db3
+constexpr int F_B1 = 0, F_B2 = F_B1 + HID, F_W3 = F_B2 + HID, F_Z = F_W3 + OUT * HID, F_DB2 = F_Z + TILE * OUT,
+              F_DB1 = F_DB2 + HID, F_DW3 = F_DB1 + HID, F_DB3 = F_DW3 + OUT * HID, F_END = F_DB3 + 4;
+constexpr uint32_t S_BAR = S_F + F_END * 4;
+constexpr uint32_t TILE_SMEM = S_BAR + 16;
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_u32(dst)), "l"(src) : "memory");
 }
-
-// ------------------------------------------------------------------ tensor-core GEMM (tcgen05)
-// C[M x N] = A[M x K] * B[N x K]^T with A and B bf16, K-major (rows lda / ldb elements apart), and
-// FP32 accumulation in TMEM: the GEMMs of the 256-wide layers.  A CTA of 128 threads owns 128 rows
-// of C and all N columns (N a multiple of 16, at most 256) and loops over K in chunks of 64:
-// every thread stages 16-byte pieces of both operands into shared memory with cp.async, in the
-// canonical K-major layout without swizzle (8-row x 16-byte core matrices, K-adjacent ones 128 bytes
-// apart, 8-row groups 1024 bytes apart), double-buffered, and one elected thread issues the
-// M = 128, N, K = 16 MMAs of a chunk and commits them to that buffer's mbarrier.  Elements past M or
-// K are zero-filled.  With ksplit > 1, CTA column kz of the grid takes every ksplit-th chunk and adds
-// its partial sums into Cf (zeroed by the caller) with atomics; the bias, ReLU, mask and bf16 outputs
-// need ksplit = 1.  Epilogue per row (a thread per TMEM lane): + bias[n], ReLU, zero where mask <= 0,
-// then FP32 (Cf), bf16 (Cb) and transposed bf16 (CbT[n * ldt + m]) outputs, each optional.  Every
-// barrier wait is bounded; a CTA that gives up waits (bounded) for its own MMAs, raises *err, frees
-// its TMEM and writes nothing.
-constexpr int TCK = 64;  // K elements per staged chunk: 128 bytes of bf16 per operand row
-template <int N>
-struct TcGemm {
-    static constexpr int ABYTES = 128 * TCK * 2, BBYTES = N * TCK * 2, STAGE = ABYTES + BBYTES;
-    static constexpr int SMEM = 2 * STAGE + 64;
-    static constexpr uint32_t TCOLS = N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256));
-    static_assert(N % 16 == 0 && N >= 16 && N <= 256, "MMA N");
-};
-
-__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc::smem_u32(dst)), "l"(src), "r"(src_bytes)
+__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
                  : "memory");
 }
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ uint4 pack8(const float* v) {
+    return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+}
+// Sums of 32 per-lane values over the warp's lanes: lane l gets the sum of the lanes' v[l] (each
+// step folds half of the remaining columns onto the other half's lanes).
+__device__ __forceinline__ float column_sums(float* v) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int w = 16; w >= 1; w >>= 1) {
+#pragma unroll
+        for (int i = 0; i < w; i++) {
+            const bool up = lane & w;
+            const float send = up ? v[i] : v[i + w], keep = up ? v[i + w] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+        }
+    }
+    return v[0];
+}
 
-template <int N>
-__global__ void __launch_bounds__(128, 1)
-    gemm_tc(const bf16* __restrict__ A, int lda, const bf16* __restrict__ B, int ldb, int M, int K, int ksplit,
-            const float* __restrict__ bias, int relu, const bf16* __restrict__ mask, float* __restrict__ Cf,
-            bf16* __restrict__ Cb, bf16* __restrict__ CbT, int ldt, int* __restrict__ err) {
-    using P = TcGemm<N>;
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * P::STAGE);  // MMA done, per buffer
-    uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 2);
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int m0 = blockIdx.x * 128, kz = blockIdx.y;
-    const int nchunks_all = (K + TCK - 1) / TCK;
-    const int nchunks = nchunks_all > kz ? (nchunks_all - kz + ksplit - 1) / ksplit : 0;  // this CTA's chunks
+// rows [first, first + n) of W2 (bf16 [256][256]) into an operand region, n a multiple of 8: eight rows of
+// one 16-byte column piece per eight lanes, 128 contiguous bytes of shared memory
+__device__ __forceinline__ void load_w2(uint8_t* dst, const bf16* __restrict__ w2, int first, int n) {
+    for (int e = threadIdx.x; e < n * (HID / 8); e += NTHR) {
+        const int r = (e >> 8) * 8 + (e & 7), kg = (e >> 3) & 31;
+        cp_async16(dst + tc::kmajor_offset(r, 8 * kg, HID, 2), w2 + (size_t)(first + r) * HID + 8 * kg);
+    }
+}
+
+template <bool GRAD>
+__global__ void __launch_bounds__(NTHR, 1)
+    mlp_tile(const float* __restrict__ x, const float* __restrict__ y, int B, const float* __restrict__ w,
+             const bf16* __restrict__ wb, float* __restrict__ probs, float* __restrict__ g,
+             float* __restrict__ loss_rows, int* __restrict__ err) {
+    extern __shared__ __align__(1024) uint8_t sm[];
+    uint8_t *R0 = sm, *R1 = sm + REGION, *R2 = sm + 2 * REGION, *W1s = sm + S_W1, *Xs = sm + S_X;
+    float* F = reinterpret_cast<float*>(sm + S_F);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + S_BAR);
+    uint32_t* slot = reinterpret_cast<uint32_t*>(bar + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row = (warp & 3) * 32 + lane, half = warp >> 2;  // this thread's tile row and column half
+    const int ntiles = (B + TILE - 1) / TILE;
+    const bf16* w2 = wb + P_W2;
+
+    for (int e = tid; e < HID * 2; e += NTHR)
+        cp_async16(W1s + tc::kmajor_offset(e >> 1, 8 * (e & 1), IN, 2), wb + P_W1 + (e >> 1) * IN + 8 * (e & 1));
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    load_w2(R0, w2, 0, HID);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int e = tid; e < HID; e += NTHR) F[F_B1 + e] = w[P_B1 + e], F[F_B2 + e] = w[P_B2 + e];
+    for (int e = tid; e < OUT * HID; e += NTHR) F[F_W3 + e] = __bfloat162float(wb[P_W3 + e]);
+    if (GRAD)
+        for (int e = F_DB2 + tid; e < F_END; e += NTHR) F[e] = 0.f;
     if (tid == 0) {
-        tc::mbar_init(bars, 1);
-        tc::mbar_init(bars + 1, 1);
+        tc::mbar_init(bar, 1);
         tc::fence_barrier_init();
     }
-    if (warp == 0) tc::tmem_alloc(slot, P::TCOLS);
+    if (warp == 0) tc::tmem_alloc(slot, 512);
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    const uint32_t tmem = *slot;
+    const uint32_t tmem = *slot, mine = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t r0 = tc::smem_u32(R0), r1 = tc::smem_u32(R1), r2 = tc::smem_u32(R2), xs = tc::smem_u32(Xs),
+                   w1s = tc::smem_u32(W1s);
+    constexpr uint32_t ID_FWD = tc::instr_desc(1, 128, HID), ID_DH1 = tc::instr_desc(1, 128, HID, false, true),
+                       ID_DW2 = tc::instr_desc(1, 128, HID, true, true), ID_DW1 = tc::instr_desc(1, 128, IN, true, true);
 
-    // stage chunk `ci` (the ci-th of this CTA) into buffer b
-    auto load = [&](int ci, int b) {
-        uint8_t* sa = smem + b * P::STAGE;
-        uint8_t* sb = sa + P::ABYTES;
-        const int k0 = (kz + ci * ksplit) * TCK;
-        constexpr int PIECES = (128 + N) * (TCK / 8);
-        for (int idx = tid; idx < PIECES; idx += 128) {
-            const int row = idx / (TCK / 8), kg = idx % (TCK / 8), k = k0 + 8 * kg;
-            const bool is_a = row < 128;
-            const int r = is_a ? row : row - 128;
-            const int grow = is_a ? m0 + r : r;
-            const bool valid = (!is_a || grow < M) && k < K;
-            uint8_t* dst = (is_a ? sa : sb) + tc::kmajor_offset(r, 8 * kg, TCK, 2);
-            if (valid && k + 8 <= K) {
-                cp_async16_zfill(dst, (is_a ? A + (size_t)grow * lda : B + (size_t)grow * ldb) + k, 16);
-            } else if (valid) {
-                // the last piece of a row whose K is not a multiple of 8: element by element
-                const uint16_t* src = reinterpret_cast<const uint16_t*>((is_a ? A + (size_t)grow * lda : B + (size_t)grow * ldb) + k);
-                uint16_t h[8];
-                for (int i = 0; i < 8; i++) h[i] = k + i < K ? src[i] : (uint16_t)0;
-                *reinterpret_cast<uint4*>(dst) = make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16,
-                                                            h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
-            } else {
-                *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    uint32_t phase = 0;
+    bool pending = false;  // a commit that no wait has seen (uniform across the CTA)
+    auto commit = [&]() {  // thread 0
+        tc::mma_commit(bar);
     };
-    constexpr uint32_t IDESC = tc::instr_desc(1, 128, N);
-    constexpr uint32_t SBO = TCK * 2 * 8;
-    bool ok = true;
-    int issued = 0;  // chunks whose MMAs were issued
-    if (nchunks > 0) load(0, 0);
-    for (int ci = 0; ci < nchunks && ok; ci++) {
-        if (ci + 1 < nchunks) {
-            // the buffer of chunk ci + 1 was read by the MMAs of chunk ci - 1
-            if (ci >= 1 && __syncthreads_or(!tc::mbar_wait(bars + ((ci + 1) & 1), ((ci - 1) >> 1) & 1))) {
-                ok = false;
-                break;
-            }
-            load(ci + 1, (ci + 1) & 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+    // wait for the last commit; false (for the whole CTA) if it did not come
+    auto wait = [&]() -> bool {
+        const bool gave_up = __syncthreads_or(!tc::mbar_wait(bar, phase));
+        phase ^= 1;
+        pending = gave_up;
+        tc::tc_fence_after();
+        return !gave_up;
+    };
+    // shared-memory operands written and TMEM read: thread 0 may issue MMAs
+    auto publish = [&]() {
+        tc::tc_fence_before();
         tc::fence_async_smem();
         __syncthreads();
-        if (tid == 0) {
-            tc::tc_fence_after();
-            const uint32_t sa = tc::smem_u32(smem + (ci & 1) * P::STAGE), sb = sa + P::ABYTES;
-            const int k0 = (kz + ci * ksplit) * TCK;
-            const int ksteps = (min(TCK, K - k0) + 15) / 16;
-            for (int s = 0; s < ksteps; s++)
-                tc::mma<false>(tmem, tc::smem_desc(sa + 256u * s, 128, SBO), tc::smem_desc(sb + 256u * s, 128, SBO),
-                               IDESC, (ci > 0 || s > 0) ? 1u : 0u);
-            tc::mma_commit(bars + (ci & 1));
+        tc::tc_fence_after();
+    };
+
+    // this thread's eight inputs of a tile: row tid / 2, half a row each
+    float xin[8];
+    auto fetch = [&](int t) {
+        const int r = t * TILE + (tid >> 1);
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (r < B) {
+            const float4* p = reinterpret_cast<const float4*>(x + (size_t)r * IN + 8 * (tid & 1));
+            a = p[0], b = p[1];
         }
-        issued = ci + 1;
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // the last issued chunk's commit covers every earlier MMA
-    if (ok && issued > 0 && __syncthreads_or(!tc::mbar_wait(bars + ((issued - 1) & 1), ((issued - 1) >> 1) & 1)))
-        ok = false;
-    tc::tc_fence_after();
-    if (ok && issued > 0) {
-        const int row = m0 + tid;
-        for (int n0 = 0; n0 < N; n0 += 32) {
+        xin[0] = a.x, xin[1] = a.y, xin[2] = a.z, xin[3] = a.w, xin[4] = b.x, xin[5] = b.y, xin[6] = b.z, xin[7] = b.w;
+    };
+    bool ok = true, first = true;
+    fetch(blockIdx.x);
+    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, first = false) {
+        if (GRAD && !first) load_w2(R0, w2, 0, HID);  // the backward pass of the last tile took its place
+        *reinterpret_cast<uint4*>(Xs + tc::kmajor_offset(tid >> 1, 8 * (tid & 1), IN, 2)) = pack8(xin);
+        if (first) asm volatile("cp.async.wait_group 1;" ::: "memory");  // W1
+        publish();
+        if (tid == 0) {
+            tc::mma<false>(tmem, tc::smem_desc(xs, 128, XGROUP), tc::smem_desc(w1s, 128, XGROUP), ID_FWD, 0u);
+            commit();
+        }
+        pending = true;
+        if (t + (int)gridDim.x < ntiles) fetch(t + gridDim.x);
+        if (!(ok = wait())) break;
+        // rows past the batch are zeros in every product (a row that is not there meets no infinite weight)
+        const int b = t * TILE + row;
+        const bool valid = b < B;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int n0 = half * 128 + 32 * c;
             float v[32];
-            tc::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)n0, v);
-            if (row >= M) continue;
-            const int nn = N - n0 < 32 ? N - n0 : 32;
-            for (int i = 0; i < nn; i++) {
-                const int n = n0 + i;
-                float x = v[i];
-                if (ksplit > 1) {
-                    atomicAdd(Cf + (size_t)row * N + n, x);
-                    continue;
-                }
-                if (bias) x += bias[n];
-                if (relu) x = fmaxf(x, 0.f);
-                if (mask && __bfloat162float(mask[(size_t)row * N + n]) <= 0.f) x = 0.f;
-                if (Cf) Cf[(size_t)row * N + n] = x;
-                const bf16 xb = __float2bfloat16_rn(x);
-                if (Cb) Cb[(size_t)row * N + n] = xb;
-                if (CbT) CbT[(size_t)n * ldt + row] = xb;
+            tc::tmem_ld32(mine + n0, v);
+#pragma unroll
+            for (int i = 0; i < 32; i++) v[i] = valid ? fmaxf(v[i] + F[F_B1 + n0 + i], 0.f) : 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                *reinterpret_cast<uint4*>(R2 + tc::kmajor_offset(row, n0 + 8 * i, HID, 2)) = pack8(v + 8 * i);
+        }
+        if (GRAD || first) cp_async_wait0();  // W2
+        publish();
+        if (tid == 0) {
+            for (uint32_t s = 0; s < HID / 16; s++)
+                tc::mma<false>(tmem + HID, tc::smem_desc(r2 + 256u * s, 128, GROUP), tc::smem_desc(r0 + 256u * s, 128, GROUP),
+                               ID_FWD, s > 0);
+            commit();
+        }
+        pending = true;
+        if (!(ok = wait())) break;
+        float z[OUT] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int n0 = half * 128 + 32 * c;
+            float v[32];
+            tc::tmem_ld32(mine + HID + n0, v);
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+                const float h = __bfloat162float(__float2bfloat16_rn(fmaxf(v[i] + F[F_B2 + n0 + i], 0.f)));
+#pragma unroll
+                for (int o = 0; o < OUT; o++) z[o] = fmaf(h, F[F_W3 + o * HID + n0 + i], z[o]);
             }
         }
+        if (half == 1)
+            for (int o = 0; o < OUT; o++) F[F_Z + row * OUT + o] = z[o];
+        tc::tc_fence_before();
+        __syncthreads();
+        tc::tc_fence_after();
+        if (half == 0) {
+            float l = 0.f, dz[OUT];
+#pragma unroll
+            for (int o = 0; o < OUT; o++) {
+                const float zz = z[o] + F[F_Z + row * OUT + o] + w[P_B3 + o];
+                const float p = 1.f / (1.f + expf(-zz));
+                if (!GRAD) {
+                    if (valid) probs[(size_t)b * OUT + o] = p;
+                } else {
+                    const float yy = valid ? y[(size_t)b * OUT + o] : 0.f;
+                    l += fmaxf(zz, 0.f) - zz * yy + log1pf(expf(-fabsf(zz)));
+                    dz[o] = valid ? (p - yy) / (float)(B * OUT) : 0.f;
+                    F[F_Z + row * OUT + o] = __bfloat162float(__float2bfloat16_rn(dz[o]));
+                }
+            }
+            if (GRAD) {
+                if (valid) loss_rows[b] = l / OUT;
+#pragma unroll
+                for (int o = 0; o < OUT; o++) {
+                    for (int d = 16; d > 0; d >>= 1) dz[o] += __shfl_xor_sync(0xffffffffu, dz[o], d);
+                    if (lane == 0) atomicAdd(&F[F_DB3 + o], dz[o]);
+                }
+            }
+        }
+        if (!GRAD) continue;
+
+        __syncthreads();
+        float dzb[OUT];
+        for (int o = 0; o < OUT; o++) dzb[o] = F[F_Z + row * OUT + o];
+#pragma unroll 1
+        for (int c = 0; c < 4; c++) {
+            const int n0 = half * 128 + 32 * c;
+            float v[32], q[32];
+            tc::tmem_ld32(mine + HID + n0, v);
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+                v[i] = valid ? __bfloat162float(__float2bfloat16_rn(fmaxf(v[i] + F[F_B2 + n0 + i], 0.f))) : 0.f;
+#pragma unroll
+            for (int o = 0; o < OUT; o++) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) q[i] = dzb[o] * v[i];
+                atomicAdd(&F[F_DW3 + o * HID + n0 + lane], column_sums(q));
+            }
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+                float d = 0.f;
+#pragma unroll
+                for (int o = 0; o < OUT; o++) d = fmaf(dzb[o], F[F_W3 + o * HID + n0 + i], d);
+                v[i] = v[i] > 0.f ? d : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                *reinterpret_cast<uint4*>(R1 + tc::kmajor_offset(row, n0 + 8 * i, HID, 2)) = pack8(v + 8 * i);
+            atomicAdd(&F[F_DB2 + n0 + lane], column_sums(v));
+        }
+        publish();
+        if (tid == 0) {
+            for (uint32_t s = 0; s < 8; s++)
+                tc::mma<false>(tmem, tc::smem_desc(r1 + 256u * s, 128, GROUP), tc::smem_desc(r0 + 2 * GROUP * s, GROUP, 128),
+                               ID_DH1, s > 0);
+            commit();
+        }
+        pending = true;
+        if (!(ok = wait())) break;
+        load_w2(R0, w2, 128, 128);
+        cp_async_wait0();
+        publish();
+        if (tid == 0) {
+            for (uint32_t s = 0; s < 8; s++)
+                tc::mma<false>(tmem, tc::smem_desc(r1 + 256u * (8 + s), 128, GROUP),
+                               tc::smem_desc(r0 + 2 * GROUP * s, GROUP, 128), ID_DH1, 1u);
+            for (uint32_t s = 0; s < 8; s++)  // dW2, outputs 128..255
+                tc::mma<false>(tmem + HID, tc::smem_desc(r1 + 16 * 128 + 2 * GROUP * s, GROUP, 128),
+                               tc::smem_desc(r2 + 2 * GROUP * s, GROUP, 128), ID_DW2, s > 0);
+            commit();
+        }
+        pending = true;
+        if (!(ok = wait())) break;
+#pragma unroll 1
+        for (int c = 0; c < 4; c++) {
+            const int n0 = half * 128 + 32 * c;
+            float v[32];
+            tc::tmem_ld32(mine + n0, v);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint4 h = *reinterpret_cast<const uint4*>(R2 + tc::kmajor_offset(row, n0 + 8 * i, HID, 2));
+                const uint32_t hw[4] = {h.x, h.y, h.z, h.w};
+                // h1 is a ReLU's output: zero where its bits (sign aside) are
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (((hw[k / 2] >> (16 * (k & 1))) & 0x7fffu) == 0u) v[8 * i + k] = 0.f;
+                *reinterpret_cast<uint4*>(R0 + tc::kmajor_offset(row, n0 + 8 * i, HID, 2)) = pack8(v + 8 * i);
+            }
+            atomicAdd(&F[F_DB1 + n0 + lane], column_sums(v));
+        }
+        publish();
+        if (tid == 0) {
+            for (uint32_t s = 0; s < 8; s++)  // dW2, outputs 0..127
+                tc::mma<false>(tmem, tc::smem_desc(r1 + 2 * GROUP * s, GROUP, 128),
+                               tc::smem_desc(r2 + 2 * GROUP * s, GROUP, 128), ID_DW2, s > 0);
+            commit();
+        }
+        pending = true;
+        auto add_dw2 = [&](uint32_t col0, int out0) {
+#pragma unroll 1
+            for (int c = 0; c < 4; c++) {
+                const int n0 = half * 128 + 32 * c;
+                float v[32];
+                tc::tmem_ld32(mine + col0 + n0, v);
+                float* p = g + P_W2 + (size_t)(out0 + row) * HID + n0;
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) red_add4(p + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
+            }
+        };
+        add_dw2(HID, 128);
+        if (!(ok = wait())) break;
+        publish();  // the second accumulator is read
+        if (tid == 0) {
+            for (uint32_t m = 0; m < 2; m++)
+                for (uint32_t s = 0; s < 8; s++)
+                    tc::mma<false>(tmem + HID + IN * m, tc::smem_desc(r0 + 16 * 128 * m + 2 * GROUP * s, GROUP, 128),
+                                   tc::smem_desc(xs + 2 * XGROUP * s, XGROUP, 128), ID_DW1, s > 0);
+            commit();
+        }
+        pending = true;
+        add_dw2(0, 0);
+        if (!(ok = wait())) break;
+        {
+            float v[16];  // column half h: units 128 h + row
+            tc::tmem_ld16(mine + HID + IN * half, v);
+            float* p = g + P_W1 + (size_t)(128 * half + row) * IN;
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) red_add4(p + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+        tc::tc_fence_before();
+        __syncthreads();
+        tc::tc_fence_after();
+    }
+    cp_async_wait0();
+    __syncthreads();
+    if (GRAD && ok && (int)blockIdx.x < ntiles) {
+        for (int e = tid; e < HID; e += NTHR) {
+            atomicAdd(g + P_B2 + e, F[F_DB2 + e]);
+            atomicAdd(g + P_B1 + e, F[F_DB1 + e]);
+        }
+        for (int e = tid; e < OUT * HID; e += NTHR) atomicAdd(g + P_W3 + e, F[F_DW3 + e]);
+        if (tid < OUT) atomicAdd(g + P_B3 + tid, F[F_DB3 + tid]);
     }
     if (!ok && tid == 0) {
-        if (issued > 0) tc::mbar_wait(bars + ((issued - 1) & 1), ((issued - 1) >> 1) & 1);  // drain, bounded
+        if (pending) tc::mbar_wait(bar, phase ^ 1);  // drain the commit that did not come in time, bounded
         atomicExch(err, 1);
     }
     tc::tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         tc::tc_fence_after();
-        tc::tmem_dealloc(tmem, P::TCOLS);
+        tc::tmem_dealloc(tmem, 512);
     }
 }
 
 __global__ void to_bf16(const float* __restrict__ x, bf16* __restrict__ y, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) y[i] = __float2bfloat16_rn(x[i]);
-}
-
-// The batch's inputs (B x IN, f32) as bf16, row-major and transposed (IN x ldt).
-__global__ void inputs_bf16(const float* __restrict__ x, bf16* __restrict__ xb, bf16* __restrict__ xt, int B, int ldt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * IN) return;
-    const bf16 v = __float2bfloat16_rn(x[i]);
-    xb[i] = v;
-    xt[(size_t)(i % IN) * ldt + i / IN] = v;
-}
-
-// W2 (FP32 master, [out][in]) as bf16 transposed, [in][out]: the B operand of dh1 = dh2 W2.
-__global__ void w2_transposed(const float* __restrict__ w2, bf16* __restrict__ w2t) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= HID * HID) return;
-    const int o = i / HID, in = i % HID;
-    w2t[(size_t)in * HID + o] = __float2bfloat16_rn(w2[i]);
-}
-
-// BCE with logits: dz = (sigmoid(z) - y) / (B * OUT); per-row losses for the host to average.
-__global__ void bce_loss(const float* __restrict__ z, const float* __restrict__ y, int B, float* __restrict__ dz,
-                         bf16* __restrict__ dzb, float* __restrict__ loss_rows) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    float l = 0.f;
-    for (int j = 0; j < OUT; j++) {
-        const float zz = z[b * OUT + j], yy = y[b * OUT + j];
-        const float p = 1.f / (1.f + expf(-zz));
-        l += fmaxf(zz, 0.f) - zz * yy + log1pf(expf(-fabsf(zz)));
-        const float g = (p - yy) / (float)(B * OUT);
-        dz[b * OUT + j] = g;
-        dzb[b * OUT + j] = __float2bfloat16_rn(g);
-    }
-    loss_rows[b] = l / OUT;
-}
-
-// Column sums of g [B x N] (bias gradients), FP32.
-__global__ void col_sum(const float* __restrict__ g, int B, int N, float* __restrict__ out) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.f;
-    for (int b = 0; b < B; b++) s += g[(size_t)b * N + n];
-    out[n] = s;
-}
-
-__global__ void sigmoid_k(const float* __restrict__ z, float* __restrict__ p, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = 1.f / (1.f + expf(-z[i]));
 }
 
 // Adam on the FP32 master weights, refreshing their BF16 copies.
@@ -319,17 +434,15 @@ using namespace lenia::mlp;
 
 struct LeniaMlp {
     int max_batch = 0;
-    int t = 0;
+    int t = 0, sms = 0;
     cudaStream_t stream = nullptr;
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // FP32 master, grads, Adam moments
     bf16* wb = nullptr;                                             // BF16 copy of the parameters
-    float *x = nullptr, *y = nullptr, *z = nullptr, *dz = nullptr, *dh = nullptr, *loss = nullptr, *p = nullptr;
-    bf16 *xb = nullptr, *h1 = nullptr, *h2 = nullptr, *dzb = nullptr, *dh2b = nullptr, *dh1b = nullptr;
-    // transposed copies (feature-major, batch contiguous, ldt apart): the K-major operands of the
-    // weight-gradient GEMMs, whose K is the batch; and W2 transposed for dh1 = dh2 W2
-    int ldt = 0;
-    bf16 *xt = nullptr, *h1t = nullptr, *dh2t = nullptr, *dh1t = nullptr, *w2t = nullptr;
-    int* err = nullptr;  // set by a tensor-core GEMM that gave up waiting on a barrier
+    float *x = nullptr, *y = nullptr, *loss = nullptr;  // a batch: inputs, labels, per-row losses
+    int* err = nullptr;  // set by a tile that gave up waiting on a barrier
+    // ranking: two halves of PREDICT_ROWS rows of inputs and probabilities, each on a stream of its own
+    cudaStream_t ps[2] = {};
+    float *px = nullptr, *pp = nullptr;
     std::vector<void*> allocs;
 };
 
@@ -349,61 +462,20 @@ int err(const char* msg) {
     return LENIA_ECUDA;
 }
 
-dim3 grid_for(int M, int N) { return dim3((N + 63) / 64, (M + 63) / 64); }
+// rows of inputs that lenia_mlp_predict has on the device at a time, in two halves: a copy of one half
+// overlaps the other's tiles
+constexpr int PREDICT_ROWS = 1 << 16;
 
-// One tensor-core GEMM launch (see gemm_tc): C [M x N] = A [M x K] B[N x K]^T.
-template <int N>
-void tc_gemm(LeniaMlp* n, const bf16* A, int lda, const bf16* B, int ldb, int M, int K, int ksplit, const float* bias,
-             int relu, const bf16* mask, float* Cf, bf16* Cb, bf16* CbT) {
-    static int configured = 0;
-    if (!configured) {
-        cudaFuncSetAttribute(gemm_tc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcGemm<N>::SMEM);
-        configured = 1;
-    }
-    const dim3 grid((M + 127) / 128, ksplit);
-    gemm_tc<N><<<grid, 128, TcGemm<N>::SMEM, n->stream>>>(A, lda, B, ldb, M, K, ksplit, bias, relu, mask, Cf, Cb, CbT,
-                                                          n->ldt, n->err);
+int tiles_grid(const LeniaMlp* n, int B) {
+    const int t = (B + TILE - 1) / TILE;
+    return t < n->sms ? t : n->sms;
 }
 
-// K-splits of a weight-gradient GEMM whose K is the batch: enough CTAs to spread the batch over SMs
-int ksplit_for(int B) {
-    const int chunks = (B + TCK - 1) / TCK;
-    return chunks < 32 ? chunks : 32;
-}
-
-// forward pass of `B` rows already in n->x; logits into n->z.  The 16 -> 256 and 256 -> 256 layers
-// run on the tensor cores; the 256 -> 3 layer on the CUDA cores.
-void forward(LeniaMlp* n, int B) {
-    cudaStream_t s = n->stream;
-    inputs_bf16<<<(B * IN + 255) / 256, 256, 0, s>>>(n->x, n->xb, n->xt, B, n->ldt);
-    tc_gemm<HID>(n, n->xb, IN, n->wb + P_W1, IN, B, IN, 1, n->w + P_B1, 1, nullptr, nullptr, n->h1, n->h1t);
-    tc_gemm<HID>(n, n->h1, HID, n->wb + P_W2, HID, B, HID, 1, n->w + P_B2, 1, nullptr, nullptr, n->h2, nullptr);
-    gemm_bf16<false, false><<<grid_for(B, OUT), 256, 0, s>>>(n->h2, n->wb + P_W3, B, OUT, HID, n->w + P_B3, 0, n->z,
-                                                              nullptr, nullptr);
-}
-
-// gradients of the mean BCE into n->g; per-row losses into n->loss
-void backward(LeniaMlp* n, int B) {
-    cudaStream_t s = n->stream;
-    bce_loss<<<(B + 127) / 128, 128, 0, s>>>(n->z, n->y, B, n->dz, n->dzb, n->loss);
-    // layer 3: dW3 = dz^T h2 [3 x 256], db3 = sum dz, dh2 = (dz W3) * (h2 > 0)
-    gemm_bf16<true, true><<<grid_for(OUT, HID), 256, 0, s>>>(n->dzb, n->h2, OUT, HID, B, nullptr, 0, n->g + P_W3,
-                                                             nullptr, nullptr);
-    col_sum<<<1, 32, 0, s>>>(n->dz, B, OUT, n->g + P_B3);
-    gemm_bf16<false, true><<<grid_for(B, HID), 256, 0, s>>>(n->dzb, n->wb + P_W3, B, HID, OUT, nullptr, 0, n->dh,
-                                                            n->dh2b, n->h2, n->dh2t, n->ldt);
-    // layer 2 (tensor cores): dW2 = dh2^T h1 (K = the batch, split over CTAs), db2 = sum dh2,
-    // dh1 = (dh2 W2) * (h1 > 0)
-    cudaMemsetAsync(n->g + P_W2, 0, (size_t)HID * HID * sizeof(float), s);
-    tc_gemm<HID>(n, n->dh2t, n->ldt, n->h1t, n->ldt, HID, B, ksplit_for(B), nullptr, 0, nullptr, n->g + P_W2, nullptr,
-                 nullptr);
-    col_sum<<<(HID + 127) / 128, 128, 0, s>>>(n->dh, B, HID, n->g + P_B2);
-    tc_gemm<HID>(n, n->dh2b, HID, n->w2t, HID, B, HID, 1, nullptr, 0, n->h1, n->dh, n->dh1b, n->dh1t);
-    // layer 1 (tensor cores): dW1 = dh1^T x, db1 = sum dh1
-    cudaMemsetAsync(n->g + P_W1, 0, (size_t)HID * IN * sizeof(float), s);
-    tc_gemm<IN>(n, n->dh1t, n->ldt, n->xt, n->ldt, HID, B, ksplit_for(B), nullptr, 0, nullptr, n->g + P_W1, nullptr,
-                nullptr);
-    col_sum<<<(HID + 127) / 128, 128, 0, s>>>(n->dh, B, HID, n->g + P_B1);
+// gradients of the mean BCE of the batch in n->x, n->y into n->g; per-row losses into n->loss
+void gradients(LeniaMlp* n, int B) {
+    cudaMemsetAsync(n->g, 0, (size_t)NPARAM * sizeof(float), n->stream);
+    mlp_tile<true><<<tiles_grid(n, B), NTHR, TILE_SMEM, n->stream>>>(n->x, n->y, B, n->w, n->wb, nullptr, n->g, n->loss,
+                                                                     n->err);
 }
 
 int check_err(LeniaMlp* n) {
@@ -411,7 +483,7 @@ int check_err(LeniaMlp* n) {
     if (cudaMemcpy(&h, n->err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return err("mlp: error flag read failed");
     if (h) {
         cudaMemset(n->err, 0, sizeof(int));
-        return err("mlp: a tensor-core GEMM gave up waiting on a barrier; results are invalid");
+        return err("mlp: a tile gave up waiting on a barrier; results are invalid");
     }
     return 0;
 }
@@ -444,16 +516,17 @@ LENIA_API int lenia_mlp_create(uint32_t seed, uint32_t max_batch, LeniaMlp** out
     LeniaMlp* n = new LeniaMlp();
     n->max_batch = (int)max_batch;
     const size_t B = max_batch;
-    bool ok = cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) == cudaSuccess && mal(n, &n->w, NPARAM) &&
+    int dev = 0;
+    bool ok = cudaGetDevice(&dev) == cudaSuccess &&
+              cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+              cudaFuncSetAttribute(mlp_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM) == cudaSuccess &&
+              cudaFuncSetAttribute(mlp_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&n->ps[0], cudaStreamNonBlocking) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&n->ps[1], cudaStreamNonBlocking) == cudaSuccess && mal(n, &n->w, NPARAM) &&
               mal(n, &n->g, NPARAM) && mal(n, &n->m, NPARAM) && mal(n, &n->v, NPARAM) && mal(n, &n->wb, NPARAM) &&
-              mal(n, &n->x, B * IN) && mal(n, &n->y, B * OUT) && mal(n, &n->z, B * OUT) && mal(n, &n->dz, B * OUT) &&
-              mal(n, &n->dh, B * HID) && mal(n, &n->loss, B) && mal(n, &n->p, B * OUT) && mal(n, &n->xb, B * IN) &&
-              mal(n, &n->h1, B * HID) && mal(n, &n->h2, B * HID) && mal(n, &n->dzb, B * OUT) &&
-              mal(n, &n->dh2b, B * HID) && mal(n, &n->dh1b, B * HID);
-    n->ldt = (int)((B + 15) / 16 * 16);
-    const size_t T = (size_t)n->ldt;
-    ok = ok && mal(n, &n->xt, T * IN) && mal(n, &n->h1t, T * HID) && mal(n, &n->dh2t, T * HID) &&
-         mal(n, &n->dh1t, T * HID) && mal(n, &n->w2t, (size_t)HID * HID) && mal(n, &n->err, 1);
+              mal(n, &n->x, B * IN) && mal(n, &n->y, B * OUT) && mal(n, &n->loss, B) && mal(n, &n->err, 1) &&
+              mal(n, &n->px, (size_t)PREDICT_ROWS * IN) && mal(n, &n->pp, (size_t)PREDICT_ROWS * OUT);
     if (!ok) {
         lenia_mlp_destroy(n);
         set_thread_error("mlp: device allocation failed");
@@ -494,9 +567,11 @@ LENIA_API int lenia_mlp_create(uint32_t seed, uint32_t max_batch, LeniaMlp** out
 
 LENIA_API int lenia_mlp_destroy(LeniaMlp* n) {
     if (!n) return 0;
-    if (n->stream) cudaStreamSynchronize(n->stream);
+    for (cudaStream_t s : {n->stream, n->ps[0], n->ps[1]})
+        if (s) cudaStreamSynchronize(s);
     for (void* p : n->allocs) cudaFree(p);
-    if (n->stream) cudaStreamDestroy(n->stream);
+    for (cudaStream_t s : {n->stream, n->ps[0], n->ps[1]})
+        if (s) cudaStreamDestroy(s);
     delete n;
     return 0;
 }
@@ -515,7 +590,6 @@ LENIA_API int lenia_mlp_set_params(LeniaMlp* n, const float* host, size_t count)
     if (cudaMemcpyAsync(n->w, host, NPARAM * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess)
         return err("mlp: upload failed");
     to_bf16<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->w, n->wb, NPARAM);
-    w2_transposed<<<(HID * HID + 255) / 256, 256, 0, n->stream>>>(n->w + P_W2, n->w2t);
     n->t = 0;
     return cudaStreamSynchronize(n->stream) == cudaSuccess ? 0 : err("mlp: set_params failed");
 }
@@ -538,8 +612,7 @@ LENIA_API int lenia_mlp_gradients(LeniaMlp* n, const float* x, const float* y, u
         return LENIA_EINVAL;
     }
     if (upload_batch(n, x, y, batch)) return err("mlp: upload failed");
-    forward(n, (int)batch);
-    backward(n, (int)batch);
+    gradients(n, (int)batch);
     if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
     cudaMemcpyAsync(grads, n->g, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream);
     const float l = mean_loss(n, batch);
@@ -554,13 +627,11 @@ LENIA_API int lenia_mlp_train_step(LeniaMlp* n, const float* x, const float* y, 
         return LENIA_EINVAL;
     }
     if (upload_batch(n, x, y, batch)) return err("mlp: upload failed");
-    forward(n, (int)batch);
-    backward(n, (int)batch);
+    gradients(n, (int)batch);
     n->t++;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)n->t), c2 = 1.f - std::pow(b2, (float)n->t);
     adam<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->w, n->g, n->m, n->v, n->wb, NPARAM, lr, b1, b2, 1e-8f, c1, c2);
-    w2_transposed<<<(HID * HID + 255) / 256, 256, 0, n->stream>>>(n->w + P_W2, n->w2t);
     if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
     const float l = mean_loss(n, batch);
     if (loss) *loss = l;
@@ -572,14 +643,30 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
         set_thread_error("mlp: NULL argument");
         return LENIA_EINVAL;
     }
-    for (uint32_t off = 0; off < count; off += (uint32_t)n->max_batch) {
-        const uint32_t B = count - off < (uint32_t)n->max_batch ? count - off : (uint32_t)n->max_batch;
-        if (upload_batch(n, x + (size_t)off * IN, nullptr, B)) return err("mlp: upload failed");
-        forward(n, (int)B);
-        sigmoid_k<<<(B * OUT + 255) / 256, 256, 0, n->stream>>>(n->z, n->p, (int)(B * OUT));
-        cudaMemcpyAsync(probs + (size_t)off * OUT, n->p, (size_t)B * OUT * 4, cudaMemcpyDeviceToHost, n->stream);
+    // chunk c runs on stream c % 2; its results leave after the next chunk has been queued, so that a copy
+    // to or from pageable memory, which blocks this thread, overlaps a chunk's tiles
+    constexpr uint32_t HALF = PREDICT_ROWS / 2;
+    const uint32_t chunks = (uint32_t)(((uint64_t)count + HALF - 1) / HALF);
+    auto rows = [&](uint32_t c) { return c + 1 < chunks ? HALF : count - c * HALF; };
+    for (uint32_t c = 0; c <= chunks; c++) {
+        if (c < chunks) {
+            const int h = c & 1;
+            float *px = n->px + (size_t)h * HALF * IN, *pp = n->pp + (size_t)h * HALF * OUT;
+            if (cudaMemcpyAsync(px, x + (size_t)c * HALF * IN, (size_t)rows(c) * IN * 4, cudaMemcpyHostToDevice, n->ps[h]) !=
+                cudaSuccess)
+                return err("mlp: upload failed");
+            mlp_tile<false><<<tiles_grid(n, (int)rows(c)), NTHR, TILE_SMEM, n->ps[h]>>>(px, nullptr, (int)rows(c), n->w, n->wb,
+                                                                                       pp, nullptr, nullptr, n->err);
+        }
+        if (c > 0) {
+            const uint32_t d = c - 1;
+            if (cudaMemcpyAsync(probs + (size_t)d * HALF * OUT, n->pp + (size_t)(d & 1) * HALF * OUT, (size_t)rows(d) * OUT * 4,
+                                cudaMemcpyDeviceToHost, n->ps[d & 1]) != cudaSuccess)
+                return err("mlp: download failed");
+        }
     }
-    if (cudaStreamSynchronize(n->stream) != cudaSuccess) return err("mlp: predict failed");
+    if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess || cudaStreamSynchronize(n->ps[1]) != cudaSuccess)
+        return err("mlp: predict failed");
     return check_err(n);
 }
 

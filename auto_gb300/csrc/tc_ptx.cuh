@@ -45,12 +45,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
            ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
 
-// Instruction descriptor, dense, D = f32, B K-major: kind::f16 with bf16 operands (format 1) or
-// kind::tf32 (format 2); A K-major, or MN-major with a_mn (bit 15); N >> 3 in bits 17-22, M >> 4 in
-// bits 24-28.
-__host__ __device__ constexpr uint32_t instr_desc(int fmt, int M, int N, bool a_mn = false) {
+// Instruction descriptor, dense, D = f32: kind::f16 with bf16 operands (format 1) or
+// kind::tf32 (format 2); A and B K-major, or MN-major with a_mn (bit 15) and b_mn (bit 16); N >> 3 in
+// bits 17-22, M >> 4 in bits 24-28.
+__host__ __device__ constexpr uint32_t instr_desc(int fmt, int M, int N, bool a_mn = false, bool b_mn = false) {
     return (1u << 4) | ((uint32_t)fmt << 7) | ((uint32_t)fmt << 10) | ((a_mn ? 1u : 0u) << 15) |
-           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+           ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // ----------------------------------------------------------------- mbarriers
