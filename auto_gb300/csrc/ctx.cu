@@ -784,14 +784,16 @@ int setup_fused(LeniaCtx* ctx) {
                         planes);
         cl.general = general;
         cl.planes = planes;
-        // Default launch variant: the 64-register form (more resident CTAs) unless it spills more
-        // than 128 bytes a thread and the 128-register form spills less than half as much.  Columns
-        // of 4096 and more take the paired build (measured 8% faster at 4096 x 4096; at 128 to 1024
-        // the scalar builds were faster); the autotuner times all three.
-        auto pick = [](int v0, int v1) { return (v0 > 128 && v1 >= 0 && v1 < v0 / 2) ? 1 : 0; };
-        cl.var_col = cl.H >= 4096 ? 2 : pick(fp32_local_bytes(0, cl.H, 0), fp32_local_bytes(0, cl.H, 1));
-        const int g2 = general ? 2 : 0;
-        cl.var_row = pick(fp32_local_bytes(1, cl.W, g2), fp32_local_bytes(1, cl.W, 1 | g2));
+        // Default launch variants (per generation; the autotuner times the others).
+        // Columns: the 64-register scalar build, but the 128-register one where a thread holds 24 or 32
+        // elements (55 worlds of 1024 x 1024 253 -> 233 us and one 13.5 -> 10.7, 43 of 768 x 768 115 -> 112; equal at
+        // 384) and at 192 (63 worlds 16.1 -> 15.0); at 4096 and 6144 the paired build (one 4096 x 4096 world 108.5 -> 107.2,
+        // but 8192 x 8192 590 against 564).
+        cl.var_col = cl.H == 4096 || cl.H == 6144 ? 2 : (col_wide(cl.H) && cl.H != 384) || cl.H == 192 ? 1 : 0;
+        // Rows: at 64 registers (768 x 768, 43 worlds: 121 us against 139) unless the launch leaves the occupancy that
+        // buys unused -- at most three items for two SMs -- (one 384 x 384 world 10.5 -> 7.0 us, 768 x 768 11.3 -> 11.0,
+        // 1536 x 768 15.5 -> 14.7) or the general step, which spills there (SmoothLife 2048 x 2048 56 -> 50 us, 512 x 512 13.4 -> 12.6).
+        cl.var_row = general || 2 * row.size() <= 3 * (size_t)ctx->sms ? 1 : 0;
         cl.ncol = (int)col.size();
         cl.nrow = (int)row.size();
         cl.ntcg = (int)tcg.size();

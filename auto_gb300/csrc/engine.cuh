@@ -96,8 +96,10 @@ size_t row_smem_bytes(int W, int acc_planes);
 constexpr int COL_VARIANTS = 4;
 // whether the scalar column pass of height H has a radix-16 build beside its radix-32 one (variant 3)
 bool col_has_r16_variant(int H);
+// whether the scalar column pass of height H holds 24 or 32 elements a thread (radix-32 plans, the
+// larger two-stage transforms)
+bool col_wide(int H);
 int row_item_rows(int W, int general);  // rows per row-pass item: 4, or 2 (general step, W >= 2048)
-int fp32_local_bytes(int row, int n, int variant);  // spill/stack bytes per thread of a pass instantiation
 int max_smem_optin();
 
 // Cluster-resident step (resident.cu): one launch advances every world of a square size class of

@@ -240,6 +240,28 @@ template <int R1, int R2, bool INV, class T> FFT_HD void dft_split(T* v) {
     }
 }
 
+// R = R1 * R2, coprime (Good-Thomas): with n = (R2 n1 + R1 n2) mod R the DFT is an R1 x R2 two-dimensional
+// one without twiddles, and output k sits at (k mod R1, k mod R2).
+template <int R1, int R2, bool INV, class T> FFT_HD void dft_coprime(T* v) {
+    constexpr int R = R1 * R2;
+    T u[R];
+#pragma unroll
+    for (int n2 = 0; n2 < R2; n2++) {
+        T a[R1];
+#pragma unroll
+        for (int n1 = 0; n1 < R1; n1++) a[n1] = v[(R2 * n1 + R1 * n2) % R];
+        Dft<R1, INV>::run(a);
+#pragma unroll
+        for (int k1 = 0; k1 < R1; k1++) u[k1 * R2 + n2] = a[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < R1; k1++) Dft<R2, INV>::run(u + k1 * R2);
+#pragma unroll
+    for (int k = 0; k < R; k++) v[k] = u[(k % R1) * R2 + k % R2];
+}
+
+template <bool INV> struct Dft<12, INV> { template <class T> FFT_HD static void run(T* v) { dft_coprime<4, 3, INV>(v); } };
+template <bool INV> struct Dft<24, INV> { template <class T> FFT_HD static void run(T* v) { dft_coprime<8, 3, INV>(v); } };
 template <bool INV> struct Dft<8, INV> { template <class T> FFT_HD static void run(T* v) { dft_split<4, 2, INV>(v); } };
 template <bool INV> struct Dft<16, INV> { template <class T> FFT_HD static void run(T* v) { dft_split<4, 4, INV>(v); } };
 template <bool INV> struct Dft<32, INV> { template <class T> FFT_HD static void run(T* v) { dft_split<8, 4, INV>(v); } };
@@ -342,7 +364,7 @@ FFT_HD int pad(int i) { return i + (i >> 4); }
 // 4 interleaved columns fall into different banks
 FFT_CHD constexpr int seq_stride(int n) { return n + n / 16 + 4; }
 
-// Twiddles w^m, m = 1..R-1, of one butterfly from w, (R >= 8) w^4 and (R >= 32) w^16; the other
+// Twiddles w^m, m = 1..R-1, of one butterfly from w, (R >= 8) w^4 and (R >= 24) w^16; the other
 // powers are products of at most four factors, so each stays within a few float ulps of the exactly
 // rounded value (checked against numpy by the host test).
 template <int R, class W>
@@ -356,19 +378,23 @@ FFT_HD void twiddle_powers(W w1, W w4, W w16, W* w) {
         w[6] = cmul(w[4], w[2]);
         w[7] = cmul(w[4], w[3]);
     }
-    if (R >= 16) {
+    if (R >= 12) {
         w[8] = cmul(w[4], w[4]);
 #pragma unroll
         for (int m = 9; m < 12; m++) w[m] = cmul(w[8], w[m - 8]);
+    }
+    if (R >= 16) {
         w[12] = cmul(w[8], w[4]);
 #pragma unroll
         for (int m = 13; m < 16; m++) w[m] = cmul(w[12], w[m - 12]);
     }
-    if (R >= 32) {
+    if (R >= 24) {
         w[16] = w16;
-        w[24] = cmul(w[16], w[8]);
 #pragma unroll
         for (int m = 17; m < 24; m++) w[m] = cmul(w[16], w[m - 16]);
+    }
+    if (R >= 32) {
+        w[24] = cmul(w[16], w[8]);
 #pragma unroll
         for (int m = 25; m < 32; m++) w[m] = cmul(w[24], w[m - 24]);
     }
@@ -419,6 +445,65 @@ FFT_HD void stage_store(T* seq, int j, const T* v) {
 #pragma unroll
         for (int m = 0; m < R; m++) seq[pad(base + m * L)] = v[m];
     }
+}
+
+// ------------------------------------------------------------------ two-stage transforms
+// N = RA * RB as two stages, for the sides whose single plan with equal outer radices needs three or
+// four (192 = 8.3.8, 384 = 8.3.2.8, and in the column pass, maxr = 32, 768 = 16.3.16).  Of two chained
+// transforms the first runs RA then RB and the second RB then RA, so the chained stages in the middle still
+// share a radix (RB, the smaller: the row pass holds its state values beside it).
+// Between its stages a transform is an RB x RA (or RA x RB) transposition: butterfly j of the first stage leaves
+// its R results as row j of a matrix with R + 1 columns, and butterfly j of the second reads column
+// j.  Every address is one base and compile-time offsets, and the odd row length keeps both sides
+// free of bank conflicts.
+// A side is here where the fewer, larger stages win: per generation, 60 worlds of 384 x 384 55 -> 39 us (one
+// world 6.9 -> 7.0), 63 of 192 x 192 17.6 -> 15.0, 43 of 768 x 768 120 -> 112 with the column pass alone
+// (one world 9.6 -> 9.8); with the row pass as well 110, but one world 10.4 and SmoothLife at 768 x 768 15.1 ->
+// 20.6: 168 registers a thread.  512 as 32.16 was slower everywhere (41 worlds 44.5 -> 46.6).
+struct TwoStage {
+    int ra, rb;  // 0: no two-stage transform
+};
+FFT_CHD constexpr TwoStage two_stage(int n, int maxr = 16) {
+    return n == 192 ? TwoStage{12, 16} : n == 384 ? TwoStage{24, 16}
+         : maxr == 32 && n == 768 ? TwoStage{32, 24} : TwoStage{0, 0};
+}
+FFT_CHD constexpr bool is_two_stage(int n, int maxr = 16) { return two_stage(n, maxr).ra != 0; }
+// Twiddle table of a two-stage transform: w^k, w^4k and w^16k, w = exp(-2 pi i / N), k below the larger radix
+// (either order's second stage, of radix R, needs w^(k m) for k < N/R and m < R).
+FFT_CHD constexpr int two_tw_len(int n) {
+    return two_stage(n, 32).ra > two_stage(n, 32).rb ? two_stage(n, 32).ra : two_stage(n, 32).rb;
+}
+FFT_CHD constexpr int two_tw_size(int n) { return 3 * two_tw_len(n); }
+template <int N, class W>
+FFT_HD void fill_two_twiddles(W* stw, const float2* tw, int tid, int nth) {
+    constexpr int M = two_tw_len(N), step = TWN / N;
+    for (int e = tid; e < 3 * M; e += nth) {
+        const int k = e % M, p = e / M;  // powers 1, 4, 16
+        set_twiddle(stw[e], tw[((k << (2 * p)) * step) % TWN]);
+    }
+}
+// First stage's results, row j of the exchange matrix; second stage's operands (column j, with its twiddles).
+template <int R, class T>
+FFT_HD void two_store(T* x, int j, const T* v) {
+    T* p = x + j * (R + 1);
+#pragma unroll
+    for (int m = 0; m < R; m++) p[m] = v[m];
+}
+template <int N, int R, bool INV, class T, class W>
+FFT_HD void two_load(const T* x, int j, T* v, const W* stw) {
+    constexpr int M = two_tw_len(N), L = N / R;
+    const T* p = x + j;
+#pragma unroll
+    for (int m = 0; m < R; m++) v[m] = p[m * (L + 1)];
+    W w[R];
+    twiddle_powers<R>(stw[j], stw[M + j], stw[2 * M + j], w);
+#pragma unroll
+    for (int m = 1; m < R; m++) v[m] = INV ? cmulc(v[m], w[m]) : cmul(v[m], w[m]);
+    Dft<R, INV>::run(v);
+}
+// values of one sequence's exchange matrix, either way round
+FFT_CHD constexpr int two_exchange(int n) {
+    return n + two_tw_len(n);
 }
 
 }  // namespace lfft

@@ -21,8 +21,8 @@
 //     is assumed, so cudaDeviceReset, or a non-primary driver-API context made current, is not
 //     supported between calls;
 //   * the kernel spectrum arrives with lenia_kernel_spectrum's row stride H/2+1, not the 16-byte
-//     aligned stride the engine's own contexts use, so every column item takes the column pass's
-//     unchained form (transform, multiply, transform in three sweeps) instead of the chained one.
+//     aligned stride the engine's own contexts use, so the column items fetch it with plain loads
+//     instead of asynchronous 16-byte copies (copy_khat).
 #include <cuda_runtime.h>
 
 #include <cmath>

@@ -64,9 +64,9 @@ __global__ void __launch_bounds__(NT, MINB)
     float2* X = reinterpret_cast<float2*>(smem_raw);
     float2* stw = X + persist_seq_floats2<N>();  // after the column pass's tile sequences and the row pass's packed rows
     // the row items' stage tables, then the column items' (their plans may differ: CMR)
-    float2* stwc = stw + tw_table_size(N) + 1;
-    fill_stage_twiddles<N>(stw, tw, threadIdx.x, NT);
-    fill_stage_twiddles<N, float2, 0, CMR>(stwc, tw, threadIdx.x, NT);
+    float2* stwc = stw + tables_size<N>() + 1;
+    fill_tables<N>(stw, tw, NT);
+    fill_tables<N, CMR>(stwc, tw, NT);
     int* cols_done = ctl + PST_COUNTERS;
     int* rows_done = cols_done + nw;
     const long long per_gen = (long long)nw * (nc + nr), total = per_gen * gens;

@@ -95,7 +95,7 @@ struct Res {
     static constexpr int G = N / 32;                 // CTAs per cluster (one world)
     static constexpr int ROWS = 32;                  // rows a CTA owns
     static constexpr int COLS = 16;                  // spectrum columns a CTA owns
-    static constexpr int R0 = plan_radix(N, 0), NB = N / R0;
+    static constexpr int R0 = chain_radix<N>(), NB = N / R0;
     static constexpr int S = S_, MINB = MINB_;
     static constexpr int NT = S * NB;                // one first-stage butterfly per thread
     static constexpr int GATHER = S * (N / 2) / NT;  // remote elements a thread gathers (and scatters) per batch
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(Res<N, S_, MINB_>::NT, MINB_)
     const int kx0 = COLS * q, r0q = P::ROWS * q;
     const uint32_t cs_addr = tc::smem_u32(CS);
 
-    fill_stage_twiddles<N>(stw, tw, threadIdx.x, NT);
+    fill_tables<N>(stw, tw, NT);
     if (threadIdx.x == 0) {
         tc::mbar_init(bar, P::G);
         tc::fence_barrier_init();
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(Res<N, S_, MINB_>::NT, MINB_)
         if (!cs.dead) {
             if (q == 0) {
                 // columns 0 and 1: column 0 packs the real DC and Nyquist columns, which pair ky with
-                // N - ky in the khat multiply; they take the two-pass step's unchained form in WK
+                // N - ky in the khat multiply; they run whole transforms in WK
                 for (int e = threadIdx.x; e < TC * N; e += NT) {
                     const int c = e / N, y = e - c * N;
                     WK[c * SEQ + pad(y)] = CS[c * SEQ + pad(y)];
@@ -203,10 +203,10 @@ __global__ void __launch_bounds__(Res<N, S_, MINB_>::NT, MINB_)
                 });
             }
             if (q == 0) {
-                fft_seqs<N, TC, NT, false>(WK, stw);
-                multiply_khat<N, NT>(WK, WK, wd.khat, wd.HQ, N, 0);
+                fft_seqs<N, TC, NT, false, false>(WK, stw);
+                multiply_khat<N, NT>(WK, wd.khat, wd.HQ, N);
                 __syncthreads();
-                fft_seqs<N, TC, NT, true>(WK, stw);
+                fft_seqs<N, TC, NT, true, true>(WK, stw);
                 for (int e = threadIdx.x; e < TC * N; e += NT) {
                     const int c = e / N, y = e - c * N;
                     CS[c * SEQ + pad(y)] = WK[c * SEQ + pad(y)];

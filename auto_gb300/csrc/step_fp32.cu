@@ -15,11 +15,10 @@ static size_t col_khat_bytes_of(int H) {
 // the largest of the scalar builds' (radix-32 and radix-16 plans) and the paired build's (same
 // sequence bytes; the paired stage tables hold each twiddle twice)
 size_t col_smem_bytes(int H) {
-    const int t32 = lfft::tw_table_size(H, CMR), t16 = lfft::tw_table_size(H);
+    const int t32 = lfft::is_two_stage(H, CMR) ? lfft::two_tw_size(H) : lfft::tw_table_size(H, CMR), t16 = lfft::tw_table_size(H);
     const size_t scalar_tables = ((t32 > t16 ? t32 : t16) + 1) * sizeof(float2);
     const size_t paired_tables = (lfft::tw_table_size(H, PMR) + 1) * sizeof(lfft::tw2);
-    const int stride = col_stride(H) > lfft::seq_stride(H) ? col_stride(H) : lfft::seq_stride(H);
-    return (size_t)TC * stride * sizeof(float2) + (scalar_tables > paired_tables ? scalar_tables : paired_tables) +
+    return (size_t)TC * col_stride(H) * sizeof(float2) + (scalar_tables > paired_tables ? scalar_tables : paired_tables) +
            col_khat_bytes_of(H);
 }
 size_t row_smem_bytes(int W, int acc_planes) {
@@ -33,6 +32,8 @@ size_t row_smem_bytes(int W, int acc_planes) {
 }
 
 int row_item_rows(int W, int general) { return 2 * row_seqs(W, general != 0); }
+
+bool col_wide(int H) { return lfft::plan_radix(H, 0, CMR) == 32 || lfft::two_stage(H, CMR).ra >= 24; }
 
 bool col_has_r16_variant(int H) { return lfft::plan_radix(H, 0, CMR) == 32; }
 
@@ -56,16 +57,6 @@ bool launch_row_fp32(int W, int variant, int mode, int general, const DevWorld* 
                launch_row_group_large_general(W, variant, mode, general, acc_planes, worlds, items, nitems, tw, s);
     return launch_row_group_small_simple(W, variant, mode, general, acc_planes, worlds, items, nitems, tw, s) ||
            launch_row_group_large_simple(W, variant, mode, general, acc_planes, worlds, items, nitems, tw, s);
-}
-
-int fp32_local_bytes(int row, int n, int variant) {
-    if (!row) {
-        const int a = col_local_bytes_small(n, variant);
-        return a >= 0 ? a : col_local_bytes_large(n, variant);
-    }
-    // row: variant bit 1 asks for the general build
-    const int a = (variant & 2) ? row_local_bytes_small_general(n, variant) : row_local_bytes_small_simple(n, variant);
-    return a >= 0 ? a : ((variant & 2) ? row_local_bytes_large_general(n, variant) : row_local_bytes_large_simple(n, variant));
 }
 
 }  // namespace lenia

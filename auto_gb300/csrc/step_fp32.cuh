@@ -95,41 +95,119 @@ __device__ __forceinline__ void fft_stages(T* buf, const W* stw) {
     }
 }
 
-template <int N, int S, int NT, bool INV, int MR = 16, class T, class W>
-__device__ __forceinline__ void fft_seqs(T* buf, const W* stw) {
-    fft_stages<N, S, NT, INV, 0, plan_len(N, MR), MR>(buf, stw);
-}
-
-// Two transforms back to back (A, then B) with work on the values in between.  When the plan's
-// first and last radix are equal, the last stage of A leaves butterfly j holding the elements
-// j + m*N/R (m < R) in natural order -- exactly the inputs of butterfly j of B's first stage.  So
-// `mid(s, j, v)` runs on those registers (sequence s, elements j + m*N/R) and B's first stage
-// follows without a round trip through shared memory: two barriers and one shared-memory
-// read/write sweep fewer than A, mid-pass, B.  `pre(s, j)` runs just before the last stage of A.
+// ------------------------------------------------------------------ chained transforms
+// Two transforms back to back (A, then B) with work on the values in between.  The last stage of A and
+// the first of B share a radix R: A's leaves butterfly j holding the elements j + m*N/R (m < R) in
+// natural order -- exactly the inputs of butterfly j of B's first stage.  So the work runs on those
+// registers and B's first stage follows without a round trip through shared memory: two barriers and one
+// shared-memory read/write sweep fewer than A, mid-pass, B.
+// Scalar transforms of the sides fft_core.cuh's two_stage lists run A as RA, RB and B as RB, RA; the others run a
+// plan whose first and last radix are equal, both ways.  The pieces, for either kind (sequences in
+// shared memory in padded natural order before A and after B, stride seq_stride(N)):
+//   chain_radix   R
+//   fft_head      A's stages before its last one; ends with a barrier
+//   chain_load    butterfly j of A's last stage
+//   chain_store   the results of butterfly j of B's first stage (after a barrier, and before one)
+//   fft_tail      B's other stages; ends with a barrier
 template <int N, int MR = 16>
 FFT_CHD constexpr bool fusable() {
-    return plan_len(N, MR) >= 2 && plan_radix(N, 0, MR) == plan_radix(N, plan_len(N, MR) - 1, MR);
+    return is_two_stage(N, MR) || (plan_len(N, MR) >= 2 && plan_radix(N, 0, MR) == plan_radix(N, plan_len(N, MR) - 1, MR));
+}
+template <int N, int MR = 16>
+FFT_CHD constexpr int chain_radix() { return is_two_stage(N, MR) ? two_stage(N, MR).rb : plan_radix(N, 0, MR); }
+// Twiddle tables of a scalar transform: two-stage or per stage of the plan.
+template <int N, int MR = 16>
+FFT_CHD constexpr int tables_size() { return is_two_stage(N, MR) ? two_tw_size(N) : tw_table_size(N, MR); }
+template <int N, int MR = 16>
+__device__ __forceinline__ void fill_tables(float2* stw, const float2* tw, int nth) {
+    if constexpr (is_two_stage(N, MR)) fill_two_twiddles<N>(stw, tw, threadIdx.x, nth);
+    else fill_stage_twiddles<N, float2, 0, MR>(stw, tw, threadIdx.x, nth);
+}
+
+// One stage of S two-stage sequences, of radix R: the first of a transform (natural order in, exchange matrix out) or its
+// second (exchange matrix in, natural order out).
+template <int N, int R, int S, int NT, bool INV, bool SECOND>
+__device__ __forceinline__ void two_stage_pass(float2* buf, const float2* stw) {
+    constexpr int NB = N / R, TOT = NB * S, PER = (TOT + NT - 1) / NT, SEQ = seq_stride(N);
+    static_assert(two_exchange(N) <= SEQ, "the exchange matrix takes the sequence's place");
+    float2 v[PER][R];
+#pragma unroll
+    for (int p = 0; p < PER; p++) {
+        const int b = threadIdx.x + p * NT;
+        if ((TOT % NT) == 0 || b < TOT) {
+            const int s = b / NB, j = b - s * NB;
+            if constexpr (SECOND) two_load<N, R, INV>(buf + s * SEQ, j, v[p], stw);
+            else stage_load<N, R, 1, INV>(buf + s * SEQ, j, v[p], stw);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < PER; p++) {
+        const int b = threadIdx.x + p * NT;
+        if ((TOT % NT) == 0 || b < TOT) {
+            const int s = b / NB, j = b - s * NB;
+            if constexpr (SECOND) stage_store<N, R, NB>(buf + s * SEQ, j, v[p]);
+            else two_store<R>(buf + s * SEQ, j, v[p]);
+        }
+    }
+    __syncthreads();
+}
+
+// Whole transforms in place.  SWAP: the order of B (RB, RA).
+template <int N, int S, int NT, bool INV, bool SWAP, int MR = 16, class T, class W>
+__device__ __forceinline__ void fft_seqs(T* buf, const W* stw) {
+    if constexpr (is_two_stage(N, MR) && sizeof(T) == sizeof(float2)) {
+        constexpr int R1 = SWAP ? two_stage(N, MR).rb : two_stage(N, MR).ra, R2 = N / R1;
+        two_stage_pass<N, R1, S, NT, INV, false>(buf, stw);
+        two_stage_pass<N, R2, S, NT, INV, true>(buf, stw);
+    } else {
+        fft_stages<N, S, NT, INV, 0, plan_len(N, MR), MR>(buf, stw);
+    }
+}
+
+template <int N, int S, int NT, bool INV, int MR = 16>
+__device__ __forceinline__ void fft_head(float2* buf, const float2* stw) {
+    if constexpr (is_two_stage(N, MR)) two_stage_pass<N, two_stage(N, MR).ra, S, NT, INV, false>(buf, stw);
+    else fft_stages<N, S, NT, INV, 0, plan_len(N, MR) - 1, MR>(buf, stw);
+}
+template <int N, bool INV, int MR = 16>
+__device__ __forceinline__ void chain_load(const float2* seq, int j, float2* v, const float2* stw) {
+    constexpr int LAST = plan_len(N, MR) - 1, R = chain_radix<N, MR>();
+    if constexpr (is_two_stage(N, MR)) two_load<N, R, INV>(seq, j, v, stw);
+    else stage_load<N, R, N / R, INV>(seq, j, v, stw + stage_tw_offset(N, LAST, MR));
+}
+template <int N, int MR = 16>
+__device__ __forceinline__ void chain_store(float2* seq, int j, const float2* v) {
+    constexpr int R = chain_radix<N, MR>();
+    if constexpr (is_two_stage(N, MR)) two_store<R>(seq, j, v);
+    else stage_store<N, R, 1>(seq, j, v);
+}
+template <int N, int S, int NT, bool INV, int MR = 16>
+__device__ __forceinline__ void fft_tail(float2* buf, const float2* stw) {
+    if constexpr (is_two_stage(N, MR)) two_stage_pass<N, two_stage(N, MR).ra, S, NT, INV, true>(buf, stw);
+    else fft_stages<N, S, NT, INV, 1, plan_len(N, MR), MR>(buf, stw);
 }
 
 struct NoPre {
     __device__ void operator()(int, int) const {}
 };
 
-template <int N, int S, int NT, bool INV_A, bool INV_B, int MR = 16, class T, class W, class Mid, class Pre = NoPre>
-__device__ __forceinline__ void fft_fused(T* buf, const W* stw, Mid mid, Pre pre = Pre()) {
-    constexpr int LAST = plan_len(N, MR) - 1;
-    constexpr int R = plan_radix(N, LAST, MR), L = plan_L(N, LAST, MR), NB = N / R;
-    static_assert(L == NB && plan_radix(N, 0, MR) == R, "fusable plans only");
+// A, mid(s, j, v) on the registers between (sequence s, elements j + m*N/R), B.  `pre(s, j)` runs just before
+// the last stage of A.
+template <int N, int S, int NT, bool INV_A, bool INV_B, int MR = 16, class Mid, class Pre = NoPre>
+__device__ __forceinline__ void fft_fused(float2* buf, const float2* stw, Mid mid, Pre pre = Pre()) {
+    static_assert(fusable<N, MR>(), "fusable plans only");
+    constexpr int R = chain_radix<N, MR>(), NB = N / R;
     constexpr int TOT = NB * S, PER = (TOT + NT - 1) / NT, SEQ = seq_stride(N);
-    fft_stages<N, S, NT, INV_A, 0, LAST, MR>(buf, stw);
-    T v[PER][R];
+    fft_head<N, S, NT, INV_A, MR>(buf, stw);
+    float2 v[PER][R];
 #pragma unroll
     for (int p = 0; p < PER; p++) {
         const int b = threadIdx.x + p * NT;
         if ((TOT % NT) == 0 || b < TOT) {
             const int s = b / NB, j = b - s * NB;
             pre(s, j);  // global loads that mid needs, issued before the last stage of A
-            stage_load<N, R, L, INV_A>(buf + s * SEQ, j, v[p], stw + stage_tw_offset(N, LAST, MR));
+            chain_load<N, INV_A, MR>(buf + s * SEQ, j, v[p], stw);
             mid(s, j, v[p]);
             Dft<R, INV_B>::run(v[p]);  // B's first stage: L = 1, no twiddle
         }
@@ -138,15 +216,15 @@ __device__ __forceinline__ void fft_fused(T* buf, const W* stw, Mid mid, Pre pre
 #pragma unroll
     for (int p = 0; p < PER; p++) {
         const int b = threadIdx.x + p * NT;
-        if ((TOT % NT) == 0 || b < TOT) stage_store<N, R, 1>(buf + (b / NB) * SEQ, b % NB, v[p]);
+        if ((TOT % NT) == 0 || b < TOT) chain_store<N, MR>(buf + (b / NB) * SEQ, b % NB, v[p]);
     }
     __syncthreads();
-    fft_stages<N, S, NT, INV_B, 1, plan_len(N, MR), MR>(buf, stw);
+    fft_tail<N, S, NT, INV_B, MR>(buf, stw);
 }
 
-// Shared memory of a pass: the sequences, then (float2-aligned) the stage twiddle tables.
+// Shared memory of a pass: the sequences, then (float2-aligned) the twiddle tables.
 template <int N, int MR = 16>
-constexpr size_t stage_table_bytes() { return (size_t)(tw_table_size(N, MR) + 1) * sizeof(float2); }
+constexpr size_t stage_table_bytes() { return (size_t)(tables_size<N, MR>() + 1) * sizeof(float2); }
 
 // The scalar column pass's radix cap: radix-32 plans where they save a stage (1024 = 32.32 against
 // 16.4.16: one shared-memory round trip fewer per transform; 3072, 8192), the radix-16 plan elsewhere.
@@ -158,10 +236,10 @@ constexpr int CMR = 32;
 template <int H>
 FFT_CHD constexpr int khat_cols_stride() { return (H / 2 + 1 + 3) / 4 * 4; }
 template <int H>
-constexpr size_t col_khat_bytes() { return fusable<H, CMR>() ? (size_t)TC * khat_cols_stride<H>() * sizeof(float) : 0; }
+constexpr size_t col_khat_bytes() { return (size_t)TC * khat_cols_stride<H>() * sizeof(float); }
 template <int H, int MR = CMR>
 __device__ __forceinline__ float* col_khat_smem(float2* stw) {
-    constexpr int TWS = tw_table_size(H, MR);
+    constexpr int TWS = tables_size<H, MR>();
     return reinterpret_cast<float*>(((uintptr_t)(stw + TWS) + 15) & ~(uintptr_t)15);
 }
 
@@ -236,14 +314,16 @@ __device__ __forceinline__ float mnca_update(float s, float c0, float c1) {
 // sequences ran its radix-3 stage in six rounds, the last a third full, and needed 128 registers a
 // thread; with 256 it fits 64, and the batched workload's 768 x 768 row pass went from 104 to 89 us a
 // generation (the step from 1.87e11 to 1.93e11 cell-updates/s).
+// Two-stage sides: one butterfly of either stage.
 FFT_CHD constexpr int seq_threads(int N, int S) {
+    if (is_two_stage(N)) return S * two_tw_len(N);
     return N % 3 == 0 && S * N / 12 > S * N / plan_radix(N, 0) ? S * N / 12 : S * N / plan_radix(N, 0);
 }
 FFT_CHD constexpr int row_seqs(int W, bool gen) { return gen ? (W >= 2048 ? 1 : (W <= 1024 ? 4 : 2)) : (W <= 1024 ? 4 : 2); }
 template <int W, bool GEN>
 constexpr int row_nt() {
     constexpr int n = seq_threads(W, row_seqs(W, GEN));
-    return n < 64 ? 64 : (n > 1024 ? 1024 : n);
+    return n < 32 ? 32 : (n > 1024 ? 1024 : n);
 }
 // variant 0: at most 1024 threads' worth of registers per SM (64 a thread at 512 threads);
 // variant 1: at most 128 a thread
@@ -256,7 +336,7 @@ constexpr int row_minb() {
 // the general path.
 template <int W>
 __device__ __forceinline__ float* row_extra_smem(float2* stw) {
-    constexpr int TWS = tw_table_size(W);
+    constexpr int TWS = tables_size<W>();
     return reinterpret_cast<float*>(((uintptr_t)(stw + TWS) + 15) & ~(uintptr_t)15);
 }
 
@@ -364,7 +444,7 @@ __device__ __noinline__ void row_item_forward(float2* Z, const float2* stw, cons
             if (IT * NT == S * W || e < S * W) Z[p * SEQ + pad(x)] = make_float2(a[i], b[i]);
         }
         __syncthreads();
-        fft_seqs<W, S, NT, false>(Z, stw);
+        fft_seqs<W, S, NT, false, true>(Z, stw);
         store_rows_spectrum<W, S, NT>(Z, wd.spec + d * cplane, H, r0);
         __syncthreads();
     }
@@ -379,7 +459,7 @@ __device__ __noinline__ void row_item_u(float2* Z, const float2* stw, const DevW
         if (per_chan && wd.kern[k].dst != d0) continue;
         load_rows_spectrum<W, S, NT>(Z, wd.conv + k * cplane, H, r0);
         __syncthreads();
-        fft_seqs<W, S, NT, true>(Z, stw);
+        fft_seqs<W, S, NT, true, false>(Z, stw);
         float* u = wd.u_out + k * plane + (size_t)r0 * W;
         for (int e = threadIdx.x; e < S * W; e += NT) {
             const int p = e / W, x = e - p * W;
@@ -409,7 +489,7 @@ __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, floa
     // pulled into L2 when the CTA starts, and each thread's 2 x R state values are loaded into
     // registers just before the last inverse stage.
     static_assert(fusable<W>(), "row widths need a plan with equal first and last radix");
-    constexpr int R = plan_radix(W, 0), NB = W / R;
+    constexpr int R = chain_radix<W>(), NB = W / R;
     static_assert(S * NB <= NT, "one butterfly per thread in the fused stage");
     if (threadIdx.x == 0) tc::bulk_prefetch_l2(st, ROWS * W * (uint32_t)sizeof(float));
     if constexpr (!CG) grid_wait();
@@ -454,7 +534,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     float* extra = row_extra_smem<W>(stw);
     const RowItem it = items[blockIdx.x];
     const DevWorld& wd = worlds[it.world];
-    fill_stage_twiddles<W>(stw, tw, threadIdx.x, NT);
+    fill_tables<W>(stw, tw, NT);
     const int H = wd.H, C = wd.C, K = wd.K, r0 = it.row0;
     const size_t plane = (size_t)W * H, cplane = (size_t)(W / 2) * H;
     // Lenia items cover one target channel; SmoothLife and MNCA items every channel
@@ -485,7 +565,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     // registers.  A thread owns the same cells (sequence s, x = j + m*N/R) in all of these stages,
     // so the plane needs no barrier of its own.
     const int rule = wd.rule;
-    constexpr int R = plan_radix(W, 0), NB = W / R, LAST = plan_len(W) - 1;
+    constexpr int R = chain_radix<W>(), NB = W / R;
     static_assert(fusable<W>(), "row widths need a plan with equal first and last radix");
     static_assert(S * NB <= NT, "one butterfly per thread in the chained stages");
     float* acc = extra;  // [ROWS][W]
@@ -508,11 +588,11 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
         const Growth growth(kp.mu, kp.sigma);
         load_rows_spectrum<W, S, NT>(Z, wd.conv + k * cplane, H, r0);
         __syncthreads();
-        fft_stages<W, S, NT, true, 0, LAST>(Z, stw);
+        fft_head<W, S, NT, true>(Z, stw);
         if ((int)threadIdx.x < S * NB) {
             const int s = threadIdx.x / NB, j = threadIdx.x - s * NB;
             float2 v[R];
-            stage_load<W, R, NB, true>(Z + s * SEQ, j, v, stw + stage_tw_offset(W, LAST));
+            chain_load<W, true>(Z + s * SEQ, j, v, stw);
             float* a = acc + (2 * s) * W + j;
 #pragma unroll
             for (int m = 0; m < R; m++) {
@@ -576,89 +656,35 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
 
 // ---------------------------------------------------------------------------- column pass
 
-// X (TC sequences of length H, forward spectrum of tile `t`) times khat -> T.  Column 0 of
-// tile 0 packs the DC column (real part) and the Nyquist column (imaginary part): both are
-// real sequences, so with Z = FFT_y(packed), Z' = Z*(K0+KN)/2 + conj(Z[-ky])*(K0-KN)/2.
+// Column 0 of tile 0 packs the DC column (real part) and the Nyquist column (imaginary part): both are
+// real sequences, so with Z = FFT_y(packed), K0 and KN their kernel spectra,
+// Z'[ky] = Z[ky] (K0 + KN)/2 + conj(Z[-ky]) (K0 - KN)/2.  One rounding order, whoever computes it.
+__device__ __forceinline__ float2 packed_times_khat(float2 z, float2 zm, float K0, float KN) {
+    const float a = 0.5f * (K0 + KN), b = 0.5f * (K0 - KN);
+    return make_float2(__fmaf_rn(z.x, a, __fmul_rn(zm.x, b)), __fmaf_rn(z.y, a, -__fmul_rn(zm.y, b)));
+}
+
+// X (TC sequences of length H in padded natural order, the forward spectrum of tile 0) times khat, in place.
 template <int H, int NT>
-__device__ __forceinline__ void multiply_khat(const float2* X, float2* T, const float* __restrict__ kh, int HQ,
-                                              int W, int t) {
+__device__ __forceinline__ void multiply_khat(float2* X, const float* __restrict__ kh, int HQ, int W) {
     constexpr int SEQ = seq_stride(H);
-    for (int e = threadIdx.x; e < TC * H; e += NT) {
-        const int col = e / H, ky = e - col * H;
-        if (t == 0 && col == 0) continue;
-        const int kx = TC * t + col;
-        const float kv = kh[(size_t)kx * HQ + (ky <= H / 2 ? ky : H - ky)];
-        T[col * SEQ + pad(ky)] = cscale(X[col * SEQ + pad(ky)], kv);
+    for (int ky = threadIdx.x; ky < H; ky += NT) {
+        float2& z = X[SEQ + pad(ky)];
+        z = cscale(z, kh[HQ + (ky <= H / 2 ? ky : H - ky)]);
     }
-    if (t == 0) {
-        for (int ky = threadIdx.x; ky <= H / 2; ky += NT) {
-            const float K0 = kh[ky], KN = kh[(size_t)(W / 2) * HQ + ky];
-            const float a = 0.5f * (K0 + KN), b = 0.5f * (K0 - KN);
-            const int km = (H - ky) % H;
-            const float2 z = X[pad(ky)], zm = X[pad(km)];
-            T[pad(ky)] = make_float2(z.x * a + zm.x * b, z.y * a - zm.y * b);
-            if (km != ky) T[pad(km)] = make_float2(zm.x * a + z.x * b, zm.y * a - z.y * b);
-        }
+    for (int ky = threadIdx.x; ky <= H / 2; ky += NT) {
+        const float K0 = kh[ky], KN = kh[(size_t)(W / 2) * HQ + ky];
+        const int km = (H - ky) % H;
+        const float2 z = X[pad(ky)], zm = X[pad(km)];
+        X[pad(ky)] = packed_times_khat(z, zm, K0, KN);
+        if (km != ky) X[pad(km)] = packed_times_khat(zm, z, K0, KN);
     }
-}
-
-// One tile (H rows x TC columns, contiguous) <-> TC sequences in shared memory.
-template <int H, int NT, bool CG = false>
-__device__ __forceinline__ void load_tile(float2* X, const float2* __restrict__ src) {
-    static_assert(TC == 2, "tile loads move one float4 (two columns) per row");
-    constexpr int SEQ = seq_stride(H);
-    constexpr int IT = (H + NT - 1) / NT;
-    const float4* s4 = reinterpret_cast<const float4*>(src);
-    float4 v[IT];
-#pragma unroll
-    for (int i = 0; i < IT; i++) {
-        const int y = threadIdx.x + i * NT;
-        if (IT * NT == H || y < H) v[i] = hint::ld4c<CG>(s4 + y, hint::policy_keep());
-    }
-    // pad(tid + i NT) = pad(tid) + i (NT + NT / 16) when NT is a multiple of 16
-    float2* x0 = X + pad(threadIdx.x);
-#pragma unroll
-    for (int i = 0; i < IT; i++) {
-        const int y = threadIdx.x + i * NT;
-        if (IT * NT == H || y < H) {
-            float2* x = NT % 16 == 0 ? x0 + i * (NT + NT / 16) : X + pad(y);
-            x[0] = make_float2(v[i].x, v[i].y);
-            x[SEQ] = make_float2(v[i].z, v[i].w);
-        }
-    }
-}
-
-template <int H, int NT>
-__device__ __forceinline__ void store_tile(const float2* X, float2* __restrict__ dst) {
-    constexpr int SEQ = seq_stride(H);
-    float4* d4 = reinterpret_cast<float4*>(dst);
-    const float2* x = X + pad(threadIdx.x);
-    for (int y = threadIdx.x; y < H; y += NT, x += NT + NT / 16) {
-        if (NT % 16 != 0) x = X + pad(y);
-        const float2 a = x[0], b = x[SEQ];
-        hint::st4(d4 + y, make_float4(a.x, a.y, b.x, b.y), hint::policy_keep());
-    }
-}
-
-// Unchained column item: tile 0 (its column 0 packs the DC and Nyquist columns, paired ky with
-// H - ky in the khat multiply) or a khat array that is not 16-byte aligned.  Not inlined: one item
-// in W/4 takes this path, and as a separate function its registers do not add to the chained path's.
-template <int H, int NT, bool CG = false, int MR = CMR>
-__device__ __noinline__ void col_item_unchained(float2* X, const float2* stw, const float2* src, float2* dst,
-                                                const float* kh, int HQ, int W, int t, bool early) {
-    load_tile<H, NT, CG>(X, src);
-    __syncthreads();
-    fft_seqs<H, TC, NT, false, MR>(X, stw);
-    multiply_khat<H, NT>(X, X, kh, HQ, W, t);
-    __syncthreads();
-    if (!CG && early) grid_trigger();
-    fft_seqs<H, TC, NT, true, MR>(X, stw);
-    store_tile<H, NT>(X, dst);
 }
 
 // Stride between a column item's two sequences in shared memory: 8 mod 16 float2, so that the eight
 // butterflies of both columns that a half-warp works on (see col_chained) touch all 32 banks once.
-FFT_CHD constexpr int col_stride(int n) { return n + n / 16 + ((24 - (n + n / 16) % 16) % 16); }
+FFT_CHD constexpr int col_values(int n) { return n + (is_two_stage(n, 32) && two_tw_len(n) > n / 16 ? two_tw_len(n) : n / 16); }
+FFT_CHD constexpr int col_stride(int n) { return col_values(n) + (24 - col_values(n) % 16) % 16; }
 
 // Stages [I, I1) of both columns of a tile in shared memory, as fft_stages, but with the column in the
 // lowest bit of the butterfly index.
@@ -693,46 +719,90 @@ __device__ __forceinline__ void col_stages(float2* X, const float2* stw) {
 // 4 stages - 5 barriers, two sweeps and four barriers fewer than staging the tile both ways.  The item is
 // bound by shared-memory instructions and barriers; measured, per generation: 60 worlds of 384 x 384
 // 60.7 -> 55.3 us, 41 of 512 x 512 47.2 -> 44.7, one of 4096 x 4096 107.5 -> 103.3, of 8192 x 8192 576 -> 552.
+// Tile 0, whose column 0 packs two real columns, runs the same way with one exchange through shared memory in
+// the middle (khn: the Nyquist column's kernel spectrum; null in every other tile).  As a separate item of whole
+// transforms and tile sweeps it took about twice as long as the others and was the last to finish in every launch
+// that fits the GPU: one 512 x 512 world 8.9 -> 7.1 us a generation, 1024 x 1024 13.8 -> 10.7, 2048 x 1024 20.2 -> 16.0.
 template <int H, int NT, bool CG, int MR>
 __device__ __forceinline__ void col_chained(float2* X, const float2* stw, const float2* __restrict__ src,
-                                            float2* __restrict__ dst, const float* ksm, bool early) {
-    constexpr int LAST = plan_len(H, MR) - 1, R = plan_radix(H, 0, MR), NB = H / R, CS = col_stride(H);
+                                            float2* __restrict__ dst, const float* ksm, const float* __restrict__ khn,
+                                            bool early) {
+    constexpr bool TWO = is_two_stage(H, MR);
+    // radix of the stages at the tile (first of the forward transform, last of the inverse) and in the middle
+    constexpr int RT = TWO ? two_stage(H, MR).ra : plan_radix(H, 0, MR), RM = chain_radix<H, MR>();
+    constexpr int NT0 = H / RT, NM = H / RM, LAST = plan_len(H, MR) - 1, CS = col_stride(H);
     constexpr int HQC = khat_cols_stride<H>();
-    static_assert(TC == 2 && fusable<H, MR>() && TC * NB <= NT, "one outer butterfly per thread, two columns");
+    static_assert(TC == 2 && fusable<H, MR>() && TC * NT0 <= NT && TC * NM <= NT, "one outer butterfly per thread, two columns");
     const int c = threadIdx.x & 1, j = threadIdx.x >> 1;
-    const bool on = TC * NB == NT || threadIdx.x < TC * NB;
+    const bool tile = TC * NT0 == NT || threadIdx.x < TC * NT0, mid = TC * NM == NT || threadIdx.x < TC * NM;
     float2* Xc = X + c * CS;
-    float2 v[R];
-    if (on) {
+    if (tile) {
+        float2 v[RT];
         const uint64_t keep = hint::policy_keep();
 #pragma unroll
-        for (int m = 0; m < R; m++) v[m] = hint::ld2c<CG>(src + threadIdx.x + TC * NB * m, keep);
-        Dft<R, false>::run(v);
-        stage_store<H, R, 1>(Xc, j, v);
+        for (int m = 0; m < RT; m++) v[m] = hint::ld2c<CG>(src + threadIdx.x + TC * NT0 * m, keep);
+        Dft<RT, false>::run(v);
+        if constexpr (TWO) two_store<RT>(Xc, j, v);
+        else stage_store<H, RT, 1>(Xc, j, v);
     }
     cp_async_wait_all();  // the khat columns
     __syncthreads();
-    col_stages<H, NT, false, 1, LAST, MR>(X, stw);
-    if (on) {
-        stage_load<H, R, NB, false>(Xc, j, v, stw + stage_tw_offset(H, LAST, MR));
+    if constexpr (!TWO) col_stages<H, NT, false, 1, LAST, MR>(X, stw);
+    float2 v[RM];
+    if (mid) {
+        chain_load<H, false, MR>(Xc, j, v, stw);
         const float* kc = ksm + c * HQC;
+        if (khn == nullptr || c == 1) {
 #pragma unroll
-        for (int m = 0; m < R; m++) {
-            const int ky = j + m * NB;
-            v[m] = cscale(v[m], kc[ky <= H / 2 ? ky : H - ky]);
+            for (int m = 0; m < RM; m++) {
+                const int ky = j + m * NM;
+                v[m] = cscale(v[m], kc[ky <= H / 2 ? ky : H - ky]);
+            }
         }
-        Dft<R, true>::run(v);
     }
+    if (khn != nullptr) {
+        // tile 0 (the same for the whole CTA): column 0's values meet their mirrors through shared memory
+        __syncthreads();
+        if (mid && c == 0)
+#pragma unroll
+            for (int m = 0; m < RM; m++) X[j + m * NM] = v[m];
+        __syncthreads();
+        if (mid && c == 0)
+#pragma unroll
+            for (int m = 0; m < RM; m++) {
+                const int ky = j + m * NM, kk = ky <= H / 2 ? ky : H - ky;
+                v[m] = packed_times_khat(v[m], X[(H - ky) % H], ksm[kk], khn[kk]);
+            }
+    }
+    if (mid) Dft<RM, true>::run(v);
     __syncthreads();
-    if (on) stage_store<H, R, 1>(Xc, j, v);
+    if (mid) chain_store<H, MR>(Xc, j, v);
     __syncthreads();
     if (!CG && early) grid_trigger();
-    col_stages<H, NT, true, 1, LAST, MR>(X, stw);
-    if (on) {
-        stage_load<H, R, NB, true>(Xc, j, v, stw + stage_tw_offset(H, LAST, MR));
+    if constexpr (!TWO) col_stages<H, NT, true, 1, LAST, MR>(X, stw);
+    if (tile) {
+        float2 u[RT];
+        if constexpr (TWO) two_load<H, RT, true>(Xc, j, u, stw);
+        else stage_load<H, RT, NT0, true>(Xc, j, u, stw + stage_tw_offset(H, LAST, MR));
         const uint64_t keep = hint::policy_keep();
 #pragma unroll
-        for (int m = 0; m < R; m++) hint::st2(dst + threadIdx.x + TC * NB * m, v[m], keep);
+        for (int m = 0; m < RT; m++) hint::st2(dst + threadIdx.x + TC * NT0 * m, u[m], keep);
+    }
+}
+
+// A tile's two khat columns (rows of HQ floats) into shared memory, khat_cols_stride apart: asynchronous
+// 16-byte copies where the rows allow it (khat_stride rows; the caller waits), else plain loads (lenia_step_noalloc's
+// callers pass rows of H/2 + 1).
+template <int H, int NT>
+__device__ __forceinline__ void copy_khat(float* ksm, const float* __restrict__ kh, int HQ) {
+    constexpr int HQC = khat_cols_stride<H>();
+    if (HQ == HQC && ((uintptr_t)kh & 15) == 0) {
+        for (int e = threadIdx.x; e < TC * HQC / 4; e += NT) cp_async16(ksm + 4 * e, kh + 4 * e);
+    } else {
+        for (int e = threadIdx.x; e < TC * (H / 2 + 1); e += NT) {
+            const int c = e / (H / 2 + 1), y = e - c * (H / 2 + 1);
+            ksm[c * HQC + y] = kh[(size_t)c * HQ + y];
+        }
     }
 }
 
@@ -746,27 +816,21 @@ __device__ __forceinline__ void col_item(const DevWorld& wd, const ColItem it, f
     const int W = wd.W, c = it.chan, t = it.tile, k = it.kernel, HQ = wd.HQ;
     const size_t cplane = (size_t)(W / 2) * H;
     const float2* src = wd.spec + c * cplane + (size_t)t * H * TC;
-    // Tiles without the packed DC/Nyquist column: the khat multiply runs in registers between the
-    // forward and the inverse column FFT, and the tile's two khat columns (contiguous, HQ floats
-    // each) are copied to shared memory while the first stage runs.
+    // The khat multiply runs in registers between the forward and the inverse column FFT; the tile's two
+    // khat columns (HQ floats each) are copied to shared memory while the first stage runs.
     constexpr int HQC = khat_cols_stride<H>();
-    const float* kh = wd.khat + ((size_t)k * (W / 2 + 1) + (size_t)TC * t) * HQC;
-    if (fusable<H, MR>() && t != 0 && wd.HQ == HQC && ((uintptr_t)kh & 15) == 0) {
-        float* ksm = col_khat_smem<H, MR>(stw);
-        for (int e = threadIdx.x; e < TC * HQC / 4; e += NT) cp_async16(ksm + 4 * e, kh + 4 * e);
-        if constexpr (!CG) grid_wait();
-        // the stage tables are read after col_chained's first barrier
-        col_chained<H, NT, CG, MR>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC, ksm, early);
-        return;
-    }
+    const float* kh0 = wd.khat + (size_t)k * (W / 2 + 1) * HQ;
+    float* ksm = col_khat_smem<H, MR>(stw);
+    copy_khat<H, NT>(ksm, kh0 + (size_t)TC * t * HQ, HQ);
     if constexpr (!CG) grid_wait();
-    col_item_unchained<H, NT, CG, MR>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC,
-                                  wd.khat + (size_t)k * (W / 2 + 1) * HQ, HQ, W, t, early);
+    // the twiddle tables are read after col_chained's first barrier
+    col_chained<H, NT, CG, MR>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC, ksm,
+                               t == 0 ? kh0 + (size_t)(W / 2) * HQ : nullptr, early);
 }
 
-// Shared memory of a column item's two sequences (the unchained item strides them by seq_stride).
+// float2s of a column item's two sequences.
 template <int H>
-FFT_CHD constexpr int col_seq_floats2() { return TC * (col_stride(H) > seq_stride(H) ? col_stride(H) : seq_stride(H)); }
+FFT_CHD constexpr int col_seq_floats2() { return TC * col_stride(H); }
 
 // MR: the radix cap of the build's plans (CMR; 16 for the radix-16 build of sizes whose CMR plan has
 // radix 32, launch variant 3)
@@ -777,7 +841,7 @@ __global__ void __launch_bounds__(NT, MINB) col_pass(const DevWorld* __restrict_
     float2* X = reinterpret_cast<float2*>(smem_raw);
     float2* stw = X + col_seq_floats2<H>();
     const ColItem it = items[blockIdx.x];
-    fill_stage_twiddles<H, float2, 0, MR>(stw, tw, threadIdx.x, NT);
+    fill_tables<H, MR>(stw, tw, NT);
     col_item<H, NT, false, MR>(worlds[it.world], it, X, stw, early);
 }
 
@@ -794,80 +858,12 @@ __device__ __forceinline__ float* col_khat_smem_pair(tw2* stw) {
     return reinterpret_cast<float*>(stw + TWS + 1);
 }
 
-template <int H, int NT>
-__device__ __forceinline__ void load_tile_pair(cpair* X, const float2* __restrict__ src) {
-    constexpr int IT = (H + NT - 1) / NT;
-    const float4* s4 = reinterpret_cast<const float4*>(src);
-    float4 v[IT];
-#pragma unroll
-    for (int i = 0; i < IT; i++) {
-        const int y = threadIdx.x + i * NT;
-        if (IT * NT == H || y < H) v[i] = hint::ld4(s4 + y, hint::policy_keep());
-    }
-    cpair* x0 = X + pad(threadIdx.x);
-#pragma unroll
-    for (int i = 0; i < IT; i++) {
-        const int y = threadIdx.x + i * NT;
-        if (IT * NT == H || y < H)
-            (NT % 16 == 0 ? x0[i * (NT + NT / 16)] : X[pad(y)]) =
-                cpair{make_float2(v[i].x, v[i].z), make_float2(v[i].y, v[i].w)};
-    }
-}
-
-template <int H, int NT>
-__device__ __forceinline__ void store_tile_pair(const cpair* X, float2* __restrict__ dst) {
-    float4* d4 = reinterpret_cast<float4*>(dst);
-    const cpair* x = X + pad(threadIdx.x);
-    for (int y = threadIdx.x; y < H; y += NT, x += NT + NT / 16) {
-        const cpair a = NT % 16 == 0 ? *x : X[pad(y)];
-        hint::st4(d4 + y, make_float4(a.re.x, a.im.x, a.re.y, a.im.y), hint::policy_keep());
-    }
-}
-
-// The khat multiply of an unchained item (see multiply_khat): column 1 (lane y) by its khat
-// column; in tile 0, column 0 (lane x) packs the DC and Nyquist columns and pairs ky with H - ky.
-template <int H, int NT>
-__device__ __forceinline__ void multiply_khat_pair(cpair* X, const float* __restrict__ kh, int HQ, int W, int t) {
-    const float* k0 = kh + (size_t)(TC * t) * HQ;
-    const float* k1 = k0 + HQ;
-    if (t != 0) {
-        for (int ky = threadIdx.x; ky < H; ky += NT) {
-            const int kk = ky <= H / 2 ? ky : H - ky;
-            X[pad(ky)] = cscale2(X[pad(ky)], make_float2(k0[kk], k1[kk]));
-        }
-        return;
-    }
-    for (int ky = threadIdx.x; ky <= H / 2; ky += NT) {
-        const float K0 = kh[ky], KN = kh[(size_t)(W / 2) * HQ + ky], kv = k1[ky];
-        const float a = 0.5f * (K0 + KN), b = 0.5f * (K0 - KN);
-        const int km = (H - ky) % H;
-        const cpair z = X[pad(ky)], zm = X[pad(km)];
-        X[pad(ky)] = cpair{make_float2(z.re.x * a + zm.re.x * b, z.re.y * kv),
-                           make_float2(z.im.x * a - zm.im.x * b, z.im.y * kv)};
-        if (km != ky)
-            X[pad(km)] = cpair{make_float2(zm.re.x * a + z.re.x * b, zm.re.y * kv),
-                               make_float2(zm.im.x * a - z.im.x * b, zm.im.y * kv)};
-    }
-}
-
-template <int H, int NT>
-__device__ __noinline__ void col_item_unchained_pair(cpair* X, const tw2* stw, const float2* src, float2* dst,
-                                                     const float* kh, int HQ, int W, int t, bool early) {
-    load_tile_pair<H, NT>(X, src);
-    __syncthreads();
-    fft_seqs<H, 1, NT, false>(X, stw);
-    multiply_khat_pair<H, NT>(X, kh, HQ, W, t);
-    __syncthreads();
-    if (early) grid_trigger();
-    fft_seqs<H, 1, NT, true>(X, stw);
-    store_tile_pair<H, NT>(X, dst);
-}
-
 // The chained paired item: as col_chained, with one butterfly of both columns per thread (a warp's access
 // to the tile is 512 contiguous bytes).
 template <int H, int NT>
 __device__ __forceinline__ void col_chained_pair(cpair* X, const tw2* stw, const float2* __restrict__ src,
-                                                 float2* __restrict__ dst, const float* ksm, bool early) {
+                                                 float2* __restrict__ dst, const float* ksm,
+                                                 const float* __restrict__ khn, bool early) {
     constexpr int LAST = plan_len(H, PMR) - 1, R = plan_radix(H, 0, PMR), NB = H / R;
     constexpr int HQC = khat_cols_stride<H>();
     static_assert(fusable<H, PMR>() && NB <= NT, "one outer butterfly per thread");
@@ -891,13 +887,32 @@ __device__ __forceinline__ void col_chained_pair(cpair* X, const tw2* stw, const
     fft_stages<H, 1, NT, false, 1, LAST>(X, stw);
     if (on) {
         stage_load<H, R, NB, false>(X, j, v, last);
+        if (khn == nullptr) {
 #pragma unroll
-        for (int m = 0; m < R; m++) {
-            const int ky = j + m * NB, kk = ky <= H / 2 ? ky : H - ky;
-            v[m] = cscale2(v[m], make_float2(ksm[kk], ksm[HQC + kk]));
+            for (int m = 0; m < R; m++) {
+                const int ky = j + m * NB, kk = ky <= H / 2 ? ky : H - ky;
+                v[m] = cscale2(v[m], make_float2(ksm[kk], ksm[HQC + kk]));
+            }
         }
-        Dft<R, true>::run(v);
     }
+    if (khn != nullptr) {  // tile 0, see col_chained
+        __syncthreads();
+        if (on)
+#pragma unroll
+            for (int m = 0; m < R; m++) X[j + m * NB] = v[m];
+        __syncthreads();
+        if (on)
+#pragma unroll
+            for (int m = 0; m < R; m++) {
+                const int ky = j + m * NB, kk = ky <= H / 2 ? ky : H - ky;
+                const cpair zm = X[(H - ky) % H];
+                const float2 p = packed_times_khat(make_float2(v[m].re.x, v[m].im.x), make_float2(zm.re.x, zm.im.x),
+                                                   ksm[kk], khn[kk]);
+                const float k1 = ksm[HQC + kk];
+                v[m] = cpair{make_float2(p.x, v[m].re.y * k1), make_float2(p.y, v[m].im.y * k1)};
+            }
+    }
+    if (on) Dft<R, true>::run(v);
     __syncthreads();
     if (on) stage_store<H, R, 1>(X, j, v);
     __syncthreads();
@@ -926,28 +941,22 @@ __global__ void __launch_bounds__(NT, MINB) col_pass_pair(const DevWorld* __rest
     const size_t cplane = (size_t)(W / 2) * H;
     const float2* src = wd.spec + c * cplane + (size_t)t * H * TC;
     float2* dst = wd.conv + k * cplane + (size_t)t * H * TC;
-    constexpr int HQC = khat_cols_stride<H>();
-    const float* kh = wd.khat + ((size_t)k * (W / 2 + 1) + (size_t)TC * t) * HQC;
-    if (fusable<H, PMR>() && t != 0 && wd.HQ == HQC && ((uintptr_t)kh & 15) == 0) {
-        float* ksm = col_khat_smem_pair<H>(stw);
-        for (int e = threadIdx.x; e < TC * HQC / 4; e += NT) cp_async16(ksm + 4 * e, kh + 4 * e);
-        grid_wait();
-        col_chained_pair<H, NT>(X, stw, src, dst, ksm, early);
-        return;
-    }
+    const float* kh0 = wd.khat + (size_t)k * (W / 2 + 1) * HQ;
+    float* ksm = col_khat_smem_pair<H>(stw);
+    copy_khat<H, NT>(ksm, kh0 + (size_t)TC * t * HQ, HQ);
     grid_wait();
-    col_item_unchained_pair<H, NT>(X, stw, src, dst, wd.khat + (size_t)k * (W / 2 + 1) * HQ, HQ, W, t, early);
+    col_chained_pair<H, NT>(X, stw, src, dst, ksm, t == 0 ? kh0 + (size_t)(W / 2) * HQ : nullptr, early);
 }
 
 // Sizes built: each TU instantiates one group.  Threads per CTA: one first-stage butterfly per
-// thread for the two sequences a CTA holds (2N / first radix), between 64 and 1024.
+// thread for the two sequences a CTA holds (2N / outer radix), in whole warps, at most 1024.  (With at least 64
+// the columns of 64 to 256 left half of every CTA idle: 1024 worlds of 256 x 256 311 -> 249 us a generation.)
 #define LENIA_SIZES_SMALL(X) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768)
 #define LENIA_SIZES_LARGE(X) X(1024) X(1536) X(2048) X(3072) X(4096) X(6144) X(8192)
-// (The column pass keeps one first-stage butterfly per thread at every size: at 768 the balanced count,
-// 128 threads, made it slower, 66 -> 73 us a generation on the batched workload's class.)
 template <int N, int MR = CMR> constexpr int nt_of() {
-    constexpr int n = 2 * N / plan_radix(N, 0, MR);  // one first-stage butterfly per thread, two sequences
-    return n < 64 ? 64 : (n > 1024 ? 1024 : n);
+    // one outer butterfly per thread, two sequences, whole warps
+    constexpr int n = (2 * (is_two_stage(N, MR) ? two_tw_len(N) : N / plan_radix(N, 0, MR)) + 31) / 32 * 32;
+    return n > 1024 ? 1024 : n;
 }
 // whether the scalar column build's plan has radix 32 (1024, 3072, 8192): those sizes also build the
 // radix-16 plan (launch variant 3)
@@ -955,7 +964,7 @@ template <int N> constexpr bool col_r32() { return plan_radix(N, 0, CMR) == 32; 
 // variant 0: at most 64 registers per thread (80 for radix-32 plans: the 1024 build spilled 508 B at
 // 64 and needs none at 80); variant 1: at most 128
 template <int N, int V, int MR = CMR> constexpr int minb_threads() {
-    return V == 0 ? (plan_radix(N, 0, MR) == 32 ? 768 : 1024) : 512;
+    return V == 0 ? (plan_radix(N, 0, MR) == 32 || two_stage(N, MR).ra > 16 ? 768 : 1024) : 512;
 }
 template <int N, int V, int MR = CMR> constexpr int minb_of() {
     return minb_threads<N, V, MR>() / nt_of<N, MR>() < 1 ? 1 : minb_threads<N, V, MR>() / nt_of<N, MR>();
@@ -1051,36 +1060,6 @@ bool col_go_variant(int variant, const DevWorld* worlds, const ColItem* items, i
                    : row_go<N, row_nt<N, G>(), row_minb<N, 0, G>(), G>(mode, general, planes, worlds, items, nitems, tw, s);
 #define LENIA_ROW_CASE_SIMPLE(N) LENIA_ROW_CASE_G(N, false)
 #define LENIA_ROW_CASE_GENERAL(N) LENIA_ROW_CASE_G(N, true)
-
-// Local memory (spills and stack) of one instantiation, bytes per thread; -1 if unknown.
-template <class F>
-int local_bytes_of(F* f) {
-    cudaFuncAttributes a;
-    return cudaFuncGetAttributes(&a, f) == cudaSuccess ? (int)a.localSizeBytes : -1;
-}
-template <int N>
-int col_local_bytes_variant(int variant) {
-    if (variant == 2) return local_bytes_of(col_pass_pair<N, nt_pair_of<N>(), minb_pair_of<N>()>);
-    if (variant == 1) return local_bytes_of(col_pass<N, nt_of<N>(), minb_of<N, 1>()>);
-    if constexpr (col_r32<N>())
-        if (variant == 3) return local_bytes_of(col_pass<N, nt_of<N, 16>(), minb_of<N, 0, 16>(), 16>);
-    return local_bytes_of(col_pass<N, nt_of<N>(), minb_of<N, 0>()>);
-}
-#define LENIA_COL_LOCAL_CASE(N) \
-    case N: return col_local_bytes_variant<N>(variant);
-#define LENIA_ROW_LOCAL_CASE_G(N, G)                                                    \
-    case N:                                                                             \
-        return (variant & 1) ? local_bytes_of(row_pass<N, row_nt<N, G>(), row_minb<N, 1, G>(), G>) \
-                             : local_bytes_of(row_pass<N, row_nt<N, G>(), row_minb<N, 0, G>(), G>);
-#define LENIA_ROW_LOCAL_CASE_SIMPLE(N) LENIA_ROW_LOCAL_CASE_G(N, false)
-#define LENIA_ROW_LOCAL_CASE_GENERAL(N) LENIA_ROW_LOCAL_CASE_G(N, true)
-int col_local_bytes_small(int H, int variant);
-int col_local_bytes_large(int H, int variant);
-// row builds: one function per (size group, single-kernel or general) translation unit
-int row_local_bytes_small_simple(int W, int variant);
-int row_local_bytes_small_general(int W, int variant);
-int row_local_bytes_large_simple(int W, int variant);
-int row_local_bytes_large_general(int W, int variant);
 
 bool launch_col_group_small(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
                             const float2* tw, LaunchOn s);

@@ -10,9 +10,4 @@ bool launch_row_group_large_simple(int W, int variant, int mode, int general, in
     return false;
 }
 
-int row_local_bytes_large_simple(int W, int variant) {
-    switch (W) { LENIA_SIZES_LARGE(LENIA_ROW_LOCAL_CASE_SIMPLE) }
-    return -1;
-}
-
 }  // namespace lenia

@@ -10,9 +10,4 @@ bool launch_row_group_large_general(int W, int variant, int mode, int general, i
     return false;
 }
 
-int row_local_bytes_large_general(int W, int variant) {
-    switch (W) { LENIA_SIZES_LARGE(LENIA_ROW_LOCAL_CASE_GENERAL) }
-    return -1;
-}
-
 }  // namespace lenia

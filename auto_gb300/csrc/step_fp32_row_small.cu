@@ -10,9 +10,4 @@ bool launch_row_group_small_simple(int W, int variant, int mode, int general, in
     return false;
 }
 
-int row_local_bytes_small_simple(int W, int variant) {
-    switch (W) { LENIA_SIZES_SMALL(LENIA_ROW_LOCAL_CASE_SIMPLE) }
-    return -1;
-}
-
 }  // namespace lenia

@@ -10,9 +10,4 @@ bool launch_row_group_small_general(int W, int variant, int mode, int general, i
     return false;
 }
 
-int row_local_bytes_small_general(int W, int variant) {
-    switch (W) { LENIA_SIZES_SMALL(LENIA_ROW_LOCAL_CASE_GENERAL) }
-    return -1;
-}
-
 }  // namespace lenia
