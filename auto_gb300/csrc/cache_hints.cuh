@@ -66,6 +66,50 @@ __device__ __forceinline__ float4 ld4_cg(const float4* p, uint64_t pol) {
                  : "l"(p), "l"(pol));
     return v;
 }
+// 32 bytes a lane (32-byte aligned), kept in L2 as policy_keep's: one 256-bit access (WIDE) or two of 128 bits.
+// 256-bit accesses stay out of functions that are called rather than inlined: ptxas 13.0 wrote only the first
+// element of such a store there (and the right bytes wherever the code was inlined into the kernel).
+__device__ __forceinline__ unsigned long long pack2(float2 v) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+template <bool CG, bool WIDE>
+__device__ __forceinline__ void ld8c(float2* r, const float2* p) {
+    if constexpr (WIDE && !CG) {
+        unsigned long long a, b, c, d;
+        asm volatile("ld.global.L2::evict_last.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+        r[0] = unpack2(a);
+        r[1] = unpack2(b);
+        r[2] = unpack2(c);
+        r[3] = unpack2(d);
+    } else {
+        const uint64_t pol = policy_keep();
+        const float4* q = reinterpret_cast<const float4*>(p);
+        const float4 a = CG ? ld4_cg(q, pol) : ld4(q, pol), b = CG ? ld4_cg(q + 1, pol) : ld4(q + 1, pol);
+        r[0] = make_float2(a.x, a.y);
+        r[1] = make_float2(a.z, a.w);
+        r[2] = make_float2(b.x, b.y);
+        r[3] = make_float2(b.z, b.w);
+    }
+}
+template <bool WIDE>
+__device__ __forceinline__ void st8(float2* p, float2 a, float2 b, float2 c, float2 d) {
+    if constexpr (WIDE) {
+        asm volatile("st.global.L2::evict_last.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(pack2(a)), "l"(pack2(b)),
+                     "l"(pack2(c)), "l"(pack2(d))
+                     : "memory");
+    } else {
+        const uint64_t pol = policy_keep();
+        st4(reinterpret_cast<float4*>(p), make_float4(a.x, a.y, b.x, b.y), pol);
+        st4(reinterpret_cast<float4*>(p) + 1, make_float4(c.x, c.y, d.x, d.y), pol);
+    }
+}
 template <bool CG>
 __device__ __forceinline__ float2 ld2c(const float2* p, uint64_t pol) { return CG ? ld2_cg(p, pol) : ld2(p, pol); }
 template <bool CG>

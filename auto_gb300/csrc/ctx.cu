@@ -784,16 +784,22 @@ int setup_fused(LeniaCtx* ctx) {
                         planes);
         cl.general = general;
         cl.planes = planes;
-        // Default launch variants (per generation; the autotuner times the others).
+        // Default launch variants (per generation; the autotuner times the others).  A height's choice
+        // never changes the arithmetic with the number of worlds: variants 0, 1 and, from 2048 up, 3 run the same plan.
         // Columns: the 64-register scalar build, but the 128-register one where a thread holds 24 or 32
-        // elements (55 worlds of 1024 x 1024 253 -> 233 us and one 13.5 -> 10.7, 43 of 768 x 768 115 -> 112; equal at
-        // 384) and at 192 (63 worlds 16.1 -> 15.0); at 4096 and 6144 the paired build (one 4096 x 4096 world 108.5 -> 107.2,
-        // but 8192 x 8192 590 against 564).
-        cl.var_col = cl.H == 4096 || cl.H == 6144 ? 2 : (col_wide(cl.H) && cl.H != 384) || cl.H == 192 ? 1 : 0;
-        // Rows: at 64 registers (768 x 768, 43 worlds: 121 us against 139) unless the launch leaves the occupancy that
-        // buys unused -- at most three items for two SMs -- (one 384 x 384 world 10.5 -> 7.0 us, 768 x 768 11.3 -> 11.0,
-        // 1536 x 768 15.5 -> 14.7) or the general step, which spills there (SmoothLife 2048 x 2048 56 -> 50 us, 512 x 512 13.4 -> 12.6).
-        cl.var_row = general || 2 * row.size() <= 3 * (size_t)ctx->sms ? 1 : 0;
+        // elements (55 worlds of 1024 x 1024 245 -> 221 us and one 13.3 -> 10.3, 43 of 768 x 768 117 -> 112; equal at
+        // 384) and at 192 (one world 6.3 -> 6.1); from 3072 to 6144 the paired build (one 3072 x 3072 world 66.3 -> 62.4,
+        // 4096 x 4096 104.9 -> 103.0, 6144 x 6144 354 -> 333, but 8192 x 8192 556 against 528); at 2048 and 8192 one
+        // column a CTA where that is at most one CTA an SM (256 x 8192 21.0 -> 16.1, 256 x 2048 8.4 -> 7.4, but 512 x 8192
+        // 32.0 against 29.9).
+        if (cl.H >= 3072 && cl.H <= 6144) cl.var_col = 2;
+        else if (cl.H >= 2048 && 2 * col.size() <= (size_t)ctx->sms) cl.var_col = 3;
+        else cl.var_col = (col_wide(cl.H) && cl.H != 384) || cl.H == 192 ? 1 : 0;
+        // Rows: at 64 registers (43 worlds of 768 x 768 112 us against 129, one of 4096 x 4096 103 against 114) unless the
+        // launch leaves the occupancy that buys unused -- at most three items for two SMs -- (one 384 x 384 world 10.1 ->
+        // 6.8 us, 768 x 768 9.9 -> 9.4, 1536 x 768 13.2 -> 12.9), or those builds spill: at 512 (41 worlds 55 -> 45 us, one
+        // 11.2 -> 6.6) and in the general step (SmoothLife 2048 x 2048 55 -> 47 us, 1024 x 1024 17.5 -> 16.2).
+        cl.var_row = general || cl.W == 512 || 2 * row.size() <= 3 * (size_t)ctx->sms ? 1 : 0;
         cl.ncol = (int)col.size();
         cl.nrow = (int)row.size();
         cl.ntcg = (int)tcg.size();
@@ -1921,7 +1927,7 @@ static int autotune_search(LeniaCtx* ctx) {
                     for (int vc = 0; vc < COL_VARIANTS; vc++)
                         for (int vr = 0; vr < 2; vr++)
                             if (!(li == 0 && ln == c[0].lanes && vc == c[0].var_col && vr == c[0].var_row) &&
-                                (vc != 3 || col_has_r16_variant(cl.H))) {
+                                (vc != 3 || col_has_variant3(cl.H))) {
                                 c.push_back(Shape{vc, vr, cl.var_tc, &lists[li], ln});
                                 which.push_back(li);
                             }

@@ -92,10 +92,10 @@ bool launch_row_fp32(int W, int variant, int mode, int general, const DevWorld* 
 size_t col_smem_bytes(int H);
 size_t row_smem_bytes(int W, int acc_planes);
 // Column-pass launch variants (launch_col_fp32): 0, 1 scalar builds at two register caps, 2 the paired
-// build, 3 the scalar radix-16 build where the scalar plan has radix 32
+// build, 3 the scalar radix-16 build (1024) or the scalar build with one column a CTA (2048 and more)
 constexpr int COL_VARIANTS = 4;
-// whether the scalar column pass of height H has a radix-16 build beside its radix-32 one (variant 3)
-bool col_has_r16_variant(int H);
+// whether variant 3 is a build of its own at height H
+bool col_has_variant3(int H);
 // whether the scalar column pass of height H holds 24 or 32 elements a thread (radix-32 plans, the
 // larger two-stage transforms)
 bool col_wide(int H);

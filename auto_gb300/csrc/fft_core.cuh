@@ -260,6 +260,7 @@ template <int R1, int R2, bool INV, class T> FFT_HD void dft_coprime(T* v) {
     for (int k = 0; k < R; k++) v[k] = u[(k % R1) * R2 + k % R2];
 }
 
+template <bool INV> struct Dft<6, INV> { template <class T> FFT_HD static void run(T* v) { dft_coprime<2, 3, INV>(v); } };
 template <bool INV> struct Dft<12, INV> { template <class T> FFT_HD static void run(T* v) { dft_coprime<4, 3, INV>(v); } };
 template <bool INV> struct Dft<24, INV> { template <class T> FFT_HD static void run(T* v) { dft_coprime<8, 3, INV>(v); } };
 template <bool INV> struct Dft<8, INV> { template <class T> FFT_HD static void run(T* v) { dft_split<4, 2, INV>(v); } };
@@ -304,7 +305,18 @@ FFT_CHD constexpr Plan make_plan_capped(int n, int maxr) {
     P.r[P.len++] = outer;
     return P;
 }
+// Plans of the device passes, as caps beyond the radices: ROW_PLAN is the radix-16 plan with the 3 and the factor of two
+// beside it as one middle stage of radix 6, 12 or 24 (Good-Thomas: 1536 = 16.6.16, 3072 = 16.12.16, 6144 =
+// 16.24.16, 96 = 4.6.4); COL_PLAN takes those at sides with a 3 and the radix-32 cap elsewhere.
+constexpr int ROW_PLAN = 24, COL_PLAN = 40;
+FFT_CHD constexpr Plan make_plan_merged(int n) {
+    const Plan P = make_plan_capped(n, 16);
+    if (!(P.len == 4 && P.r[1] == 3 && P.r[2] < 16)) return P;
+    return Plan{3, {P.r[0], 3 * P.r[2], P.r[3], 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0}};
+}
 FFT_CHD constexpr Plan make_plan(int n, int maxr = 16) {
+    if (maxr == ROW_PLAN) return make_plan_merged(n);
+    if (maxr == COL_PLAN && n % 3 == 0) return make_plan_merged(n);
     return maxr <= 16 ? make_plan_capped(n, maxr)
          : (make_plan_capped(n, 32).len < make_plan_capped(n, 16).len ? make_plan_capped(n, 32)
                                                                       : make_plan_capped(n, 16));
@@ -322,11 +334,11 @@ FFT_CHD constexpr bool size_ok(int n) {
 }
 
 // Per-stage twiddle tables.  A stage with L > 1 needs w = exp(-2 pi i k / (L R)) for k < L and,
-// when R >= 8, w^4 (and when R >= 32, w^16); they are copied once per CTA from the global table into
+// when R >= 8, w^4 (and when R >= 24, w^16); they are copied once per CTA from the global table into
 // shared memory.
 FFT_CHD constexpr int stage_tw_count(int n, int i, int maxr = 16) {
     return plan_L(n, i, maxr) > 1
-               ? (plan_radix(n, i, maxr) >= 32 ? 3 : plan_radix(n, i, maxr) >= 8 ? 2 : 1) * plan_L(n, i, maxr)
+               ? (plan_radix(n, i, maxr) >= 24 ? 3 : plan_radix(n, i, maxr) >= 8 ? 2 : 1) * plan_L(n, i, maxr)
                : 0;
 }
 FFT_CHD constexpr int stage_tw_offset(int n, int i, int maxr = 16) {
@@ -351,7 +363,7 @@ FFT_HD void fill_stage_twiddles(W* stw, const float2* tw, int tid, int nth) {
             for (int k = tid; k < L; k += nth) {
                 set_twiddle(stw[off + k], tw[k * step]);
                 if (R >= 8) set_twiddle(stw[off + L + k], tw[4 * k * step]);
-                if (R >= 32) set_twiddle(stw[off + 2 * L + k], tw[16 * k * step]);
+                if (R >= 24) set_twiddle(stw[off + 2 * L + k], tw[16 * k * step]);
             }
         }
         fill_stage_twiddles<N, W, I + 1, MR>(stw, tw, tid, nth);
@@ -360,9 +372,9 @@ FFT_HD void fill_stage_twiddles(W* stw, const float2* tw, int tid, int nth) {
 
 // padded shared-memory index: one float2 of padding per 16 keeps radix-16 stores conflict-free
 FFT_HD int pad(int i) { return i + (i >> 4); }
-// stride between sequences held in one shared buffer: padded length, +4 so that loads of
-// 4 interleaved columns fall into different banks
-FFT_CHD constexpr int seq_stride(int n) { return n + n / 16 + 4; }
+// stride between sequences held in one shared buffer: padded length, 1 mod 16 so that four neighbouring
+// sequences fall into different banks (the row pass's spectrum unpack and pack)
+FFT_CHD constexpr int seq_stride(int n) { return n + n / 16 + 4 + (29 - (n + n / 16) % 16) % 16; }
 
 // Twiddles w^m, m = 1..R-1, of one butterfly from w, (R >= 8) w^4 and (R >= 24) w^16; the other
 // powers are products of at most four factors, so each stays within a few float ulps of the exactly
@@ -372,6 +384,10 @@ FFT_HD void twiddle_powers(W w1, W w4, W w16, W* w) {
     w[1] = w1;
     if (R >= 3) w[2] = cmul(w[1], w[1]);
     if (R >= 4) w[3] = cmul(w[2], w[1]);
+    if (R == 6) {
+        w[4] = cmul(w[2], w[2]);
+        w[5] = cmul(w[3], w[2]);
+    }
     if (R >= 8) {
         w[4] = w4;
         w[5] = cmul(w[4], w[1]);
@@ -418,7 +434,7 @@ FFT_HD void stage_load(const T* seq, int j, T* v, const W* stw) {
     }
     if (L > 1) {
         W w[R];
-        twiddle_powers<R>(stw[k], R >= 8 ? stw[L + k] : stw[k], R >= 32 ? stw[2 * L + k] : stw[k], w);
+        twiddle_powers<R>(stw[k], R >= 8 ? stw[L + k] : stw[k], R >= 24 ? stw[2 * L + k] : stw[k], w);
 #pragma unroll
         for (int m = 1; m < R; m++) v[m] = INV ? cmulc(v[m], w[m]) : cmul(v[m], w[m]);
     }
@@ -449,7 +465,7 @@ FFT_HD void stage_store(T* seq, int j, const T* v) {
 
 // ------------------------------------------------------------------ two-stage transforms
 // N = RA * RB as two stages, for the sides whose single plan with equal outer radices needs three or
-// four (192 = 8.3.8, 384 = 8.3.2.8, and in the column pass, maxr = 32, 768 = 16.3.16).  Of two chained
+// four (192 = 8.3.8, 384 = 8.3.2.8, and in the column pass 768 = 16.3.16).  Of two chained
 // transforms the first runs RA then RB and the second RB then RA, so the chained stages in the middle still
 // share a radix (RB, the smaller: the row pass holds its state values beside it).
 // Between its stages a transform is an RB x RA (or RA x RB) transposition: butterfly j of the first stage leaves
@@ -465,13 +481,13 @@ struct TwoStage {
 };
 FFT_CHD constexpr TwoStage two_stage(int n, int maxr = 16) {
     return n == 192 ? TwoStage{12, 16} : n == 384 ? TwoStage{24, 16}
-         : maxr == 32 && n == 768 ? TwoStage{32, 24} : TwoStage{0, 0};
+         : maxr == COL_PLAN && n == 768 ? TwoStage{32, 24} : TwoStage{0, 0};
 }
 FFT_CHD constexpr bool is_two_stage(int n, int maxr = 16) { return two_stage(n, maxr).ra != 0; }
 // Twiddle table of a two-stage transform: w^k, w^4k and w^16k, w = exp(-2 pi i / N), k below the larger radix
 // (either order's second stage, of radix R, needs w^(k m) for k < N/R and m < R).
 FFT_CHD constexpr int two_tw_len(int n) {
-    return two_stage(n, 32).ra > two_stage(n, 32).rb ? two_stage(n, 32).ra : two_stage(n, 32).rb;
+    return two_stage(n, COL_PLAN).ra > two_stage(n, COL_PLAN).rb ? two_stage(n, COL_PLAN).ra : two_stage(n, COL_PLAN).rb;
 }
 FFT_CHD constexpr int two_tw_size(int n) { return 3 * two_tw_len(n); }
 template <int N, class W>

@@ -35,7 +35,7 @@ int row_item_rows(int W, int general) { return 2 * row_seqs(W, general != 0); }
 
 bool col_wide(int H) { return lfft::plan_radix(H, 0, CMR) == 32 || lfft::two_stage(H, CMR).ra >= 24; }
 
-bool col_has_r16_variant(int H) { return lfft::plan_radix(H, 0, CMR) == 32; }
+bool col_has_variant3(int H) { return lfft::plan_radix(H, 0, CMR) == 32 || H >= 2048; }
 
 int max_smem_optin() {
     int dev = 0, v = 0;

@@ -62,9 +62,9 @@ __device__ __forceinline__ void static_for(F&& f) {
 // seq_stride(N)), in place, by NT threads; stw holds the per-stage twiddle tables
 // (fill_stage_twiddles).  Starts after the caller's barrier; ends with a barrier.
 // MR: the plan's radix cap (make_plan); 16 for every pass but the scalar column pass.
-template <int N, int S, int NT, bool INV, int I, int I1, int MR = 16, class T, class W>
+template <int N, int S, int NT, bool INV, int I, int I1, int MR = ROW_PLAN, class T, class W>
 __device__ __forceinline__ void fft_stages(T* buf, const W* stw) {
-    static_assert(MR == 32 || MR == max_radix<T>(), "radix-32 plans are built for scalar elements only");
+    static_assert(MR != COL_PLAN || sizeof(T) == sizeof(float2), "radix-32 plans are built for scalar elements only");
     if constexpr (I < I1) {
         constexpr int R = plan_radix(N, I, MR);
         constexpr int L = plan_L(N, I, MR);
@@ -109,16 +109,16 @@ __device__ __forceinline__ void fft_stages(T* buf, const W* stw) {
 //   chain_load    butterfly j of A's last stage
 //   chain_store   the results of butterfly j of B's first stage (after a barrier, and before one)
 //   fft_tail      B's other stages; ends with a barrier
-template <int N, int MR = 16>
+template <int N, int MR = ROW_PLAN>
 FFT_CHD constexpr bool fusable() {
     return is_two_stage(N, MR) || (plan_len(N, MR) >= 2 && plan_radix(N, 0, MR) == plan_radix(N, plan_len(N, MR) - 1, MR));
 }
-template <int N, int MR = 16>
+template <int N, int MR = ROW_PLAN>
 FFT_CHD constexpr int chain_radix() { return is_two_stage(N, MR) ? two_stage(N, MR).rb : plan_radix(N, 0, MR); }
 // Twiddle tables of a scalar transform: two-stage or per stage of the plan.
-template <int N, int MR = 16>
+template <int N, int MR = ROW_PLAN>
 FFT_CHD constexpr int tables_size() { return is_two_stage(N, MR) ? two_tw_size(N) : tw_table_size(N, MR); }
-template <int N, int MR = 16>
+template <int N, int MR = ROW_PLAN>
 __device__ __forceinline__ void fill_tables(float2* stw, const float2* tw, int nth) {
     if constexpr (is_two_stage(N, MR)) fill_two_twiddles<N>(stw, tw, threadIdx.x, nth);
     else fill_stage_twiddles<N, float2, 0, MR>(stw, tw, threadIdx.x, nth);
@@ -154,7 +154,7 @@ __device__ __forceinline__ void two_stage_pass(float2* buf, const float2* stw) {
 }
 
 // Whole transforms in place.  SWAP: the order of B (RB, RA).
-template <int N, int S, int NT, bool INV, bool SWAP, int MR = 16, class T, class W>
+template <int N, int S, int NT, bool INV, bool SWAP, int MR = ROW_PLAN, class T, class W>
 __device__ __forceinline__ void fft_seqs(T* buf, const W* stw) {
     if constexpr (is_two_stage(N, MR) && sizeof(T) == sizeof(float2)) {
         constexpr int R1 = SWAP ? two_stage(N, MR).rb : two_stage(N, MR).ra, R2 = N / R1;
@@ -165,24 +165,24 @@ __device__ __forceinline__ void fft_seqs(T* buf, const W* stw) {
     }
 }
 
-template <int N, int S, int NT, bool INV, int MR = 16>
+template <int N, int S, int NT, bool INV, int MR = ROW_PLAN>
 __device__ __forceinline__ void fft_head(float2* buf, const float2* stw) {
     if constexpr (is_two_stage(N, MR)) two_stage_pass<N, two_stage(N, MR).ra, S, NT, INV, false>(buf, stw);
     else fft_stages<N, S, NT, INV, 0, plan_len(N, MR) - 1, MR>(buf, stw);
 }
-template <int N, bool INV, int MR = 16>
+template <int N, bool INV, int MR = ROW_PLAN>
 __device__ __forceinline__ void chain_load(const float2* seq, int j, float2* v, const float2* stw) {
     constexpr int LAST = plan_len(N, MR) - 1, R = chain_radix<N, MR>();
     if constexpr (is_two_stage(N, MR)) two_load<N, R, INV>(seq, j, v, stw);
     else stage_load<N, R, N / R, INV>(seq, j, v, stw + stage_tw_offset(N, LAST, MR));
 }
-template <int N, int MR = 16>
+template <int N, int MR = ROW_PLAN>
 __device__ __forceinline__ void chain_store(float2* seq, int j, const float2* v) {
     constexpr int R = chain_radix<N, MR>();
     if constexpr (is_two_stage(N, MR)) two_store<R>(seq, j, v);
     else stage_store<N, R, 1>(seq, j, v);
 }
-template <int N, int S, int NT, bool INV, int MR = 16>
+template <int N, int S, int NT, bool INV, int MR = ROW_PLAN>
 __device__ __forceinline__ void fft_tail(float2* buf, const float2* stw) {
     if constexpr (is_two_stage(N, MR)) two_stage_pass<N, two_stage(N, MR).ra, S, NT, INV, true>(buf, stw);
     else fft_stages<N, S, NT, INV, 1, plan_len(N, MR), MR>(buf, stw);
@@ -194,7 +194,7 @@ struct NoPre {
 
 // A, mid(s, j, v) on the registers between (sequence s, elements j + m*N/R), B.  `pre(s, j)` runs just before
 // the last stage of A.
-template <int N, int S, int NT, bool INV_A, bool INV_B, int MR = 16, class Mid, class Pre = NoPre>
+template <int N, int S, int NT, bool INV_A, bool INV_B, int MR = ROW_PLAN, class Mid, class Pre = NoPre>
 __device__ __forceinline__ void fft_fused(float2* buf, const float2* stw, Mid mid, Pre pre = Pre()) {
     static_assert(fusable<N, MR>(), "fusable plans only");
     constexpr int R = chain_radix<N, MR>(), NB = N / R;
@@ -223,14 +223,14 @@ __device__ __forceinline__ void fft_fused(float2* buf, const float2* stw, Mid mi
 }
 
 // Shared memory of a pass: the sequences, then (float2-aligned) the twiddle tables.
-template <int N, int MR = 16>
+template <int N, int MR = ROW_PLAN>
 constexpr size_t stage_table_bytes() { return (size_t)(tables_size<N, MR>() + 1) * sizeof(float2); }
 
 // The scalar column pass's radix cap: radix-32 plans where they save a stage (1024 = 32.32 against
 // 16.4.16: one shared-memory round trip fewer per transform; 3072, 8192), the radix-16 plan elsewhere.
 // The column item holds its 32 elements a thread in registers between stages; the row pass, which also
 // holds the state values of its rows there, keeps radix 16.
-constexpr int CMR = 32;
+constexpr int CMR = COL_PLAN;
 
 // Column pass, fused form: after the stage tables (16-byte aligned), the tile's TC khat columns.
 template <int H>
@@ -317,9 +317,9 @@ __device__ __forceinline__ float mnca_update(float s, float c0, float c1) {
 // Two-stage sides: one butterfly of either stage.
 FFT_CHD constexpr int seq_threads(int N, int S) {
     if (is_two_stage(N)) return S * two_tw_len(N);
-    return N % 3 == 0 && S * N / 12 > S * N / plan_radix(N, 0) ? S * N / 12 : S * N / plan_radix(N, 0);
+    return N % 3 == 0 && N < 6144 && S * N / 12 > S * N / plan_radix(N, 0) ? S * N / 12 : S * N / plan_radix(N, 0);
 }
-FFT_CHD constexpr int row_seqs(int W, bool gen) { return gen ? (W >= 2048 ? 1 : (W <= 1024 ? 4 : 2)) : (W <= 1024 ? 4 : 2); }
+FFT_CHD constexpr int row_seqs(int W, bool gen) { return gen ? (W >= 2048 ? 1 : (W <= 1024 ? 4 : 2)) : (W <= 1024 ? 4 : W >= 6144 ? 1 : 2); }
 template <int W, bool GEN>
 constexpr int row_nt() {
     constexpr int n = seq_threads(W, row_seqs(W, GEN));
@@ -332,6 +332,11 @@ constexpr int row_minb() {
     constexpr int t = V == 0 ? 1024 : 512;
     return t / row_nt<W, GEN>() < 1 ? 1 : t / row_nt<W, GEN>();
 }
+// 256-bit spectrum accesses, but 128-bit ones in the builds for a few rows of small worlds, whose launches wait for
+// a single access's latency: one 256 x 256 world 5.9 -> 5.5 us a generation, 384 x 384 7.1 -> 6.8; against them
+// 1024 worlds of 256 x 256 233 -> 222, one of 1024 x 1024 11.1 -> 10.3, 4096 x 4096 109.7 -> 103.0.
+template <int W, int V>
+constexpr bool row_wide() { return !(V == 1 && W <= 384); }
 // Shared memory after the sequences and stage tables: the accumulation planes ([planes][2S][W]) of
 // the general path.
 template <int W>
@@ -340,82 +345,102 @@ __device__ __forceinline__ float* row_extra_smem(float2* stw) {
     return reinterpret_cast<float*>(((uintptr_t)(stw + TWS) + 15) & ~(uintptr_t)15);
 }
 
-// Half-spectra of rows r0..r0+2S-1 (tile layout) -> S packed complex sequences
-// Z_p = A + iB with A = row r0+2p, B = row r0+2p+1, using Hermitian symmetry for k > W/2.
-// One element per lane and column, consecutive lanes on consecutive columns: the shared-memory
-// writes of a warp are contiguous (a tile per lane, with both its columns, would write at
-// stride 2 and conflict; measured 4% slower at 4096 x 4096).
-template <int W, int S, int NT, bool CG = false>
+// Half-spectra of rows r0..r0+2S-1 (tile layout) <-> S packed complex sequences Z_p = A + iB with A = row
+// r0+2p, B = row r0+2p+1, using Hermitian symmetry for k > W/2.
+// A lane moves 32 bytes: both columns (kx = 2t, 2t+1) of one tile t for one row pair p, consecutive lanes on the
+// pairs of a tile.  A half-warp's shared-memory accesses have stride 2 within a pair; with the sequences 1 mod 16
+// apart, and at S = 4 the even tiles in one half-warp and the odd in the other, they touch all banks once (at S = 1
+// every other eight lanes take their second column first instead).  The row pass is bound by L1 wavefronts
+// (67-77% of their peak at 4096 and 8192), and as 8-byte accesses -- a lane per column and row -- the spectrum
+// took twice the wavefronts and four times the instructions.
+template <int W, int S, int NT>
+struct RowLanes {
+    static constexpr int TILES = W / 4, G = S == 4 ? 8 : 1;  // tiles are dealt in groups of G
+    static constexpr int E = (TILES + G - 1) / G * G * S, IT = (E + NT - 1) / NT;
+    // kx moves by D an iteration; a multiple of 16 moves padded positions by D + D / 16
+    static constexpr int D = 2 * NT / S, O = D + D / 16;
+    static constexpr bool STEP = NT % (G * S) == 0 && D % 16 == 0;
+    static constexpr bool FULL = TILES % G == 0 && IT * NT == E;
+};
+template <int S>
+__device__ __forceinline__ int row_tile(int e) {
+    return S == 4 ? (e >> 5) * 8 + 2 * ((e >> 2) & 3) + ((e >> 4) & 1) : e / S;
+}
+
+template <int W, int S, int NT, bool CG = false, bool WIDE = true>
 __device__ __forceinline__ void load_rows_spectrum(float2* Z, const float2* __restrict__ sp, int H, int r0) {
+    using L = RowLanes<W, S, NT>;
     constexpr int SEQ = seq_stride(W);
-    constexpr int E = W / 2 * S, IT = (E + NT - 1) / NT;
-    float2 A[IT], B[IT];
+    float2 v[L::IT][4];
 #pragma unroll
-    for (int i = 0; i < IT; i++) {
-        const int e = threadIdx.x + i * NT;
-        if (IT * NT == E || e < E) {
-            const int t = e / (S * TC), p = (e / TC) % S, c = e % TC;
-            const float2* src = sp + ((size_t)t * H + r0 + 2 * p) * TC + c;
-            const uint64_t keep = hint::policy_keep();
-            A[i] = hint::ld2c<CG>(src, keep);
-            B[i] = hint::ld2c<CG>(src + TC, keep);
-        }
+    for (int i = 0; i < L::IT; i++) {
+        const int e = threadIdx.x + i * NT, t = row_tile<S>(e), p = e % S;
+        if (L::FULL || t < L::TILES)
+            hint::ld8c<CG, WIDE>(v[i], sp + ((size_t)t * H + r0 + 2 * p) * TC);
     }
-    // When every iteration moves kx by the same multiple of 16 (D), the padded positions of kx and
-    // W - kx move by D + D/16: two base pointers and compile-time offsets.
-    constexpr int D = NT / S;
-    constexpr bool STEP = NT % (S * TC) == 0 && D % 16 == 0;
-    const int kx0 = TC * (threadIdx.x / (S * TC)) + threadIdx.x % TC, p0 = (threadIdx.x / TC) % S;
-    float2* za = Z + p0 * SEQ + pad(kx0);
-    float2* zb = Z + p0 * SEQ + pad(W - kx0);
+    const int t0 = row_tile<S>(threadIdx.x), p0 = threadIdx.x % S;
+    float2* za0 = Z + p0 * SEQ + pad(2 * t0);
+    float2* zb0 = Z + p0 * SEQ + pad(W - 2 * t0);
+    float2* zc0 = Z + p0 * SEQ + pad(W - 2 * t0 - 1);
 #pragma unroll
-    for (int i = 0; i < IT; i++) {
-        const int e = threadIdx.x + i * NT;
-        if (IT * NT == E || e < E) {
-            const int t = e / (S * TC), p = (e / TC) % S, c = e % TC, kx = TC * t + c;
-            float2* z = Z + p * SEQ;
-            if (kx == 0) {
-                z[pad(0)] = make_float2(A[i].x, B[i].x);
-                z[pad(W / 2)] = make_float2(A[i].y, B[i].y);
-            } else if constexpr (STEP) {
-                za[i * (D + D / 16)] = make_float2(A[i].x - B[i].y, A[i].y + B[i].x);
-                zb[-i * (D + D / 16)] = make_float2(A[i].x + B[i].y, B[i].x - A[i].y);
-            } else {
-                z[pad(kx)] = make_float2(A[i].x - B[i].y, A[i].y + B[i].x);
-                z[pad(W - kx)] = make_float2(A[i].x + B[i].y, B[i].x - A[i].y);
-            }
+    for (int i = 0; i < L::IT; i++) {
+        const int e = threadIdx.x + i * NT, t = row_tile<S>(e), p = e % S;
+        const bool swap = S == 1 && (threadIdx.x & 8);
+        if (!L::FULL && t >= L::TILES) continue;
+        float2* z = Z + p * SEQ;
+        // kx = 2t at za and (mirrored) zb, kx = 2t + 1 at za + 1 and zc
+        float2* za = L::STEP ? za0 + i * L::O : z + pad(2 * t);
+        float2* zb = L::STEP ? zb0 - i * L::O : z + pad(W - 2 * t);
+        float2* zc = L::STEP ? zc0 - i * L::O : z + pad(W - 2 * t - 1);
+        const float2 A0 = v[i][0], A1 = v[i][1], B0 = v[i][2], B1 = v[i][3];
+        const float2 p0_ = make_float2(A0.x - B0.y, A0.y + B0.x), m0 = make_float2(A0.x + B0.y, B0.x - A0.y);
+        const float2 p1 = make_float2(A1.x - B1.y, A1.y + B1.x), m1 = make_float2(A1.x + B1.y, B1.x - A1.y);
+        if (t == 0) {  // column 0 packs DC and Nyquist
+            z[pad(0)] = make_float2(A0.x, B0.x);
+            z[pad(W / 2)] = make_float2(A0.y, B0.y);
+            za[1] = p1;
+            *zc = m1;
+        } else {
+            za[swap ? 1 : 0] = swap ? p1 : p0_;
+            za[swap ? 0 : 1] = swap ? p0_ : p1;
+            *(swap ? zc : zb) = swap ? m1 : m0;
+            *(swap ? zb : zc) = swap ? m0 : m1;
         }
     }
 }
 
 // S packed complex spectra Z_p = FFT(a + ib) -> half-spectra of rows r0+2p (A) and r0+2p+1 (B).
-template <int W, int S, int NT>
+template <int W, int S, int NT, bool WIDE = true>
 __device__ __forceinline__ void store_rows_spectrum(const float2* Z, float2* __restrict__ sp, int H, int r0) {
+    using L = RowLanes<W, S, NT>;
     constexpr int SEQ = seq_stride(W);
-    constexpr int E = W / 2 * S;
-    // as in load_rows_spectrum: the padded positions of kx and W - kx move by a constant
-    constexpr int D = NT / S;
-    constexpr bool STEP = NT % (S * TC) == 0 && D % 16 == 0;
-    const int kx0 = TC * (threadIdx.x / (S * TC)) + threadIdx.x % TC, p0 = (threadIdx.x / TC) % S;
-    const float2* za = Z + p0 * SEQ + pad(kx0);
-    const float2* zb = Z + p0 * SEQ + pad(W - kx0);
-    for (int e = threadIdx.x; e < E; e += NT, za += STEP ? D + D / 16 : 0, zb -= STEP ? D + D / 16 : 0) {
-        const int t = e / (S * TC), p = (e / TC) % S, c = e % TC, kx = TC * t + c;
+    const int t0 = row_tile<S>(threadIdx.x), p0 = threadIdx.x % S;
+    const float2* za0 = Z + p0 * SEQ + pad(2 * t0);
+    const float2* zb0 = Z + p0 * SEQ + pad(W - 2 * t0);
+    const float2* zc0 = Z + p0 * SEQ + pad(W - 2 * t0 - 1);
+#pragma unroll
+    for (int i = 0; i < L::IT; i++) {
+        const int e = threadIdx.x + i * NT, t = row_tile<S>(e), p = e % S;
+        const bool swap = S == 1 && (threadIdx.x & 8);
+        if (!L::FULL && t >= L::TILES) continue;
         const float2* z = Z + p * SEQ;
+        const float2* za = L::STEP ? za0 + i * L::O : z + pad(2 * t);
+        const float2* zb = L::STEP ? zb0 - i * L::O : z + pad(W - 2 * t);
+        const float2* zc = L::STEP ? zc0 - i * L::O : z + pad(W - 2 * t - 1);
+        const float2* zm = t == 0 ? za : zb;  // column 0 has no mirror
+        const float2 f = za[swap ? 1 : 0], s = za[swap ? 0 : 1], g = *(swap ? zc : zm), h = *(swap ? zm : zc);
+        const float2 a0 = swap ? s : f, a1 = swap ? f : s, b0 = swap ? h : g, b1 = swap ? g : h;
         float2 A, B;
-        if (kx == 0) {
-            const float2 z0 = z[pad(0)], zn = z[pad(W / 2)];
-            A = make_float2(z0.x, zn.x);
-            B = make_float2(z0.y, zn.y);
+        if (t == 0) {
+            const float2 zn = z[pad(W / 2)];
+            A = make_float2(a0.x, zn.x);
+            B = make_float2(a0.y, zn.y);
         } else {
-            const float2 a = STEP ? *za : z[pad(kx)], b = STEP ? *zb : z[pad(W - kx)];
-            A = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
-            B = make_float2(0.5f * (a.y + b.y), -0.5f * (a.x - b.x));
+            A = make_float2(0.5f * (a0.x + b0.x), 0.5f * (a0.y - b0.y));
+            B = make_float2(0.5f * (a0.y + b0.y), -0.5f * (a0.x - b0.x));
         }
-        float2* dst = sp + ((size_t)t * H + r0 + 2 * p) * TC + c;
-        const uint64_t keep = hint::policy_keep();
-        hint::st2(dst, A, keep);
-        hint::st2(dst + TC, B, keep);
+        hint::st8<WIDE>(sp + ((size_t)t * H + r0 + 2 * p) * TC, A, make_float2(0.5f * (a1.x + b1.x), 0.5f * (a1.y - b1.y)), B,
+                  make_float2(0.5f * (a1.y + b1.y), -0.5f * (a1.x - b1.x)));
     }
 }
 
@@ -445,7 +470,7 @@ __device__ __noinline__ void row_item_forward(float2* Z, const float2* stw, cons
         }
         __syncthreads();
         fft_seqs<W, S, NT, false, true>(Z, stw);
-        store_rows_spectrum<W, S, NT>(Z, wd.spec + d * cplane, H, r0);
+        store_rows_spectrum<W, S, NT, false>(Z, wd.spec + d * cplane, H, r0);
         __syncthreads();
     }
 }
@@ -457,7 +482,7 @@ __device__ __noinline__ void row_item_u(float2* Z, const float2* stw, const DevW
     const size_t plane = (size_t)W * H, cplane = (size_t)(W / 2) * H;
     for (int k = 0; k < K; k++) {
         if (per_chan && wd.kern[k].dst != d0) continue;
-        load_rows_spectrum<W, S, NT>(Z, wd.conv + k * cplane, H, r0);
+        load_rows_spectrum<W, S, NT, false, false>(Z, wd.conv + k * cplane, H, r0);
         __syncthreads();
         fft_seqs<W, S, NT, true, false>(Z, stw);
         float* u = wd.u_out + k * plane + (size_t)r0 * W;
@@ -475,7 +500,7 @@ __device__ __noinline__ void row_item_u(float2* Z, const float2* stw, const DevW
 // dt update and clamp against the state, forward row FFT of the new rows.  Z: the two packed
 // sequences, stw: the stage tables.  CG: spectrum and state loads bypass L1 (the persistent step,
 // where another CTA of the same launch wrote them).
-template <int W, int NT, bool CG>
+template <int W, int NT, bool CG, bool WIDE = true>
 __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, float2* Z, const float2* stw, bool early = false) {
     constexpr int S = row_seqs(W, false), ROWS = 2 * S;
     const int H = wd.H;
@@ -493,7 +518,7 @@ __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, floa
     static_assert(S * NB <= NT, "one butterfly per thread in the fused stage");
     if (threadIdx.x == 0) tc::bulk_prefetch_l2(st, ROWS * W * (uint32_t)sizeof(float));
     if constexpr (!CG) grid_wait();
-    load_rows_spectrum<W, S, NT, CG>(Z, wd.conv, H, r0);
+    load_rows_spectrum<W, S, NT, CG, WIDE>(Z, wd.conv, H, r0);
     __syncthreads();
     float sa[R], sb[R];
     fft_fused<W, S, NT, true, false>(
@@ -516,14 +541,15 @@ __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, floa
             });
         });
     if (!CG && early) grid_trigger();
-    store_rows_spectrum<W, S, NT>(Z, wd.spec, H, r0);
+    store_rows_spectrum<W, S, NT, WIDE>(Z, wd.spec, H, r0);
 }
 
 // GEN: the instantiation for size classes with worlds that need the general step (several
 // channels or kernels, SmoothLife, MNCA).  Without it the kernel carries only the one-channel,
 // one-kernel Lenia step (and the forward and U modes), so the general path's register pressure
 // does not set the budget of the common path.
-template <int W, int NT, int MINB, bool GEN>
+// WIDE: whether the spectrum moves in 256-bit accesses (row_wide).
+template <int W, int NT, int MINB, bool GEN, bool WIDE>
 __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict__ worlds, const RowItem* __restrict__ items,
                                                 int mode, int general, const float2* __restrict__ tw, bool early) {
     constexpr int S = row_seqs(W, GEN), ROWS = 2 * S;
@@ -552,7 +578,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     }
 
     if constexpr (!GEN) {
-        row_item_simple<W, NT, false>(wd, r0, Z, stw, early);
+        row_item_simple<W, NT, false, WIDE>(wd, r0, Z, stw, early);
         return;
     }
 
@@ -586,7 +612,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
         const DevKernel kp = wd.kern[k];
         if (per_chan && kp.dst != d0) continue;
         const Growth growth(kp.mu, kp.sigma);
-        load_rows_spectrum<W, S, NT>(Z, wd.conv + k * cplane, H, r0);
+        load_rows_spectrum<W, S, NT, false, WIDE>(Z, wd.conv + k * cplane, H, r0);
         __syncthreads();
         fft_head<W, S, NT, true>(Z, stw);
         if ((int)threadIdx.x < S * NB) {
@@ -614,7 +640,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     const float dt = wd.dt;
     const bool have_acc = nk > 1;
     const uint64_t stream = hint::policy_stream();
-    load_rows_spectrum<W, S, NT>(Z, wd.conv + klast * cplane, H, r0);
+    load_rows_spectrum<W, S, NT, false, WIDE>(Z, wd.conv + klast * cplane, H, r0);
     __syncthreads();
     float sa[R], sb[R];
     fft_fused<W, S, NT, true, false>(
@@ -651,7 +677,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
             }
         });
     if (early) grid_trigger();
-    store_rows_spectrum<W, S, NT>(Z, wd.spec + d0 * cplane, H, r0);
+    store_rows_spectrum<W, S, NT, WIDE>(Z, wd.spec + d0 * cplane, H, r0);
 }
 
 // ---------------------------------------------------------------------------- column pass
@@ -683,31 +709,31 @@ __device__ __forceinline__ void multiply_khat(float2* X, const float* __restrict
 
 // Stride between a column item's two sequences in shared memory: 8 mod 16 float2, so that the eight
 // butterflies of both columns that a half-warp works on (see col_chained) touch all 32 banks once.
-FFT_CHD constexpr int col_values(int n) { return n + (is_two_stage(n, 32) && two_tw_len(n) > n / 16 ? two_tw_len(n) : n / 16); }
+FFT_CHD constexpr int col_values(int n) { return n + (is_two_stage(n, CMR) && two_tw_len(n) > n / 16 ? two_tw_len(n) : n / 16); }
 FFT_CHD constexpr int col_stride(int n) { return col_values(n) + (24 - col_values(n) % 16) % 16; }
 
 // Stages [I, I1) of both columns of a tile in shared memory, as fft_stages, but with the column in the
 // lowest bit of the butterfly index.
-template <int N, int NT, bool INV, int I, int I1, int MR>
+template <int N, int NT, bool INV, int I, int I1, int MR, int NC>
 __device__ __forceinline__ void col_stages(float2* X, const float2* stw) {
     if constexpr (I < I1) {
         constexpr int R = plan_radix(N, I, MR), L = plan_L(N, I, MR);
-        constexpr int TOT = TC * (N / R), PER = (TOT + NT - 1) / NT, CS = col_stride(N);
+        constexpr int TOT = NC * (N / R), PER = (TOT + NT - 1) / NT, CS = col_stride(N);
         float2 v[PER][R];
 #pragma unroll
         for (int p = 0; p < PER; p++) {
             const int b = threadIdx.x + p * NT;
             if ((TOT % NT) == 0 || b < TOT)
-                stage_load<N, R, L, INV>(X + (b & 1) * CS, b >> 1, v[p], stw + stage_tw_offset(N, I, MR));
+                stage_load<N, R, L, INV>(X + (b % NC) * CS, b / NC, v[p], stw + stage_tw_offset(N, I, MR));
         }
         __syncthreads();
 #pragma unroll
         for (int p = 0; p < PER; p++) {
             const int b = threadIdx.x + p * NT;
-            if ((TOT % NT) == 0 || b < TOT) stage_store<N, R, L>(X + (b & 1) * CS, b >> 1, v[p]);
+            if ((TOT % NT) == 0 || b < TOT) stage_store<N, R, L>(X + (b % NC) * CS, b / NC, v[p]);
         }
         __syncthreads();
-        col_stages<N, NT, INV, I + 1, I1, MR>(X, stw);
+        col_stages<N, NT, INV, I + 1, I1, MR, NC>(X, stw);
     }
 }
 
@@ -723,35 +749,35 @@ __device__ __forceinline__ void col_stages(float2* X, const float2* stw) {
 // the middle (khn: the Nyquist column's kernel spectrum; null in every other tile).  As a separate item of whole
 // transforms and tile sweeps it took about twice as long as the others and was the last to finish in every launch
 // that fits the GPU: one 512 x 512 world 8.9 -> 7.1 us a generation, 1024 x 1024 13.8 -> 10.7, 2048 x 1024 20.2 -> 16.0.
-template <int H, int NT, bool CG, int MR>
+template <int H, int NT, bool CG, int MR, int NC>
 __device__ __forceinline__ void col_chained(float2* X, const float2* stw, const float2* __restrict__ src,
                                             float2* __restrict__ dst, const float* ksm, const float* __restrict__ khn,
-                                            bool early) {
+                                            int c0, bool early) {
     constexpr bool TWO = is_two_stage(H, MR);
     // radix of the stages at the tile (first of the forward transform, last of the inverse) and in the middle
     constexpr int RT = TWO ? two_stage(H, MR).ra : plan_radix(H, 0, MR), RM = chain_radix<H, MR>();
     constexpr int NT0 = H / RT, NM = H / RM, LAST = plan_len(H, MR) - 1, CS = col_stride(H);
     constexpr int HQC = khat_cols_stride<H>();
-    static_assert(TC == 2 && fusable<H, MR>() && TC * NT0 <= NT && TC * NM <= NT, "one outer butterfly per thread, two columns");
-    const int c = threadIdx.x & 1, j = threadIdx.x >> 1;
-    const bool tile = TC * NT0 == NT || threadIdx.x < TC * NT0, mid = TC * NM == NT || threadIdx.x < TC * NM;
-    float2* Xc = X + c * CS;
+    static_assert(TC == 2 && fusable<H, MR>() && NC * NT0 <= NT && NC * NM <= NT, "one outer butterfly per thread and column");
+    const int c = c0 + threadIdx.x % NC, j = threadIdx.x / NC;
+    const bool tile = NC * NT0 == NT || threadIdx.x < NC * NT0, mid = NC * NM == NT || threadIdx.x < NC * NM;
+    float2* Xc = X + (threadIdx.x % NC) * CS;
     if (tile) {
         float2 v[RT];
         const uint64_t keep = hint::policy_keep();
 #pragma unroll
-        for (int m = 0; m < RT; m++) v[m] = hint::ld2c<CG>(src + threadIdx.x + TC * NT0 * m, keep);
+        for (int m = 0; m < RT; m++) v[m] = hint::ld2c<CG>(src + TC * j + c + TC * NT0 * m, keep);
         Dft<RT, false>::run(v);
         if constexpr (TWO) two_store<RT>(Xc, j, v);
         else stage_store<H, RT, 1>(Xc, j, v);
     }
     cp_async_wait_all();  // the khat columns
     __syncthreads();
-    if constexpr (!TWO) col_stages<H, NT, false, 1, LAST, MR>(X, stw);
+    if constexpr (!TWO) col_stages<H, NT, false, 1, LAST, MR, NC>(X, stw);
     float2 v[RM];
     if (mid) {
         chain_load<H, false, MR>(Xc, j, v, stw);
-        const float* kc = ksm + c * HQC;
+        const float* kc = ksm + (threadIdx.x % NC) * HQC;
         if (khn == nullptr || c == 1) {
 #pragma unroll
             for (int m = 0; m < RM; m++) {
@@ -779,27 +805,27 @@ __device__ __forceinline__ void col_chained(float2* X, const float2* stw, const 
     if (mid) chain_store<H, MR>(Xc, j, v);
     __syncthreads();
     if (!CG && early) grid_trigger();
-    if constexpr (!TWO) col_stages<H, NT, true, 1, LAST, MR>(X, stw);
+    if constexpr (!TWO) col_stages<H, NT, true, 1, LAST, MR, NC>(X, stw);
     if (tile) {
         float2 u[RT];
         if constexpr (TWO) two_load<H, RT, true>(Xc, j, u, stw);
         else stage_load<H, RT, NT0, true>(Xc, j, u, stw + stage_tw_offset(H, LAST, MR));
         const uint64_t keep = hint::policy_keep();
 #pragma unroll
-        for (int m = 0; m < RT; m++) hint::st2(dst + threadIdx.x + TC * NT0 * m, u[m], keep);
+        for (int m = 0; m < RT; m++) hint::st2(dst + TC * j + c + TC * NT0 * m, u[m], keep);
     }
 }
 
 // A tile's two khat columns (rows of HQ floats) into shared memory, khat_cols_stride apart: asynchronous
 // 16-byte copies where the rows allow it (khat_stride rows; the caller waits), else plain loads (lenia_step_noalloc's
 // callers pass rows of H/2 + 1).
-template <int H, int NT>
+template <int H, int NT, int NC = TC>
 __device__ __forceinline__ void copy_khat(float* ksm, const float* __restrict__ kh, int HQ) {
     constexpr int HQC = khat_cols_stride<H>();
     if (HQ == HQC && ((uintptr_t)kh & 15) == 0) {
-        for (int e = threadIdx.x; e < TC * HQC / 4; e += NT) cp_async16(ksm + 4 * e, kh + 4 * e);
+        for (int e = threadIdx.x; e < NC * HQC / 4; e += NT) cp_async16(ksm + 4 * e, kh + 4 * e);
     } else {
-        for (int e = threadIdx.x; e < TC * (H / 2 + 1); e += NT) {
+        for (int e = threadIdx.x; e < NC * (H / 2 + 1); e += NT) {
             const int c = e / (H / 2 + 1), y = e - c * (H / 2 + 1);
             ksm[c * HQC + y] = kh[(size_t)c * HQ + y];
         }
@@ -811,8 +837,10 @@ __device__ __forceinline__ void copy_khat(float* ksm, const float* __restrict__ 
 // repeating the channel's forward column transform: that keeps every item on the chained path and
 // multiplies the items, which the multichannel world needs more than it needs the saved transforms.
 // CG: the tile loads bypass L1 (the persistent step, where another CTA of the same launch wrote them).
-template <int H, int NT, bool CG, int MR = CMR>
-__device__ __forceinline__ void col_item(const DevWorld& wd, const ColItem it, float2* X, float2* stw, bool early = false) {
+// NC: the columns of the tile this CTA takes, from c0 on.
+template <int H, int NT, bool CG, int MR = CMR, int NC = TC>
+__device__ __forceinline__ void col_item(const DevWorld& wd, const ColItem it, float2* X, float2* stw, int c0 = 0,
+                                         bool early = false) {
     const int W = wd.W, c = it.chan, t = it.tile, k = it.kernel, HQ = wd.HQ;
     const size_t cplane = (size_t)(W / 2) * H;
     const float2* src = wd.spec + c * cplane + (size_t)t * H * TC;
@@ -821,28 +849,28 @@ __device__ __forceinline__ void col_item(const DevWorld& wd, const ColItem it, f
     constexpr int HQC = khat_cols_stride<H>();
     const float* kh0 = wd.khat + (size_t)k * (W / 2 + 1) * HQ;
     float* ksm = col_khat_smem<H, MR>(stw);
-    copy_khat<H, NT>(ksm, kh0 + (size_t)TC * t * HQ, HQ);
+    copy_khat<H, NT, NC>(ksm, kh0 + (size_t)(TC * t + c0) * HQ, HQ);
     if constexpr (!CG) grid_wait();
     // the twiddle tables are read after col_chained's first barrier
-    col_chained<H, NT, CG, MR>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC, ksm,
-                               t == 0 ? kh0 + (size_t)(W / 2) * HQ : nullptr, early);
+    col_chained<H, NT, CG, MR, NC>(X, stw, src, wd.conv + k * cplane + (size_t)t * H * TC, ksm,
+                                   t == 0 ? kh0 + (size_t)(W / 2) * HQ : nullptr, c0, early);
 }
 
 // float2s of a column item's two sequences.
-template <int H>
-FFT_CHD constexpr int col_seq_floats2() { return TC * col_stride(H); }
+template <int H, int NC = TC>
+FFT_CHD constexpr int col_seq_floats2() { return NC * col_stride(H); }
 
 // MR: the radix cap of the build's plans (CMR; 16 for the radix-16 build of sizes whose CMR plan has
 // radix 32, launch variant 3)
-template <int H, int NT, int MINB, int MR = CMR>
+template <int H, int NT, int MINB, int MR = CMR, int NC = TC>
 __global__ void __launch_bounds__(NT, MINB) col_pass(const DevWorld* __restrict__ worlds, const ColItem* __restrict__ items,
                                                 const float2* __restrict__ tw, bool early) {
     extern __shared__ float4 smem_raw[];
     float2* X = reinterpret_cast<float2*>(smem_raw);
-    float2* stw = X + col_seq_floats2<H>();
-    const ColItem it = items[blockIdx.x];
+    float2* stw = X + col_seq_floats2<H, NC>();
+    const ColItem it = items[blockIdx.x / (TC / NC)];
     fill_tables<H, MR>(stw, tw, NT);
-    col_item<H, NT, false, MR>(worlds[it.world], it, X, stw, early);
+    col_item<H, NT, false, MR, NC>(worlds[it.world], it, X, stw, NC * (blockIdx.x % (TC / NC)), early);
 }
 
 // ------------------------------------------------------------------ paired column pass
@@ -851,7 +879,7 @@ __global__ void __launch_bounds__(NT, MINB) col_pass(const DevWorld* __restrict_
 // 16-byte shared-memory accesses, so the item needs half the threads and about half the
 // instructions of the scalar build.  Shared memory: the sequence, the tw2 stage tables, the khat
 // columns.
-constexpr int PMR = max_radix<cpair>();  // largest radix of the paired builds' plans
+constexpr int PMR = ROW_PLAN;  // largest radix of the paired builds' plans
 template <int H>
 __device__ __forceinline__ float* col_khat_smem_pair(tw2* stw) {
     constexpr int TWS = tw_table_size(H, PMR);
@@ -936,7 +964,7 @@ __global__ void __launch_bounds__(NT, MINB) col_pass_pair(const DevWorld* __rest
     tw2* stw = reinterpret_cast<tw2*>(X + seq_stride(H));
     const ColItem it = items[blockIdx.x];
     const DevWorld& wd = worlds[it.world];
-    fill_stage_twiddles<H>(stw, tw, threadIdx.x, NT);
+    fill_stage_twiddles<H, tw2, 0, PMR>(stw, tw, threadIdx.x, NT);
     const int W = wd.W, c = it.chan, t = it.tile, k = it.kernel, HQ = wd.HQ;
     const size_t cplane = (size_t)(W / 2) * H;
     const float2* src = wd.spec + c * cplane + (size_t)t * H * TC;
@@ -958,8 +986,7 @@ template <int N, int MR = CMR> constexpr int nt_of() {
     constexpr int n = (2 * (is_two_stage(N, MR) ? two_tw_len(N) : N / plan_radix(N, 0, MR)) + 31) / 32 * 32;
     return n > 1024 ? 1024 : n;
 }
-// whether the scalar column build's plan has radix 32 (1024, 3072, 8192): those sizes also build the
-// radix-16 plan (launch variant 3)
+// whether the scalar column build's plan has radix 32 (1024, 8192)
 template <int N> constexpr bool col_r32() { return plan_radix(N, 0, CMR) == 32; }
 // variant 0: at most 64 registers per thread (80 for radix-32 plans: the 1024 build spilled 508 B at
 // 64 and needs none at 80); variant 1: at most 128
@@ -979,17 +1006,17 @@ template <int N> constexpr int minb_pair_of() { return 512 / nt_pair_of<N>() < 1
 
 // Launch one instantiation.  Dynamic shared memory above 48 KB must be enabled per kernel before
 // its first launch and before any stream capture that contains it; a zero-item call does just that.
-template <int H, int NT, int MINB, int MR = CMR>
+template <int H, int NT, int MINB, int MR = CMR, int NC = TC>
 bool col_go(const DevWorld* worlds, const ColItem* items, int nitems, const float2* tw, LaunchOn s) {
-    const size_t smem = col_seq_floats2<H>() * sizeof(float2) + stage_table_bytes<H, MR>() + col_khat_bytes<H>();
+    const size_t smem = col_seq_floats2<H, NC>() * sizeof(float2) + stage_table_bytes<H, MR>() + col_khat_bytes<H>() / (TC / NC) + 16;
     static int attr_max = 0;
     if ((int)smem > attr_max) {
-        if (cudaFuncSetAttribute(col_pass<H, NT, MINB, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        if (cudaFuncSetAttribute(col_pass<H, NT, MINB, MR, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
             cudaSuccess)
             return false;
         attr_max = (int)smem;
     }
-    return nitems <= 0 || launch_pass(col_pass<H, NT, MINB, MR>, nitems, NT, smem, s, worlds, items, tw, s.early);
+    return nitems <= 0 || launch_pass(col_pass<H, NT, MINB, MR, NC>, nitems * (TC / NC), NT, smem, s, worlds, items, tw, s.early);
 }
 
 template <int H>
@@ -1019,30 +1046,35 @@ constexpr size_t row_smem(int general, int planes) {
            (size_t)(general ? planes : 0) * rows * W * sizeof(float);
 }
 
-template <int W, int NT, int MINB, bool GEN>
+template <int W, int NT, int MINB, bool GEN, bool WIDE>
 bool row_go(int mode, int general, int planes, const DevWorld* worlds, const RowItem* items, int nitems,
             const float2* tw, LaunchOn s) {
     const size_t smem = row_smem<W, GEN>(general, planes);
     static int attr_max = 0;
     if ((int)smem > attr_max) {
-        if (cudaFuncSetAttribute(row_pass<W, NT, MINB, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        if (cudaFuncSetAttribute(row_pass<W, NT, MINB, GEN, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
             cudaSuccess)
             return false;
         attr_max = (int)smem;
     }
-    return nitems <= 0 || launch_pass(row_pass<W, NT, MINB, GEN>, nitems, NT, smem, s, worlds, items, mode, general, tw, s.early);
+    return nitems <= 0 || launch_pass(row_pass<W, NT, MINB, GEN, WIDE>, nitems, NT, smem, s, worlds, items, mode, general, tw, s.early);
 }
 
 // Column-pass builds: variant 0 and 1 are the scalar build at 64 (80 with a radix-32 plan) and 128
 // registers a thread, variant 2 the paired build, variant 3 the scalar build with the radix-16 plan at
-// 64 registers where the scalar plan has radix 32 (elsewhere variant 0).
+// 64 registers where the scalar plan has radix 32 and the sides are below 2048, from 2048 up the
+// scalar build with one column a CTA (elsewhere variant 0).
 template <int N>
 bool col_go_variant(int variant, const DevWorld* worlds, const ColItem* items, int nitems, const float2* tw,
                     LaunchOn s) {
     if (variant == 2) return col_go_pair<N, nt_pair_of<N>(), minb_pair_of<N>()>(worlds, items, nitems, tw, s);
     if (variant == 1) return col_go<N, nt_of<N>(), minb_of<N, 1>()>(worlds, items, nitems, tw, s);
-    if constexpr (col_r32<N>())
+    if constexpr (N >= 2048) {
+        if (variant == 3)
+            return col_go<N, nt_of<N>() / TC, minb_threads<N, N == 8192>() / (nt_of<N>() / TC), CMR, 1>(worlds, items, nitems, tw, s);
+    } else if constexpr (col_r32<N>()) {
         if (variant == 3) return col_go<N, nt_of<N, 16>(), minb_of<N, 0, 16>(), 16>(worlds, items, nitems, tw, s);
+    }
     return col_go<N, nt_of<N>(), minb_of<N, 0>()>(worlds, items, nitems, tw, s);
 }
 #define LENIA_COL_CASE(N) \
@@ -1056,8 +1088,8 @@ bool col_go_variant(int variant, const DevWorld* worlds, const ColItem* items, i
 #define LENIA_ROW_CASE_G(N, G)                                                                                   \
     case N:                                                                                                      \
         return (variant & 1)                                                                                     \
-                   ? row_go<N, row_nt<N, G>(), row_minb<N, 1, G>(), G>(mode, general, planes, worlds, items, nitems, tw, s) \
-                   : row_go<N, row_nt<N, G>(), row_minb<N, 0, G>(), G>(mode, general, planes, worlds, items, nitems, tw, s);
+                   ? row_go<N, row_nt<N, G>(), row_minb<N, 1, G>(), G, row_wide<N, 1>()>(mode, general, planes, worlds, items, nitems, tw, s) \
+                   : row_go<N, row_nt<N, G>(), row_minb<N, 0, G>(), G, row_wide<N, 0>()>(mode, general, planes, worlds, items, nitems, tw, s);
 #define LENIA_ROW_CASE_SIMPLE(N) LENIA_ROW_CASE_G(N, false)
 #define LENIA_ROW_CASE_GENERAL(N) LENIA_ROW_CASE_G(N, true)
 
