@@ -157,8 +157,12 @@ struct LeniaCtx {
     char* arena = nullptr;
     size_t arena_need = 0, arena_used = 0;
     bool sizing = false;
+    // lenia_step replays graph_big for every graph_steps generations; the rest are launched one by one where a
+    // generation is two launches (direct), else replayed from graph_mid (MID_STEPS) and graph_one
+    static constexpr int MID_STEPS = 8;
     int graph_steps = 64;
-    cudaGraphExec_t graph_big = nullptr, graph_one = nullptr;
+    bool direct = false;
+    cudaGraphExec_t graph_big = nullptr, graph_mid = nullptr, graph_one = nullptr;
     TcPlan tc;
     // Worlds whose state changed since their half-spectrum was last formed.  The forward row
     // transforms run at the next call that reads spectra (flush_spectra), one launch per size class
@@ -170,6 +174,7 @@ struct LeniaCtx {
     size_t states_count = 0;
     // device error flag of the cluster-resident step (1: a cluster sync gave up)
     int* d_flags = nullptr;
+    bool flags_used = false;  // a launch that may raise it has been enqueued (the others cannot)
 };
 
 namespace {
@@ -469,6 +474,7 @@ bool early_dependents(const LeniaCtx* ctx, const Chunk& ch) {
 // `steps` steps of one size class, chunk after chunk, in the given launch shape; a resident class is
 // one launch for all its worlds and steps.
 int enqueue_class(LeniaCtx* ctx, const SizeClass& cl, const Shape& sh, int steps, cudaStream_t s) {
+    if (cl.persist || cl.resident) ctx->flags_used = true;
     if (cl.persist) {
         const int nw = (int)cl.worlds.size();
         CK(cudaMemsetAsync(cl.d_pctl, 0, persist_ctl_words(nw) * sizeof(int), s));
@@ -609,11 +615,20 @@ int capture(LeniaCtx* ctx, int steps, cudaGraphExec_t* out) {
 }
 
 int rebuild_graphs(LeniaCtx* ctx) {
-    if (ctx->graph_big) cudaGraphExecDestroy(ctx->graph_big);
-    if (ctx->graph_one) cudaGraphExecDestroy(ctx->graph_one);
-    ctx->graph_big = ctx->graph_one = nullptr;
+    for (cudaGraphExec_t* g : {&ctx->graph_big, &ctx->graph_mid, &ctx->graph_one}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
+    // One class in one chunk of FP32 passes is two launches a generation, which overlap one by one as they do in a graph
+    // where a replay a generation cannot: 20 generations of one 256 x 256 world 8.2 -> 5.8 us each, of 64 x 64 6.2 ->
+    // 3.8.  More launches a generation are replayed, eight generations at a time where that many are left, so that a
+    // chunk finds its last generation in L2 (36 generations of 1024 worlds of 256 x 256: 263 -> 231 us each, of
+    // the 384-world batch 530 -> 477).
+    const SizeClass* one = ctx->classes.size() == 1 ? &ctx->classes[0] : nullptr;
+    ctx->direct = one && one->chunks.size() == 1 && one->ntcg == 0 && !one->tc_rows && !one->resident && !one->persist;
     int rc = capture(ctx, ctx->graph_steps, &ctx->graph_big);
-    if (!rc) rc = capture(ctx, 1, &ctx->graph_one);
+    if (!rc && !ctx->direct && ctx->path != LENIA_PATH_RADIX2) rc = capture(ctx, LeniaCtx::MID_STEPS, &ctx->graph_mid);
+    if (!rc && !ctx->direct) rc = capture(ctx, 1, &ctx->graph_one);
     return rc;
 }
 
@@ -1059,7 +1074,7 @@ int time_class_graph(LeniaCtx* ctx, const SizeClass& cl, const Shape& sh, int st
 // step's (set when a bounded barrier wait gave up).  Reading them synchronises with the device.
 int check_device_errors(LeniaCtx* ctx) {
     int rc = tc_check_error(ctx->tc, &ctx->err);
-    if (rc || !ctx->d_flags) return rc;
+    if (rc || !ctx->flags_used) return rc;
     int h = 0;
     CK(cudaMemcpy(&h, ctx->d_flags, sizeof(int), cudaMemcpyDeviceToHost));
     if (h) {
@@ -1192,8 +1207,8 @@ int lenia_destroy(LeniaCtx* ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->up) cudaStreamSynchronize(ctx->up);
     if (ctx->down) cudaStreamSynchronize(ctx->down);
-    if (ctx->graph_big) cudaGraphExecDestroy(ctx->graph_big);
-    if (ctx->graph_one) cudaGraphExecDestroy(ctx->graph_one);
+    for (cudaGraphExec_t g : {ctx->graph_big, ctx->graph_mid, ctx->graph_one})
+        if (g) cudaGraphExecDestroy(g);
     tc_release(ctx->tc);
     for (void* p : ctx->allocs) cudaFree(p);
     for (cudaEvent_t e : {ctx->ev_in_ready, ctx->ev_in_free, ctx->ev_out_ready, ctx->ev_out_free})
@@ -1340,7 +1355,14 @@ int lenia_step(LeniaCtx* ctx, uint32_t steps) {
     if (frc) return frc;
     uint32_t full = steps / ctx->graph_steps, rem = steps % ctx->graph_steps;
     for (uint32_t i = 0; i < full; i++) CK(cudaGraphLaunch(ctx->graph_big, ctx->stream));
-    for (uint32_t i = 0; i < rem; i++) CK(cudaGraphLaunch(ctx->graph_one, ctx->stream));
+    if (ctx->direct && rem > 0) {
+        int rc = enqueue_steps(ctx, (int)rem);
+        if (rc) return rc;
+        rem = 0;
+    }
+    for (; ctx->graph_mid && rem >= LeniaCtx::MID_STEPS; rem -= LeniaCtx::MID_STEPS)
+        CK(cudaGraphLaunch(ctx->graph_mid, ctx->stream));
+    for (; rem > 0; rem--) CK(cudaGraphLaunch(ctx->graph_one, ctx->stream));
     ctx->tick += steps;
     return 0;
 }
@@ -1364,8 +1386,8 @@ int lenia_step_timed(LeniaCtx* ctx, uint32_t steps, float* ms) {
 int lenia_sync(LeniaCtx* ctx) {
     if (!ctx) return LENIA_EINVAL;
     CK(cudaStreamSynchronize(ctx->stream));
-    CK(cudaStreamSynchronize(ctx->up));
-    CK(cudaStreamSynchronize(ctx->down));
+    if (ctx->stage_in) CK(cudaStreamSynchronize(ctx->up));
+    if (ctx->stage_out) CK(cudaStreamSynchronize(ctx->down));
     int rc = check_device_errors(ctx);
     return rc;
 }

@@ -439,7 +439,7 @@ struct LeniaMlp {
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // FP32 master, grads, Adam moments
     bf16* wb = nullptr;                                             // BF16 copy of the parameters
     float *x = nullptr, *y = nullptr, *loss = nullptr;  // a batch: inputs, labels, per-row losses
-    int* err = nullptr;  // set by a tile that gave up waiting on a barrier
+    int* err = nullptr;  // set by a tile that gave up waiting on a barrier; the losses follow it (one copy for both)
     // ranking: two halves of PREDICT_ROWS rows of inputs and probabilities, each on a stream of its own
     cudaStream_t ps[2] = {};
     float *px = nullptr, *pp = nullptr;
@@ -494,13 +494,18 @@ int upload_batch(LeniaMlp* n, const float* x, const float* y, uint32_t B) {
     return 0;
 }
 
-float mean_loss(LeniaMlp* n, uint32_t B) {
-    std::vector<float> l(B);
-    cudaMemcpyAsync(l.data(), n->loss, B * 4, cudaMemcpyDeviceToHost, n->stream);
-    cudaStreamSynchronize(n->stream);
+// Waits for the batch; its mean loss, and the error flag that travels with the losses.
+int mean_loss(LeniaMlp* n, uint32_t B, float* loss) {
+    std::vector<float> l((size_t)B + 1);
+    if (cudaMemcpyAsync(l.data(), n->err, ((size_t)B + 1) * 4, cudaMemcpyDeviceToHost, n->stream) != cudaSuccess ||
+        cudaStreamSynchronize(n->stream) != cudaSuccess)
+        return err("mlp: download failed");
     double s = 0;
-    for (float v : l) s += v;
-    return (float)(s / B);
+    for (uint32_t i = 1; i <= B; i++) s += l[i];
+    if (loss) *loss = (float)(s / B);
+    int flag;
+    memcpy(&flag, l.data(), sizeof(flag));
+    return flag ? check_err(n) : 0;
 }
 
 }  // namespace
@@ -525,13 +530,14 @@ LENIA_API int lenia_mlp_create(uint32_t seed, uint32_t max_batch, LeniaMlp** out
               cudaStreamCreateWithFlags(&n->ps[0], cudaStreamNonBlocking) == cudaSuccess &&
               cudaStreamCreateWithFlags(&n->ps[1], cudaStreamNonBlocking) == cudaSuccess && mal(n, &n->w, NPARAM) &&
               mal(n, &n->g, NPARAM) && mal(n, &n->m, NPARAM) && mal(n, &n->v, NPARAM) && mal(n, &n->wb, NPARAM) &&
-              mal(n, &n->x, B * IN) && mal(n, &n->y, B * OUT) && mal(n, &n->loss, B) && mal(n, &n->err, 1) &&
+              mal(n, &n->x, B * IN) && mal(n, &n->y, B * OUT) && mal(n, &n->err, B + 1) &&
               mal(n, &n->px, (size_t)PREDICT_ROWS * IN) && mal(n, &n->pp, (size_t)PREDICT_ROWS * OUT);
     if (!ok) {
         lenia_mlp_destroy(n);
         set_thread_error("mlp: device allocation failed");
         return LENIA_ENOMEM;
     }
+    n->loss = reinterpret_cast<float*>(n->err + 1);
     // He-uniform initialisation from the PCG hash, biases zero
     std::vector<float> w(NPARAM, 0.f);
     auto pcg = [](uint32_t v) {
@@ -615,10 +621,7 @@ LENIA_API int lenia_mlp_gradients(LeniaMlp* n, const float* x, const float* y, u
     gradients(n, (int)batch);
     if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
     cudaMemcpyAsync(grads, n->g, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream);
-    const float l = mean_loss(n, batch);
-    if (loss) *loss = l;
-    if (cudaGetLastError() != cudaSuccess) return err("mlp: gradients failed");
-    return check_err(n);
+    return mean_loss(n, batch, loss);
 }
 
 LENIA_API int lenia_mlp_train_step(LeniaMlp* n, const float* x, const float* y, uint32_t batch, float lr, float* loss) {
@@ -633,9 +636,7 @@ LENIA_API int lenia_mlp_train_step(LeniaMlp* n, const float* x, const float* y, 
     const float c1 = 1.f - std::pow(b1, (float)n->t), c2 = 1.f - std::pow(b2, (float)n->t);
     adam<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->w, n->g, n->m, n->v, n->wb, NPARAM, lr, b1, b2, 1e-8f, c1, c2);
     if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
-    const float l = mean_loss(n, batch);
-    if (loss) *loss = l;
-    return check_err(n);
+    return mean_loss(n, batch, loss);
 }
 
 LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, float* probs) {

@@ -1,6 +1,6 @@
-"""Overlapped launches of the step (programmatic dependent launches in the step graph) against the same
-passes launched one after another (lenia_profile_step): the arithmetic is the same, so the states
-must be equal bit for bit."""
+"""Overlapped launches of the step (programmatic dependent launches, in the step graphs or one by one)
+against the same passes launched one after another (lenia_profile_step): the arithmetic is the same, so
+the states must be equal bit for bit."""
 import numpy as np
 import pytest
 
@@ -32,7 +32,7 @@ def test_overlapped_step_gives_the_bits_of_separate_launches(worlds):
     got = []
     for overlapped in (True, False):
         with ag.Sim(made, seed=3) as sim:
-            for steps in (70, 3):  # a whole graph, then single steps
+            for steps in (75, 3):  # a whole graph, eight generations and single ones (or direct launches), then single ones
                 sim.step(steps) if overlapped else sim.profile(steps)
             got.append(sim.read_states())
     assert np.array_equal(got[0], got[1])
