@@ -632,6 +632,24 @@ int rebuild_graphs(LeniaCtx* ctx) {
     return rc;
 }
 
+// The default branch split of the step graph (lenia_set_branch_split).  While all classes together fit L2, no
+// class's launches fill the GPU, and every class but the largest gets a branch of its own: the first 8, 24 and 48
+// worlds of the batched workload (10, 61, 120 MB) take 22, 34 and 74 us a generation against 46, 71 and 99 one class
+// after another, on the BF16x3 path 29, 45 and 91 against 61, 94 and 139.  Up to twice that the classes of at most 384 x
+// 384 go on one side branch (96 worlds, 245 MB: 139 against 146 us).  Beyond, the large classes' chunks fill the GPU and a
+// side branch only takes L2 from them (192 worlds 239 against 249 us, 384 worlds 465 against 537).
+void default_branches(LeniaCtx* ctx) {
+    size_t bytes = 0;
+    int64_t largest = 0;
+    for (const SizeClass& cl : ctx->classes) {
+        bytes += cl.bytes;
+        largest = std::max(largest, (int64_t)cl.W * cl.H);
+    }
+    if (ctx->classes.size() < 2 || bytes > (256u << 20)) return;
+    ctx->branch_each = bytes <= (128u << 20);
+    ctx->branch_cells = ctx->branch_each ? largest - 1 : std::min<int64_t>(largest - 1, 384 * 384);
+}
+
 int setup_fused(LeniaCtx* ctx) {
     const int nw = (int)ctx->desc.size();
     ctx->hw.resize(nw);
@@ -911,6 +929,7 @@ int setup_fused(LeniaCtx* ctx) {
             !launch_row_tc(ctx->tc, ctx->path, cl.W, ctx->d_worlds, cl.d_row, cl.tc_row_stride, 0, ctx->d_tw, ctx->stream))
             return fail(ctx, LENIA_ECUDA, "cannot configure the tensor-core row pass for W=%d", cl.W);
     }
+    default_branches(ctx);
     return 0;
 }
 
