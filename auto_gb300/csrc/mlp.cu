@@ -36,8 +36,7 @@ constexpr int P_W1 = 0, P_B1 = P_W1 + HID * IN, P_W2 = P_B1 + HID, P_B2 = P_W2 +
 using bf16 = __nv_bfloat16;
 
 // ------------------------------------------------------------------ the network on a tile of rows
-// One CTA takes 128 rows through the whole network: forward to the logits and, with GRAD, back to every
-// gradient.  Nothing but the inputs, the weights and the results touches global memory.
+// One CTA takes 128 rows through the whole network, forward to the logits and back to every gradient.  Nothing but the inputs, the weights and the results touches global memory.
 //
 // All operands sit in shared memory in the canonical layout without swizzle (8-row x 16-byte core
 // matrices, K-adjacent ones 128 bytes apart, 8-row groups one after another: tc::kmajor_offset).  A
@@ -56,27 +55,25 @@ using bf16 = __nv_bfloat16;
 //   dW1   += dh1^T x                      A dh1 (MN-major)  B x (MN-major)   M = 2 x 128, N = 16,  K = 128 rows
 //
 // The bias gradients are column sums of the unrounded FP32 dh2 and dh1 (transposed by shuffles), dW3
-// of dz h2; weight gradients of several tiles meet in global memory with vector reductions.  256
-// threads: warp w reads TMEM lanes 32 (w % 4) .. + 31 (the tile's rows) and columns 128 (w / 4) .. + 127.
+// of dz h2; weight gradients of several tiles meet in global memory with vector reductions.  512
+// threads: warp w reads TMEM lanes 32 (w % 4) .. + 31 (the tile's rows) and columns 64 (w / 4) .. + 63.
 //
 // W2 takes R0 and R1 (128 KB); the backward pass needs R1 for dh2 and fetches W2's rows 128..255
-// again into R0.  One CTA per SM (214 KB of shared memory, all 512 TMEM columns).  A tile is a chain of
-// two (five) waits on the tensor cores with a hand-over after each, so it is bound by that latency: 71
-// tiles forward take 14 us (W2's load included), 8 tiles forward and back 40 us.  As separate GEMM
-// launches, whose hand-overs wrote h1 and h2 (and their transposes) to global memory with 2-byte stores
-// one row stride apart per lane, a 4096-row chunk took 155 us forward and 1000 rows 520 us forward and
-// back: lenia_mlp_predict of 250001 rows went from 11.1 to 0.39 ms, lenia_mlp_gradients of 1000 from 560
-// to 98 us (the rest is copies and synchronisation).
+// again into R0.  One CTA per SM (224 KB of shared memory, all 512 TMEM columns).  A tile is a chain of
+// five waits on the tensor cores with a hand-over after each, so it is bound by that latency, and a batch of
+// 1000 rows by one tile's: with a thread for every 64 columns of a row instead of every 128,
+// lenia_mlp_gradients of 1000 rows went from 77 to 66 us.  As separate GEMM launches, whose hand-overs wrote
+// h1 and h2 (and their transposes) to global memory with 2-byte stores one row stride apart per lane, it took 560.
 //
 // Every barrier wait is bounded; a CTA that gives up waits (bounded) for its MMAs and copies, raises *err,
 // frees its TMEM and returns.
-constexpr int TILE = 128, NTHR = 256;
+constexpr int TILE = 128, NTHR = 512, NCOL = TILE * HID / NTHR;  // columns of a row per thread
 constexpr uint32_t GROUP = HID * 2 * 8;    // bytes of eight 256-wide rows
 constexpr uint32_t XGROUP = IN * 2 * 8;    // bytes of eight 16-wide rows
 constexpr uint32_t REGION = TILE * HID * 2;  // 64 KB
 constexpr uint32_t S_W1 = 3 * REGION, S_X = S_W1 + HID * IN * 2, S_F = S_X + TILE * IN * 2;
-// floats from S_F: b1, b2, W3, the second column half's logits (then dz), and the sums db2, db1, dW3, db3
-constexpr int F_B1 = 0, F_B2 = F_B1 + HID, F_W3 = F_B2 + HID, F_Z = F_W3 + OUT * HID, F_DB2 = F_Z + TILE * OUT,
+// floats from S_F: b1, b2, W3, the other column quarters' logits (then dz), and the sums db2, db1, dW3, db3
+constexpr int F_B1 = 0, F_B2 = F_B1 + HID, F_W3 = F_B2 + HID, F_Z = F_W3 + OUT * HID, F_DB2 = F_Z + (HID / NCOL - 1) * TILE * OUT,
               F_DB1 = F_DB2 + HID, F_DW3 = F_DB1 + HID, F_DB3 = F_DW3 + OUT * HID, F_END = F_DB3 + 4;
 constexpr uint32_t S_BAR = S_F + F_END * 4;
 constexpr uint32_t TILE_SMEM = S_BAR + 16;
@@ -114,25 +111,24 @@ __device__ __forceinline__ float column_sums(float* v) {
 
 // rows [first, first + n) of W2 (bf16 [256][256]) into an operand region, n a multiple of 8: eight rows of
 // one 16-byte column piece per eight lanes, 128 contiguous bytes of shared memory
+template <int NT = NTHR>
 __device__ __forceinline__ void load_w2(uint8_t* dst, const bf16* __restrict__ w2, int first, int n) {
-    for (int e = threadIdx.x; e < n * (HID / 8); e += NTHR) {
+    for (int e = threadIdx.x; e < n * (HID / 8); e += NT) {
         const int r = (e >> 8) * 8 + (e & 7), kg = (e >> 3) & 31;
         cp_async16(dst + tc::kmajor_offset(r, 8 * kg, HID, 2), w2 + (size_t)(first + r) * HID + 8 * kg);
     }
 }
 
-template <bool GRAD>
 __global__ void __launch_bounds__(NTHR, 1)
     mlp_tile(const float* __restrict__ x, const float* __restrict__ y, int B, const float* __restrict__ w,
-             const bf16* __restrict__ wb, float* __restrict__ probs, float* __restrict__ g,
-             float* __restrict__ loss_rows, int* __restrict__ err) {
+             const bf16* __restrict__ wb, float* __restrict__ g, float* __restrict__ loss_rows, int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t sm[];
     uint8_t *R0 = sm, *R1 = sm + REGION, *R2 = sm + 2 * REGION, *W1s = sm + S_W1, *Xs = sm + S_X;
     float* F = reinterpret_cast<float*>(sm + S_F);
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + S_BAR);
     uint32_t* slot = reinterpret_cast<uint32_t*>(bar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int row = (warp & 3) * 32 + lane, half = warp >> 2;  // this thread's tile row and column half
+    const int row = (warp & 3) * 32 + lane, part = warp >> 2;  // this thread's tile row and column quarter
     const int ntiles = (B + TILE - 1) / TILE;
     const bf16* w2 = wb + P_W2;
 
@@ -143,8 +139,7 @@ __global__ void __launch_bounds__(NTHR, 1)
     asm volatile("cp.async.commit_group;" ::: "memory");
     for (int e = tid; e < HID; e += NTHR) F[F_B1 + e] = w[P_B1 + e], F[F_B2 + e] = w[P_B2 + e];
     for (int e = tid; e < OUT * HID; e += NTHR) F[F_W3 + e] = __bfloat162float(wb[P_W3 + e]);
-    if (GRAD)
-        for (int e = F_DB2 + tid; e < F_END; e += NTHR) F[e] = 0.f;
+    for (int e = F_DB2 + tid; e < F_END; e += NTHR) F[e] = 0.f;
     if (tid == 0) {
         tc::mbar_init(bar, 1);
         tc::fence_barrier_init();
@@ -180,12 +175,13 @@ __global__ void __launch_bounds__(NTHR, 1)
         tc::tc_fence_after();
     };
 
-    // this thread's eight inputs of a tile: row tid / 2, half a row each
+    // eight inputs of a tile for each of the first 256 threads: row tid / 2, half a row each
     float xin[8];
+    const bool loads = tid < 2 * TILE;
     auto fetch = [&](int t) {
         const int r = t * TILE + (tid >> 1);
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-        if (r < B) {
+        if (loads && r < B) {
             const float4* p = reinterpret_cast<const float4*>(x + (size_t)r * IN + 8 * (tid & 1));
             a = p[0], b = p[1];
         }
@@ -194,8 +190,8 @@ __global__ void __launch_bounds__(NTHR, 1)
     bool ok = true, first = true;
     fetch(blockIdx.x);
     for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, first = false) {
-        if (GRAD && !first) load_w2(R0, w2, 0, HID);  // the backward pass of the last tile took its place
-        *reinterpret_cast<uint4*>(Xs + tc::kmajor_offset(tid >> 1, 8 * (tid & 1), IN, 2)) = pack8(xin);
+        if (!first) load_w2(R0, w2, 0, HID);  // the backward pass of the last tile took its place
+        if (loads) *reinterpret_cast<uint4*>(Xs + tc::kmajor_offset(tid >> 1, 8 * (tid & 1), IN, 2)) = pack8(xin);
         if (first) asm volatile("cp.async.wait_group 1;" ::: "memory");  // W1
         publish();
         if (tid == 0) {
@@ -208,9 +204,13 @@ __global__ void __launch_bounds__(NTHR, 1)
         // rows past the batch are zeros in every product (a row that is not there meets no infinite weight)
         const int b = t * TILE + row;
         const bool valid = b < B;
+        float yy[OUT] = {0.f, 0.f, 0.f};  // labels, wanted after the second layer
+        if (part == 0 && valid)
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int n0 = half * 128 + 32 * c;
+            for (int o = 0; o < OUT; o++) yy[o] = y[(size_t)b * OUT + o];
+#pragma unroll
+        for (int c = 0; c < NCOL / 32; c++) {
+            const int n0 = part * NCOL + 32 * c;
             float v[32];
             tc::tmem_ld32(mine + n0, v);
 #pragma unroll
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(NTHR, 1)
             for (int i = 0; i < 4; i++)
                 *reinterpret_cast<uint4*>(R2 + tc::kmajor_offset(row, n0 + 8 * i, HID, 2)) = pack8(v + 8 * i);
         }
-        if (GRAD || first) cp_async_wait0();  // W2
+        cp_async_wait0();  // W2
         publish();
         if (tid == 0) {
             for (uint32_t s = 0; s < HID / 16; s++)
@@ -231,8 +231,8 @@ __global__ void __launch_bounds__(NTHR, 1)
         if (!(ok = wait())) break;
         float z[OUT] = {0.f, 0.f, 0.f};
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int n0 = half * 128 + 32 * c;
+        for (int c = 0; c < NCOL / 32; c++) {
+            const int n0 = part * NCOL + 32 * c;
             float v[32];
             tc::tmem_ld32(mine + HID + n0, v);
 #pragma unroll
@@ -242,43 +242,36 @@ __global__ void __launch_bounds__(NTHR, 1)
                 for (int o = 0; o < OUT; o++) z[o] = fmaf(h, F[F_W3 + o * HID + n0 + i], z[o]);
             }
         }
-        if (half == 1)
-            for (int o = 0; o < OUT; o++) F[F_Z + row * OUT + o] = z[o];
+        if (part > 0)
+            for (int o = 0; o < OUT; o++) F[F_Z + ((part - 1) * TILE + row) * OUT + o] = z[o];
         tc::tc_fence_before();
         __syncthreads();
         tc::tc_fence_after();
-        if (half == 0) {
+        if (part == 0) {
             float l = 0.f, dz[OUT];
 #pragma unroll
             for (int o = 0; o < OUT; o++) {
-                const float zz = z[o] + F[F_Z + row * OUT + o] + w[P_B3 + o];
+                float zz = z[o];
+                for (int q = 0; q < HID / NCOL - 1; q++) zz += F[F_Z + (q * TILE + row) * OUT + o];
+                zz += w[P_B3 + o];
                 const float p = 1.f / (1.f + expf(-zz));
-                if (!GRAD) {
-                    if (valid) probs[(size_t)b * OUT + o] = p;
-                } else {
-                    const float yy = valid ? y[(size_t)b * OUT + o] : 0.f;
-                    l += fmaxf(zz, 0.f) - zz * yy + log1pf(expf(-fabsf(zz)));
-                    dz[o] = valid ? (p - yy) / (float)(B * OUT) : 0.f;
-                    F[F_Z + row * OUT + o] = __bfloat162float(__float2bfloat16_rn(dz[o]));
-                }
+                l += fmaxf(zz, 0.f) - zz * yy[o] + log1pf(expf(-fabsf(zz)));
+                dz[o] = valid ? (p - yy[o]) / (float)(B * OUT) : 0.f;
+                F[F_Z + row * OUT + o] = __bfloat162float(__float2bfloat16_rn(dz[o]));
             }
-            if (GRAD) {
-                if (valid) loss_rows[b] = l / OUT;
+            if (valid) loss_rows[b] = l / OUT;
 #pragma unroll
-                for (int o = 0; o < OUT; o++) {
-                    for (int d = 16; d > 0; d >>= 1) dz[o] += __shfl_xor_sync(0xffffffffu, dz[o], d);
-                    if (lane == 0) atomicAdd(&F[F_DB3 + o], dz[o]);
-                }
+            for (int o = 0; o < OUT; o++) {
+                for (int d = 16; d > 0; d >>= 1) dz[o] += __shfl_xor_sync(0xffffffffu, dz[o], d);
+                if (lane == 0) atomicAdd(&F[F_DB3 + o], dz[o]);
             }
         }
-        if (!GRAD) continue;
-
         __syncthreads();
         float dzb[OUT];
         for (int o = 0; o < OUT; o++) dzb[o] = F[F_Z + row * OUT + o];
 #pragma unroll 1
-        for (int c = 0; c < 4; c++) {
-            const int n0 = half * 128 + 32 * c;
+        for (int c = 0; c < NCOL / 32; c++) {
+            const int n0 = part * NCOL + 32 * c;
             float v[32], q[32];
             tc::tmem_ld32(mine + HID + n0, v);
 #pragma unroll
@@ -326,8 +319,8 @@ __global__ void __launch_bounds__(NTHR, 1)
         pending = true;
         if (!(ok = wait())) break;
 #pragma unroll 1
-        for (int c = 0; c < 4; c++) {
-            const int n0 = half * 128 + 32 * c;
+        for (int c = 0; c < NCOL / 32; c++) {
+            const int n0 = part * NCOL + 32 * c;
             float v[32];
             tc::tmem_ld32(mine + n0, v);
 #pragma unroll
@@ -352,8 +345,8 @@ __global__ void __launch_bounds__(NTHR, 1)
         pending = true;
         auto add_dw2 = [&](uint32_t col0, int out0) {
 #pragma unroll 1
-            for (int c = 0; c < 4; c++) {
-                const int n0 = half * 128 + 32 * c;
+            for (int c = 0; c < NCOL / 32; c++) {
+                const int n0 = part * NCOL + 32 * c;
                 float v[32];
                 tc::tmem_ld32(mine + col0 + n0, v);
                 float* p = g + P_W2 + (size_t)(out0 + row) * HID + n0;
@@ -374,10 +367,10 @@ __global__ void __launch_bounds__(NTHR, 1)
         pending = true;
         add_dw2(0, 0);
         if (!(ok = wait())) break;
-        {
-            float v[16];  // column half h: units 128 h + row
-            tc::tmem_ld16(mine + HID + IN * half, v);
-            float* p = g + P_W1 + (size_t)(128 * half + row) * IN;
+        if (part < 2) {
+            float v[16];  // part p: units 128 p + row
+            tc::tmem_ld16(mine + HID + IN * part, v);
+            float* p = g + P_W1 + (size_t)(128 * part + row) * IN;
 #pragma unroll
             for (int i = 0; i < 16; i += 4) red_add4(p + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
         }
@@ -387,7 +380,7 @@ __global__ void __launch_bounds__(NTHR, 1)
     }
     cp_async_wait0();
     __syncthreads();
-    if (GRAD && ok && (int)blockIdx.x < ntiles) {
+    if (ok && (int)blockIdx.x < ntiles) {
         for (int e = tid; e < HID; e += NTHR) {
             atomicAdd(g + P_B2 + e, F[F_DB2 + e]);
             atomicAdd(g + P_B1 + e, F[F_DB1 + e]);
@@ -397,8 +390,161 @@ __global__ void __launch_bounds__(NTHR, 1)
     }
     if (!ok && tid == 0) {
         if (pending) tc::mbar_wait(bar, phase ^ 1);  // drain the commit that did not come in time, bounded
-        atomicExch(err, 1);
+        *(volatile int*)err = 1;
     }
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc::tc_fence_after();
+        tc::tmem_dealloc(tmem, 512);
+    }
+}
+
+// ------------------------------------------------------------------ ranking: the forward pass alone
+// The same tile and operands as mlp_tile, as a pipeline of two groups of eight warps.  Group A takes a tile through the
+// first layer (x W1^T, then h1 into R2) and issues the second layer's MMAs; group B takes the second layer's accumulator to
+// the probabilities.  A works on tile t + 1 while B works on tile t: h1 may be overwritten once the
+// second layer's MMAs of tile t have completed (bar2), its accumulator once B has read it (free2).
+// lenia_mlp_predict of 250001 rows: 11.1 ms as separate GEMM launches of 4096 rows, 372 us with one group running a tile's
+// hand-overs one after the other and copied inputs, 336 with two groups, 175 with the inputs read in place (in_place).
+// A wait that gives up ends its own group, and the other group's next wait gives up in turn.
+constexpr int NGROUP = 256, NRANK = 2 * NGROUP;
+constexpr uint32_t RANK_SMEM = S_BAR + 32;
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
+}
+
+__global__ void __launch_bounds__(NRANK, 1)
+    mlp_rank(const float* __restrict__ x, int B, const float* __restrict__ w, const bf16* __restrict__ wb,
+             float* __restrict__ probs, int* __restrict__ err) {
+    extern __shared__ __align__(1024) uint8_t sm[];
+    uint8_t *R0 = sm, *R2 = sm + 2 * REGION, *W1s = sm + S_W1, *Xs = sm + S_X;
+    float* F = reinterpret_cast<float*>(sm + S_F);
+    uint64_t *bar1 = reinterpret_cast<uint64_t*>(sm + S_BAR), *bar2 = bar1 + 1, *free2 = bar1 + 2;
+    uint32_t* slot = reinterpret_cast<uint32_t*>(bar1 + 3);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row = (warp & 3) * 32 + lane, half = (warp >> 2) & 1;
+    const int ntiles = (B + TILE - 1) / TILE;
+    const bf16* w2 = wb + P_W2;
+
+    for (int e = tid; e < HID * 2; e += NRANK)
+        cp_async16(W1s + tc::kmajor_offset(e >> 1, 8 * (e & 1), IN, 2), wb + P_W1 + (e >> 1) * IN + 8 * (e & 1));
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    load_w2<NRANK>(R0, w2, 0, HID);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int e = tid; e < HID; e += NRANK) F[F_B1 + e] = w[P_B1 + e], F[F_B2 + e] = w[P_B2 + e];
+    for (int e = tid; e < OUT * HID; e += NRANK) F[F_W3 + e] = __bfloat162float(wb[P_W3 + e]);
+    if (tid == 0) {
+        tc::mbar_init(bar1, 1);
+        tc::mbar_init(bar2, 1);
+        tc::mbar_init(free2, NGROUP);
+        tc::fence_barrier_init();
+    }
+    if (warp == 0) tc::tmem_alloc(slot, 512);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    tc::fence_async_smem();
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = *slot, mine = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t r0 = tc::smem_u32(R0), r2 = tc::smem_u32(R2), xs = tc::smem_u32(Xs), w1s = tc::smem_u32(W1s);
+    constexpr uint32_t IDESC = tc::instr_desc(1, 128, HID);
+    const int group = warp >> 3;  // A: 0, B: 1
+    // a wait of the whole group (its barrier: 1 + group)
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+        const bool ok = !tc::named_sync_or(1 + group, NGROUP, !tc::mbar_wait(bar, parity));
+        tc::tc_fence_after();
+        return ok;
+    };
+    bool ok = true;
+    uint32_t n = 0;  // tiles this group has begun
+    uint32_t issued2 = 0;
+    if (group == 0) {
+        const int r = tid >> 1, kg = tid & 1;  // this thread's eight inputs of a tile
+        float xin[8];
+        auto fetch = [&](int t) {
+            const int g = t * TILE + r;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+            if (g < B) {
+                const float4* p = reinterpret_cast<const float4*>(x + (size_t)g * IN + 8 * kg);
+                a = p[0], b = p[1];
+            }
+            xin[0] = a.x, xin[1] = a.y, xin[2] = a.z, xin[3] = a.w, xin[4] = b.x, xin[5] = b.y, xin[6] = b.z, xin[7] = b.w;
+        };
+        auto publish = [&]() {
+            tc::tc_fence_before();
+            tc::fence_async_smem();
+            tc::named_sync(1, NGROUP);
+            tc::tc_fence_after();
+        };
+        fetch(blockIdx.x);
+        for (int t = blockIdx.x; t < ntiles; t += gridDim.x, n++) {
+            *reinterpret_cast<uint4*>(Xs + tc::kmajor_offset(r, 8 * kg, IN, 2)) = pack8(xin);
+            publish();
+            if (tid == 0) {
+                tc::mma<false>(tmem, tc::smem_desc(xs, 128, XGROUP), tc::smem_desc(w1s, 128, XGROUP), IDESC, 0u);
+                tc::mma_commit(bar1);
+            }
+            if (t + (int)gridDim.x < ntiles) fetch(t + gridDim.x);
+            if (!(ok = wait(bar1, n & 1))) break;
+            if (n > 0 && !(ok = wait(bar2, (n - 1) & 1))) break;  // h1 of the last tile has been read
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const int n0 = half * 128 + 32 * c;
+                float v[32];
+                tc::tmem_ld32(mine + n0, v);
+#pragma unroll
+                for (int i = 0; i < 32; i++) v[i] = fmaxf(v[i] + F[F_B1 + n0 + i], 0.f);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    *reinterpret_cast<uint4*>(R2 + tc::kmajor_offset(row, n0 + 8 * i, HID, 2)) = pack8(v + 8 * i);
+            }
+            if (n > 0 && !(ok = wait(free2, (n - 1) & 1))) break;  // the last tile's accumulator has been read
+            publish();
+            if (tid == 0) {
+                for (uint32_t s = 0; s < HID / 16; s++)
+                    tc::mma<false>(tmem + HID, tc::smem_desc(r2 + 256u * s, 128, GROUP), tc::smem_desc(r0 + 256u * s, 128, GROUP),
+                                   IDESC, s > 0);
+                tc::mma_commit(bar2);
+            }
+            issued2 = n + 1;
+        }
+        // the CTA's last MMAs: waited for by B, and here before TMEM is freed
+        if (issued2 > 0 && tid == 0) tc::mbar_wait(bar2, (issued2 - 1) & 1);
+        if (!ok && tid == 0) tc::mbar_wait(bar1, n & 1);
+    } else {
+        for (int t = blockIdx.x; t < ntiles; t += gridDim.x, n++) {
+            if (!(ok = wait(bar2, n & 1))) break;
+            float z[OUT] = {0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const int n0 = half * 128 + 32 * c;
+                float v[32];
+                tc::tmem_ld32(mine + HID + n0, v);
+#pragma unroll
+                for (int i = 0; i < 32; i++) {
+                    const float h = __bfloat162float(__float2bfloat16_rn(fmaxf(v[i] + F[F_B2 + n0 + i], 0.f)));
+#pragma unroll
+                    for (int o = 0; o < OUT; o++) z[o] = fmaf(h, F[F_W3 + o * HID + n0 + i], z[o]);
+                }
+            }
+            if (half == 1)
+                for (int o = 0; o < OUT; o++) F[F_Z + row * OUT + o] = z[o];
+            tc::named_sync(2, NGROUP);
+            const int b = t * TILE + row;
+            if (half == 0) {
+#pragma unroll
+                for (int o = 0; o < OUT; o++) z[o] += F[F_Z + row * OUT + o];
+            }
+            tc::tc_fence_before();
+            mbar_arrive(free2);
+            if (half == 0 && b < B) {
+#pragma unroll
+                for (int o = 0; o < OUT; o++) probs[(size_t)b * OUT + o] = 1.f / (1.f + expf(-(z[o] + w[P_B3 + o])));
+            }
+        }
+    }
+    if (!ok) *(volatile int*)err = 1;
     tc::tc_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -435,11 +581,12 @@ using namespace lenia::mlp;
 struct LeniaMlp {
     int max_batch = 0;
     int t = 0, sms = 0;
+    int reads_host = 0;  // whether kernels may read pageable host memory in place
     cudaStream_t stream = nullptr;
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // FP32 master, grads, Adam moments
     bf16* wb = nullptr;                                             // BF16 copy of the parameters
     float *x = nullptr, *y = nullptr, *loss = nullptr;  // a batch: inputs, labels, per-row losses
-    int* err = nullptr;  // set by a tile that gave up waiting on a barrier; the losses follow it (one copy for both)
+    int* err = nullptr;  // set by a tile that gave up waiting on a barrier; page-locked host memory, the losses after it
     // ranking: two halves of PREDICT_ROWS rows of inputs and probabilities, each on a stream of its own
     cudaStream_t ps[2] = {};
     float *px = nullptr, *pp = nullptr;
@@ -463,49 +610,58 @@ int err(const char* msg) {
 }
 
 // rows of inputs that lenia_mlp_predict has on the device at a time, in two halves: a copy of one half
-// overlaps the other's tiles
-constexpr int PREDICT_ROWS = 1 << 16;
+// overlaps the other's tiles.  A half is two tiles for each of the GPU's 152 SMs, about as long on the SMs as on the
+// host link.
+constexpr int PREDICT_ROWS = 2 * 2 * 152 * TILE;
+// rows of one launch where the kernel reads them in host memory
+constexpr int DIRECT_ROWS = 1 << 20;
 
 int tiles_grid(const LeniaMlp* n, int B) {
     const int t = (B + TILE - 1) / TILE;
     return t < n->sms ? t : n->sms;
 }
 
-// gradients of the mean BCE of the batch in n->x, n->y into n->g; per-row losses into n->loss
-void gradients(LeniaMlp* n, int B) {
+// gradients of the mean BCE of the batch (x, y on the device, or in host memory in_place) into n->g; per-row losses
+// into n->loss
+void gradients(LeniaMlp* n, const float* x, const float* y, int B) {
     cudaMemsetAsync(n->g, 0, (size_t)NPARAM * sizeof(float), n->stream);
-    mlp_tile<true><<<tiles_grid(n, B), NTHR, TILE_SMEM, n->stream>>>(n->x, n->y, B, n->w, n->wb, nullptr, n->g, n->loss,
-                                                                     n->err);
+    mlp_tile<<<tiles_grid(n, B), NTHR, TILE_SMEM, n->stream>>>(x, y, B, n->w, n->wb, n->g, n->loss, n->err);
 }
 
+// After the streams have been waited for.
 int check_err(LeniaMlp* n) {
-    int h = 0;
-    if (cudaMemcpy(&h, n->err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return err("mlp: error flag read failed");
-    if (h) {
-        cudaMemset(n->err, 0, sizeof(int));
+    volatile int* flag = n->err;
+    if (*flag) {
+        *flag = 0;
         return err("mlp: a tile gave up waiting on a barrier; results are invalid");
     }
     return 0;
 }
 
-int upload_batch(LeniaMlp* n, const float* x, const float* y, uint32_t B) {
-    if (cudaMemcpyAsync(n->x, x, (size_t)B * IN * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess) return -1;
-    if (y && cudaMemcpyAsync(n->y, y, (size_t)B * OUT * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess) return -1;
+// Whether a kernel may read host rows where they are: the GPU walks the host's page tables (Grace) and the rows are
+// aligned for its 16-byte loads.  Against copying them first, lenia_mlp_predict of 250001 rows 336 -> 188 us, of
+// 1000 rows 50 -> 42, lenia_mlp_gradients of 1000 rows 84 -> 72.
+bool in_place(const LeniaMlp* n, const float* rows) { return n->reads_host && ((uintptr_t)rows & 15) == 0; }
+
+// The batch's gradients from host rows, copied first where they cannot be read in place.
+int batch_gradients(LeniaMlp* n, const float* x, const float* y, uint32_t B) {
+    if (!in_place(n, x)) {
+        if (cudaMemcpyAsync(n->x, x, (size_t)B * IN * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess ||
+            cudaMemcpyAsync(n->y, y, (size_t)B * OUT * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess)
+            return err("mlp: upload failed");
+        x = n->x, y = n->y;
+    }
+    gradients(n, x, y, (int)B);
     return 0;
 }
 
-// Waits for the batch; its mean loss, and the error flag that travels with the losses.
+// Waits for the batch; its mean loss.
 int mean_loss(LeniaMlp* n, uint32_t B, float* loss) {
-    std::vector<float> l((size_t)B + 1);
-    if (cudaMemcpyAsync(l.data(), n->err, ((size_t)B + 1) * 4, cudaMemcpyDeviceToHost, n->stream) != cudaSuccess ||
-        cudaStreamSynchronize(n->stream) != cudaSuccess)
-        return err("mlp: download failed");
+    if (cudaStreamSynchronize(n->stream) != cudaSuccess) return err("mlp: the batch failed");
     double s = 0;
-    for (uint32_t i = 1; i <= B; i++) s += l[i];
+    for (uint32_t i = 0; i < B; i++) s += n->loss[i];
     if (loss) *loss = (float)(s / B);
-    int flag;
-    memcpy(&flag, l.data(), sizeof(flag));
-    return flag ? check_err(n) : 0;
+    return check_err(n);
 }
 
 }  // namespace
@@ -524,20 +680,23 @@ LENIA_API int lenia_mlp_create(uint32_t seed, uint32_t max_batch, LeniaMlp** out
     int dev = 0;
     bool ok = cudaGetDevice(&dev) == cudaSuccess &&
               cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-              cudaFuncSetAttribute(mlp_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM) == cudaSuccess &&
-              cudaFuncSetAttribute(mlp_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM) == cudaSuccess &&
+              cudaDeviceGetAttribute(&n->reads_host, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) == cudaSuccess &&
+              cudaFuncSetAttribute(mlp_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM) == cudaSuccess &&
+              cudaFuncSetAttribute(mlp_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, RANK_SMEM) == cudaSuccess &&
               cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaStreamCreateWithFlags(&n->ps[0], cudaStreamNonBlocking) == cudaSuccess &&
               cudaStreamCreateWithFlags(&n->ps[1], cudaStreamNonBlocking) == cudaSuccess && mal(n, &n->w, NPARAM) &&
               mal(n, &n->g, NPARAM) && mal(n, &n->m, NPARAM) && mal(n, &n->v, NPARAM) && mal(n, &n->wb, NPARAM) &&
-              mal(n, &n->x, B * IN) && mal(n, &n->y, B * OUT) && mal(n, &n->err, B + 1) &&
-              mal(n, &n->px, (size_t)PREDICT_ROWS * IN) && mal(n, &n->pp, (size_t)PREDICT_ROWS * OUT);
+              mal(n, &n->x, B * IN) && mal(n, &n->y, B * OUT) &&
+              cudaHostAlloc((void**)&n->err, (B + 4) * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess &&
+              mal(n, &n->px, (size_t)PREDICT_ROWS * IN) && mal(n, &n->pp, (size_t)DIRECT_ROWS * OUT);
     if (!ok) {
         lenia_mlp_destroy(n);
         set_thread_error("mlp: device allocation failed");
         return LENIA_ENOMEM;
     }
-    n->loss = reinterpret_cast<float*>(n->err + 1);
+    *n->err = 0;
+    n->loss = reinterpret_cast<float*>(n->err + 4);
     // He-uniform initialisation from the PCG hash, biases zero
     std::vector<float> w(NPARAM, 0.f);
     auto pcg = [](uint32_t v) {
@@ -562,7 +721,6 @@ LENIA_API int lenia_mlp_create(uint32_t seed, uint32_t max_batch, LeniaMlp** out
     }
     cudaMemsetAsync(n->m, 0, NPARAM * 4, n->stream);
     cudaMemsetAsync(n->v, 0, NPARAM * 4, n->stream);
-    cudaMemsetAsync(n->err, 0, sizeof(int), n->stream);
     if (cudaStreamSynchronize(n->stream) != cudaSuccess) {
         lenia_mlp_destroy(n);
         return err("mlp: initialisation failed");
@@ -576,6 +734,7 @@ LENIA_API int lenia_mlp_destroy(LeniaMlp* n) {
     for (cudaStream_t s : {n->stream, n->ps[0], n->ps[1]})
         if (s) cudaStreamSynchronize(s);
     for (void* p : n->allocs) cudaFree(p);
+    if (n->err) cudaFreeHost(n->err);
     for (cudaStream_t s : {n->stream, n->ps[0], n->ps[1]})
         if (s) cudaStreamDestroy(s);
     delete n;
@@ -617,8 +776,7 @@ LENIA_API int lenia_mlp_gradients(LeniaMlp* n, const float* x, const float* y, u
         set_thread_error("mlp: bad batch");
         return LENIA_EINVAL;
     }
-    if (upload_batch(n, x, y, batch)) return err("mlp: upload failed");
-    gradients(n, (int)batch);
+    if (int rc = batch_gradients(n, x, y, batch)) return rc;
     if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
     cudaMemcpyAsync(grads, n->g, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream);
     return mean_loss(n, batch, loss);
@@ -629,8 +787,7 @@ LENIA_API int lenia_mlp_train_step(LeniaMlp* n, const float* x, const float* y, 
         set_thread_error("mlp: bad batch or learning rate");
         return LENIA_EINVAL;
     }
-    if (upload_batch(n, x, y, batch)) return err("mlp: upload failed");
-    gradients(n, (int)batch);
+    if (int rc = batch_gradients(n, x, y, batch)) return rc;
     n->t++;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)n->t), c2 = 1.f - std::pow(b2, (float)n->t);
@@ -644,6 +801,17 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
         set_thread_error("mlp: NULL argument");
         return LENIA_EINVAL;
     }
+    if (in_place(n, x)) {
+        for (uint64_t off = 0; off < count; off += DIRECT_ROWS) {
+            const uint32_t B = count - off < DIRECT_ROWS ? (uint32_t)(count - off) : DIRECT_ROWS;
+            mlp_rank<<<tiles_grid(n, (int)B), NRANK, RANK_SMEM, n->ps[0]>>>(x + off * IN, (int)B, n->w, n->wb, n->pp, n->err);
+            if (cudaMemcpyAsync(probs + off * OUT, n->pp, (size_t)B * OUT * 4, cudaMemcpyDeviceToHost, n->ps[0]) !=
+                cudaSuccess)
+                return err("mlp: download failed");
+        }
+        if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess) return err("mlp: predict failed");
+        return check_err(n);
+    }
     // chunk c runs on stream c % 2; its results leave after the next chunk has been queued, so that a copy
     // to or from pageable memory, which blocks this thread, overlaps a chunk's tiles
     constexpr uint32_t HALF = PREDICT_ROWS / 2;
@@ -656,8 +824,7 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
             if (cudaMemcpyAsync(px, x + (size_t)c * HALF * IN, (size_t)rows(c) * IN * 4, cudaMemcpyHostToDevice, n->ps[h]) !=
                 cudaSuccess)
                 return err("mlp: upload failed");
-            mlp_tile<false><<<tiles_grid(n, (int)rows(c)), NTHR, TILE_SMEM, n->ps[h]>>>(px, nullptr, (int)rows(c), n->w, n->wb,
-                                                                                       pp, nullptr, nullptr, n->err);
+            mlp_rank<<<tiles_grid(n, (int)rows(c)), NRANK, RANK_SMEM, n->ps[h]>>>(px, (int)rows(c), n->w, n->wb, pp, n->err);
         }
         if (c > 0) {
             const uint32_t d = c - 1;

@@ -44,8 +44,9 @@ def test_gradients_at_tile_edges(proposer, batch):
         assert err < 1e-2, (a, b, err)
 
 
-# no rows, partial and full tiles, and the edges of the two halves that overlap (32768 rows each)
-@pytest.mark.parametrize("count", [0, 1, 128, 129, 32768, 32769, 65537])
+# no rows, partial and full tiles, the second tile of a CTA's pipeline, and the edges of the two halves that
+# overlap (38912 rows each: two tiles for each of 152 SMs)
+@pytest.mark.parametrize("count", [0, 1, 128, 129, 19457, 38912, 38913, 77825])
 def test_predict_at_half_edges(proposer, count):
     x = np.random.default_rng(count).random((count, M.IN)).astype(np.float32)
     got = proposer.predict(x)
