@@ -320,17 +320,23 @@ FFT_CHD constexpr int seq_threads(int N, int S) {
     return N % 3 == 0 && N < 6144 && S * N / 12 > S * N / plan_radix(N, 0) ? S * N / 12 : S * N / plan_radix(N, 0);
 }
 FFT_CHD constexpr int row_seqs(int W, bool gen) { return gen ? (W >= 2048 ? 1 : (W <= 1024 ? 4 : 2)) : (W <= 1024 ? 4 : W >= 6144 ? 1 : 2); }
-template <int W, bool GEN>
+// Sequences a CTA holds: an item's, or from 768 up in variant 1 of the single-kernel step, which runs where the items
+// leave SMs idle, half of them (two CTAs an item): one 4096 x 256 world 13.3 -> 10.0 us a generation, 1536 x 768 12.9 ->
+// 11.8, 1024 x 256 8.2 -> 7.1, 768 x 768 9.4 -> 9.1, but 384 x 384 6.8 -> 9.8 and 256 x 256 5.5 -> 6.0.
+FFT_CHD constexpr int row_cta_seqs(int W, int V, bool gen) {
+    return V == 1 && !gen && W >= 768 && row_seqs(W, gen) > 1 ? row_seqs(W, gen) / 2 : row_seqs(W, gen);
+}
+template <int W, bool GEN, int V = 0>
 constexpr int row_nt() {
-    constexpr int n = seq_threads(W, row_seqs(W, GEN));
+    constexpr int n = seq_threads(W, row_cta_seqs(W, V, GEN));
     return n < 32 ? 32 : (n > 1024 ? 1024 : n);
 }
-// variant 0: at most 1024 threads' worth of registers per SM (64 a thread at 512 threads);
-// variant 1: at most 128 a thread
+// variant 0: at most 64 registers a thread (1024 threads an SM), 80 at 512 (which spills 36 bytes at 64: one world 11.2 ->
+// 6.6 us a generation, 41 worlds 55.5 -> 42.7); variant 1: at most 128
 template <int W, int V, bool GEN>
 constexpr int row_minb() {
-    constexpr int t = V == 0 ? 1024 : 512;
-    return t / row_nt<W, GEN>() < 1 ? 1 : t / row_nt<W, GEN>();
+    constexpr int t = V == 0 ? (W == 512 && !GEN ? 768 : 1024) : 512, b = t / row_nt<W, GEN, V>();
+    return b < 1 ? 1 : b > 32 ? 32 : b;
 }
 // 256-bit spectrum accesses, but 128-bit ones in the builds for a few rows of small worlds, whose launches wait for
 // a single access's latency: one 256 x 256 world 5.9 -> 5.5 us a generation, 384 x 384 7.1 -> 6.8; against them
@@ -500,9 +506,9 @@ __device__ __noinline__ void row_item_u(float2* Z, const float2* stw, const DevW
 // dt update and clamp against the state, forward row FFT of the new rows.  Z: the two packed
 // sequences, stw: the stage tables.  CG: spectrum and state loads bypass L1 (the persistent step,
 // where another CTA of the same launch wrote them).
-template <int W, int NT, bool CG, bool WIDE = true>
+template <int W, int NT, int S, bool CG, bool WIDE = true>
 __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, float2* Z, const float2* stw, bool early = false) {
-    constexpr int S = row_seqs(W, false), ROWS = 2 * S;
+    constexpr int ROWS = 2 * S;
     const int H = wd.H;
     const DevKernel kp = wd.kern[0];
     const float dtw = wd.dt * kp.weight;
@@ -549,19 +555,19 @@ __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, floa
 // one-kernel Lenia step (and the forward and U modes), so the general path's register pressure
 // does not set the budget of the common path.
 // WIDE: whether the spectrum moves in 256-bit accesses (row_wide).
-template <int W, int NT, int MINB, bool GEN, bool WIDE>
+template <int W, int NT, int MINB, int S, bool GEN, bool WIDE>
 __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict__ worlds, const RowItem* __restrict__ items,
                                                 int mode, int general, const float2* __restrict__ tw, bool early) {
-    constexpr int S = row_seqs(W, GEN), ROWS = 2 * S;
+    constexpr int ROWS = 2 * S, SPLIT = row_seqs(W, GEN) / S;  // CTAs an item
     extern __shared__ float4 smem_raw[];
     constexpr int SEQ = seq_stride(W);
     float2* Z = reinterpret_cast<float2*>(smem_raw);
     float2* stw = Z + S * SEQ;
     float* extra = row_extra_smem<W>(stw);
-    const RowItem it = items[blockIdx.x];
+    const RowItem it = items[blockIdx.x / SPLIT];
     const DevWorld& wd = worlds[it.world];
     fill_tables<W>(stw, tw, NT);
-    const int H = wd.H, C = wd.C, K = wd.K, r0 = it.row0;
+    const int H = wd.H, C = wd.C, K = wd.K, r0 = it.row0 + ROWS * (blockIdx.x % SPLIT);
     const size_t plane = (size_t)W * H, cplane = (size_t)(W / 2) * H;
     // Lenia items cover one target channel; SmoothLife and MNCA items every channel
     const bool per_chan = wd.rule == LENIA_RULE_LENIA;
@@ -578,7 +584,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     }
 
     if constexpr (!GEN) {
-        row_item_simple<W, NT, false, WIDE>(wd, r0, Z, stw, early);
+        row_item_simple<W, NT, S, false, WIDE>(wd, r0, Z, stw, early);
         return;
     }
 
@@ -1040,24 +1046,26 @@ bool col_go_pair(const DevWorld* worlds, const ColItem* items, int nitems, const
 // Shared memory of a row-pass launch: sequences, stage tables, then the general path's
 // accumulation planes.
 template <int W, bool GEN>
-constexpr size_t row_smem(int general, int planes) {
-    const int rows = 2 * row_seqs(W, GEN);
-    return (size_t)row_seqs(W, GEN) * seq_stride(W) * sizeof(float2) + stage_table_bytes<W>() +
+constexpr size_t row_smem(int general, int planes, int seqs = row_seqs(W, GEN)) {
+    const int rows = 2 * seqs;
+    return (size_t)seqs * seq_stride(W) * sizeof(float2) + stage_table_bytes<W>() +
            (size_t)(general ? planes : 0) * rows * W * sizeof(float);
 }
 
-template <int W, int NT, int MINB, bool GEN, bool WIDE>
+template <int W, int V, bool GEN>
 bool row_go(int mode, int general, int planes, const DevWorld* worlds, const RowItem* items, int nitems,
             const float2* tw, LaunchOn s) {
-    const size_t smem = row_smem<W, GEN>(general, planes);
+    constexpr int S = row_cta_seqs(W, V, GEN), NT = row_nt<W, GEN, V>();
+    constexpr auto kernel = row_pass<W, NT, row_minb<W, V, GEN>(), S, GEN, row_wide<W, V>()>;
+    const size_t smem = row_smem<W, GEN>(general, planes, S);
     static int attr_max = 0;
     if ((int)smem > attr_max) {
-        if (cudaFuncSetAttribute(row_pass<W, NT, MINB, GEN, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
             cudaSuccess)
             return false;
         attr_max = (int)smem;
     }
-    return nitems <= 0 || launch_pass(row_pass<W, NT, MINB, GEN, WIDE>, nitems, NT, smem, s, worlds, items, mode, general, tw, s.early);
+    return nitems <= 0 || launch_pass(kernel, nitems * (row_seqs(W, GEN) / S), NT, smem, s, worlds, items, mode, general, tw, s.early);
 }
 
 // Column-pass builds: variant 0 and 1 are the scalar build at 64 (80 with a radix-32 plan) and 128
@@ -1085,11 +1093,10 @@ bool col_go_variant(int variant, const DevWorld* worlds, const ColItem* items, i
 // unit's compile time down.  (A paired row build, two packed sequences per thread as in the
 // column pass, measured 15% slower at 4096 x 4096: its stores and growth had half the warps to
 // hide behind.)
-#define LENIA_ROW_CASE_G(N, G)                                                                                   \
-    case N:                                                                                                      \
-        return (variant & 1)                                                                                     \
-                   ? row_go<N, row_nt<N, G>(), row_minb<N, 1, G>(), G, row_wide<N, 1>()>(mode, general, planes, worlds, items, nitems, tw, s) \
-                   : row_go<N, row_nt<N, G>(), row_minb<N, 0, G>(), G, row_wide<N, 0>()>(mode, general, planes, worlds, items, nitems, tw, s);
+#define LENIA_ROW_CASE_G(N, G)                                                                     \
+    case N:                                                                                        \
+        return (variant & 1) ? row_go<N, 1, G>(mode, general, planes, worlds, items, nitems, tw, s) \
+                             : row_go<N, 0, G>(mode, general, planes, worlds, items, nitems, tw, s);
 #define LENIA_ROW_CASE_SIMPLE(N) LENIA_ROW_CASE_G(N, false)
 #define LENIA_ROW_CASE_GENERAL(N) LENIA_ROW_CASE_G(N, true)
 
