@@ -830,9 +830,10 @@ int setup_fused(LeniaCtx* ctx) {
         else cl.var_col = (col_wide(cl.H) && cl.H != 384) || cl.H == 192 ? 1 : 0;
         // Rows: at 64 registers (43 worlds of 768 x 768 112 us against 129, one of 4096 x 4096 103 against 114) unless the
         // launch leaves the occupancy that buys unused -- at most three items for two SMs -- (one 384 x 384 world 10.1 ->
-        // 6.8 us, 1536 x 768 12.9 -> 11.8, but 2048 x 1024, 256 items, 14.4 against 15.9) or the general step, which
-        // spills there (SmoothLife 2048 x 2048 55 -> 47 us, 1024 x 1024 17.5 -> 16.2).
-        cl.var_row = general || 2 * row.size() <= 3 * (size_t)ctx->sms ? 1 : 0;
+        // 6.8 us, 1536 x 768 12.9 -> 11.8, but 2048 x 1024, 256 items, 14.4 against 15.9), at 384 (384 x 2048 12.3 -> 9.5,
+        // 60 worlds the same) or in the general step, which spills there (SmoothLife 2048 x 2048 55 -> 47 us, 1024 x 1024
+        // 17.5 -> 16.2).
+        cl.var_row = general || cl.W == 384 || 2 * row.size() <= 3 * (size_t)ctx->sms ? 1 : 0;
         cl.ncol = (int)col.size();
         cl.nrow = (int)row.size();
         cl.ntcg = (int)tcg.size();

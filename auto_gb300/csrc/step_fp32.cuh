@@ -331,11 +331,11 @@ constexpr int row_nt() {
     constexpr int n = seq_threads(W, row_cta_seqs(W, V, GEN));
     return n < 32 ? 32 : (n > 1024 ? 1024 : n);
 }
-// variant 0: at most 64 registers a thread (1024 threads an SM), 80 at 512 (which spills 36 bytes at 64: one world 11.2 ->
-// 6.6 us a generation, 41 worlds 55.5 -> 42.7); variant 1: at most 128
+// variant 0: at most 64 registers a thread (1024 threads an SM), 80 at 192 and 512 (which spill 40 bytes at 64: 63 worlds of
+// 192 x 192 14.0 -> 13.5 us a generation, 41 of 512 x 512 55.5 -> 42.7, one 11.2 -> 6.6); variant 1: at most 128
 template <int W, int V, bool GEN>
 constexpr int row_minb() {
-    constexpr int t = V == 0 ? (W == 512 && !GEN ? 768 : 1024) : 512, b = t / row_nt<W, GEN, V>();
+    constexpr int t = V == 0 ? ((W == 192 || W == 512) && !GEN ? 768 : 1024) : 512, b = t / row_nt<W, GEN, V>();
     return b < 1 ? 1 : b > 32 ? 32 : b;
 }
 // 256-bit spectrum accesses, but 128-bit ones in the builds for a few rows of small worlds, whose launches wait for
