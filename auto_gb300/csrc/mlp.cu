@@ -62,7 +62,8 @@ using bf16 = __nv_bfloat16;
 // again into R0.  One CTA per SM (224 KB of shared memory, all 512 TMEM columns).  A tile is a chain of
 // five waits on the tensor cores with a hand-over after each, so it is bound by that latency, and a batch of
 // 1000 rows by one tile's: with a thread for every 64 columns of a row instead of every 128,
-// lenia_mlp_gradients of 1000 rows went from 77 to 66 us.  As separate GEMM launches, whose hand-overs wrote
+// lenia_mlp_gradients of 1000 rows went from 77 to 66 us; with the gradient reductions on whole 128-byte runs
+// (transpose_pieces) to 65, lenia_mlp_train_step from 58 to 55.  As separate GEMM launches, whose hand-overs wrote
 // h1 and h2 (and their transposes) to global memory with 2-byte stores one row stride apart per lane, it took 560.
 //
 // Every barrier wait is bounded; a CTA that gives up waits (bounded) for its MMAs and copies, raises *err,
@@ -107,6 +108,25 @@ __device__ __forceinline__ float column_sums(float* v) {
         }
     }
     return v[0];
+}
+
+// Eight lanes' eight float4s each (v[4 i ..]: piece i of a row) transposed among them: lane l of eight then holds
+// piece l of rows 0..7 in v[4 r ..].
+__device__ __forceinline__ void transpose_pieces(float* v) {
+#pragma unroll
+    for (int w = 4; w >= 1; w >>= 1) {
+        const bool up = threadIdx.x & w;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (!(i & w))
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    float &lo = v[4 * i + k], &hi = v[4 * (i + w) + k];
+                    const float got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, w);
+                    if (up) lo = got;
+                    else hi = got;
+                }
+    }
 }
 
 // rows [first, first + n) of W2 (bf16 [256][256]) into an operand region, n a multiple of 8: eight rows of
@@ -349,9 +369,11 @@ __global__ void __launch_bounds__(NTHR, 1)
                 const int n0 = part * NCOL + 32 * c;
                 float v[32];
                 tc::tmem_ld32(mine + col0 + n0, v);
-                float* p = g + P_W2 + (size_t)(out0 + row) * HID + n0;
+                // eight lanes on 128 contiguous bytes of a row instead of 32 lanes on 32 rows
+                transpose_pieces(v);
+                float* p = g + P_W2 + (size_t)(out0 + (row & ~7)) * HID + n0 + 4 * (lane & 7);
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) red_add4(p + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
+                for (int r = 0; r < 8; r++) red_add4(p + r * HID, v[4 * r], v[4 * r + 1], v[4 * r + 2], v[4 * r + 3]);
             }
         };
         add_dw2(HID, 128);
