@@ -831,9 +831,15 @@ int setup_fused(LeniaCtx* ctx) {
         // Rows: at 64 registers (43 worlds of 768 x 768 112 us against 129, one of 4096 x 4096 103 against 114) unless the
         // launch leaves the occupancy that buys unused -- at most three items for two SMs -- (one 384 x 384 world 10.1 ->
         // 6.8 us, 1536 x 768 12.9 -> 11.8, but 2048 x 1024, 256 items, 14.4 against 15.9), at 384 (384 x 2048 12.3 -> 9.5,
-        // 60 worlds the same) or in the general step, which spills there (SmoothLife 2048 x 2048 55 -> 47 us, 1024 x 1024
-        // 17.5 -> 16.2).
-        cl.var_row = general || cl.W == 384 || 2 * row.size() <= 3 * (size_t)ctx->sms ? 1 : 0;
+        // 60 worlds the same).  The general step has 80 registers there and is better off with 128 (SmoothLife 2048 x 2048
+        // 54 us against 47, 2048 x 1024 27.4 against 25.2) unless that makes two waves of what three CTAs an SM hold in
+        // one: from 768 to 1536 wide, with more than two items an SM and at most three (three channels of 1024 x 1024
+        // 43.4 -> 41.8 us, 768 x 1024 37.8 -> 33.5, SmoothLife 1536 x 1536 35.1 -> 31.7, but 1024 x 1024, 128 items,
+        // 15.6 against 16.5).
+        if (general)
+            cl.var_row = !(cl.W >= 768 && cl.W <= 1536 && row.size() > 2 * (size_t)ctx->sms && row.size() <= 3 * (size_t)ctx->sms);
+        else
+            cl.var_row = cl.W == 384 || 2 * row.size() <= 3 * (size_t)ctx->sms ? 1 : 0;
         cl.ncol = (int)col.size();
         cl.nrow = (int)row.size();
         cl.ntcg = (int)tcg.size();

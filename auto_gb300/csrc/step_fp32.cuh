@@ -332,10 +332,12 @@ constexpr int row_nt() {
     return n < 32 ? 32 : (n > 1024 ? 1024 : n);
 }
 // variant 0: at most 64 registers a thread (1024 threads an SM), 80 at 192 and 512 (which spill 40 bytes at 64: 63 worlds of
-// 192 x 192 14.0 -> 13.5 us a generation, 41 of 512 x 512 55.5 -> 42.7, one 11.2 -> 6.6); variant 1: at most 128
+// 192 x 192 14.0 -> 13.5 us a generation, 41 of 512 x 512 55.5 -> 42.7, one 11.2 -> 6.6) and in the general step (which
+// spilled at 64 at most sizes; three 256-thread CTAs an SM: three channels of 1024 x 1024 with nine kernels 43.4 -> 41.8);
+// variant 1: at most 128
 template <int W, int V, bool GEN>
 constexpr int row_minb() {
-    constexpr int t = V == 0 ? ((W == 192 || W == 512) && !GEN ? 768 : 1024) : 512, b = t / row_nt<W, GEN, V>();
+    constexpr int t = V == 0 ? (GEN || W == 192 || W == 512 ? 768 : 1024) : 512, b = t / row_nt<W, GEN, V>();
     return b < 1 ? 1 : b > 32 ? 32 : b;
 }
 // 256-bit spectrum accesses, but 128-bit ones in the builds for a few rows of small worlds, whose launches wait for
