@@ -1579,7 +1579,10 @@ int lenia_read_spectrum(LeniaCtx* ctx, int32_t world, int32_t channel, float* ho
 int lenia_world_stats(LeniaCtx* ctx, float* host_out, size_t count) {
     if (!ctx) return LENIA_EINVAL;
     if (!host_out || count != 3 * ctx->desc.size()) return fail(ctx, LENIA_EINVAL, "need 3 floats per world");
-    launch_world_stats(ctx->d_worlds, (int)ctx->desc.size(), ctx->d_stats, ctx->stream);
+    uint32_t sides = 0;
+    for (const auto& d : ctx->desc) sides = std::max(sides, d.width + d.height);
+    if (!launch_world_stats(ctx->d_worlds, (int)ctx->desc.size(), (int)sides, ctx->d_stats, ctx->stream))
+        return fail(ctx, LENIA_ECUDA, "launch configuration failed");
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(host_out, ctx->d_stats, count * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));

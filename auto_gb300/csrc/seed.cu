@@ -125,21 +125,38 @@ __global__ void render_kernel(const float* __restrict__ state, int W, int H, flo
     out[(size_t)py * out_w + px] = make_uchar4(u8(sqrtf(ar * inv)), u8(sqrtf(ag * inv)), u8(sqrtf(ab * inv)), 255);
 }
 
-// Mass of channel 0 and toroidal centroid (circular mean per axis), one CTA per world.
-__global__ void world_stats_kernel(const DevWorld* __restrict__ worlds, float* out) {
+// Mass of channel 0 and toroidal centroid (circular mean per axis), one CTA per world; a thread adds its
+// cells, 1024 apart, in order.  Bound by load latency (eight loads are in flight a thread) and the work per cell:
+// the angles' sines come from a table per axis instead of two sincospif a cell and the cell's column and row from a running
+// pair instead of a division, with equal bits.  lenia_world_stats of 1024 worlds of 256 x 256 462 -> 229 us, of one
+// 1024 x 1024 world 585 -> 165.
+constexpr int STATS_NT = 1024, STATS_LOADS = 8;
+__global__ void __launch_bounds__(STATS_NT) world_stats_kernel(const DevWorld* __restrict__ worlds, float* out) {
+    extern __shared__ float2 axis[];  // (sin, cos) of the columns' angles, then of the rows'
     const DevWorld& wd = worlds[blockIdx.x];
-    const int W = wd.W, H = wd.H;
-    const size_t n = (size_t)W * H;
+    const int W = wd.W, H = wd.H, n = W * H;
+    const float* __restrict__ state = wd.state;
     float m = 0.f, cxs = 0.f, cxc = 0.f, cys = 0.f, cyc = 0.f;
     const float ax = 2.0f / W, ay = 2.0f / H;
-    for (size_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const float s = wd.state[i];
-        if (s == 0.0f) continue;
-        const int x = (int)(i % W), y = (int)(i / W);
-        float sx, cx, sy, cy;
-        sincospif(ax * x, &sx, &cx);
-        sincospif(ay * y, &sy, &cy);
-        m += s; cxs += s * sx; cxc += s * cx; cys += s * sy; cyc += s * cy;
+    for (int i = threadIdx.x; i < W + H; i += STATS_NT)
+        sincospif(i < W ? ax * i : ay * (i - W), &axis[i].x, &axis[i].y);
+    __syncthreads();
+    const int dx = STATS_NT % W, dy = STATS_NT / W;
+    int x = threadIdx.x % W, y = threadIdx.x / W;
+    for (int i = threadIdx.x; i < n; i += STATS_LOADS * STATS_NT) {
+        float v[STATS_LOADS];
+#pragma unroll
+        for (int q = 0; q < STATS_LOADS; q++) v[q] = i + q * STATS_NT < n ? state[i + q * STATS_NT] : 0.f;
+#pragma unroll
+        for (int q = 0; q < STATS_LOADS; q++) {
+            const float s = v[q];
+            if (s != 0.0f) {
+                const float2 a = axis[x], b = axis[W + y];
+                m += s; cxs += s * a.x; cxc += s * a.y; cys += s * b.x; cyc += s * b.y;
+            }
+            x += dx, y += dy;
+            if (x >= W) x -= W, y++;
+        }
     }
     __shared__ double red[5][32];
     double v[5] = {m, cxs, cxc, cys, cyc};
@@ -187,8 +204,13 @@ void launch_render(const float* state, int W, int H, float ox, float oy, float s
     render_kernel<<<grd, blk, 0, s>>>(state, W, H, ox, oy, scale, n, out_w, out_h, palette, out);
 }
 
-void launch_world_stats(const DevWorld* worlds, int nworlds, float* out, cudaStream_t s) {
-    world_stats_kernel<<<nworlds, 1024, 0, s>>>(worlds, out);
+bool launch_world_stats(const DevWorld* worlds, int nworlds, int max_sides, float* out, cudaStream_t s) {
+    const int smem = max_sides * (int)sizeof(float2);
+    if (smem > 40 * 1024 &&
+        cudaFuncSetAttribute(world_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return false;
+    world_stats_kernel<<<nworlds, STATS_NT, smem, s>>>(worlds, out);
+    return true;
 }
 
 }  // namespace lenia
