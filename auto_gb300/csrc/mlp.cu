@@ -63,7 +63,7 @@ using bf16 = __nv_bfloat16;
 // five waits on the tensor cores with a hand-over after each, so it is bound by that latency, and a batch of
 // 1000 rows by one tile's: with a thread for every 64 columns of a row instead of every 128,
 // lenia_mlp_gradients of 1000 rows went from 77 to 66 us; with the gradient reductions on whole 128-byte runs
-// (transpose_pieces) to 65, lenia_mlp_train_step from 58 to 55.  As separate GEMM launches, whose hand-overs wrote
+// (transpose_pieces) lenia_mlp_train_step of 1000 rows from 57.8 to 55.4, of 4096 from 60.1 to 57.5.  As separate GEMM launches, whose hand-overs wrote
 // h1 and h2 (and their transposes) to global memory with 2-byte stores one row stride apart per lane, it took 560.
 //
 // Every barrier wait is bounded; a CTA that gives up waits (bounded) for its MMAs and copies, raises *err,
