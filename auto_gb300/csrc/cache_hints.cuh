@@ -112,8 +112,6 @@ __device__ __forceinline__ void st8(float2* p, float2 a, float2 b, float2 c, flo
 }
 template <bool CG>
 __device__ __forceinline__ float2 ld2c(const float2* p, uint64_t pol) { return CG ? ld2_cg(p, pol) : ld2(p, pol); }
-template <bool CG>
-__device__ __forceinline__ float4 ld4c(const float4* p, uint64_t pol) { return CG ? ld4_cg(p, pol) : ld4(p, pol); }
 
 // The same with a compile-time byte offset folded into the address ([p + OFF]), so that a run of
 // accesses off one base pointer does not need a 64-bit register pair per address.

@@ -79,10 +79,10 @@ bool launch_pass(void (*kernel)(P...), int grid, int threads, size_t smem, Launc
     return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
 }
 
-// Fused FP32 path (step_fp32_*.cu).  Every size is built in two launch variants with the same
-// threads per CTA: variant 0 caps registers at 64 per thread (more resident CTAs), variant 1 at
-// 128.  The column pass has a third, variant 2: the paired build (both columns of a tile in one
-// sequence of f32x2 pairs, half the threads).  The autotuner picks per size class.  The row
+// Fused FP32 path (step_fp32_*.cu).  Every size is built in two launch variants: variant 0 caps registers
+// at 64 or 80 per thread (more resident CTAs), variant 1 at 128 (and gives a row item from 768 wide up
+// two CTAs, see row_cta_seqs).  The column pass has two more: variant 2, the paired build (both columns of a tile
+// in one sequence of f32x2 pairs, half the threads), and variant 3 (COL_VARIANTS).  The row
 // launcher picks its general build from its `general` argument.  Launchers return false if the
 // size is not built.
 bool launch_col_fp32(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
@@ -99,7 +99,7 @@ bool col_has_variant3(int H);
 // whether the scalar column pass of height H holds 24 or 32 elements a thread (radix-32 plans, the
 // larger two-stage transforms)
 bool col_wide(int H);
-int row_item_rows(int W, int general);  // rows per row-pass item: 4, or 2 (general step, W >= 2048)
+int row_item_rows(int W, int general);  // rows per row-pass item: 2, 4 or 8 (row_seqs)
 int max_smem_optin();
 
 // Cluster-resident step (resident.cu): one launch advances every world of a square size class of

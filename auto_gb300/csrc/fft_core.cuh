@@ -1,4 +1,4 @@
-// Shared-memory Stockham FFT building blocks (mixed radix 2/3/4/8/16), FP32.
+// Shared-memory Stockham FFT building blocks (mixed radix 2 to 32), FP32.
 //
 // The reference runs one radix-2 Stockham stage per dispatch over global memory
 // (crates/auto-core/src/automata/spectral.rs:14-64: src p and p+n/2, dst 2p-k and 2p-k+m,

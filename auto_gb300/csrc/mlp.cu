@@ -36,7 +36,8 @@ constexpr int P_W1 = 0, P_B1 = P_W1 + HID * IN, P_W2 = P_B1 + HID, P_B2 = P_W2 +
 using bf16 = __nv_bfloat16;
 
 // ------------------------------------------------------------------ the network on a tile of rows
-// One CTA takes 128 rows through the whole network, forward to the logits and back to every gradient.  Nothing but the inputs, the weights and the results touches global memory.
+// One CTA takes 128 rows through the whole network, forward to the logits and back to every gradient.
+// Nothing but the inputs, the weights and the results touches global memory.
 //
 // All operands sit in shared memory in the canonical layout without swizzle (8-row x 16-byte core
 // matrices, K-adjacent ones 128 bytes apart, 8-row groups one after another: tc::kmajor_offset).  A
@@ -63,8 +64,9 @@ using bf16 = __nv_bfloat16;
 // five waits on the tensor cores with a hand-over after each, so it is bound by that latency, and a batch of
 // 1000 rows by one tile's: with a thread for every 64 columns of a row instead of every 128,
 // lenia_mlp_gradients of 1000 rows went from 77 to 66 us; with the gradient reductions on whole 128-byte runs
-// (transpose_pieces) lenia_mlp_train_step of 1000 rows from 57.8 to 55.4, of 4096 from 60.1 to 57.5.  As separate GEMM launches, whose hand-overs wrote
-// h1 and h2 (and their transposes) to global memory with 2-byte stores one row stride apart per lane, it took 560.
+// (transpose_pieces) lenia_mlp_train_step of 1000 rows from 57.8 to 55.4, of 4096 from 60.1 to 57.5.  As separate
+// GEMM launches, whose hand-overs wrote h1 and h2 (and their transposes) to global memory with 2-byte stores one
+// row stride apart per lane, the gradients took 560.
 //
 // Every barrier wait is bounded; a CTA that gives up waits (bounded) for its MMAs and copies, raises *err,
 // frees its TMEM and returns.

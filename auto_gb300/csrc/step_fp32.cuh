@@ -7,7 +7,7 @@
 //
 //   column pass (per world, channel, tile of TC = 2 spectrum columns, kernel k reading it):
 //       forward FFT along y  ->  x khat_k (real, even; includes 1/(W*H))  ->  inverse FFT along y
-//   row pass (per world, block of 4 rows; Lenia: and target channel):
+//   row pass (per world, block of 2 to 8 rows; Lenia: and target channel):
 //       inverse real FFT along x of U_k  ->  growth, dt, clamp (spectral.rs:337-345)  ->
 //       write state  ->  forward real FFT along x of the new rows  ->  write spectrum
 //
@@ -17,7 +17,8 @@
 //
 // The column pass is built twice: scalar (col_pass: a thread runs a butterfly of one column) and
 // paired (col_pass_pair: a thread runs the same butterfly of both columns of the tile as f32x2
-// pairs, half the threads and instructions); launch variant 2 selects the paired build.
+// pairs, half the threads and instructions); launch variant 2 selects the paired build, the default from
+// 3072 to 6144.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -61,7 +62,7 @@ __device__ __forceinline__ void static_for(F&& f) {
 // Stages [I, I1) of the transform of S sequences of length N in shared memory (stride
 // seq_stride(N)), in place, by NT threads; stw holds the per-stage twiddle tables
 // (fill_stage_twiddles).  Starts after the caller's barrier; ends with a barrier.
-// MR: the plan's radix cap (make_plan); 16 for every pass but the scalar column pass.
+// MR: the plans (ROW_PLAN, COL_PLAN, or make_plan's radix cap): COL_PLAN in the scalar column pass only.
 template <int N, int S, int NT, bool INV, int I, int I1, int MR = ROW_PLAN, class T, class W>
 __device__ __forceinline__ void fft_stages(T* buf, const W* stw) {
     static_assert(MR != COL_PLAN || sizeof(T) == sizeof(float2), "radix-32 plans are built for scalar elements only");
