@@ -135,6 +135,8 @@ void launch_seed_patches(float* state, int W, int H, uint32_t seed, const int4* 
                          cudaStream_t s);
 void launch_seed_tiles(float* state, int W, int H, uint32_t seed, const float* pattern, int pw, int ph,
                        int spacing, cudaStream_t s);
+// count floats, a multiple of 4, between 16-byte aligned places
+void launch_copy_words(float* dst, const float* src, size_t count, cudaStream_t s);
 // max_sides: the largest W + H of the worlds
 bool launch_world_stats(const DevWorld* worlds, int nworlds, int max_sides, float* out, cudaStream_t s);
 void launch_seed_rule(float* state, int W, int H, uint32_t seed, int kind, cudaStream_t s);

@@ -180,6 +180,12 @@ __global__ void __launch_bounds__(STATS_NT) world_stats_kernel(const DevWorld* _
     }
 }
 
+// States between device memory and the caller's pageable memory in place (see in_place in ctx.cu), one 16-byte word a
+// thread so that enough are in flight to cover the link's latency.
+__global__ void copy_words_kernel(float4* __restrict__ dst, const float4* __restrict__ src, unsigned n) {
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
+}
+
 static int grid_for(size_t n) {
     size_t g = (n + 255) / 256;
     return (int)(g > 152 * 32 ? 152 * 32 : (g < 1 ? 1 : g));
@@ -202,6 +208,11 @@ void launch_render(const float* state, int W, int H, float ox, float oy, float s
                    int palette, uchar4* out, cudaStream_t s) {
     const dim3 blk(16, 16), grd((out_w + 15) / 16, (out_h + 15) / 16);
     render_kernel<<<grd, blk, 0, s>>>(state, W, H, ox, oy, scale, n, out_w, out_h, palette, out);
+}
+
+void launch_copy_words(float* dst, const float* src, size_t count, cudaStream_t s) {
+    copy_words_kernel<<<grid_for(count / 4), 256, 0, s>>>(reinterpret_cast<float4*>(dst), reinterpret_cast<const float4*>(src),
+                                                          (unsigned)(count / 4));
 }
 
 bool launch_world_stats(const DevWorld* worlds, int nworlds, int max_sides, float* out, cudaStream_t s) {
