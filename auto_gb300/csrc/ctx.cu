@@ -6,7 +6,6 @@
 // steps.  Worlds of one grid size form a size class; each class is one column launch and one
 // row launch per step over all of its worlds, and the graph runs the classes one after another.
 #include <cuda_runtime.h>
-#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -994,33 +993,13 @@ int setup_radix2(LeniaCtx* ctx) {
 
 float* state_ptr(LeniaCtx* ctx, int w) { return ctx->path == LENIA_PATH_RADIX2 ? ctx->r2[w].state : ctx->hw[w].state; }
 
-// Whether a kernel copies a state from or to the caller's memory where it is: pageable memory that the GPU reaches through
-// the host's page tables, 16-byte aligned, of at most 1 MiB.  The copy itself takes as long as the driver's (14 us for 256
-// KB), but the passes before and after it follow on the same engine: a frame (state in, one generation, state out) of a 256 x
-// 256 world 49.1 -> 41.8 us, of 512 x 512 57.3 -> 52.3.  Above, the driver reaches the link's rate as well, and pages that
-// are not there yet cost more from the GPU (64 MiB read into fresh pages 3.7 -> 21.5 ms).  Up to 64 KiB the driver stages a
-// write and returns at once.
-constexpr size_t WRITE_STAGED = 64 << 10, IN_PLACE_MAX = 1 << 20;
+// Whether a kernel copies a state from or to the caller's memory where it is (pageable_in_place).  The copy itself takes as
+// long as the driver's (14 us for 256 KB), but the passes before and after it follow on the same engine: a frame (state in, one
+// generation, state out) of a 256 x 256 world 49.1 -> 41.8 us, of 512 x 512 57.3 -> 52.3.  Up to 64 KiB the driver stages
+// a write and returns at once.
+constexpr size_t WRITE_STAGED = 64 << 10;
 bool in_place(const LeniaCtx* ctx, const float* host, size_t count) {
-    if (!ctx->reads_host || ((uintptr_t)host & 15) || (count & 3) || count * sizeof(float) > IN_PLACE_MAX) return false;
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeUnregistered;
-}
-// Touches every page from the host first: pages not there yet get their place from the host and a bad range faults
-// there, not on the GPU.
-void touch_pages(float* p, size_t bytes, bool write) {
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    volatile char* c = reinterpret_cast<volatile char*>(p);
-    auto touch = [&](size_t at) {
-        const char v = c[at];
-        if (write) c[at] = v;
-    };
-    for (size_t at = 0; at < bytes; at += page) touch(at);
-    touch(bytes - 1);
+    return (count & 3) == 0 && pageable_in_place(ctx->reads_host, host, count * sizeof(float));
 }
 
 // Device time of `steps` steps of one size class in the graph's order (chunk after chunk, each for

@@ -135,6 +135,14 @@ void launch_seed_patches(float* state, int W, int H, uint32_t seed, const int4* 
                          cudaStream_t s);
 void launch_seed_tiles(float* state, int W, int H, uint32_t seed, const float* pattern, int pw, int ph,
                        int spacing, cudaStream_t s);
+// Whether kernels take a range of the caller's memory where it is: pageable memory that the GPU reaches through the host's page
+// tables (reads_host: cudaDevAttrPageableMemoryAccessUsesHostPageTables), 16-byte aligned, of at most 1 MiB.  Above, the
+// driver's copies reach the link's rate as well, and pages that are not there yet cost more from the GPU (64 MiB into
+// fresh pages 3.7 -> 21.5 ms).
+bool pageable_in_place(int reads_host, const void* p, size_t bytes);
+// Touches every page of such a range from the host first: pages not there yet get their place from the host, and a bad
+// range faults there, not on the GPU.
+void touch_pages(void* p, size_t bytes, bool write);
 // count floats, a multiple of 4, between 16-byte aligned places
 void launch_copy_words(float* dst, const float* src, size_t count, cudaStream_t s);
 // max_sides: the largest W + H of the worlds

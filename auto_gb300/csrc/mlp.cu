@@ -582,6 +582,11 @@ __global__ void to_bf16(const float* __restrict__ x, bf16* __restrict__ y, int n
     if (i < n) y[i] = __float2bfloat16_rn(x[i]);
 }
 
+__global__ void copy_out(const float* __restrict__ x, float* __restrict__ y, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) y[i] = x[i];
+}
+
 // Adam on the FP32 master weights, refreshing their BF16 copies.
 __global__ void adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                      bf16* __restrict__ wb, int n, float lr, float b1, float b2, float eps, float c1, float c2) {
@@ -802,7 +807,15 @@ LENIA_API int lenia_mlp_gradients(LeniaMlp* n, const float* x, const float* y, u
     }
     if (int rc = batch_gradients(n, x, y, batch)) return rc;
     if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
-    cudaMemcpyAsync(grads, n->g, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream);
+    // straight into the caller's memory where kernels reach it: 1000 rows 65.3 -> 62.7 us against the driver's copy, which
+    // waits for a change of engine
+    if (pageable_in_place(n->reads_host, grads, NPARAM * 4)) {
+        touch_pages(grads, NPARAM * 4, true);  // beside the tiles
+        copy_out<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->g, grads, NPARAM);
+        if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
+    } else {
+        cudaMemcpyAsync(grads, n->g, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream);
+    }
     return mean_loss(n, batch, loss);
 }
 
@@ -826,12 +839,19 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
         return LENIA_EINVAL;
     }
     if (in_place(n, x)) {
-        for (uint64_t off = 0; off < count; off += DIRECT_ROWS) {
-            const uint32_t B = count - off < DIRECT_ROWS ? (uint32_t)(count - off) : DIRECT_ROWS;
-            mlp_rank<<<tiles_grid(n, (int)B), NRANK, RANK_SMEM, n->ps[0]>>>(x + off * IN, (int)B, n->w, n->wb, n->pp, n->err);
-            if (cudaMemcpyAsync(probs + off * OUT, n->pp, (size_t)B * OUT * 4, cudaMemcpyDeviceToHost, n->ps[0]) !=
-                cudaSuccess)
-                return err("mlp: download failed");
+        if (count > 0 && pageable_in_place(n->reads_host, probs, (size_t)count * OUT * 4)) {
+            // no copy after the tiles: 1000 rows 30.5 -> 25.3 us, 19456 47.9 -> 36.0, 65536 74.0 -> 67.4
+            touch_pages(probs, (size_t)count * OUT * 4, true);
+            mlp_rank<<<tiles_grid(n, (int)count), NRANK, RANK_SMEM, n->ps[0]>>>(x, (int)count, n->w, n->wb, probs, n->err);
+            if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
+        } else {
+            for (uint64_t off = 0; off < count; off += DIRECT_ROWS) {
+                const uint32_t B = count - off < DIRECT_ROWS ? (uint32_t)(count - off) : DIRECT_ROWS;
+                mlp_rank<<<tiles_grid(n, (int)B), NRANK, RANK_SMEM, n->ps[0]>>>(x + off * IN, (int)B, n->w, n->wb, n->pp, n->err);
+                if (cudaMemcpyAsync(probs + off * OUT, n->pp, (size_t)B * OUT * 4, cudaMemcpyDeviceToHost, n->ps[0]) !=
+                    cudaSuccess)
+                    return err("mlp: download failed");
+            }
         }
         if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess) return err("mlp: predict failed");
         return check_err(n);

@@ -5,6 +5,7 @@
 // the PCG hash of program.rs:140-147; the tile seeder follows spectral.rs:313-335 with the
 // pattern passed in by the caller.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include "engine.cuh"
 
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(STATS_NT) world_stats_kernel(const DevWorld* _
     }
 }
 
-// States between device memory and the caller's pageable memory in place (see in_place in ctx.cu), one 16-byte word a
+// Words between device memory and the caller's pageable memory in place (pageable_in_place), one 16-byte word a
 // thread so that enough are in flight to cover the link's latency.
 __global__ void copy_words_kernel(float4* __restrict__ dst, const float4* __restrict__ src, unsigned n) {
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
@@ -208,6 +209,27 @@ void launch_render(const float* state, int W, int H, float ox, float oy, float s
                    int palette, uchar4* out, cudaStream_t s) {
     const dim3 blk(16, 16), grd((out_w + 15) / 16, (out_h + 15) / 16);
     render_kernel<<<grd, blk, 0, s>>>(state, W, H, ox, oy, scale, n, out_w, out_h, palette, out);
+}
+
+bool pageable_in_place(int reads_host, const void* p, size_t bytes) {
+    if (!reads_host || ((uintptr_t)p & 15) || bytes > (1u << 20)) return false;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+void touch_pages(void* p, size_t bytes, bool write) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char* c = static_cast<volatile char*>(p);
+    auto touch = [&](size_t at) {
+        const char v = c[at];
+        if (write) c[at] = v;
+    };
+    for (size_t at = 0; at < bytes; at += page) touch(at);
+    touch(bytes - 1);
 }
 
 void launch_copy_words(float* dst, const float* src, size_t count, cudaStream_t s) {

@@ -1,0 +1,63 @@
+"""The proposer's results in the caller's memory of every kind (aligned, 4 bytes off, page-locked, fresh), on both sides of the
+1 MiB up to which kernels write it in place (87,381 rows of three probabilities).
+
+Probabilities: a row's arithmetic does not depend on where it goes: equal bits.  Gradients: tiles meet in float additions of
+any order; 8 tiles of sums below 1 differ by at most 8 * 2^-24 of the sums' magnitude; bound 2e-6 of each tensor's largest."""
+import ctypes
+import mmap
+
+import numpy as np
+import pytest
+
+from auto_gb300.screen import Proposer
+
+pytestmark = pytest.mark.gpu
+P = ctypes.POINTER(ctypes.c_float)
+
+
+def memory(kind, n):
+    if kind == "aligned":
+        return np.full(n + 16, np.nan, np.float32)[:n]
+    if kind == "off":
+        a = np.full(n + 16, np.nan, np.float32)
+        k = 1 + (-(a.ctypes.data // 4)) % 4
+        return a[k:k + n]
+    if kind == "fresh":
+        return np.frombuffer(mmap.mmap(-1, 4 * n), np.float32)
+    torch = pytest.importorskip("torch")
+    return torch.full((n,), float("nan"), pin_memory=True).numpy()
+
+
+def ptr(a):
+    return ctypes.cast(a.ctypes.data, P)
+
+
+@pytest.mark.parametrize("rows", [1, 127, 1000, 87381, 87382])
+def test_probabilities(rows):
+    p = Proposer(seed=3, max_batch=1024)
+    x = np.random.default_rng(rows).random((rows, 16), dtype=np.float32)
+    got = []
+    for kind in ("off", "aligned", "fresh", "pinned"):
+        out = memory(kind, 3 * rows)
+        assert p.L.lenia_mlp_predict(p.h, ptr(x), rows, ptr(out)) == 0
+        got.append(out.copy())
+    assert np.isfinite(got[0]).all()
+    for g in got[1:]:
+        np.testing.assert_array_equal(g, got[0])
+
+
+@pytest.mark.parametrize("rows", [1, 1000])
+def test_gradients(rows):
+    p = Proposer(seed=3, max_batch=1024)
+    r = np.random.default_rng(rows)
+    x, y = r.random((rows, 16), dtype=np.float32), (r.random((rows, 3)) < 0.3).astype(np.float32)
+    got = []
+    for kind in ("off", "aligned", "fresh", "pinned"):
+        out, loss = memory(kind, p.nparam), ctypes.c_float()
+        assert p.L.lenia_mlp_gradients(p.h, ptr(x), ptr(y), rows, ptr(out), ctypes.byref(loss)) == 0
+        got.append(out.copy())
+    for lo, hi in ((0, 4096), (4096, 4352), (4352, 69888), (69888, 70144), (70144, 70912), (70912, 70915)):
+        top = np.abs(got[0][lo:hi]).max()
+        assert top > 0
+        for g in got[1:]:
+            assert np.abs(g[lo:hi] - got[0][lo:hi]).max() <= 2e-6 * top
