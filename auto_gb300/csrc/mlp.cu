@@ -667,18 +667,32 @@ int check_err(LeniaMlp* n) {
     return 0;
 }
 
-// Whether a kernel may read host rows where they are: the GPU walks the host's page tables (Grace) and the rows are
-// aligned for its 16-byte loads.  Against copying them first, lenia_mlp_predict of 250001 rows 336 -> 188 us, of
-// 1000 rows 50 -> 42, lenia_mlp_gradients of 1000 rows 84 -> 72.
-bool in_place(const LeniaMlp* n, const float* rows) { return n->reads_host && ((uintptr_t)rows & 15) == 0; }
+// Whether a kernel may read host rows where they are: the GPU walks the host's page tables (Grace), the rows are aligned
+// for its loads (16 bytes, labels 4), and they are the host's (a device pointer is for the copy to refuse).  Against copying them
+// first, lenia_mlp_predict of 250001 rows 336 -> 188 us, of 1000 rows 50 -> 42, lenia_mlp_gradients of 1000 rows 84 -> 72.
+bool in_place(const LeniaMlp* n, const float* rows, uintptr_t align = 16) {
+    if (!n->reads_host || (uintptr_t)rows % align) return false;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, rows) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type != cudaMemoryTypeDevice;
+}
+
+// Reads the last of a range that a kernel will read in place: a range that is too short faults on the host.
+void touch_last(const float* p, size_t count) { touch_pages(const_cast<float*>(p) + count - 1, sizeof(float), false); }
 
 // The batch's gradients from host rows, copied first where they cannot be read in place.
 int batch_gradients(LeniaMlp* n, const float* x, const float* y, uint32_t B) {
-    if (!in_place(n, x)) {
+    if (!in_place(n, x) || !in_place(n, y, 4)) {
         if (cudaMemcpyAsync(n->x, x, (size_t)B * IN * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess ||
             cudaMemcpyAsync(n->y, y, (size_t)B * OUT * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess)
             return err("mlp: upload failed");
         x = n->x, y = n->y;
+    } else {
+        touch_last(x, (size_t)B * IN);
+        touch_last(y, (size_t)B * OUT);
     }
     gradients(n, x, y, (int)B);
     return 0;
@@ -839,6 +853,7 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
         return LENIA_EINVAL;
     }
     if (in_place(n, x)) {
+        if (count > 0) touch_last(x, (size_t)count * IN);
         if (count > 0 && pageable_in_place(n->reads_host, probs, (size_t)count * OUT * 4)) {
             // no copy after the tiles: 1000 rows 30.5 -> 25.3 us, 19456 47.9 -> 36.0, 65536 74.0 -> 67.4
             touch_pages(probs, (size_t)count * OUT * 4, true);

@@ -61,3 +61,28 @@ def test_gradients(rows):
         assert top > 0
         for g in got[1:]:
             assert np.abs(g[lo:hi] - got[0][lo:hi]).max() <= 2e-6 * top
+
+
+@pytest.mark.parametrize("shift", [1, 2, 4, 8])
+def test_rows_and_labels_at_any_address(shift):
+    """Inputs `shift` bytes past a 16-byte boundary give what aligned ones give."""
+    rows, r = 300, np.random.default_rng(shift)
+    x, y = r.random((rows, 16), dtype=np.float32), (r.random((rows, 3)) < 0.3).astype(np.float32)
+    p = Proposer(seed=3, max_batch=512)
+
+    def moved(a):
+        b = np.zeros(a.nbytes + 64, np.uint8)
+        k = -b.ctypes.data % 16 + shift
+        b[k:k + a.nbytes] = a.view(np.uint8).reshape(-1)
+        return b, ctypes.cast(b.ctypes.data + k, P)
+
+    (bx, px), (by, py) = moved(x), moved(y)
+    got = []
+    for ax, ay in ((ptr(x), ptr(y)), (px, ptr(y)), (ptr(x), py), (px, py)):
+        out, probs, loss = np.empty(p.nparam, np.float32), np.empty(3 * rows, np.float32), ctypes.c_float()
+        assert p.L.lenia_mlp_gradients(p.h, ax, ay, rows, ptr(out), ctypes.byref(loss)) == 0
+        assert p.L.lenia_mlp_predict(p.h, ax, rows, ptr(probs)) == 0
+        got.append((out, probs, loss.value))
+    for g, q, l in got[1:]:
+        np.testing.assert_array_equal(q, got[0][1])
+        assert np.abs(g - got[0][0]).max() <= 2e-6 * np.abs(got[0][0]).max() and abs(l - got[0][2]) <= 1e-6
