@@ -24,7 +24,7 @@ size_t col_smem_bytes(int H) {
 size_t row_smem_bytes(int W, int acc_planes) {
     switch (W) {
 #define RS_CASE(N) \
-    case N: return acc_planes > 0 ? row_smem<N, true>(1, acc_planes) : row_smem<N, false>(0, 0);
+    case N: return acc_planes > 0 ? row_smem<N, true>() : row_smem<N, false>();
         LENIA_SIZES_SMALL(RS_CASE) LENIA_SIZES_LARGE(RS_CASE)
 #undef RS_CASE
     }

@@ -346,14 +346,6 @@ constexpr int row_minb() {
 // 1024 worlds of 256 x 256 233 -> 222, one of 1024 x 1024 11.1 -> 10.3, 4096 x 4096 109.7 -> 103.0.
 template <int W, int V>
 constexpr bool row_wide() { return !(V == 1 && W <= 384); }
-// Shared memory after the sequences and stage tables: the accumulation planes ([planes][2S][W]) of
-// the general path.
-template <int W>
-__device__ __forceinline__ float* row_extra_smem(float2* stw) {
-    constexpr int TWS = tables_size<W>();
-    return reinterpret_cast<float*>(((uintptr_t)(stw + TWS) + 15) & ~(uintptr_t)15);
-}
-
 // Half-spectra of rows r0..r0+2S-1 (tile layout) <-> S packed complex sequences Z_p = A + iB with A = row
 // r0+2p, B = row r0+2p+1, using Hermitian symmetry for k > W/2.
 // A lane moves 32 bytes: both columns (kx = 2t, 2t+1) of one tile t for one row pair p, consecutive lanes on the
@@ -565,8 +557,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     extern __shared__ float4 smem_raw[];
     constexpr int SEQ = seq_stride(W);
     float2* Z = reinterpret_cast<float2*>(smem_raw);
-    float2* stw = Z + S * SEQ;
-    float* extra = row_extra_smem<W>(stw);
+    float2* stw = Z + (GEN ? 2 : 1) * S * SEQ;
     const RowItem it = items[blockIdx.x / SPLIT];
     const DevWorld& wd = worlds[it.world];
     fill_tables<W>(stw, tw, NT);
@@ -598,12 +589,12 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     // MNCA keep the first kernel's U.  The last kernel runs chained (fft_fused): its last inverse
     // stage, the rule's update with the plane and the state, and the first forward stage stay in
     // registers.  A thread owns the same cells (sequence s, x = j + m*N/R) in all of these stages,
-    // so the plane needs no barrier of its own.
+    // so the plane needs no barrier of its own.  It lies where the second kernel's sequences do below.
     const int rule = wd.rule;
     constexpr int R = chain_radix<W>(), NB = W / R;
     static_assert(fusable<W>(), "row widths need a plan with equal first and last radix");
     static_assert(S * NB <= NT, "one butterfly per thread in the chained stages");
-    float* acc = extra;  // [ROWS][W]
+    float* acc = reinterpret_cast<float*>(Z + S * SEQ);  // [ROWS][W]
     int nk = 0, klast = -1;
     for (int k = 0; k < K; k++)
         if (!per_chan || wd.kern[k].dst == d0) nk++, klast = k;
@@ -616,6 +607,63 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
         return;
     }
     if (threadIdx.x == 0) tc::bulk_prefetch_l2(st, ROWS * W * (uint32_t)sizeof(float));
+    const uint64_t stream = hint::policy_stream();
+    // Two kernels up to 128 wide: the launch is bound by an item's latency, so both spectra are loaded at once, both inverse
+    // transforms share their barriers (2S sequences), and nothing goes through the plane.  Same bits.  SmoothLife 64 x 64
+    // 6.3 -> 5.2 us a generation, 128 x 1024 9.3 -> 8.3, two channels of 128 x 128 6.6 -> 6.0.  Wider items hold 16 elements
+    // a thread and lose: 256 x 256 10.0 -> 12.6, 512 x 512 11.5 -> 15.3, 2048 x 2048 48.5 -> 51.0.
+    constexpr bool PAIR = W <= 128 && NT * MINB <= 512;
+    if (PAIR && nk == 2) {
+        int k0 = 0;
+        while (per_chan && wd.kern[k0].dst != d0) k0++;
+        const DevKernel kp = wd.kern[k0], kq = wd.kern[klast];
+        load_rows_spectrum<W, S, NT, false, WIDE>(Z, wd.conv + k0 * cplane, H, r0);
+        load_rows_spectrum<W, S, NT, false, WIDE>(Z + S * SEQ, wd.conv + klast * cplane, H, r0);
+        __syncthreads();
+        fft_head<W, 2 * S, NT, true>(Z, stw);
+        const Growth gp(kp.mu, kp.sigma), gq(kq.mu, kq.sigma);
+        const float dt = wd.dt;
+        const int s = threadIdx.x / NB, j = threadIdx.x - s * NB;
+        const bool on = S * NB == NT || (int)threadIdx.x < S * NB;
+        float2 v[R];
+        if (on) {
+            float sa[R], sb[R];
+            float* ga = st + (2 * s) * W + j;
+#pragma unroll
+            for (int m = 0; m < R; m++) {
+                sa[m] = hint::ld1(ga + m * NB, stream);
+                sb[m] = hint::ld1(ga + W + m * NB, stream);
+            }
+            float2 u[R];
+            chain_load<W, true>(Z + s * SEQ, j, u, stw);
+            chain_load<W, true>(Z + (S + s) * SEQ, j, v, stw);
+#pragma unroll
+            for (int m = 0; m < R; m++) {
+                float n0, n1;
+                if (rule == LENIA_RULE_LENIA) {
+                    n0 = clamp01(sa[m] + dt * __fmaf_rn(kq.weight, gq(v[m].x), __fmul_rn(kp.weight, gp(u[m].x))));
+                    n1 = clamp01(sb[m] + dt * __fmaf_rn(kq.weight, gq(v[m].y), __fmul_rn(kp.weight, gp(u[m].y))));
+                } else if (rule == LENIA_RULE_SMOOTHLIFE) {
+                    n0 = smoothlife_update(sa[m], u[m].x, v[m].x);
+                    n1 = smoothlife_update(sb[m], u[m].y, v[m].y);
+                } else {
+                    n0 = mnca_update(sa[m], u[m].x, v[m].x);
+                    n1 = mnca_update(sb[m], u[m].y, v[m].y);
+                }
+                hint::st1(ga + m * NB, n0, stream);
+                hint::st1(ga + W + m * NB, n1, stream);
+                v[m] = make_float2(n0, n1);
+            }
+            Dft<R, false>::run(v);
+        }
+        __syncthreads();
+        if (on) chain_store<W>(Z + s * SEQ, j, v);
+        __syncthreads();
+        fft_tail<W, S, NT, false>(Z, stw);
+        if (early) grid_trigger();
+        store_rows_spectrum<W, S, NT, WIDE>(Z, wd.spec + d0 * cplane, H, r0);
+        return;
+    }
     bool first = true;
     for (int k = 0; k < klast; k++) {
         const DevKernel kp = wd.kern[k];
@@ -632,7 +680,7 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
 #pragma unroll
             for (int m = 0; m < R; m++) {
                 if (rule == LENIA_RULE_LENIA) {
-                    const float g0 = kp.weight * growth(v[m].x), g1 = kp.weight * growth(v[m].y);
+                    const float g0 = __fmul_rn(kp.weight, growth(v[m].x)), g1 = __fmul_rn(kp.weight, growth(v[m].y));
                     a[m * NB] = first ? g0 : a[m * NB] + g0;
                     a[W + m * NB] = first ? g1 : a[W + m * NB] + g1;
                 } else {
@@ -648,7 +696,6 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
     const Growth growth(kp.mu, kp.sigma);
     const float dt = wd.dt;
     const bool have_acc = nk > 1;
-    const uint64_t stream = hint::policy_stream();
     load_rows_spectrum<W, S, NT, false, WIDE>(Z, wd.conv + klast * cplane, H, r0);
     __syncthreads();
     float sa[R], sb[R];
@@ -661,8 +708,9 @@ __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict_
             for (int m = 0; m < R; m++) {
                 float n0, n1;
                 if (rule == LENIA_RULE_LENIA) {
-                    float t0 = kp.weight * growth(v[m].x), t1 = kp.weight * growth(v[m].y);
-                    if (have_acc) t0 = a[m * NB] + t0, t1 = a[W + m * NB] + t1;
+                    const float g0 = growth(v[m].x), g1 = growth(v[m].y);
+                    const float t0 = have_acc ? __fmaf_rn(kp.weight, g0, a[m * NB]) : kp.weight * g0;
+                    const float t1 = have_acc ? __fmaf_rn(kp.weight, g1, a[W + m * NB]) : kp.weight * g1;
                     n0 = clamp01(sa[m] + dt * t0);
                     n1 = clamp01(sb[m] + dt * t1);
                 } else if (rule == LENIA_RULE_SMOOTHLIFE) {
@@ -1049,10 +1097,8 @@ bool col_go_pair(const DevWorld* worlds, const ColItem* items, int nitems, const
 // Shared memory of a row-pass launch: sequences, stage tables, then the general path's
 // accumulation planes.
 template <int W, bool GEN>
-constexpr size_t row_smem(int general, int planes, int seqs = row_seqs(W, GEN)) {
-    const int rows = 2 * seqs;
-    return (size_t)seqs * seq_stride(W) * sizeof(float2) + stage_table_bytes<W>() +
-           (size_t)(general ? planes : 0) * rows * W * sizeof(float);
+constexpr size_t row_smem(int seqs = row_seqs(W, GEN)) {
+    return (size_t)(GEN ? 2 : 1) * seqs * seq_stride(W) * sizeof(float2) + stage_table_bytes<W>();
 }
 
 template <int W, int V, bool GEN>
@@ -1060,7 +1106,7 @@ bool row_go(int mode, int general, int planes, const DevWorld* worlds, const Row
             const float2* tw, LaunchOn s) {
     constexpr int S = row_cta_seqs(W, V, GEN), NT = row_nt<W, GEN, V>();
     constexpr auto kernel = row_pass<W, NT, row_minb<W, V, GEN>(), S, GEN, row_wide<W, V>()>;
-    const size_t smem = row_smem<W, GEN>(general, planes, S);
+    const size_t smem = row_smem<W, GEN>(S);
     static int attr_max = 0;
     if ((int)smem > attr_max) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=

@@ -1,6 +1,5 @@
-"""The general row pass (several channels or kernels) where its launch has between two and three items an SM, which
-takes the 80-register build, and the same worlds with the 128-register one: equal bits, and a step within 1e-5 of FP64,
-the parity tests' bound."""
+"""The general row pass (several channels or kernels) in its 80- and its 128-register build: the default (80 where a launch
+has between two and three items an SM), equal bits, and a step within 1e-5 of FP64, the parity tests' bound."""
 import numpy as np
 import pytest
 
@@ -12,11 +11,12 @@ pytestmark = pytest.mark.gpu
 
 
 def world(w, h, channels):
-    kernels = [ag.Kernel(radius=8.0 + 3 * s + d, beta=[1.0, 0.5][: 1 + (s + d) % 2], mu=0.3, sigma=0.06, src=s, dst=d,
+    r = 8.0 if min(w, h) >= 64 else 4.0
+    kernels = [ag.Kernel(radius=r + 3 * s + d, beta=[1.0, 0.5][: 1 + (s + d) % 2], mu=0.3, sigma=0.06, src=s, dst=d,
                          weight=1.0 / channels)
                for s in range(channels) for d in range(channels)]
     if channels == 1:
-        kernels.append(ag.Kernel(radius=15.0, mu=0.25, sigma=0.05, weight=0.5))
+        kernels.append(ag.Kernel(radius=r + 7.0, mu=0.25, sigma=0.05, weight=0.5))
     return ag.World(w, h, kernels, channels=channels, dt=0.05)
 
 
@@ -28,6 +28,15 @@ def world(w, h, channels):
     (1024, 768, 3, 1),
     (512, 1024, 3, 1),   # 384, but six CTAs of 128 threads fit an SM
     (2048, 768, 1, 1),
+    # two kernels a target at narrow widths: both inverse transforms at once in the 128-register build, one after
+    # the other through the plane in the other
+    (32, 64, 1, 1),
+    (48, 32, 2, 1),
+    (64, 64, 1, 1),
+    (96, 128, 2, 1),
+    (128, 96, 1, 1),
+    (128, 1024, 2, 1),
+    (192, 64, 1, 1),
 ])
 def test_general_row_builds(w, h, channels, default):
     wd = world(w, h, channels)
