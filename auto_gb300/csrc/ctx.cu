@@ -49,7 +49,7 @@ struct SizeClass {
     int var_col = 0, var_row = 0;  // launch variants (see launch_col_fp32)
     int var_tc = 1;                // tensor-core column pass variant (launch_col_tc): 1 measured 4-7% faster
                                    // than 0 at 512 and 1024 (batched BF16x3), equal at 256
-    int general = 0, planes = 0;
+    int general = 0;
     size_t bytes = 0;          // device bytes the class's worlds touch in a step
     size_t chunk_budget = 0;   // largest chunk in bytes (0: the whole class is one chunk)
     std::vector<Chunk> chunks;
@@ -399,14 +399,14 @@ int flush_spectra(LeniaCtx* ctx) {
         if (n == 0) continue;
         bool ok = true;
         if (n == cl.worlds.size()) {
-            ok = launch_row_fp32(cl.W, cl.var_row, MODE_FORWARD, cl.general, ctx->d_worlds, cl.d_row, cl.nrow, cl.planes,
+            ok = launch_row_fp32(cl.W, cl.var_row, MODE_FORWARD, cl.general, ctx->d_worlds, cl.d_row, cl.nrow,
                                  ctx->d_tw, ctx->stream);
         } else {
             for (int w : cl.worlds) {
                 if (!ctx->dirty[w]) continue;
                 const WorldBuffers& b = ctx->wb[w];
                 ok = ok && launch_row_fp32(cl.W, cl.var_row, MODE_FORWARD, cl.general, ctx->d_worlds, b.d_row, b.nrow,
-                                           cl.planes, ctx->d_tw, ctx->stream);
+                                           ctx->d_tw, ctx->stream);
             }
         }
         if (!ok) return fail(ctx, LENIA_ECUDA, "row transform launch failed for %dx%d", cl.W, cl.H);
@@ -449,7 +449,7 @@ bool launch_rows_step(LeniaCtx* ctx, const SizeClass& cl, int variant, const Row
         const int st = cl.tc_row_stride, ngroups = st > 0 ? nrow / st : nrow * -st;
         return launch_row_tc(ctx->tc, ctx->path, cl.W, ctx->d_worlds, items, st, ngroups, ctx->d_tw, s);
     }
-    return launch_row_fp32(cl.W, variant, MODE_STEP, cl.general, ctx->d_worlds, items, nrow, cl.planes, ctx->d_tw,
+    return launch_row_fp32(cl.W, variant, MODE_STEP, cl.general, ctx->d_worlds, items, nrow, ctx->d_tw,
                            LaunchOn(s, overlap, early));
 }
 
@@ -780,7 +780,6 @@ int setup_fused(LeniaCtx* ctx) {
             const LeniaWorldDesc& d = ctx->desc[wi];
             if (!(d.channels == 1 && d.nkernels == 1 && d.rule == LENIA_RULE_LENIA)) general = 1;
         }
-        const int planes = general;  // the general step's one shared-memory plane
         const uint32_t item_rows = (uint32_t)row_item_rows(cl.W, general);
         // tensor-core groups of CT columns, except the first group of every channel: column 0
         // packs the DC and Nyquist columns, which the FP32 pass pairs up (ky with H - ky)
@@ -813,11 +812,9 @@ int setup_fused(LeniaCtx* ctx) {
             b.nrow = (int)row.size() - first_row;
             b.ntcg = (int)tcg.size() - first_tcg;
         }
-        if ((int)col_smem_bytes(cl.H) > smem_max || (int)row_smem_bytes(cl.W, planes) > smem_max)
-            return fail(ctx, LENIA_ESIZE, "%dx%d with %d planes needs more shared memory than a CTA has", cl.W, cl.H,
-                        planes);
+        if ((int)col_smem_bytes(cl.H) > smem_max || (int)row_smem_bytes(cl.W, general) > smem_max)
+            return fail(ctx, LENIA_ESIZE, "%dx%d needs more shared memory than a CTA has", cl.W, cl.H);
         cl.general = general;
-        cl.planes = planes;
         // Default launch variants (per generation; the autotuner times the others).  A height's choice
         // never changes the arithmetic with the number of worlds: variants 0, 1 and, from 2048 up, 3 run the same plan.
         // Columns: the 64-register scalar build, but the 128-register one where a thread holds 24 or 32
@@ -927,7 +924,7 @@ int setup_fused(LeniaCtx* ctx) {
             if (!launch_col_fp32(cl.H, v, ctx->d_worlds, cl.d_col, 0, ctx->d_tw, ctx->stream))
                 return fail(ctx, LENIA_ECUDA, "cannot configure launches for %dx%d", cl.W, cl.H);
         for (int v = 0; v < 2; v++)
-            if (!launch_row_fp32(cl.W, v, MODE_STEP, cl.general, ctx->d_worlds, cl.d_row, 0, cl.planes, ctx->d_tw,
+            if (!launch_row_fp32(cl.W, v, MODE_STEP, cl.general, ctx->d_worlds, cl.d_row, 0, ctx->d_tw,
                                  ctx->stream))
                 return fail(ctx, LENIA_ECUDA, "cannot configure launches for %dx%d", cl.W, cl.H);
         for (int v = 0; v < TC_COL_VARIANTS && cl.ntcg > 0; v++)
@@ -1558,7 +1555,7 @@ int lenia_read_field_u(LeniaCtx* ctx, int32_t world, int32_t kernel, float* host
     const WorldBuffers& b = ctx->wb[world];
     const SizeClass& cl = ctx->classes[b.cls];
     bool ok = launch_columns(ctx, cl, b.d_col, b.ncol, b.d_tcg, b.ntcg, cl.var_col, cl.var_tc, ctx->stream);
-    ok = ok && launch_row_fp32(cl.W, cl.var_row, MODE_U, cl.general, ctx->d_worlds, b.d_row, b.nrow, cl.planes, ctx->d_tw,
+    ok = ok && launch_row_fp32(cl.W, cl.var_row, MODE_U, cl.general, ctx->d_worlds, b.d_row, b.nrow, ctx->d_tw,
                                ctx->stream);
     if (!ok) return fail(ctx, LENIA_ECUDA, "U launch failed");
     CK(cudaGetLastError());

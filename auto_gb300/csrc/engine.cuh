@@ -88,9 +88,9 @@ bool launch_pass(void (*kernel)(P...), int grid, int threads, size_t smem, Launc
 bool launch_col_fp32(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
                      const float2* tw, LaunchOn s);
 bool launch_row_fp32(int W, int variant, int mode, int general, const DevWorld* worlds, const RowItem* items,
-                     int nitems, int acc_planes, const float2* tw, LaunchOn s);
+                     int nitems, const float2* tw, LaunchOn s);
 size_t col_smem_bytes(int H);
-size_t row_smem_bytes(int W, int acc_planes);
+size_t row_smem_bytes(int W, int general);
 // Column-pass launch variants (launch_col_fp32): 0, 1 scalar builds at two register caps, 2 the paired
 // build, 3 the scalar radix-16 build (1024) or the scalar build with one column a CTA (2048 and more)
 constexpr int COL_VARIANTS = 4;

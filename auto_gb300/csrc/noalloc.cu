@@ -144,13 +144,13 @@ LENIA_API int lenia_step_noalloc(float* state, uint32_t width, uint32_t height, 
     const int n = ncol > nrow ? ncol : nrow;
     // Zero-item launches configure both passes (shared-memory limits) before anything is enqueued,
     // so a size the passes cannot run is reported without having advanced the state.
-    if (!launch_col_fp32((int)height, 0, dw, col, 0, tw, s) || !launch_row_fp32((int)width, 0, MODE_STEP, 0, dw, row, 0, 0, tw, s))
+    if (!launch_col_fp32((int)height, 0, dw, col, 0, tw, s) || !launch_row_fp32((int)width, 0, MODE_STEP, 0, dw, row, 0, tw, s))
         return set_error(LENIA_ECUDA, "launch configuration failed; the state is unchanged");
     noalloc_prepare<<<(n + 255) / 256, 256, 0, s>>>(dw, w, col, ncol, row, nrow, rows);
-    bool ok = launch_row_fp32((int)width, 0, MODE_FORWARD, 0, dw, row, nrow, 0, tw, s);
+    bool ok = launch_row_fp32((int)width, 0, MODE_FORWARD, 0, dw, row, nrow, tw, s);
     for (uint32_t i = 0; ok && i < steps; i++) {
         ok = launch_col_fp32((int)height, 0, dw, col, ncol, tw, s) &&
-             launch_row_fp32((int)width, 0, MODE_STEP, 0, dw, row, nrow, 0, tw, s);
+             launch_row_fp32((int)width, 0, MODE_STEP, 0, dw, row, nrow, tw, s);
     }
     if (!ok) return set_error(LENIA_ECUDA, "launch configuration failed");
     e = cudaGetLastError();

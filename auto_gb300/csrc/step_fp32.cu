@@ -21,10 +21,10 @@ size_t col_smem_bytes(int H) {
     return (size_t)TC * col_stride(H) * sizeof(float2) + (scalar_tables > paired_tables ? scalar_tables : paired_tables) +
            col_khat_bytes_of(H);
 }
-size_t row_smem_bytes(int W, int acc_planes) {
+size_t row_smem_bytes(int W, int general) {
     switch (W) {
 #define RS_CASE(N) \
-    case N: return acc_planes > 0 ? row_smem<N, true>() : row_smem<N, false>();
+    case N: return general ? row_smem<N, true>() : row_smem<N, false>();
         LENIA_SIZES_SMALL(RS_CASE) LENIA_SIZES_LARGE(RS_CASE)
 #undef RS_CASE
     }
@@ -51,12 +51,12 @@ bool launch_col_fp32(int H, int variant, const DevWorld* worlds, const ColItem* 
 }
 
 bool launch_row_fp32(int W, int variant, int mode, int general, const DevWorld* worlds, const RowItem* items,
-                     int nitems, int acc_planes, const float2* tw, LaunchOn s) {
+                     int nitems, const float2* tw, LaunchOn s) {
     if (general)
-        return launch_row_group_small_general(W, variant, mode, general, acc_planes, worlds, items, nitems, tw, s) ||
-               launch_row_group_large_general(W, variant, mode, general, acc_planes, worlds, items, nitems, tw, s);
-    return launch_row_group_small_simple(W, variant, mode, general, acc_planes, worlds, items, nitems, tw, s) ||
-           launch_row_group_large_simple(W, variant, mode, general, acc_planes, worlds, items, nitems, tw, s);
+        return launch_row_group_small_general(W, variant, mode, general, worlds, items, nitems, tw, s) ||
+               launch_row_group_large_general(W, variant, mode, general, worlds, items, nitems, tw, s);
+    return launch_row_group_small_simple(W, variant, mode, general, worlds, items, nitems, tw, s) ||
+           launch_row_group_large_simple(W, variant, mode, general, worlds, items, nitems, tw, s);
 }
 
 }  // namespace lenia

@@ -1094,15 +1094,15 @@ bool col_go_pair(const DevWorld* worlds, const ColItem* items, int nitems, const
     return nitems <= 0 || launch_pass(col_pass_pair<H, NT, MINB>, nitems, NT, smem, s, worlds, items, tw, s.early);
 }
 
-// Shared memory of a row-pass launch: sequences, stage tables, then the general path's
-// accumulation planes.
+// Shared memory of a row-pass launch: sequences (in the general step twice, for a second kernel's sequences or the plane),
+// then the stage tables.
 template <int W, bool GEN>
 constexpr size_t row_smem(int seqs = row_seqs(W, GEN)) {
     return (size_t)(GEN ? 2 : 1) * seqs * seq_stride(W) * sizeof(float2) + stage_table_bytes<W>();
 }
 
 template <int W, int V, bool GEN>
-bool row_go(int mode, int general, int planes, const DevWorld* worlds, const RowItem* items, int nitems,
+bool row_go(int mode, int general, const DevWorld* worlds, const RowItem* items, int nitems,
             const float2* tw, LaunchOn s) {
     constexpr int S = row_cta_seqs(W, V, GEN), NT = row_nt<W, GEN, V>();
     constexpr auto kernel = row_pass<W, NT, row_minb<W, V, GEN>(), S, GEN, row_wide<W, V>()>;
@@ -1144,8 +1144,8 @@ bool col_go_variant(int variant, const DevWorld* worlds, const ColItem* items, i
 // hide behind.)
 #define LENIA_ROW_CASE_G(N, G)                                                                     \
     case N:                                                                                        \
-        return (variant & 1) ? row_go<N, 1, G>(mode, general, planes, worlds, items, nitems, tw, s) \
-                             : row_go<N, 0, G>(mode, general, planes, worlds, items, nitems, tw, s);
+        return (variant & 1) ? row_go<N, 1, G>(mode, general, worlds, items, nitems, tw, s) \
+                             : row_go<N, 0, G>(mode, general, worlds, items, nitems, tw, s);
 #define LENIA_ROW_CASE_SIMPLE(N) LENIA_ROW_CASE_G(N, false)
 #define LENIA_ROW_CASE_GENERAL(N) LENIA_ROW_CASE_G(N, true)
 
@@ -1154,7 +1154,7 @@ bool launch_col_group_small(int H, int variant, const DevWorld* worlds, const Co
 bool launch_col_group_large(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
                             const float2* tw, LaunchOn s);
 #define LENIA_ROW_GROUP_DECL(NAME)                                                                       \
-    bool NAME(int W, int variant, int mode, int general, int planes, const DevWorld* worlds, const RowItem* items, \
+    bool NAME(int W, int variant, int mode, int general, const DevWorld* worlds, const RowItem* items, \
               int nitems, const float2* tw, LaunchOn s);
 LENIA_ROW_GROUP_DECL(launch_row_group_small_simple)
 LENIA_ROW_GROUP_DECL(launch_row_group_small_general)
