@@ -854,7 +854,9 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
     }
     if (in_place(n, x)) {
         if (count > 0) touch_last(x, (size_t)count * IN);
-        if (count > 0 && pageable_in_place(n->reads_host, probs, (size_t)count * OUT * 4)) {
+        // probabilities over their own rows leave by copy, after every row has been read
+        const bool apart = probs + (size_t)count * OUT <= x || x + (size_t)count * IN <= probs;
+        if (count > 0 && apart && pageable_in_place(n->reads_host, probs, (size_t)count * OUT * 4)) {
             // no copy after the tiles: 1000 rows 30.5 -> 25.3 us, 19456 47.9 -> 36.0, 65536 74.0 -> 67.4
             touch_pages(probs, (size_t)count * OUT * 4, true);
             mlp_rank<<<tiles_grid(n, (int)count), NRANK, RANK_SMEM, n->ps[0]>>>(x, (int)count, n->w, n->wb, probs, n->err);

@@ -86,3 +86,13 @@ def test_rows_and_labels_at_any_address(shift):
     for g, q, l in got[1:]:
         np.testing.assert_array_equal(q, got[0][1])
         assert np.abs(g - got[0][0]).max() <= 2e-6 * np.abs(got[0][0]).max() and abs(l - got[0][2]) <= 1e-6
+
+
+def test_probabilities_over_their_own_rows():
+    rows = 20000
+    x = np.random.default_rng(1).random((rows, 16), dtype=np.float32)
+    p = Proposer(seed=3, max_batch=512)
+    want, buf = np.empty(3 * rows, np.float32), x.reshape(-1).copy()
+    assert p.L.lenia_mlp_predict(p.h, ptr(x), rows, ptr(want)) == 0
+    assert p.L.lenia_mlp_predict(p.h, ptr(buf), rows, ptr(buf)) == 0
+    np.testing.assert_array_equal(buf[:3 * rows], want)
