@@ -334,11 +334,11 @@ FFT_CHD constexpr bool size_ok(int n) {
 }
 
 // Per-stage twiddle tables.  A stage with L > 1 needs w = exp(-2 pi i k / (L R)) for k < L and,
-// when R >= 8, w^4 (and when R >= 24, w^16); they are copied once per CTA from the global table into
+// when R >= 6, w^4 (and when R >= 24, w^16); they are copied once per CTA from the global table into
 // shared memory.
 FFT_CHD constexpr int stage_tw_count(int n, int i, int maxr = 16) {
     return plan_L(n, i, maxr) > 1
-               ? (plan_radix(n, i, maxr) >= 24 ? 3 : plan_radix(n, i, maxr) >= 8 ? 2 : 1) * plan_L(n, i, maxr)
+               ? (plan_radix(n, i, maxr) >= 24 ? 3 : plan_radix(n, i, maxr) >= 6 ? 2 : 1) * plan_L(n, i, maxr)
                : 0;
 }
 FFT_CHD constexpr int stage_tw_offset(int n, int i, int maxr = 16) {
@@ -362,7 +362,7 @@ FFT_HD void fill_stage_twiddles(W* stw, const float2* tw, int tid, int nth) {
             constexpr int step = TWN / (L * R);
             for (int k = tid; k < L; k += nth) {
                 set_twiddle(stw[off + k], tw[k * step]);
-                if (R >= 8) set_twiddle(stw[off + L + k], tw[4 * k * step]);
+                if (R >= 6) set_twiddle(stw[off + L + k], tw[4 * k * step]);
                 if (R >= 24) set_twiddle(stw[off + 2 * L + k], tw[16 * k * step]);
             }
         }
@@ -376,7 +376,7 @@ FFT_HD int pad(int i) { return i + (i >> 4); }
 // sequences fall into different banks (the row pass's spectrum unpack and pack)
 FFT_CHD constexpr int seq_stride(int n) { return n + n / 16 + 4 + (29 - (n + n / 16) % 16) % 16; }
 
-// Twiddles w^m, m = 1..R-1, of one butterfly from w, (R >= 8) w^4 and (R >= 24) w^16; the other
+// Twiddles w^m, m = 1..R-1, of one butterfly from w, (R >= 6) w^4 and (R >= 24) w^16; the other
 // powers are products of at most four factors, so each stays within a few float ulps of the exactly
 // rounded value (checked against numpy by the host test).
 template <int R, class W>
@@ -384,9 +384,9 @@ FFT_HD void twiddle_powers(W w1, W w4, W w16, W* w) {
     w[1] = w1;
     if (R >= 3) w[2] = cmul(w[1], w[1]);
     if (R >= 4) w[3] = cmul(w[2], w[1]);
-    if (R == 6) {
-        w[4] = cmul(w[2], w[2]);
-        w[5] = cmul(w[3], w[2]);
+    if (R == 6) {  // with w^4 as w^2 squared the relative error at 1536 was 1.52e-7; now 1.40e-7 (16.3.2.16: 1.38e-7)
+        w[4] = w4;
+        w[5] = cmul(w[4], w[1]);
     }
     if (R >= 8) {
         w[4] = w4;
@@ -434,7 +434,7 @@ FFT_HD void stage_load(const T* seq, int j, T* v, const W* stw) {
     }
     if (L > 1) {
         W w[R];
-        twiddle_powers<R>(stw[k], R >= 8 ? stw[L + k] : stw[k], R >= 24 ? stw[2 * L + k] : stw[k], w);
+        twiddle_powers<R>(stw[k], R >= 6 ? stw[L + k] : stw[k], R >= 24 ? stw[2 * L + k] : stw[k], w);
 #pragma unroll
         for (int m = 1; m < R; m++) v[m] = INV ? cmulc(v[m], w[m]) : cmul(v[m], w[m]);
     }
