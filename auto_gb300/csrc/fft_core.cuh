@@ -134,6 +134,7 @@ FFT_HD cpair cmul(cpair a, tw2 w) { return {f2sub(f2mul(a.re, w.rr), f2mul(a.im,
 FFT_HD cpair cmulc(cpair a, tw2 w) { return {f2fma(a.im, w.ii, f2mul(a.re, w.rr)), f2sub(f2mul(a.im, w.rr), f2mul(a.re, w.ii))}; }
 FFT_HD cpair cmul(cpair a, float2 w) { return cmul(a, splat(w)); }
 FFT_HD tw2 cmul(tw2 a, tw2 b) { return {f2sub(f2mul(a.rr, b.rr), f2mul(a.ii, b.ii)), f2fma(a.rr, b.ii, f2mul(a.ii, b.rr))}; }
+FFT_HD tw2 cmulc(tw2 a, tw2 b) { return {f2fma(a.ii, b.ii, f2mul(a.rr, b.rr)), f2sub(f2mul(a.ii, b.rr), f2mul(a.rr, b.ii))}; }
 
 // exp(sign*2*pi*i*j/R) for compile-time R in {2,4,8,16,32} and j, via the 16- or 32-entry table
 template <int R, bool INV> FFT_HD float2 wR(int j) {
@@ -383,9 +384,10 @@ template <int R, class W>
 FFT_HD void twiddle_powers(W w1, W w4, W w16, W* w) {
     w[1] = w1;
     if (R >= 3) w[2] = cmul(w[1], w[1]);
-    if (R >= 4) w[3] = cmul(w[2], w[1]);
-    if (R == 6) {  // with w^4 as w^2 squared the relative error at 1536 was 1.52e-7; now 1.40e-7 (16.3.2.16: 1.38e-7)
+    if (R >= 4 && R != 6) w[3] = cmul(w[2], w[1]);
+    if (R == 6) {  // one rounding each: by squares and their products the relative error at 1536 was 1.52e-7; now 1.38e-7
         w[4] = w4;
+        w[3] = cmulc(w[4], w[1]);
         w[5] = cmul(w[4], w[1]);
     }
     if (R >= 8) {
