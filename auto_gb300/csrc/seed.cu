@@ -239,8 +239,11 @@ void launch_copy_words(float* dst, const float* src, size_t count, cudaStream_t 
 
 bool launch_world_stats(const DevWorld* worlds, int nworlds, int max_sides, float* out, cudaStream_t s) {
     const int smem = max_sides * (int)sizeof(float2);
+    // The limit is the kernel's, for all contexts and their threads: always the largest need (two sides of 8192), so that no
+    // call lowers it between another's set and launch.
+    constexpr int LIMIT = 2 * 8192 * (int)sizeof(float2);
     if (smem > 40 * 1024 &&
-        cudaFuncSetAttribute(world_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        cudaFuncSetAttribute(world_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT) != cudaSuccess)
         return false;
     world_stats_kernel<<<nworlds, STATS_NT, smem, s>>>(worlds, out);
     return true;

@@ -1,0 +1,43 @@
+"""The host code of the proposer and of the statistics (auto_gb300/csrc/mlp.cu, seed.cu) over a stand-in for the CUDA runtime
+(tests/cpp/fake_cudart.cpp): what happens when a call of the runtime fails, and in which order copies and kernels touch the
+caller's memory.  No GPU; the kernels are simple functions of the same arguments, so every value is exact."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc) or not shutil.which("g++"):
+        pytest.skip("needs nvcc and g++")
+    d = str(tmp_path_factory.mktemp("runtime"))
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    objs = []
+    for name in ("mlp", "seed"):
+        objs.append(os.path.join(d, name + ".o"))
+        # PTX only: the kernels do not run here
+        subprocess.check_call([nvcc, "-gencode", "arch=compute_103a,code=compute_103a", "-O1", "-std=c++17", "-Xcompiler", "-fPIC",
+                               "-I" + os.path.join(ROOT, "include"), "-c", os.path.join(ROOT, "auto_gb300", "csrc", name + ".cu"),
+                               "-o", objs[-1]])
+    so = os.path.join(d, "runtime_host.so")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I" + include,
+                           "-I" + os.path.join(ROOT, "include"), os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp")] + objs +
+                          ["-o", so])
+    return ctypes.CDLL(so)
+
+
+def test_statistics_of_a_smaller_context_between_set_and_launch(lib):
+    """The shared-memory limit belongs to the kernel, which all contexts share: a call for small worlds that comes between
+    another thread's setting of the limit and its launch leaves that launch valid."""
+    small = []
+    hook = ctypes.CFUNCTYPE(None)(lambda: small.append(lib.fake_world_stats(4096 + 4096)))
+    lib.fake_on_attribute(hook)
+    assert lib.fake_world_stats(8192 + 8192)
+    assert small == [1]
+    assert lib.fake_world_stats(32 + 32)
