@@ -634,6 +634,7 @@ bool mal(LeniaMlp* n, T** p, size_t count) {
 }
 
 int err(const char* msg) {
+    cudaGetLastError();  // reported here, and by no later call
     set_thread_error(msg);
     return LENIA_ECUDA;
 }
@@ -827,8 +828,8 @@ LENIA_API int lenia_mlp_gradients(LeniaMlp* n, const float* x, const float* y, u
         touch_pages(grads, NPARAM * 4, true);  // beside the tiles
         copy_out<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->g, grads, NPARAM);
         if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
-    } else {
-        cudaMemcpyAsync(grads, n->g, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream);
+    } else if (cudaMemcpyAsync(grads, n->g, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream) != cudaSuccess) {
+        return err("mlp: download failed");
     }
     return mean_loss(n, batch, loss);
 }

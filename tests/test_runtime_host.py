@@ -6,6 +6,7 @@ import os
 import shutil
 import subprocess
 
+import numpy as np
 import pytest
 
 from conftest import ROOT
@@ -41,3 +42,53 @@ def test_statistics_of_a_smaller_context_between_set_and_launch(lib):
     assert lib.fake_world_stats(8192 + 8192)
     assert small == [1]
     assert lib.fake_world_stats(32 + 32)
+
+
+IN, OUT, NPARAM, ECUDA = 16, 3, 70915, -4
+F = ctypes.POINTER(ctypes.c_float)
+
+
+def ptr(a):
+    return ctypes.cast(a.ctypes.data, F)
+
+
+def floats(n, aligned=True):
+    """n floats, 16-byte aligned or 4 bytes past such an address (which only a copy takes)."""
+    a = np.zeros(n + 8, np.float32)
+    k = -(a.ctypes.data // 4) % 4 + (0 if aligned else 1)
+    return a[k:k + n]
+
+
+def rows(n, aligned=True):
+    """Rows whose sums are their numbers."""
+    a = floats(n * IN, aligned)
+    a[::IN] = np.arange(n)
+    return a
+
+
+def probabilities(n):
+    return np.arange(n, dtype=np.float32)[:, None] + np.arange(OUT, dtype=np.float32)
+
+
+@pytest.fixture
+def mlp(lib):
+    h = ctypes.c_void_p()
+    lib.lenia_mlp_destroy.argtypes = [ctypes.c_void_p]
+    lib.fake_reads_host(1)
+    assert lib.lenia_mlp_create(1, 4096, ctypes.byref(h)) == 0
+    yield h
+    lib.fake_fail(b"", 0)
+    lib.lenia_mlp_destroy(h)
+
+
+def test_gradients_report_a_failed_download(lib, mlp):
+    """Gradients that leave by copy: a copy that the runtime refuses is an error of this call, and of no later one."""
+    x, y, loss = rows(100), floats(100 * OUT), ctypes.c_float()
+    for aligned, want in ((False, ECUDA), (True, 0), (False, 0)):
+        g = floats(NPARAM, aligned)
+        if want:
+            lib.fake_fail(b"cudaMemcpyAsync:down", 0)
+        assert lib.lenia_mlp_gradients(mlp, ptr(x), ptr(y), 100, ptr(g), ctypes.byref(loss)) == want
+        assert lib.fake_failed()
+        if not want:
+            assert (g == x.sum()).all() and loss.value == x[::IN].mean()
