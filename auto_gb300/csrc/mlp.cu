@@ -639,6 +639,14 @@ int err(const char* msg) {
     return LENIA_ECUDA;
 }
 
+// An error after work has been queued: waits for it first, for kernels and copies of the call may still be reading or
+// writing the caller's memory.
+int abandon(LeniaMlp* n, const char* msg) {
+    for (cudaStream_t s : {n->stream, n->ps[0], n->ps[1]}) cudaStreamSynchronize(s);
+    *n->err = 0;
+    return err(msg);
+}
+
 // rows of inputs that lenia_mlp_predict has on the device at a time, in two halves: a copy of one half
 // overlaps the other's tiles.  A half is two tiles for each of the GPU's 152 SMs, about as long on the SMs as on the
 // host link.
@@ -689,7 +697,7 @@ int batch_gradients(LeniaMlp* n, const float* x, const float* y, uint32_t B) {
     if (!in_place(n, x) || !in_place(n, y, 4)) {
         if (cudaMemcpyAsync(n->x, x, (size_t)B * IN * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess ||
             cudaMemcpyAsync(n->y, y, (size_t)B * OUT * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess)
-            return err("mlp: upload failed");
+            return abandon(n, "mlp: upload failed");
         x = n->x, y = n->y;
     } else {
         touch_last(x, (size_t)B * IN);
@@ -701,7 +709,7 @@ int batch_gradients(LeniaMlp* n, const float* x, const float* y, uint32_t B) {
 
 // Waits for the batch; its mean loss.
 int mean_loss(LeniaMlp* n, uint32_t B, float* loss) {
-    if (cudaStreamSynchronize(n->stream) != cudaSuccess) return err("mlp: the batch failed");
+    if (cudaStreamSynchronize(n->stream) != cudaSuccess) return abandon(n, "mlp: the batch failed");
     double s = 0;
     for (uint32_t i = 0; i < B; i++) s += n->loss[i];
     if (loss) *loss = (float)(s / B);
@@ -797,7 +805,7 @@ LENIA_API int lenia_mlp_set_params(LeniaMlp* n, const float* host, size_t count)
         return LENIA_EINVAL;
     }
     if (cudaMemcpyAsync(n->w, host, NPARAM * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess)
-        return err("mlp: upload failed");
+        return abandon(n, "mlp: upload failed");
     to_bf16<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->w, n->wb, NPARAM);
     n->t = 0;
     return cudaStreamSynchronize(n->stream) == cudaSuccess ? 0 : err("mlp: set_params failed");
@@ -810,7 +818,7 @@ LENIA_API int lenia_mlp_get_params(LeniaMlp* n, float* host, size_t count) {
     }
     if (cudaMemcpyAsync(host, n->w, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream) != cudaSuccess ||
         cudaStreamSynchronize(n->stream) != cudaSuccess)
-        return err("mlp: download failed");
+        return abandon(n, "mlp: download failed");
     return 0;
 }
 
@@ -821,15 +829,15 @@ LENIA_API int lenia_mlp_gradients(LeniaMlp* n, const float* x, const float* y, u
         return LENIA_EINVAL;
     }
     if (int rc = batch_gradients(n, x, y, batch)) return rc;
-    if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
+    if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
     // straight into the caller's memory where kernels reach it: 1000 rows 65.3 -> 62.7 us against the driver's copy, which
     // waits for a change of engine
     if (pageable_in_place(n->reads_host, grads, NPARAM * 4)) {
         touch_pages(grads, NPARAM * 4, true);  // beside the tiles
         copy_out<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->g, grads, NPARAM);
-        if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
+        if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
     } else if (cudaMemcpyAsync(grads, n->g, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream) != cudaSuccess) {
-        return err("mlp: download failed");
+        return abandon(n, "mlp: download failed");
     }
     return mean_loss(n, batch, loss);
 }
@@ -844,7 +852,7 @@ LENIA_API int lenia_mlp_train_step(LeniaMlp* n, const float* x, const float* y, 
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)n->t), c2 = 1.f - std::pow(b2, (float)n->t);
     adam<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->w, n->g, n->m, n->v, n->wb, NPARAM, lr, b1, b2, 1e-8f, c1, c2);
-    if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
+    if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
     return mean_loss(n, batch, loss);
 }
 
@@ -861,17 +869,17 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
             // no copy after the tiles: 1000 rows 30.5 -> 25.3 us, 19456 47.9 -> 36.0, 65536 74.0 -> 67.4
             touch_pages(probs, (size_t)count * OUT * 4, true);
             mlp_rank<<<tiles_grid(n, (int)count), NRANK, RANK_SMEM, n->ps[0]>>>(x, (int)count, n->w, n->wb, probs, n->err);
-            if (cudaGetLastError() != cudaSuccess) return err("mlp: launch failed");
+            if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
         } else {
             for (uint64_t off = 0; off < count; off += DIRECT_ROWS) {
                 const uint32_t B = count - off < DIRECT_ROWS ? (uint32_t)(count - off) : DIRECT_ROWS;
                 mlp_rank<<<tiles_grid(n, (int)B), NRANK, RANK_SMEM, n->ps[0]>>>(x + off * IN, (int)B, n->w, n->wb, n->pp, n->err);
                 if (cudaMemcpyAsync(probs + off * OUT, n->pp, (size_t)B * OUT * 4, cudaMemcpyDeviceToHost, n->ps[0]) !=
                     cudaSuccess)
-                    return err("mlp: download failed");
+                    return abandon(n, "mlp: download failed");
             }
         }
-        if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess) return err("mlp: predict failed");
+        if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess) return abandon(n, "mlp: predict failed");
         return check_err(n);
     }
     // chunk c runs on stream c % 2; its results leave after the next chunk has been queued, so that a copy
@@ -885,18 +893,18 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
             float *px = n->px + (size_t)h * HALF * IN, *pp = n->pp + (size_t)h * HALF * OUT;
             if (cudaMemcpyAsync(px, x + (size_t)c * HALF * IN, (size_t)rows(c) * IN * 4, cudaMemcpyHostToDevice, n->ps[h]) !=
                 cudaSuccess)
-                return err("mlp: upload failed");
+                return abandon(n, "mlp: upload failed");
             mlp_rank<<<tiles_grid(n, (int)rows(c)), NRANK, RANK_SMEM, n->ps[h]>>>(px, (int)rows(c), n->w, n->wb, pp, n->err);
         }
         if (c > 0) {
             const uint32_t d = c - 1;
             if (cudaMemcpyAsync(probs + (size_t)d * HALF * OUT, n->pp + (size_t)(d & 1) * HALF * OUT, (size_t)rows(d) * OUT * 4,
                                 cudaMemcpyDeviceToHost, n->ps[d & 1]) != cudaSuccess)
-                return err("mlp: download failed");
+                return abandon(n, "mlp: download failed");
         }
     }
     if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess || cudaStreamSynchronize(n->ps[1]) != cudaSuccess)
-        return err("mlp: predict failed");
+        return abandon(n, "mlp: predict failed");
     return check_err(n);
 }
 

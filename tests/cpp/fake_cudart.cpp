@@ -138,6 +138,9 @@ int fake_pending() {
     for (Stream* s : streams) n += (int)s->queue.size();
     return n;
 }
+// a range of the caller's as page-locked memory
+void fake_lock(void* p, size_t n) { ranges[(uintptr_t)p] = {n, cudaMemoryTypeHost}; }
+void fake_unlock(void* p) { ranges.erase((uintptr_t)p); }
 void fake_set_error() { last = cudaErrorInvalidValue; }  // an error of somebody else's that nobody has asked for
 void fake_reads_host(int on) { reads_host = on; }
 void fake_on_attribute(void (*f)()) { on_attribute = f; }

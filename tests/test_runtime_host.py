@@ -92,3 +92,43 @@ def test_gradients_report_a_failed_download(lib, mlp):
         assert lib.fake_failed()
         if not want:
             assert (g == x.sum()).all() and loss.value == x[::IN].mean()
+
+
+# the last two: rows of more than one half (38,912 rows), page-locked, so that copies are in flight as well
+@pytest.mark.parametrize("call, count, aligned, locked, what, skip", [
+    ("predict", 1000, (True, False), False, b"cudaMemcpyAsync:down", 0),
+    ("predict", 100000, (True, True), False, b"cudaMemcpyAsync:down", 0),
+    ("predict", 1000, (False, True), True, b"cudaMemcpyAsync:down", 0),
+    ("predict", 100000, (False, True), True, b"cudaMemcpyAsync:up", 2),
+    ("predict", 100000, (False, True), True, b"cudaMemcpyAsync:down", 1),
+    ("gradients", 1000, (True, False), False, b"cudaMemcpyAsync:down", 0),
+    ("gradients", 1000, (True, True), False, b"copy_out", 0),
+    ("gradients", 1000, (False, True), True, b"cudaMemcpyAsync:up", 1),
+    ("train_step", 1000, (True, True), False, b"adam", 0),
+])
+def test_a_failed_call_leaves_nothing_running(lib, mlp, call, count, aligned, locked, what, skip):
+    """A call that fails half way waits for what it has queued: the caller may free its arrays.  The next call is
+    as good as ever."""
+    x, y = rows(count, aligned[0]), floats(count * OUT)
+    out = floats(count * OUT if call == "predict" else NPARAM, aligned[1])
+    loss = ctypes.c_float()
+    if locked:
+        lib.fake_lock(ptr(x), ctypes.c_size_t(x.nbytes))
+
+    def run():
+        if call == "predict":
+            return lib.lenia_mlp_predict(mlp, ptr(x), count, ptr(out))
+        if call == "gradients":
+            return lib.lenia_mlp_gradients(mlp, ptr(x), ptr(y), count, ptr(out), ctypes.byref(loss))
+        return lib.lenia_mlp_train_step(mlp, ptr(x), ptr(y), count, ctypes.c_float(0.1), ctypes.byref(loss))
+
+    lib.fake_fail(what, skip)
+    assert run() == ECUDA
+    assert lib.fake_failed() and lib.fake_pending() == 0
+    assert run() == 0 and lib.fake_pending() == 0
+    if call == "predict":
+        np.testing.assert_array_equal(out.reshape(-1, OUT), probabilities(count))
+    elif call == "gradients":
+        assert (out == x.sum(dtype=np.float64).astype(np.float32)).all()
+    if locked:
+        lib.fake_unlock(ptr(x))
