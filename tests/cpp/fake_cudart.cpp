@@ -148,7 +148,9 @@ void fake_on_attribute(void (*f)()) { on_attribute = f; }
 int fake_world_stats(int sides) {
     static cudaStream_t s = nullptr;
     if (!s) cudaStreamCreateWithFlags(&s, 0);
-    return lenia::launch_world_stats(nullptr, 1, sides, nullptr, s) && cudaGetLastError() == cudaSuccess;
+    const bool ok = lenia::launch_world_stats(nullptr, 1, sides, nullptr, s) && cudaGetLastError() == cudaSuccess;
+    drain(of(s));
+    return ok;
 }
 
 // -------------------------------------------------------------- the runtime
