@@ -689,8 +689,9 @@ bool in_place(const LeniaMlp* n, const float* rows, uintptr_t align = 16) {
     return a.type != cudaMemoryTypeDevice;
 }
 
-// Reads the last of a range that a kernel will read in place: a range that is too short faults on the host.
-void touch_last(const float* p, size_t count) { touch_pages(const_cast<float*>(p) + count - 1, sizeof(float), false); }
+// Reads a word of every page of a range that a kernel will read in place (touch_pages): a page that is not the caller's faults
+// on the host, and one that is not there yet gets its place from it.  256 pages of 64 KB for 250001 rows.
+void touch_rows(const float* p, size_t count) { touch_pages(const_cast<float*>(p), count * sizeof(float), false); }
 
 // The batch's gradients from host rows, copied first where they cannot be read in place.
 int batch_gradients(LeniaMlp* n, const float* x, const float* y, uint32_t B) {
@@ -700,8 +701,8 @@ int batch_gradients(LeniaMlp* n, const float* x, const float* y, uint32_t B) {
             return abandon(n, "mlp: upload failed");
         x = n->x, y = n->y;
     } else {
-        touch_last(x, (size_t)B * IN);
-        touch_last(y, (size_t)B * OUT);
+        touch_rows(x, (size_t)B * IN);
+        touch_rows(y, (size_t)B * OUT);
     }
     gradients(n, x, y, (int)B);
     return 0;
@@ -862,7 +863,7 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
         return LENIA_EINVAL;
     }
     if (in_place(n, x)) {
-        if (count > 0) touch_last(x, (size_t)count * IN);
+        if (count > 0) touch_rows(x, (size_t)count * IN);
         // probabilities over their own rows leave by copy, after every row has been read
         const bool apart = probs + (size_t)count * OUT <= x || x + (size_t)count * IN <= probs;
         if (count > 0 && apart && pageable_in_place(n->reads_host, probs, (size_t)count * OUT * 4)) {

@@ -5,6 +5,8 @@
 // waited for, or when a copy on it that blocks for pageable memory is queued.  The kernels the tests need are restated as simple
 // functions of the same arguments (fake_kernel below); the rest do nothing.  fake_fail makes a coming call fail.
 #include <cuda_runtime_api.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <cstdint>
 #include <cstring>
@@ -66,6 +68,16 @@ void drain(Stream* s) {
 }
 Stream* of(cudaStream_t s) { return reinterpret_cast<Stream*>(s); }
 
+// pages of the caller's pageable memory that a kernel was launched on and that the host had not touched
+int absent = 0;
+void expect_present(const void* p, size_t bytes) {
+    if (find(p)) return;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p / page * page, n = ((uintptr_t)p + bytes - a + page - 1) / page;
+    std::vector<unsigned char> v(n);
+    if (mincore((void*)a, n * page, v.data())) return;
+    for (unsigned char c : v) absent += !(c & 1);
+}
+
 template <class T>
 T arg(void** a, int i) { return *static_cast<T*>(a[i]); }
 
@@ -77,6 +89,8 @@ std::function<void()> fake_kernel(const std::string& name, void** a) {
         const float* x = arg<const float*>(a, 0);
         const int n = arg<int>(a, 1);
         float* p = arg<float*>(a, 4);
+        expect_present(x, (size_t)n * IN * 4);
+        expect_present(p, (size_t)n * OUT * 4);
         return [=] {
             std::vector<float> r((size_t)n * OUT);
             for (int b = 0; b < n; b++) {
@@ -91,6 +105,8 @@ std::function<void()> fake_kernel(const std::string& name, void** a) {
         const float *x = arg<const float*>(a, 0), *y = arg<const float*>(a, 1);
         const int n = arg<int>(a, 2);
         float *g = arg<float*>(a, 5), *loss = arg<float*>(a, 6);
+        expect_present(x, (size_t)n * IN * 4);
+        expect_present(y, (size_t)n * OUT * 4);
         return [=] {
             double s = 0;
             for (size_t i = 0; i < (size_t)n * IN; i++) s += x[i];
@@ -103,6 +119,7 @@ std::function<void()> fake_kernel(const std::string& name, void** a) {
         const float* x = arg<const float*>(a, 0);
         float* y = arg<float*>(a, 1);
         const int n = arg<int>(a, 2);
+        expect_present(y, (size_t)n * 4);
         return [=] { memcpy(y, x, (size_t)n * 4); };
     }
     if (name.find("copy_words") != std::string::npos) {
@@ -141,6 +158,11 @@ int fake_pending() {
 // a range of the caller's as page-locked memory
 void fake_lock(void* p, size_t n) { ranges[(uintptr_t)p] = {n, cudaMemoryTypeHost}; }
 void fake_unlock(void* p) { ranges.erase((uintptr_t)p); }
+int fake_absent() {
+    const int n = absent;
+    absent = 0;
+    return n;
+}
 void fake_set_error() { last = cudaErrorInvalidValue; }  // an error of somebody else's that nobody has asked for
 void fake_reads_host(int on) { reads_host = on; }
 void fake_on_attribute(void (*f)()) { on_attribute = f; }

@@ -2,6 +2,7 @@
 (tests/cpp/fake_cudart.cpp): what happens when a call of the runtime fails, and in which order copies and kernels touch the
 caller's memory.  No GPU; the kernels are simple functions of the same arguments, so every value is exact."""
 import ctypes
+import mmap
 import os
 import shutil
 import subprocess
@@ -132,3 +133,25 @@ def test_a_failed_call_leaves_nothing_running(lib, mlp, call, count, aligned, lo
         assert (out == x.sum(dtype=np.float64).astype(np.float32)).all()
     if locked:
         lib.fake_unlock(ptr(x))
+
+
+def fresh(n):
+    """n floats (zeros) in pages that nobody has touched."""
+    return np.frombuffer(mmap.mmap(-1, 4 * n), np.float32)
+
+
+@pytest.mark.parametrize("count", [1, 63, 64, 4000, 250001])
+def test_every_page_is_touched_from_the_host_before_a_kernel_gets_it(lib, mlp, count):
+    """A kernel that walked into a page that is not the caller's would take the GPU's context with it; the host's touch
+    faults here.  So every page of a range that goes to a kernel in place has been touched."""
+    loss = ctypes.c_float()
+    x, probs = fresh(count * IN), fresh(count * OUT)
+    assert lib.lenia_mlp_predict(mlp, ptr(x), count, ptr(probs)) == 0
+    assert lib.fake_absent() == 0
+    if count <= 4096:
+        x, y, g = fresh(count * IN), fresh(count * OUT), fresh(NPARAM)
+        assert lib.lenia_mlp_gradients(mlp, ptr(x), ptr(y), count, ptr(g), ctypes.byref(loss)) == 0
+        assert lib.fake_absent() == 0
+        x, y = fresh(count * IN), fresh(count * OUT)
+        assert lib.lenia_mlp_train_step(mlp, ptr(x), ptr(y), count, ctypes.c_float(0.1), ctypes.byref(loss)) == 0
+        assert lib.fake_absent() == 0
