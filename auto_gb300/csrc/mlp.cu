@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -651,6 +652,7 @@ int abandon(LeniaMlp* n, const char* msg) {
 // overlaps the other's tiles.  A half is two tiles for each of the GPU's 152 SMs, about as long on the SMs as on the
 // host link.
 constexpr int PREDICT_ROWS = 2 * 2 * 152 * TILE;
+constexpr uint32_t HALF = PREDICT_ROWS / 2;
 // rows of one launch where the kernel reads them in host memory
 constexpr int DIRECT_ROWS = 1 << 20;
 
@@ -714,6 +716,54 @@ int mean_loss(LeniaMlp* n, uint32_t B, float* loss) {
     double s = 0;
     for (uint32_t i = 0; i < B; i++) s += n->loss[i];
     if (loss) *loss = (float)(s / B);
+    return check_err(n);
+}
+
+// Probabilities of count rows.  A chunk's may leave before the rows of a later chunk are read.
+int rank_rows(LeniaMlp* n, const float* x, uint32_t count, float* probs) {
+    if (in_place(n, x)) {
+        if (count > 0) touch_rows(x, (size_t)count * IN);
+        // probabilities over their own rows leave by copy, after the launch has read them
+        const bool apart = probs + (size_t)count * OUT <= x || x + (size_t)count * IN <= probs;
+        if (count > 0 && apart && pageable_in_place(n->reads_host, probs, (size_t)count * OUT * 4)) {
+            // no copy after the tiles: 1000 rows 30.5 -> 25.3 us, 19456 47.9 -> 36.0, 65536 74.0 -> 67.4
+            touch_pages(probs, (size_t)count * OUT * 4, true);
+            mlp_rank<<<tiles_grid(n, (int)count), NRANK, RANK_SMEM, n->ps[0]>>>(x, (int)count, n->w, n->wb, probs, n->err);
+            if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
+        } else {
+            for (uint64_t off = 0; off < count; off += DIRECT_ROWS) {
+                const uint32_t B = count - off < DIRECT_ROWS ? (uint32_t)(count - off) : DIRECT_ROWS;
+                mlp_rank<<<tiles_grid(n, (int)B), NRANK, RANK_SMEM, n->ps[0]>>>(x + off * IN, (int)B, n->w, n->wb, n->pp, n->err);
+                if (cudaMemcpyAsync(probs + off * OUT, n->pp, (size_t)B * OUT * 4, cudaMemcpyDeviceToHost, n->ps[0]) !=
+                    cudaSuccess)
+                    return abandon(n, "mlp: download failed");
+            }
+        }
+        if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess) return abandon(n, "mlp: predict failed");
+        return check_err(n);
+    }
+    // chunk c runs on stream c % 2; its results leave after the next chunk has been queued, so that a copy
+    // to or from pageable memory, which blocks this thread, overlaps a chunk's tiles
+    const uint32_t chunks = (uint32_t)(((uint64_t)count + HALF - 1) / HALF);
+    auto rows = [&](uint32_t c) { return c + 1 < chunks ? HALF : count - c * HALF; };
+    for (uint32_t c = 0; c <= chunks; c++) {
+        if (c < chunks) {
+            const int h = c & 1;
+            float *px = n->px + (size_t)h * HALF * IN, *pp = n->pp + (size_t)h * HALF * OUT;
+            if (cudaMemcpyAsync(px, x + (size_t)c * HALF * IN, (size_t)rows(c) * IN * 4, cudaMemcpyHostToDevice, n->ps[h]) !=
+                cudaSuccess)
+                return abandon(n, "mlp: upload failed");
+            mlp_rank<<<tiles_grid(n, (int)rows(c)), NRANK, RANK_SMEM, n->ps[h]>>>(px, (int)rows(c), n->w, n->wb, pp, n->err);
+        }
+        if (c > 0) {
+            const uint32_t d = c - 1;
+            if (cudaMemcpyAsync(probs + (size_t)d * HALF * OUT, n->pp + (size_t)(d & 1) * HALF * OUT, (size_t)rows(d) * OUT * 4,
+                                cudaMemcpyDeviceToHost, n->ps[d & 1]) != cudaSuccess)
+                return abandon(n, "mlp: download failed");
+        }
+    }
+    if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess || cudaStreamSynchronize(n->ps[1]) != cudaSuccess)
+        return abandon(n, "mlp: predict failed");
     return check_err(n);
 }
 
@@ -862,51 +912,21 @@ LENIA_API int lenia_mlp_predict(LeniaMlp* n, const float* x, uint32_t count, flo
         set_thread_error("mlp: NULL argument");
         return LENIA_EINVAL;
     }
-    if (in_place(n, x)) {
-        if (count > 0) touch_rows(x, (size_t)count * IN);
-        // probabilities over their own rows leave by copy, after every row has been read
-        const bool apart = probs + (size_t)count * OUT <= x || x + (size_t)count * IN <= probs;
-        if (count > 0 && apart && pageable_in_place(n->reads_host, probs, (size_t)count * OUT * 4)) {
-            // no copy after the tiles: 1000 rows 30.5 -> 25.3 us, 19456 47.9 -> 36.0, 65536 74.0 -> 67.4
-            touch_pages(probs, (size_t)count * OUT * 4, true);
-            mlp_rank<<<tiles_grid(n, (int)count), NRANK, RANK_SMEM, n->ps[0]>>>(x, (int)count, n->w, n->wb, probs, n->err);
-            if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
-        } else {
-            for (uint64_t off = 0; off < count; off += DIRECT_ROWS) {
-                const uint32_t B = count - off < DIRECT_ROWS ? (uint32_t)(count - off) : DIRECT_ROWS;
-                mlp_rank<<<tiles_grid(n, (int)B), NRANK, RANK_SMEM, n->ps[0]>>>(x + off * IN, (int)B, n->w, n->wb, n->pp, n->err);
-                if (cudaMemcpyAsync(probs + off * OUT, n->pp, (size_t)B * OUT * 4, cudaMemcpyDeviceToHost, n->ps[0]) !=
-                    cudaSuccess)
-                    return abandon(n, "mlp: download failed");
-            }
+    // Over their own rows, behind the start (12 bytes a row never catch up with 64), the first chunk's probabilities could
+    // lie where later rows are yet to be read: they wait in a buffer.
+    if (count > HALF && probs > x && probs < x + (size_t)count * IN) {
+        const size_t bytes = (size_t)count * OUT * sizeof(float);
+        float* all = static_cast<float*>(malloc(bytes));
+        if (!all) {
+            set_thread_error("mlp: no host memory for probabilities over their own rows");
+            return LENIA_ENOMEM;
         }
-        if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess) return abandon(n, "mlp: predict failed");
-        return check_err(n);
+        const int rc = rank_rows(n, x, count, all);
+        if (!rc) memcpy(probs, all, bytes);
+        free(all);
+        return rc;
     }
-    // chunk c runs on stream c % 2; its results leave after the next chunk has been queued, so that a copy
-    // to or from pageable memory, which blocks this thread, overlaps a chunk's tiles
-    constexpr uint32_t HALF = PREDICT_ROWS / 2;
-    const uint32_t chunks = (uint32_t)(((uint64_t)count + HALF - 1) / HALF);
-    auto rows = [&](uint32_t c) { return c + 1 < chunks ? HALF : count - c * HALF; };
-    for (uint32_t c = 0; c <= chunks; c++) {
-        if (c < chunks) {
-            const int h = c & 1;
-            float *px = n->px + (size_t)h * HALF * IN, *pp = n->pp + (size_t)h * HALF * OUT;
-            if (cudaMemcpyAsync(px, x + (size_t)c * HALF * IN, (size_t)rows(c) * IN * 4, cudaMemcpyHostToDevice, n->ps[h]) !=
-                cudaSuccess)
-                return abandon(n, "mlp: upload failed");
-            mlp_rank<<<tiles_grid(n, (int)rows(c)), NRANK, RANK_SMEM, n->ps[h]>>>(px, (int)rows(c), n->w, n->wb, pp, n->err);
-        }
-        if (c > 0) {
-            const uint32_t d = c - 1;
-            if (cudaMemcpyAsync(probs + (size_t)d * HALF * OUT, n->pp + (size_t)(d & 1) * HALF * OUT, (size_t)rows(d) * OUT * 4,
-                                cudaMemcpyDeviceToHost, n->ps[d & 1]) != cudaSuccess)
-                return abandon(n, "mlp: download failed");
-        }
-    }
-    if (cudaStreamSynchronize(n->ps[0]) != cudaSuccess || cudaStreamSynchronize(n->ps[1]) != cudaSuccess)
-        return abandon(n, "mlp: predict failed");
-    return check_err(n);
+    return rank_rows(n, x, count, probs);
 }
 
 }  // extern "C"

@@ -345,7 +345,7 @@ LENIA_API int lenia_mlp_gradients(LeniaMlp* mlp, const float* x, const float* y,
 /* One Adam step (beta 0.9 / 0.999) on one batch; returns the batch's mean loss. */
 LENIA_API int lenia_mlp_train_step(LeniaMlp* mlp, const float* x, const float* y, uint32_t batch, float lr,
                                    float* loss);
-/* Sigmoid outputs for `count` rows of features (count x 3 floats). */
+/* Sigmoid outputs for `count` rows of features (count x 3 floats).  probs may lie over x. */
 LENIA_API int lenia_mlp_predict(LeniaMlp* mlp, const float* x, uint32_t count, float* probs);
 
 /* Event-timed average device time of the dominant launches of one step, in milliseconds:

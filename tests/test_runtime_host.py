@@ -155,3 +155,16 @@ def test_every_page_is_touched_from_the_host_before_a_kernel_gets_it(lib, mlp, c
         x, y = fresh(count * IN), fresh(count * OUT)
         assert lib.lenia_mlp_train_step(mlp, ptr(x), ptr(y), count, ctypes.c_float(0.1), ctypes.byref(loss)) == 0
         assert lib.fake_absent() == 0
+
+
+# in place in one launch and in two, copied in one half, two, three and four
+@pytest.mark.parametrize("count, aligned", [(1000, True), (100000, True), (1048577, True), (38912, False), (38913, False), (77825, False),
+                                            (150000, False)])
+@pytest.mark.parametrize("at", [0, 4, 0.5, 1])
+def test_probabilities_anywhere_over_their_own_rows(lib, mlp, count, aligned, at):
+    """The probabilities of the first rows may lie over rows that are yet to be read."""
+    k = int(at * (count * IN - count * OUT)) // 4 * 4 if at <= 1 else at  # floats from the rows' start; 1: at their end
+    x = rows(count, aligned)
+    assert lib.lenia_mlp_predict(mlp, ptr(x), count, ptr(x[k:])) == 0
+    np.testing.assert_array_equal(x[k:k + count * OUT].reshape(-1, OUT), probabilities(count))
+    assert lib.fake_pending() == 0
