@@ -188,6 +188,7 @@ int fail(LeniaCtx* c, int code, const char* fmt, ...) {
     va_end(ap);
     if (c) c->err = buf;
     else g_create_error = buf;
+    if (code == LENIA_ECUDA) cudaGetLastError();  // reported here, and by no later call
     return code;
 }
 
@@ -1276,8 +1277,8 @@ int lenia_write_state(LeniaCtx* ctx, int32_t world, const float* host, size_t co
                     count);
     if (count * sizeof(float) > WRITE_STAGED && in_place(ctx, host, count)) {
         touch_pages(const_cast<float*>(host), count * sizeof(float), false);
-        launch_copy_words(state_ptr(ctx, world), host, count, ctx->stream);
-        CK(cudaGetLastError());
+        if (!launch_copy_words(state_ptr(ctx, world), host, count, ctx->stream))
+            return fail(ctx, LENIA_ECUDA, "state copy launch failed");
         CK(cudaStreamSynchronize(ctx->stream));
     } else {
         CK(cudaMemcpyAsync(state_ptr(ctx, world), host, count * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
@@ -1299,8 +1300,8 @@ int lenia_read_state(LeniaCtx* ctx, int32_t world, float* host, size_t count) {
     if (!host || count != state_count(ctx->desc[world])) return fail(ctx, LENIA_EINVAL, "bad count for world %d", world);
     if (in_place(ctx, host, count)) {
         touch_pages(host, count * sizeof(float), true);
-        launch_copy_words(host, state_ptr(ctx, world), count, ctx->stream);
-        CK(cudaGetLastError());
+        if (!launch_copy_words(host, state_ptr(ctx, world), count, ctx->stream))
+            return fail(ctx, LENIA_ECUDA, "state copy launch failed");
     } else {
         CK(cudaMemcpyAsync(host, state_ptr(ctx, world), count * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     }

@@ -143,8 +143,8 @@ bool pageable_in_place(int reads_host, const void* p, size_t bytes);
 // Touches every page of such a range from the host first: pages not there yet get their place from the host, and a bad
 // range faults there, not on the GPU.
 void touch_pages(void* p, size_t bytes, bool write);
-// count floats, a multiple of 4, between 16-byte aligned places
-void launch_copy_words(float* dst, const float* src, size_t count, cudaStream_t s);
+// count floats, a multiple of 4, between 16-byte aligned places; whether this launch succeeded
+bool launch_copy_words(float* dst, const float* src, size_t count, cudaStream_t s);
 // max_sides: the largest W + H of the worlds
 bool launch_world_stats(const DevWorld* worlds, int nworlds, int max_sides, float* out, cudaStream_t s);
 void launch_seed_rule(float* state, int W, int H, uint32_t seed, int kind, cudaStream_t s);

@@ -54,6 +54,7 @@ std::mutex g_mutex;
 unsigned char* g_base[MAX_DEVICES] = {};
 // Failures are reported through lenia_last_error(NULL), like those of lenia_create.
 int set_error(int code, const std::string& msg) {
+    if (code == LENIA_ECUDA) cudaGetLastError();  // reported here, and by no later call
     set_thread_error(msg);
     return code;
 }

@@ -232,9 +232,9 @@ void touch_pages(void* p, size_t bytes, bool write) {
     touch(bytes - 1);
 }
 
-void launch_copy_words(float* dst, const float* src, size_t count, cudaStream_t s) {
-    copy_words_kernel<<<grid_for(count / 4), 256, 0, s>>>(reinterpret_cast<float4*>(dst), reinterpret_cast<const float4*>(src),
-                                                          (unsigned)(count / 4));
+bool launch_copy_words(float* dst, const float* src, size_t count, cudaStream_t s) {
+    return launch_pass(copy_words_kernel, grid_for(count / 4), 256, 0, s, reinterpret_cast<float4*>(dst),
+                       reinterpret_cast<const float4*>(src), (unsigned)(count / 4));
 }
 
 bool launch_world_stats(const DevWorld* worlds, int nworlds, int max_sides, float* out, cudaStream_t s) {

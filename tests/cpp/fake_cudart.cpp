@@ -126,6 +126,8 @@ std::function<void()> fake_kernel(const std::string& name, void** a) {
         float* d = arg<float*>(a, 0);
         const float* s = arg<const float*>(a, 1);
         const unsigned n = arg<unsigned>(a, 2);
+        expect_present(d, (size_t)n * 16);
+        expect_present(s, (size_t)n * 16);
         return [=] { memcpy(d, s, (size_t)n * 16); };
     }
     return [] {};
@@ -140,8 +142,6 @@ cudaError_t launch(const void* f, void** args, size_t smem, cudaStream_t s) {
 }
 
 }  // namespace
-
-void lenia::set_thread_error(const std::string&) {}
 
 extern "C" {
 
@@ -163,7 +163,6 @@ int fake_absent() {
     absent = 0;
     return n;
 }
-void fake_set_error() { last = cudaErrorInvalidValue; }  // an error of somebody else's that nobody has asked for
 void fake_reads_host(int on) { reads_host = on; }
 void fake_on_attribute(void (*f)()) { on_attribute = f; }
 // entries of the engine's that are not exported
@@ -255,6 +254,19 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kin
     if (!find(kind == cudaMemcpyHostToDevice ? s : d)) drain(of(st));  // pageable memory: blocks
     return cudaSuccess;
 }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+    memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemset(void* d, int v, size_t n) {
+    memset(d, v, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
+cudaError_t cudaFreeAsync(void* p, cudaStream_t s) {
+    of(s)->queue.push_back([=] { cudaFree(p); });
+    return cudaSuccess;
+}
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t st) {
     of(st)->queue.push_back([=] { memset(d, v, n); });
     return cudaSuccess;
@@ -262,6 +274,41 @@ cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t st) {
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     streams.push_back(new Stream);
     *s = reinterpret_cast<cudaStream_t>(streams.back());
+    return cudaSuccess;
+}
+// events and graphs: every queue is drained where an order is asked for
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) {
+    *e = reinterpret_cast<cudaEvent_t>(&last);
+    return cudaSuccess;
+}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t s) {
+    drain(of(s));
+    return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
+    *ms = 1;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
+    *g = nullptr;
+    return cudaSuccess;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+    *e = reinterpret_cast<cudaGraphExec_t>(&last);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+const char* cudaGetErrorString(cudaError_t) { return "refused"; }
+cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int) {
+    memset(p, 0, sizeof(*p));
+    p->major = 10, p->minor = 3, p->multiProcessorCount = 152;
     return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t s) {

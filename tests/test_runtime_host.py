@@ -1,5 +1,5 @@
-"""The host code of the proposer and of the statistics (auto_gb300/csrc/mlp.cu, seed.cu) over a stand-in for the CUDA runtime
-(tests/cpp/fake_cudart.cpp): what happens when a call of the runtime fails, and in which order copies and kernels touch the
+"""The host code of the context, the proposer and the statistics (auto_gb300/csrc/ctx.cu, mlp.cu, seed.cu) over stand-ins for
+the CUDA runtime and the passes (tests/cpp/fake_cudart.cpp, fake_passes.cpp): what happens when a call of the runtime fails, and in which order copies and kernels touch the
 caller's memory.  No GPU; the kernels are simple functions of the same arguments, so every value is exact."""
 import ctypes
 import mmap
@@ -12,6 +12,9 @@ import pytest
 
 from conftest import ROOT
 
+from auto_gb300 import _lib
+from auto_gb300.program import Kernel, World
+
 
 @pytest.fixture(scope="module")
 def lib(tmp_path_factory):
@@ -21,7 +24,7 @@ def lib(tmp_path_factory):
     d = str(tmp_path_factory.mktemp("runtime"))
     include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
     objs = []
-    for name in ("mlp", "seed"):
+    for name in ("ctx", "mlp", "seed"):
         objs.append(os.path.join(d, name + ".o"))
         # PTX only: the kernels do not run here
         subprocess.check_call([nvcc, "-gencode", "arch=compute_103a,code=compute_103a", "-O1", "-std=c++17", "-Xcompiler", "-fPIC",
@@ -29,8 +32,8 @@ def lib(tmp_path_factory):
                                "-o", objs[-1]])
     so = os.path.join(d, "runtime_host.so")
     subprocess.check_call(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I" + include,
-                           "-I" + os.path.join(ROOT, "include"), os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp")] + objs +
-                          ["-o", so])
+                           "-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(ROOT, "auto_gb300", "csrc")] +
+                          [os.path.join(ROOT, "tests", "cpp", f) for f in ("fake_cudart.cpp", "fake_passes.cpp")] + objs + ["-o", so])
     return ctypes.CDLL(so)
 
 
@@ -168,3 +171,56 @@ def test_probabilities_anywhere_over_their_own_rows(lib, mlp, count, aligned, at
     assert lib.lenia_mlp_predict(mlp, ptr(x), count, ptr(x[k:])) == 0
     np.testing.assert_array_equal(x[k:k + count * OUT].reshape(-1, OUT), probabilities(count))
     assert lib.fake_pending() == 0
+
+
+# ---------------------------------------------------------------------- states
+
+@pytest.fixture
+def context(lib):
+    """make(worlds): a context of one-kernel worlds of these (width, height)."""
+    made = []
+    lib.lenia_destroy.argtypes = [ctypes.c_void_p]
+    lib.fake_reads_host(1)
+
+    def make(worlds):
+        descs = (_lib.LeniaWorldDesc * len(worlds))(*[World(w, h, [Kernel(radius=5.0)]).to_desc() for w, h in worlds])
+        made.append(ctypes.c_void_p())
+        assert lib.lenia_create(descs, len(worlds), 0, ctypes.byref(made[-1])) == 0
+        return made[-1]
+
+    yield make
+    lib.fake_fail(b"", 0)
+    for c in made:
+        lib.lenia_destroy(c)
+
+
+def size(n):
+    return ctypes.c_size_t(n)
+
+
+@pytest.mark.parametrize("refused", ["lenia_read_states", "lenia_mlp_get_params"])
+def test_a_reported_error_does_not_come_back(lib, mlp, context, refused):
+    """An error that a call has reported is not found again by a later, valid one."""
+    n = 256 * 256
+    ctx, state, out = context([(256, 256)]), floats(n), floats(n)
+    state[:] = np.arange(n)
+    lib.fake_fail(b"cudaMemcpyAsync:down", 0)
+    if refused == "lenia_read_states":
+        assert lib.lenia_read_states(ctx, ptr(out), size(n)) == ECUDA
+    else:
+        assert lib.lenia_mlp_get_params(mlp, ptr(floats(NPARAM)), size(NPARAM)) == ECUDA
+    assert lib.fake_failed()
+    assert lib.lenia_write_state(ctx, 0, ptr(state), size(n)) == 0
+    assert lib.lenia_read_state(ctx, 0, ptr(out), size(n)) == 0
+    np.testing.assert_array_equal(out, state)
+    x, probs = rows(100), floats(100 * OUT)
+    assert lib.lenia_mlp_predict(mlp, ptr(x), 100, ptr(probs)) == 0
+
+
+@pytest.mark.parametrize("w, h", [(96, 32), (128, 128), (192, 128), (256, 256), (512, 512)])
+def test_states_copied_in_place_are_touched_first(lib, context, w, h):
+    n = w * h
+    ctx, state, out = context([(w, h)]), fresh(n), fresh(n)
+    assert lib.lenia_write_state(ctx, 0, ptr(state), size(n)) == 0
+    assert lib.lenia_read_state(ctx, 0, ptr(out), size(n)) == 0
+    assert lib.fake_absent() == 0 and lib.fake_pending() == 0
