@@ -96,3 +96,45 @@ def test_probabilities_over_their_own_rows():
     assert p.L.lenia_mlp_predict(p.h, ptr(x), rows, ptr(want)) == 0
     assert p.L.lenia_mlp_predict(p.h, ptr(buf), rows, ptr(buf)) == 0
     np.testing.assert_array_equal(buf[:3 * rows], want)
+
+
+# copied where the rows are not 16-byte aligned, in halves of 38,912 rows that overlap: one, two, three (the first half's
+# buffers used again) and four of them, with a short last one
+@pytest.mark.parametrize("count", [1, 38912, 38913, 77824, 77825, 116737, 150001])
+def test_copied_halves_give_the_bits_of_rows_in_place(count):
+    p = Proposer(seed=3, max_batch=64)
+    x = np.random.default_rng(count).random((count, 16), dtype=np.float32)
+    off = memory("off", 16 * count)
+    off[:] = x.reshape(-1)
+    got = []
+    for rows in (x, off):
+        for kind in ("aligned", "pinned"):
+            out = memory(kind, 3 * count)
+            assert p.L.lenia_mlp_predict(p.h, ptr(rows), count, ptr(out)) == 0
+            got.append(out.copy())
+    assert np.isfinite(got[0]).all()
+    for g in got[1:]:
+        np.testing.assert_array_equal(g, got[0])
+
+
+def test_rows_in_place_in_two_launches():
+    """One row more than a launch takes (2^20): the rows of both launches give what they give in a call of their own."""
+    count, cut = (1 << 20) + 1, 1 << 19
+    p = Proposer(seed=3, max_batch=64)
+    x = np.random.default_rng(2).random((count, 16), dtype=np.float32)
+    got = p.predict(x)
+    np.testing.assert_array_equal(got[:cut], p.predict(x[:cut]))
+    np.testing.assert_array_equal(got[cut:], p.predict(x[cut:]))
+
+
+@pytest.mark.parametrize("count, at", [(20000, 0.5), (150001, 1.0), ((1 << 20) + 1, 1.0)])
+def test_probabilities_over_later_rows(count, at):
+    """Probabilities from the middle or at the end of their own rows."""
+    p = Proposer(seed=3, max_batch=64)
+    x = np.random.default_rng(3).random((count, 16), dtype=np.float32)
+    want, k = p.predict(x), int(at * 13 * count) // 4 * 4
+    for kind in ("aligned", "off"):
+        buf = memory(kind, 16 * count)
+        buf[:] = x.reshape(-1)
+        assert p.L.lenia_mlp_predict(p.h, ptr(buf), count, ptr(buf[k:])) == 0
+        np.testing.assert_array_equal(buf[k:k + 3 * count].reshape(-1, 3), want)
