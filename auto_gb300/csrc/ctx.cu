@@ -572,9 +572,9 @@ int enqueue_steps(LeniaCtx* ctx, int steps) {
     // Size classes one after another, and within a class its chunks one after another, each chunk for
     // all its steps: a chunk's states and spectra then stay in L2 across its generations.  Measured on
     // the 384-world batched workload, running every class as its own concurrent graph branch was 6%
-    // slower than one after another.  With branch_cells set, the small classes (latency-bound: little
-    // work a launch) run one after another on a second branch beside the large ones, whose launches
-    // fill the GPU; lenia_autotune decides whether that pays.
+    // slower than one after another.  With branch_cells set, the classes of at most that many cells (latency-bound:
+    // little work a launch) run beside the large ones, whose launches fill the GPU, one after another on a second branch
+    // or (branch_each) each on its own: where default_branches, lenia_set_branch_split or lenia_autotune says so.
     cudaStream_t s = ctx->stream;
     const bool split = ctx->branch_cells > 0;
     int used = 0;  // side branches in use

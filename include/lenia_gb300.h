@@ -226,8 +226,10 @@ LENIA_API int lenia_set_chunk_lanes(LeniaCtx* ctx, int32_t lanes);
 /* Branches of the step graph (FP32, TF32 and BF16X3 paths): size classes of at most `cells` cells a world run on graph
  * branches beside the larger classes -- one after another on one side branch (each = 0), or each on
  * a branch of its own (each = 1) -- so that the small classes' latency-bound launches share the GPU
- * with the large classes' (cells = 0: one branch, every class in turn, the default).  lenia_autotune
- * tries every split between class sizes, both ways.  Results do not depend on it (bit for bit).
+ * with the large classes' (cells = 0: one branch, every class in turn).  The default of a context with
+ * several classes goes by the bytes that its worlds touch in a step: up to 128 MiB every class but the
+ * largest has a branch of its own, up to 256 MiB the classes of at most 384 x 384 cells (or all but the
+ * largest) share a side branch, beyond that cells = 0.  lenia_autotune tries every split between class sizes, both ways.  Results do not depend on it (bit for bit).
  * Rebuilds the step graphs.  lenia_branch_split reports the current choice.  No reference
  * counterpart. */
 LENIA_API int lenia_set_branch_split(LeniaCtx* ctx, int64_t cells, int32_t each);

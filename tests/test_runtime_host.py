@@ -224,3 +224,28 @@ def test_states_copied_in_place_are_touched_first(lib, context, w, h):
     assert lib.lenia_write_state(ctx, 0, ptr(state), size(n)) == 0
     assert lib.lenia_read_state(ctx, 0, ptr(out), size(n)) == 0
     assert lib.fake_absent() == 0 and lib.fake_pending() == 0
+
+
+@pytest.mark.parametrize("worlds, want", [
+    ([(256, 256)] * 4, (0, False)),                                  # one class
+    ([(256, 256)] * 4 + [(512, 512)] * 2, (512 * 512 - 1, True)),     # within 128 MiB
+    ([(512, 512)] * 2 + [(256, 512)], (512 * 512 - 1, True)),
+    ([(1024, 1024)] * 16 + [(256, 256)], (384 * 384, False)),         # within 256 MiB
+    ([(384, 256)] * 110 + [(256, 256)], (384 * 256 - 1, True)),
+    ([(384, 256)] * 200 + [(256, 256)], (384 * 256 - 1, False)),
+    ([(1024, 1024)] * 30 + [(256, 256)], (0, False)),                 # beyond
+])
+def test_the_default_branch_split(lib, context, worlds, want):
+    """lenia_branch_split of a new context, by the bytes that its worlds touch in a step (9 a cell and a bit); lenia_set_branch_split
+    replaces it, and cells = 0 turns it off."""
+    ctx, cells, each = context(worlds), ctypes.c_int64(), ctypes.c_int32()
+
+    def split():
+        assert lib.lenia_branch_split(ctx, ctypes.byref(cells), ctypes.byref(each)) == 0
+        return cells.value, bool(each.value)
+
+    assert split() == want
+    assert lib.lenia_set_branch_split(ctx, ctypes.c_int64(128 * 128), 1) == 0
+    assert split() == (128 * 128, True)
+    assert lib.lenia_set_branch_split(ctx, ctypes.c_int64(0), 0) == 0
+    assert split() == (0, False)
