@@ -97,7 +97,9 @@ struct Res {
     static constexpr int COLS = 16;                  // spectrum columns a CTA owns
     static constexpr int R0 = chain_radix<N>(), NB = N / R0;
     static constexpr int S = S_, MINB = MINB_;
-    static constexpr int NT = S * NB;                // one first-stage butterfly per thread
+    // one butterfly of the widest stage per thread: at 192 = 12.16 the chained stage's 12 a sequence ran the other stages' 16
+    // in two rounds and spilled 580 bytes (63 worlds of 192 x 192 52 / 54 / 48 -> 44 / 45 / 33 us a generation for S = 16 / 8 / 4)
+    static constexpr int NT = S * (is_two_stage(N) ? two_tw_len(N) : NB);
     static constexpr int GATHER = S * (N / 2) / NT;  // remote elements a thread gathers (and scatters) per batch
     static constexpr int SEQ = seq_stride(N);
     static constexpr int HQC = khat_cols_stride<N>();
