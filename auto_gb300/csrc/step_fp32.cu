@@ -53,10 +53,10 @@ bool launch_col_fp32(int H, int variant, const DevWorld* worlds, const ColItem* 
 bool launch_row_fp32(int W, int variant, int mode, int general, const DevWorld* worlds, const RowItem* items,
                      int nitems, const float2* tw, LaunchOn s) {
     if (general)
-        return launch_row_group_small_general(W, variant, mode, general, worlds, items, nitems, tw, s) ||
-               launch_row_group_large_general(W, variant, mode, general, worlds, items, nitems, tw, s);
-    return launch_row_group_small_simple(W, variant, mode, general, worlds, items, nitems, tw, s) ||
-           launch_row_group_large_simple(W, variant, mode, general, worlds, items, nitems, tw, s);
+        return launch_row_group_small_general(W, variant, mode, worlds, items, nitems, tw, s) ||
+               launch_row_group_large_general(W, variant, mode, worlds, items, nitems, tw, s);
+    return launch_row_group_small_simple(W, variant, mode, worlds, items, nitems, tw, s) ||
+           launch_row_group_large_simple(W, variant, mode, worlds, items, nitems, tw, s);
 }
 
 }  // namespace lenia

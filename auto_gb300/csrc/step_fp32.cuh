@@ -552,7 +552,7 @@ __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, floa
 // WIDE: whether the spectrum moves in 256-bit accesses (row_wide).
 template <int W, int NT, int MINB, int S, bool GEN, bool WIDE>
 __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict__ worlds, const RowItem* __restrict__ items,
-                                                int mode, int general, const float2* __restrict__ tw, bool early) {
+                                                int mode, const float2* __restrict__ tw, bool early) {
     constexpr int ROWS = 2 * S, SPLIT = row_seqs(W, GEN) / S;  // CTAs an item
     extern __shared__ float4 smem_raw[];
     constexpr int SEQ = seq_stride(W);
@@ -1102,8 +1102,7 @@ constexpr size_t row_smem(int seqs = row_seqs(W, GEN)) {
 }
 
 template <int W, int V, bool GEN>
-bool row_go(int mode, int general, const DevWorld* worlds, const RowItem* items, int nitems,
-            const float2* tw, LaunchOn s) {
+bool row_go(int mode, const DevWorld* worlds, const RowItem* items, int nitems, const float2* tw, LaunchOn s) {
     constexpr int S = row_cta_seqs(W, V, GEN), NT = row_nt<W, GEN, V>();
     constexpr auto kernel = row_pass<W, NT, row_minb<W, V, GEN>(), S, GEN, row_wide<W, V>()>;
     const size_t smem = row_smem<W, GEN>(S);
@@ -1114,7 +1113,7 @@ bool row_go(int mode, int general, const DevWorld* worlds, const RowItem* items,
             return false;
         attr_max = (int)smem;
     }
-    return nitems <= 0 || launch_pass(kernel, nitems * (row_seqs(W, GEN) / S), NT, smem, s, worlds, items, mode, general, tw, s.early);
+    return nitems <= 0 || launch_pass(kernel, nitems * (row_seqs(W, GEN) / S), NT, smem, s, worlds, items, mode, tw, s.early);
 }
 
 // Column-pass builds: variant 0 and 1 are the scalar build at 64 (80 with a radix-32 plan) and 128
@@ -1144,8 +1143,8 @@ bool col_go_variant(int variant, const DevWorld* worlds, const ColItem* items, i
 // hide behind.)
 #define LENIA_ROW_CASE_G(N, G)                                                                     \
     case N:                                                                                        \
-        return (variant & 1) ? row_go<N, 1, G>(mode, general, worlds, items, nitems, tw, s) \
-                             : row_go<N, 0, G>(mode, general, worlds, items, nitems, tw, s);
+        return (variant & 1) ? row_go<N, 1, G>(mode, worlds, items, nitems, tw, s) \
+                             : row_go<N, 0, G>(mode, worlds, items, nitems, tw, s);
 #define LENIA_ROW_CASE_SIMPLE(N) LENIA_ROW_CASE_G(N, false)
 #define LENIA_ROW_CASE_GENERAL(N) LENIA_ROW_CASE_G(N, true)
 
@@ -1154,7 +1153,7 @@ bool launch_col_group_small(int H, int variant, const DevWorld* worlds, const Co
 bool launch_col_group_large(int H, int variant, const DevWorld* worlds, const ColItem* items, int nitems,
                             const float2* tw, LaunchOn s);
 #define LENIA_ROW_GROUP_DECL(NAME)                                                                       \
-    bool NAME(int W, int variant, int mode, int general, const DevWorld* worlds, const RowItem* items, \
+    bool NAME(int W, int variant, int mode, const DevWorld* worlds, const RowItem* items, \
               int nitems, const float2* tw, LaunchOn s);
 LENIA_ROW_GROUP_DECL(launch_row_group_small_simple)
 LENIA_ROW_GROUP_DECL(launch_row_group_small_general)

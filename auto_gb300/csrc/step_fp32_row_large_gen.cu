@@ -4,7 +4,7 @@
 
 namespace lenia {
 
-bool launch_row_group_large_general(int W, int variant, int mode, int general, const DevWorld* worlds,
+bool launch_row_group_large_general(int W, int variant, int mode, const DevWorld* worlds,
                                 const RowItem* items, int nitems, const float2* tw, LaunchOn s) {
     switch (W) { LENIA_SIZES_LARGE(LENIA_ROW_CASE_GENERAL) }
     return false;
