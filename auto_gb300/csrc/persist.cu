@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(NT, MINB)
             col_item<N, NT, true>(worlds[it.world], it, X, stwc);
         } else {
             const RowItem it = rows[(size_t)w * nr + idx];
-            row_item_simple<N, NT, row_seqs(N, false), true>(worlds[it.world], it.row0, X, stw);
+            row_item_simple<N, NT, row_seqs(N, false), true, true>(worlds[it.world], it.row0, X, stw);
         }
         __syncthreads();  // every thread's stores of this item are issued
         if (threadIdx.x == 0) {

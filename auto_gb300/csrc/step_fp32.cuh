@@ -227,10 +227,11 @@ __device__ __forceinline__ void fft_fused(float2* buf, const float2* stw, Mid mi
 template <int N, int MR = ROW_PLAN>
 constexpr size_t stage_table_bytes() { return (size_t)(tables_size<N, MR>() + 1) * sizeof(float2); }
 
-// The scalar column pass's radix cap: radix-32 plans where they save a stage (1024 = 32.32 against
-// 16.4.16: one shared-memory round trip fewer per transform; 3072, 8192), the radix-16 plan elsewhere.
-// The column item holds its 32 elements a thread in registers between stages; the row pass, which also
-// holds the state values of its rows there, keeps radix 16.
+// The scalar column pass's plans: radix 32 where that saves a stage (1024 = 32.32 against 16.4.16: one
+// shared-memory round trip fewer per transform; 8192 = 32.8.32), two stages at 192, 384 and 768, the merged plans at 96 and
+// from 1536 up where the side has a 3 (3072 = 16.12.16), radix 16 elsewhere.  The column item holds its up to 32
+// elements a thread in registers between stages; the row pass, which also holds the state values of its rows there, keeps
+// radix 16 in its chained stages.
 constexpr int CMR = COL_PLAN;
 
 // Column pass, fused form: after the stage tables (16-byte aligned), the tile's TC khat columns.
@@ -303,9 +304,10 @@ __device__ __forceinline__ float mnca_update(float s, float c0, float c1) {
 // 1024 wide: an item then reads and writes each tile's spectrum as 128 contiguous bytes (8 rows x 16
 // B) instead of 64, and on the 384-world batched workload the row pass went from 189 to 166 us a
 // generation for the 1024 x 1024 class (512: 41 -> 34 us), the step from 1.75e11 to 1.87e11 cell-updates/s.
-// Wider rows keep S = 2: measured at 4096 x 4096, S = 4 (1024 threads, one CTA per SM) was 10% slower
-// (row pass 76 against 68 us) and S = 1 (256 threads, three or four CTAs per SM) 5-30% slower than
-// S = 2 (512 threads, two CTAs per SM).  The general step keeps a plane of W x 2S floats besides
+// Rows of 1536 to 4096 take S = 2: measured at 4096 x 4096, S = 4 (1024 threads, one CTA per SM) was 10% slower
+// (row pass 76 against 68 us) and S = 1 (256 threads, three or four CTAs per SM) 4% slower (107 against 103 us a
+// generation) than S = 2 (512 threads, two CTAs per SM).  From 6144 up S = 2 leaves one CTA an SM and S = 1 wins (6144 x 6144
+// 378 -> 333 us a generation, 8192 x 8192 569 -> 528, with one-column columns at 8192).  The general step keeps a plane of W x 2S floats besides
 // the sequences; from W = 2048 up it uses S = 1 (at S = 2 a 4096-wide item needed 138 KB of shared
 // memory, one CTA per SM; MNCA at 4096 x 4096 measured 7% faster at S = 1), up to 1024 wide S = 4 (the
 // 3-channel 1024 x 1024 world: 5.97e10 -> 6.33e10 channel-cell updates/s from S = 2, and 5% slower at
@@ -368,7 +370,7 @@ __device__ __forceinline__ int row_tile(int e) {
     return S == 4 ? (e >> 5) * 8 + 2 * ((e >> 2) & 3) + ((e >> 4) & 1) : e / S;
 }
 
-template <int W, int S, int NT, bool CG = false, bool WIDE = true>
+template <int W, int S, int NT, bool CG, bool WIDE>
 __device__ __forceinline__ void load_rows_spectrum(float2* Z, const float2* __restrict__ sp, int H, int r0) {
     using L = RowLanes<W, S, NT>;
     constexpr int SEQ = seq_stride(W);
@@ -411,7 +413,7 @@ __device__ __forceinline__ void load_rows_spectrum(float2* Z, const float2* __re
 }
 
 // S packed complex spectra Z_p = FFT(a + ib) -> half-spectra of rows r0+2p (A) and r0+2p+1 (B).
-template <int W, int S, int NT, bool WIDE = true>
+template <int W, int S, int NT, bool WIDE>
 __device__ __forceinline__ void store_rows_spectrum(const float2* Z, float2* __restrict__ sp, int H, int r0) {
     using L = RowLanes<W, S, NT>;
     constexpr int SEQ = seq_stride(W);
@@ -497,11 +499,11 @@ __device__ __noinline__ void row_item_u(float2* Z, const float2* stw, const DevW
     }
 }
 
-// The one-channel, one-kernel Lenia row step of rows r0..r0+3 of world wd: inverse row FFT of U, growth,
-// dt update and clamp against the state, forward row FFT of the new rows.  Z: the two packed
+// The one-channel, one-kernel Lenia row step of rows r0..r0+2S-1 of world wd: inverse row FFT of U, growth,
+// dt update and clamp against the state, forward row FFT of the new rows.  Z: the S packed
 // sequences, stw: the stage tables.  CG: spectrum and state loads bypass L1 (the persistent step,
 // where another CTA of the same launch wrote them).
-template <int W, int NT, int S, bool CG, bool WIDE = true>
+template <int W, int NT, int S, bool CG, bool WIDE>
 __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, float2* Z, const float2* stw, bool early = false) {
     constexpr int ROWS = 2 * S;
     const int H = wd.H;
@@ -549,7 +551,7 @@ __device__ __forceinline__ void row_item_simple(const DevWorld& wd, int r0, floa
 // channels or kernels, SmoothLife, MNCA).  Without it the kernel carries only the one-channel,
 // one-kernel Lenia step (and the forward and U modes), so the general path's register pressure
 // does not set the budget of the common path.
-// WIDE: whether the spectrum moves in 256-bit accesses (row_wide).
+// WIDE: whether the spectrum moves in 256-bit accesses (row_wide; never in the noinline modes above, see hint::st8).
 template <int W, int NT, int MINB, int S, bool GEN, bool WIDE>
 __global__ void __launch_bounds__(NT, MINB) row_pass(const DevWorld* __restrict__ worlds, const RowItem* __restrict__ items,
                                                 int mode, const float2* __restrict__ tw, bool early) {
