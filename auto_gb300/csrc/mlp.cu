@@ -875,7 +875,7 @@ LENIA_API int lenia_mlp_get_params(LeniaMlp* n, float* host, size_t count) {
 
 LENIA_API int lenia_mlp_gradients(LeniaMlp* n, const float* x, const float* y, uint32_t batch, float* grads,
                                   float* loss) {
-    if (!n || !x || !y || !grads || batch < 1 || (int)batch > n->max_batch) {
+    if (!n || !x || !y || !grads || batch < 1 || batch > (uint32_t)n->max_batch) {
         set_thread_error("mlp: bad batch");
         return LENIA_EINVAL;
     }
@@ -894,7 +894,7 @@ LENIA_API int lenia_mlp_gradients(LeniaMlp* n, const float* x, const float* y, u
 }
 
 LENIA_API int lenia_mlp_train_step(LeniaMlp* n, const float* x, const float* y, uint32_t batch, float lr, float* loss) {
-    if (!n || !x || !y || batch < 1 || (int)batch > n->max_batch || !(lr > 0.f)) {
+    if (!n || !x || !y || batch < 1 || batch > (uint32_t)n->max_batch || !(lr > 0.f)) {
         set_thread_error("mlp: bad batch or learning rate");
         return LENIA_EINVAL;
     }

@@ -48,7 +48,7 @@ def test_statistics_of_a_smaller_context_between_set_and_launch(lib):
     assert lib.fake_world_stats(32 + 32)
 
 
-IN, OUT, NPARAM, ECUDA = 16, 3, 70915, -4
+IN, OUT, NPARAM, EINVAL, ECUDA = 16, 3, 70915, -1, -4
 F = ctypes.POINTER(ctypes.c_float)
 
 
@@ -249,3 +249,11 @@ def test_the_default_branch_split(lib, context, worlds, want):
     assert split() == (128 * 128, True)
     assert lib.lenia_set_branch_split(ctx, ctypes.c_int64(0), 0) == 0
     assert split() == (0, False)
+
+
+@pytest.mark.parametrize("batch", [0, 4097, 0x7fffffff, 0x80000000, 0xffffffff])
+def test_batches_beyond_the_handle_are_refused(lib, mlp, batch):
+    x, y, g, loss = rows(1), floats(OUT), floats(NPARAM), ctypes.c_float()
+    b = ctypes.c_uint32(batch)
+    assert lib.lenia_mlp_gradients(mlp, ptr(x), ptr(y), b, ptr(g), ctypes.byref(loss)) == EINVAL
+    assert lib.lenia_mlp_train_step(mlp, ptr(x), ptr(y), b, ctypes.c_float(0.1), ctypes.byref(loss)) == EINVAL
