@@ -663,9 +663,20 @@ int tiles_grid(const LeniaMlp* n, int B) {
 
 // gradients of the mean BCE of the batch (x, y on the device, or in host memory in_place) into n->g; per-row losses
 // into n->loss
-void gradients(LeniaMlp* n, const float* x, const float* y, int B) {
-    cudaMemsetAsync(n->g, 0, (size_t)NPARAM * sizeof(float), n->stream);
-    mlp_tile<<<tiles_grid(n, B), NTHR, TILE_SMEM, n->stream>>>(x, y, B, n->w, n->wb, n->g, n->loss, n->err);
+bool gradients(LeniaMlp* n, const float* x, const float* y, int B) {
+    return cudaMemsetAsync(n->g, 0, (size_t)NPARAM * sizeof(float), n->stream) == cudaSuccess &&
+           launch_pass(mlp_tile, tiles_grid(n, B), NTHR, TILE_SMEM, n->stream, x, y, B, n->w, n->wb, n->g, n->loss, n->err);
+}
+
+// probabilities of B rows on s (x, probs on the device, or in host memory in_place)
+bool rank(LeniaMlp* n, cudaStream_t s, const float* x, uint32_t B, float* probs) {
+    return launch_pass(mlp_rank, tiles_grid(n, (int)B), NRANK, RANK_SMEM, s, x, (int)B, n->w, n->wb, probs, n->err);
+}
+
+// a kernel with a thread for every parameter
+template <class... P, class... A>
+bool each_param(LeniaMlp* n, void (*kernel)(P...), A... args) {
+    return launch_pass(kernel, (NPARAM + 255) / 256, 256, 0, n->stream, args...);
 }
 
 // After the streams have been waited for.
@@ -706,8 +717,7 @@ int batch_gradients(LeniaMlp* n, const float* x, const float* y, uint32_t B) {
         touch_rows(x, (size_t)B * IN);
         touch_rows(y, (size_t)B * OUT);
     }
-    gradients(n, x, y, (int)B);
-    return 0;
+    return gradients(n, x, y, (int)B) ? 0 : abandon(n, "mlp: launch failed");
 }
 
 // Waits for the batch; its mean loss.
@@ -728,12 +738,11 @@ int rank_rows(LeniaMlp* n, const float* x, uint32_t count, float* probs) {
         if (count > 0 && apart && pageable_in_place(n->reads_host, probs, (size_t)count * OUT * 4)) {
             // no copy after the tiles: 1000 rows 30.5 -> 25.3 us, 19456 47.9 -> 36.0, 65536 74.0 -> 67.4
             touch_pages(probs, (size_t)count * OUT * 4, true);
-            mlp_rank<<<tiles_grid(n, (int)count), NRANK, RANK_SMEM, n->ps[0]>>>(x, (int)count, n->w, n->wb, probs, n->err);
-            if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
+            if (!rank(n, n->ps[0], x, count, probs)) return abandon(n, "mlp: launch failed");
         } else {
             for (uint64_t off = 0; off < count; off += DIRECT_ROWS) {
                 const uint32_t B = count - off < DIRECT_ROWS ? (uint32_t)(count - off) : DIRECT_ROWS;
-                mlp_rank<<<tiles_grid(n, (int)B), NRANK, RANK_SMEM, n->ps[0]>>>(x + off * IN, (int)B, n->w, n->wb, n->pp, n->err);
+                if (!rank(n, n->ps[0], x + off * IN, B, n->pp)) return abandon(n, "mlp: launch failed");
                 if (cudaMemcpyAsync(probs + off * OUT, n->pp, (size_t)B * OUT * 4, cudaMemcpyDeviceToHost, n->ps[0]) !=
                     cudaSuccess)
                     return abandon(n, "mlp: download failed");
@@ -753,7 +762,7 @@ int rank_rows(LeniaMlp* n, const float* x, uint32_t count, float* probs) {
             if (cudaMemcpyAsync(px, x + (size_t)c * HALF * IN, (size_t)rows(c) * IN * 4, cudaMemcpyHostToDevice, n->ps[h]) !=
                 cudaSuccess)
                 return abandon(n, "mlp: upload failed");
-            mlp_rank<<<tiles_grid(n, (int)rows(c)), NRANK, RANK_SMEM, n->ps[h]>>>(px, (int)rows(c), n->w, n->wb, pp, n->err);
+            if (!rank(n, n->ps[h], px, rows(c), pp)) return abandon(n, "mlp: launch failed");
         }
         if (c > 0) {
             const uint32_t d = c - 1;
@@ -857,7 +866,7 @@ LENIA_API int lenia_mlp_set_params(LeniaMlp* n, const float* host, size_t count)
     }
     if (cudaMemcpyAsync(n->w, host, NPARAM * 4, cudaMemcpyHostToDevice, n->stream) != cudaSuccess)
         return abandon(n, "mlp: upload failed");
-    to_bf16<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->w, n->wb, NPARAM);
+    if (!each_param(n, to_bf16, n->w, n->wb, NPARAM)) return abandon(n, "mlp: launch failed");
     n->t = 0;
     return cudaStreamSynchronize(n->stream) == cudaSuccess ? 0 : err("mlp: set_params failed");
 }
@@ -880,13 +889,11 @@ LENIA_API int lenia_mlp_gradients(LeniaMlp* n, const float* x, const float* y, u
         return LENIA_EINVAL;
     }
     if (int rc = batch_gradients(n, x, y, batch)) return rc;
-    if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
     // straight into the caller's memory where kernels reach it: 1000 rows 65.3 -> 62.7 us against the driver's copy, which
     // waits for a change of engine
     if (pageable_in_place(n->reads_host, grads, NPARAM * 4)) {
         touch_pages(grads, NPARAM * 4, true);  // beside the tiles
-        copy_out<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->g, grads, NPARAM);
-        if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
+        if (!each_param(n, copy_out, n->g, grads, NPARAM)) return abandon(n, "mlp: launch failed");
     } else if (cudaMemcpyAsync(grads, n->g, NPARAM * 4, cudaMemcpyDeviceToHost, n->stream) != cudaSuccess) {
         return abandon(n, "mlp: download failed");
     }
@@ -902,8 +909,7 @@ LENIA_API int lenia_mlp_train_step(LeniaMlp* n, const float* x, const float* y, 
     n->t++;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)n->t), c2 = 1.f - std::pow(b2, (float)n->t);
-    adam<<<(NPARAM + 255) / 256, 256, 0, n->stream>>>(n->w, n->g, n->m, n->v, n->wb, NPARAM, lr, b1, b2, 1e-8f, c1, c2);
-    if (cudaGetLastError() != cudaSuccess) return abandon(n, "mlp: launch failed");
+    if (!each_param(n, adam, n->w, n->g, n->m, n->v, n->wb, NPARAM, lr, b1, b2, 1e-8f, c1, c2)) return abandon(n, "mlp: launch failed");
     return mean_loss(n, batch, loss);
 }
 

@@ -158,6 +158,7 @@ int fake_pending() {
 // a range of the caller's as page-locked memory
 void fake_lock(void* p, size_t n) { ranges[(uintptr_t)p] = {n, cudaMemoryTypeHost}; }
 void fake_unlock(void* p) { ranges.erase((uintptr_t)p); }
+void fake_leave_error() { last = cudaErrorInvalidValue; }  // an error that nobody has asked for
 int fake_absent() {
     const int n = absent;
     absent = 0;

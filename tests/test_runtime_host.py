@@ -173,6 +173,25 @@ def test_probabilities_anywhere_over_their_own_rows(lib, mlp, count, aligned, at
     assert lib.fake_pending() == 0
 
 
+@pytest.mark.parametrize("count, aligned", [(1000, True), (100000, True), (100000, False)])
+def test_a_launch_is_judged_by_its_own_status(lib, mlp, count, aligned):
+    """An older error of the runtime's is no failure of this call; a refused launch is, on every route."""
+    x, probs, y, g, loss = rows(count, aligned), floats(count * OUT), floats(4096 * OUT), floats(NPARAM), ctypes.c_float()
+
+    def calls():
+        yield b"mlp_rank", lambda: lib.lenia_mlp_predict(mlp, ptr(x), count, ptr(probs))
+        yield b"mlp_tile", lambda: lib.lenia_mlp_gradients(mlp, ptr(x), ptr(y), 1000, ptr(g), ctypes.byref(loss))
+        yield b"adam", lambda: lib.lenia_mlp_train_step(mlp, ptr(x), ptr(y), 1000, ctypes.c_float(0.1), ctypes.byref(loss))
+
+    for kernel, call in calls():
+        lib.fake_leave_error()
+        assert call() == 0
+        lib.fake_fail(kernel, 0)
+        assert call() == ECUDA and lib.fake_failed() and lib.fake_pending() == 0
+        assert call() == 0
+    np.testing.assert_array_equal(probs.reshape(-1, OUT), probabilities(count))
+
+
 # ---------------------------------------------------------------------- states
 
 @pytest.fixture
