@@ -690,7 +690,7 @@ int check_err(LeniaMlp* n) {
 }
 
 // Whether a kernel may read host rows where they are: the GPU walks the host's page tables (Grace), the rows are aligned
-// for its loads (16 bytes, labels 4), and they are the host's (a device pointer is for the copy to refuse).  Against copying them
+// for its loads (16 bytes, labels 4), and they are the host's (device memory is no valid argument and stays with the copy).  Against copying them
 // first, lenia_mlp_predict of 250001 rows 336 -> 188 us, of 1000 rows 50 -> 42, lenia_mlp_gradients of 1000 rows 84 -> 72.
 bool in_place(const LeniaMlp* n, const float* rows, uintptr_t align = 16) {
     if (!n->reads_host || (uintptr_t)rows % align) return false;
