@@ -690,8 +690,9 @@ int check_err(LeniaMlp* n) {
 }
 
 // Whether a kernel may read host rows where they are: the GPU walks the host's page tables (Grace), the rows are aligned
-// for its loads (16 bytes, labels 4), and they are the host's (device memory is no valid argument and stays with the copy).  Against copying them
-// first, lenia_mlp_predict of 250001 rows 336 -> 188 us, of 1000 rows 50 -> 42, lenia_mlp_gradients of 1000 rows 84 -> 72.
+// for its loads (16 bytes, labels 4), and they are the host's (device memory is no valid argument and stays with the copy).
+// Against copying them first, lenia_mlp_predict of 250001 rows 336 -> 188 us, of 1000 rows 50 -> 42, lenia_mlp_gradients of
+// 1000 rows 84 -> 72.
 bool in_place(const LeniaMlp* n, const float* rows, uintptr_t align = 16) {
     if (!n->reads_host || (uintptr_t)rows % align) return false;
     cudaPointerAttributes a;
@@ -909,7 +910,8 @@ LENIA_API int lenia_mlp_train_step(LeniaMlp* n, const float* x, const float* y, 
     n->t++;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)n->t), c2 = 1.f - std::pow(b2, (float)n->t);
-    if (!each_param(n, adam, n->w, n->g, n->m, n->v, n->wb, NPARAM, lr, b1, b2, 1e-8f, c1, c2)) return abandon(n, "mlp: launch failed");
+    if (!each_param(n, adam, n->w, n->g, n->m, n->v, n->wb, NPARAM, lr, b1, b2, 1e-8f, c1, c2))
+        return abandon(n, "mlp: launch failed");
     return mean_loss(n, batch, loss);
 }
 
